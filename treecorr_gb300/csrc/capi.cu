@@ -274,6 +274,7 @@ int field_build(tc_field* f)
     TC_TRY(stream_get(&st));
     const int64_t n = f->n;
     if (n == 0) { f->built = true; return 0; }
+    TC_TRY(noalloc_preload());
     const int64_t ncap = 2 * n - 1;
     TC_TRY(alloc_cells(f->cells, ncap));
     TC_TRY(dalloc(&f->tcells, ncap));

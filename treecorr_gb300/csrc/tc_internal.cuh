@@ -87,7 +87,7 @@ struct BuildParams {
 
 static constexpr int CH = 4096;        // points per chunk in the cooperative levels
 static constexpr int CB = 256;         // threads per chunk block
-static constexpr int SMALL = 2048;     // cells at most this big are finished by one warp
+static constexpr int SMALL = 2048;     // cells at most this big are finished by one block
 
 struct Part1 {   // chunk partial of pass 1
     double sx, sy, sz, swp, sw;

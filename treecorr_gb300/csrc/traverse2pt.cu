@@ -1190,6 +1190,16 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
 static void* g_noalloc_ptr[64] = {nullptr};
 
+// CUDA loads a kernel's code to the device on its first use, which may allocate: the kernels
+// of the allocation-free call are loaded when a field is built.
+int noalloc_preload()
+{
+    cudaFuncAttributes at;
+    TC_CU(cudaFuncGetAttributes(&at, k_traverse));
+    TC_CU(cudaFuncGetAttributes(&at, k_reduce_acc));
+    return 0;
+}
+
 int noalloc_scratch(void** base)
 {
     int dev = 0;

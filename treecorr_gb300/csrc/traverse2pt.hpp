@@ -117,6 +117,7 @@ static constexpr size_t NOALLOC_BYTES = NOALLOC_OFF_ERR + 256;
 
 // Device address of the fixed scratch on the current device (looked up on first use).
 int noalloc_scratch(void** base);
+int noalloc_preload();
 
 // Device-side schedule of the level-by-level expansion: a one-thread kernel picks the next
 // chunk (the deepest non-empty level first) so that launches need no host round trip.

@@ -12,8 +12,8 @@
 // GB300 layout: the build is level-synchronous.  Cells with more than SMALL points are
 // processed cooperatively by many blocks (fixed chunks of CH points, deterministic two-stage
 // FP64 reductions, a stable scatter into the other of two point buffers).  Cells with at
-// most SMALL points are finished by one warp each, which builds the whole subtree with warp
-// reductions and ballot-based stable partitions, ping-ponging inside its own point range.
+// most SMALL points are finished by one block each, which keeps the points in shared memory
+// and builds the whole subtree on them.
 // Cell ids are positional, so no allocation counter is needed: an internal cell that
 // splits [s,e) at m gets id m-1, a leaf starting at point s gets id (n-1)+s.
 #include <cfloat>
@@ -37,12 +37,33 @@ __device__ __forceinline__ double coord3(const Points& P, int i, int axis)
 __device__ __forceinline__ void set_err(int* err, int code)
 { atomicCAS(err, 0, code); }
 
+// a / n for several a: one division, then Markstein's correction of a * (1 / n), which gives
+// the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34, 1990) for operands
+// without over- or underflow; other quotients (0, infinities, NaN, tiny or huge values) take
+// the division itself.
+struct Divisor {
+    double n, inv;
+    bool plain;
+    __device__ __forceinline__ explicit Divisor(double n_) : n(n_), inv(1. / n_)
+    { const double a = fabs(n_); plain = a > 1e-100 && a < 1e100; }
+    __device__ __forceinline__ double operator()(double a) const
+    {
+        const double b = fabs(a);
+        if (!(plain && b > 1e-100 && b < 1e100)) return a / n;
+        const double q = a * inv;
+        return fma(fma(-q, n, a), inv, q);
+    }
+};
+
 // Position<Sphere>::normalize, include/Position.h:258-263.
 __device__ __forceinline__ void normalize3(double& x, double& y, double& z)
 {
     double n = sqrt(x * x + y * y + z * z);
     if (n == 0.) { x = 1.; y = 0.; z = 0.; }
-    else { x /= n; y /= n; z /= n; }
+    else {
+        const Divisor by(n);
+        x = by(x); y = by(y); z = by(z);
+    }
 }
 
 // Bounds::getSplit, include/Bounds.h:65-66 (Flat) and 133-141 (ThreeD/Sphere).
@@ -180,44 +201,7 @@ __global__ void k_prepare(int n, int coords, int dkind, const double* x, const d
 }
 
 // ---------------------------------------------------------------------------------------
-// Deterministic block reductions (warp butterfly, then warps in a fixed order).
-
-template <int NT>
-__device__ __forceinline__ double block_sum(double v, double* sh)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    double t = 0.;
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NT / 32; ++k) t += sh[k];
-        sh[0] = t;
-    }
-    __syncthreads();
-    return sh[0];
-}
-
-template <int NT, bool MAX>
-__device__ __forceinline__ double block_ext(double v, double* sh)
-{
-    for (int o = 16; o > 0; o >>= 1) {
-        double u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = MAX ? fmax(v, u) : fmin(v, u);
-    }
-    int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = sh[0];
-        for (int k = 1; k < NT / 32; ++k) t = MAX ? fmax(t, sh[k]) : fmin(t, sh[k]);
-        sh[0] = t;
-    }
-    __syncthreads();
-    return sh[0];
-}
+// Deterministic warp reductions (butterflies).
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -240,33 +224,143 @@ __device__ __forceinline__ int warp_isum(int v)
     return v;
 }
 
+// Doubles as integers of the same order: a comparison is two ALU instructions, where FP64
+// comparisons share the FP64 pipe (1/64 of the FP32 rate) that bounds the build.
+__device__ __forceinline__ long long dkey(double v)
+{
+    const long long b = __double_as_longlong(v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double dunkey(long long k)
+{ return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL)); }
+
+__device__ __forceinline__ long long warp_kmin(long long v)
+{
+    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ long long warp_kmax(long long v)
+{
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Sums v[0..N) over the warp by a reduce-scatter (N <= 8, half of the values travel per
+// step) and hands every lane all totals: 9 FP64 adds per lane for five values where five
+// butterflies take 25.
+template <int N>
+__device__ __forceinline__ void warp_sums(double (&v)[N], int lane)
+{
+    static_assert(N <= 8, "");
+    double a[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) a[q] = q < N ? v[q] : 0.;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        const int half = 4 >> s, o = 16 >> s;
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < half; ++q) {
+            if (q >= N) continue;                      // both partners hold zeros
+            const double send = up ? a[q] : a[q + half];
+            const double keep = up ? a[q + half] : a[q];
+            a[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    // Lane bits 4, 3, 2 picked the upper half at each step: value q sits at lanes 4 q.
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = __shfl_sync(0xffffffffu, a[0], 4 * q);
+}
+
+// transport_add for a point at squared distance dsq from the centre; the spin-2 phase takes
+// one reciprocal for its two divisions.
+__device__ __forceinline__ void transport_near(int coords, int spin, double cx, double cy,
+                                               double cz, double cz_raw, double px, double py,
+                                               double pz, double dsq, double wr, double wi,
+                                               double& sr, double& si)
+{
+    if (spin != 2 || coords == THREED) {
+        transport_add(coords, spin, cx, cy, cz, cz_raw, px, py, pz, wr, wi, sr, si);
+        return;
+    }
+    if (dsq < 1.e-12) { sr += wr; si += wi; return; }
+    const double cosA = (cz - pz) + 0.5 * pz * dsq;
+    const double sinA = cy * px - cx * py;
+    const double cosB = (pz - cz) + 0.5 * cz * dsq;
+    const double cb = -cosA * cosB + sinA * sinA;
+    const double sb = sinA * cosB + cosA * sinA;
+    double nrm = cb * cb + sb * sb;
+    if (!(nrm > 0.)) nrm = 1.;
+    const double inv = 1. / nrm;
+    const double er = (cb * cb - sb * sb) * inv;
+    const double ei = -(2. * cb * sb) * inv;
+    sr += wr * er - wi * ei;
+    si += wr * ei + wi * er;
+}
+
 // ---------------------------------------------------------------------------------------
 // Cooperative levels (cells with more than SMALL points).
 
 __global__ void __launch_bounds__(CB) k_chunk_pass1(const Chunk* chunks, const BuildTask* tasks,
                                                      Points P0, Points P1, int coords, Part1* out)
 {
-    __shared__ double sh[CB / 32];
+    __shared__ double sh[CB / 32][5];
+    __shared__ long long shk[CB / 32][6];
     const Chunk ch = chunks[blockIdx.x];
     const Points& P = tasks[ch.task].buf ? P1 : P0;
-    double sx = 0., sy = 0., sz = 0., swp = 0., sw = 0.;
-    double xmin = DBL_MAX, ymin = DBL_MAX, zmin = DBL_MAX;
-    double xmax = -DBL_MAX, ymax = -DBL_MAX, zmax = -DBL_MAX;
+    double s[5] = {0., 0., 0., 0., 0.};
+    long long k[6];                       // minima and, negated, maxima
+    const long long big = dkey(DBL_MAX);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { k[2 * q] = big; k[2 * q + 1] = ~dkey(-DBL_MAX); }
+    const bool flat = coords == FLAT;
+    if (flat) { k[4] = 0; k[5] = ~0ll; }
+#pragma unroll 4
     for (int i = ch.cs + threadIdx.x; i < ch.ce; i += CB) {
-        double px = P.x[i], py = P.y[i], pz = P.z[i], wp = P.wp[i];
-        sx += px * wp; sy += py * wp; sz += pz * wp; swp += wp; sw += P.w[i];
-        xmin = fmin(xmin, px); xmax = fmax(xmax, px);
-        ymin = fmin(ymin, py); ymax = fmax(ymax, py);
-        zmin = fmin(zmin, pz); zmax = fmax(zmax, pz);
+        const double px = P.x[i], py = P.y[i], wp = P.wp[i];
+        s[0] += px * wp; s[1] += py * wp; s[3] += wp; s[4] += P.w[i];
+        const long long kx = dkey(px), ky = dkey(py);
+        k[0] = min(k[0], kx); k[1] = min(k[1], ~kx);
+        k[2] = min(k[2], ky); k[3] = min(k[3], ~ky);
+        if (!flat) {
+            const double pz = P.z[i];
+            s[2] += pz * wp;
+            const long long kz = dkey(pz);
+            k[4] = min(k[4], kz); k[5] = min(k[5], ~kz);
+        }
     }
-    Part1 r;
-    r.sx = block_sum<CB>(sx, sh); r.sy = block_sum<CB>(sy, sh); r.sz = block_sum<CB>(sz, sh);
-    r.swp = block_sum<CB>(swp, sh); r.sw = block_sum<CB>(sw, sh);
-    r.xmin = block_ext<CB, false>(xmin, sh); r.xmax = block_ext<CB, true>(xmax, sh);
-    r.ymin = block_ext<CB, false>(ymin, sh); r.ymax = block_ext<CB, true>(ymax, sh);
-    r.zmin = block_ext<CB, false>(zmin, sh); r.zmax = block_ext<CB, true>(zmax, sh);
-    if (threadIdx.x == 0) out[blockIdx.x] = r;
-    (void)coords;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    warp_sums<5>(s, lane);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) k[q] = warp_kmin(k[q]);
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) sh[wid][q] = s[q];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) shk[wid][q] = k[q];
+    }
+    __syncthreads();
+    // Thread q combines quantity q over the warps, in their order.
+    if (threadIdx.x < 5) {
+        double t = 0.;
+        for (int w = 0; w < CB / 32; ++w) t += sh[w][threadIdx.x];
+        sh[0][threadIdx.x] = t;
+    } else if (threadIdx.x >= 32 && threadIdx.x < 38) {
+        long long t = shk[0][threadIdx.x - 32];
+        for (int w = 1; w < CB / 32; ++w) t = min(t, shk[w][threadIdx.x - 32]);
+        shk[0][threadIdx.x - 32] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        Part1 r;
+        r.sx = sh[0][0]; r.sy = sh[0][1]; r.sz = sh[0][2]; r.swp = sh[0][3]; r.sw = sh[0][4];
+        r.xmin = dunkey(shk[0][0]); r.xmax = dunkey(~shk[0][1]);
+        r.ymin = dunkey(shk[0][2]); r.ymax = dunkey(~shk[0][3]);
+        r.zmin = dunkey(shk[0][4]); r.zmax = dunkey(~shk[0][5]);
+        out[blockIdx.x] = r;
+    }
 }
 
 // One warp per cooperative task: centroid, weight, split axis and value.
@@ -324,7 +418,7 @@ __global__ void __launch_bounds__(CB) k_chunk_pass2(const Chunk* chunks, const B
                                                      const TaskStats* st, Points P0, Points P1,
                                                      int coords, int dkind, int spin, Part2* out)
 {
-    __shared__ double sh[CB / 32];
+    __shared__ double sh[CB / 32][3];
     __shared__ int shi[CB / 32];
     const Chunk ch = chunks[blockIdx.x];
     const TaskStats s = st[ch.task];
@@ -345,21 +439,25 @@ __global__ void __launch_bounds__(CB) k_chunk_pass2(const Chunk* chunks, const B
             pr += P.d1[i];
         } else if (dkind == DG) {
             if (coords == FLAT) { pr += P.d1[i]; pi += P.d2[i]; }
-            else transport_add(coords, spin, tcx, tcy, tcz, cz, px, py, pz, P.d1[i], P.d2[i], pr, pi);
+            else transport_near(coords, spin, tcx, tcy, tcz, cz, px, py, pz, d, P.d1[i], P.d2[i], pr, pi);
         }
     }
-    Part2 r;
-    r.sizesq = block_ext<CB, true>(sizesq, sh);
-    r.pr = block_sum<CB>(pr, sh);
-    r.pi = block_sum<CB>(pi, sh);
-    for (int o = 16; o > 0; o >>= 1) nleft += __shfl_xor_sync(0xffffffffu, nleft, o);
-    if ((threadIdx.x & 31) == 0) shi[threadIdx.x >> 5] = nleft;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    sizesq = dunkey(warp_kmax(dkey(sizesq)));
+    double pp[2] = {pr, pi};
+    if (dkind != DN) warp_sums<2>(pp, lane);
+    nleft = warp_isum(nleft);
+    if (lane == 0) { sh[wid][0] = sizesq; sh[wid][1] = pp[0]; sh[wid][2] = pp[1]; shi[wid] = nleft; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        int t = 0;
-        for (int k = 0; k < CB / 32; ++k) t += shi[k];
-        r.nleft = t;
-        r.pad = 0;
+        Part2 r;
+        r.sizesq = 0.; r.pr = 0.; r.pi = 0.;
+        r.nleft = 0; r.pad = 0;
+        for (int w = 0; w < CB / 32; ++w) {
+            r.sizesq = fmax(r.sizesq, sh[w][0]);
+            r.pr += sh[w][1]; r.pi += sh[w][2];
+            r.nleft += shi[w];
+        }
         out[blockIdx.x] = r;
     }
 }
@@ -486,7 +584,7 @@ __global__ void __launch_bounds__(CB) k_chunk_scatter(const Chunk* chunks, const
 }
 
 // ---------------------------------------------------------------------------------------
-// Warp-finished subtrees (cells with at most SMALL points, or every cell for Median).
+// Block-finished subtrees (cells with at most SMALL points).
 
 __device__ __forceinline__ int pack_meta(int side, int intop, int buf, int mintop, int maxtop)
 {
@@ -495,131 +593,464 @@ __device__ __forceinline__ int pack_meta(int side, int intop, int buf, int minto
     return side | (intop << 1) | (buf << 2) | (mintop << 8) | (maxtop << 20);
 }
 
-// Cells of at most THREAD_T points are finished by one thread: the steps of the warp loop
-// below (src/Cell.cpp:170-200, 520-615) with the sums taken in point order.  Small cells
-// are ~94% of a subtree's cells, and a warp spends the same reductions on a 2-point cell
-// as on a 2048-point one.
+// Cells of at most THREAD_T points are finished by one thread, sums in point order.  Small
+// cells are ~94% of a subtree's cells, and a warp spends the same reductions on a 2-point
+// cell as on a 2048-point one.
 constexpr int THREAD_T = 32;
+constexpr int SB = 256;             // threads of a subtree block
+constexpr int SW = SB / 32;
+constexpr unsigned NOT_SINGLE = ~0u;
+constexpr int SBIG = SMALL / (THREAD_T + 1) + 1;   // cells above THREAD_T points at one depth
 
-__device__ void subtree_by_thread(WTask root, Points P0, Points P1, const BuildParams& BP,
-                                  const Cells& C, int* tops, int* ntop, int* err)
+// One subtree's points, in shared memory for the whole build of the subtree: the points stay
+// where they are and the cells permute 16-bit indices, so a level moves 2 bytes per point
+// instead of 48.
+struct SubPoints {
+    double x[SMALL], y[SMALL], z[SMALL], wp[SMALL];
+    float w[SMALL], d1[SMALL], d2[SMALL];
+    unsigned short perm[2][SMALL];
+    unsigned single[SMALL];         // position of a one-point cell: (parent + 1, index buffer,
+                                    // side) packed, or NOT_SINGLE
+};
+struct SubPart {                    // one warp's share of a cell that several warps work on
+    double sum[5];                  // x wp, y wp, z wp, wp, w
+    long long lo[3], hi[3];         // bounds as ordered keys
+    double sizesq, pr, pi;
+    int nleft;
+};
+struct SubShared {
+    SubPoints P;
+    WTask cell[2][SBIG];            // cells above THREAD_T points of this and the next depth
+    int ncell[2], nsmall[2];
+    SubPart part[SW];
+};
+
+// The first pass over the points i0, i0 + step, .. < e of a cell: sums and bounds.
+template <bool FLATC>
+__device__ __forceinline__ void sub_pass1(const SubPoints& P, const unsigned short* perm, int i0,
+                                          int e, int step, double (&s)[5], long long (&lo)[3],
+                                          long long (&hi)[3])
 {
-    WTask stk[THREAD_T + 1];
-    int sp = 0;
-    stk[sp++] = root;
-    while (sp > 0) {
-        const WTask w = stk[--sp];
-        const int s = w.s, e = w.e, n = e - s;
-        const int side = w.meta & 1, buf = (w.meta >> 2) & 1;
-        int intop = (w.meta >> 1) & 1;
-        const int mintop = ((w.meta >> 8) & 0xfff) - 2048;
-        const int maxtop = ((w.meta >> 20) & 0xfff) - 2048;
-        const Points& A = buf ? P1 : P0;
-        const Points& B = buf ? P0 : P1;
-        if (n == 1) {
-            const int id = (BP.n - 1) + s;
-            write_cell(C, id, A.x[s], A.y[s], A.z[s], 0.f, A.w[s], A.d1[s], A.d2[s], 1, s,
-                       w.parent, side);
-            if (intop) add_top(tops, ntop, id, s);
-            if (buf) move_point(A, s, P0, s);
-            continue;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) s[q] = 0.;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { lo[q] = dkey(DBL_MAX); hi[q] = dkey(-DBL_MAX); }
+    if (FLATC) { lo[2] = 0; hi[2] = 0; }
+    for (int i = i0; i < e; i += step) {
+        const int p = perm[i];
+        const double px = P.x[p], py = P.y[p], wp = P.wp[p];
+        s[0] += px * wp; s[1] += py * wp; s[3] += wp; s[4] += P.w[p];
+        const long long kx = dkey(px), ky = dkey(py);
+        lo[0] = min(lo[0], kx); hi[0] = max(hi[0], kx);
+        lo[1] = min(lo[1], ky); hi[1] = max(hi[1], ky);
+        if (!FLATC) {
+            const double pz = P.z[p];
+            s[2] += pz * wp;
+            const long long kz = dkey(pz);
+            lo[2] = min(lo[2], kz); hi[2] = max(hi[2], kz);
         }
-        double sx = 0., sy = 0., sz = 0., swp = 0., sw = 0.;
-        double xmin = DBL_MAX, ymin = DBL_MAX, zmin = DBL_MAX;
-        double xmax = -DBL_MAX, ymax = -DBL_MAX, zmax = -DBL_MAX;
-        for (int i = s; i < e; ++i) {
-            const double px = A.x[i], py = A.y[i], pz = A.z[i], wp = A.wp[i];
-            sx += px * wp; sy += py * wp; sz += pz * wp; swp += wp; sw += A.w[i];
-            xmin = fmin(xmin, px); xmax = fmax(xmax, px);
-            ymin = fmin(ymin, py); ymax = fmax(ymax, py);
-            zmin = fmin(zmin, pz); zmax = fmax(zmax, pz);
-        }
-        double cx, cy, cz;
-        if (swp != 0.) {
-            cx = sx / swp; cy = sy / swp; cz = sz / swp;
-            if (BP.coords == SPHERE) normalize3(cx, cy, cz);
-        } else {
-            cx = A.x[s]; cy = A.y[s]; cz = A.z[s];
-        }
-        const int axis = split_axis(BP.coords, xmax - xmin, ymax - ymin, zmax - zmin);
-        double splitval;
-        if (BP.split == MIDDLE)
-            splitval = axis == 2 ? (zmax + zmin) / 2. : axis == 1 ? (ymax + ymin) / 2.
-                                                                   : (xmax + xmin) / 2.;
-        else
-            splitval = axis == 2 ? cz : axis == 1 ? cy : cx;
-        double tcx = cx, tcy = cy, tcz = cz;
-        if (BP.coords == THREED) normalize3(tcx, tcy, tcz);
-        double sizesq = 0., pr = 0., pi = 0.;
-        int nleft = 0;
-        for (int i = s; i < e; ++i) {
-            const double px = A.x[i], py = A.y[i], pz = A.z[i];
-            double d = (cx - px) * (cx - px) + (cy - py) * (cy - py);
-            if (BP.coords != FLAT) d += (cz - pz) * (cz - pz);
-            sizesq = fmax(sizesq, d);
-            const double c = axis == 2 ? pz : axis == 1 ? py : px;
-            nleft += (c < splitval) ? 1 : 0;
-            if (BP.dkind == DK) pr += A.d1[i];
-            else if (BP.dkind == DG) {
-                if (BP.coords == FLAT) { pr += A.d1[i]; pi += A.d2[i]; }
-                else transport_add(BP.coords, BP.spin, tcx, tcy, tcz, cz, px, py, pz, A.d1[i],
-                                   A.d2[i], pr, pi);
-            }
-        }
-        bool is_top;
-        const bool split = decide_split(BP, intop, mintop, maxtop, sizesq, is_top);
-        bool use_rank = (BP.split == MEDIAN);
-        int mid = s + nleft;
-        if (split && !use_rank && (nleft == 0 || nleft == n)) use_rank = true;
-        if (split && use_rank) mid = (s + e) / 2;   // SplitDataCore<Median>, src/Cell.cpp:464-479
-        float d1 = float(pr), d2 = float(pi);
-        if (BP.dkind == DN) { d1 = 0.f; d2 = 0.f; }
-        if (BP.dkind == DK) d2 = 0.f;
-        const int id = split ? mid - 1 : (BP.n - 1) + s;
-        write_cell(C, id, cx, cy, cz, split ? cell_size(BP, sizesq) : 0.f, float(sw), d1, d2, n,
-                   s, w.parent, side);
-        if (is_top) add_top(tops, ntop, id, s);
-        if (!split) {
-            if (buf) for (int i = s; i < e; ++i) move_point(A, i, P0, i);
-            continue;
-        }
-        // Stable partition into the other buffer.
-        int lo = s, hi = mid;
-        for (int i = s; i < e; ++i) {
-            const double c = axis == 2 ? A.z[i] : axis == 1 ? A.y[i] : A.x[i];
-            bool left;
-            if (!use_rank) {
-                left = c < splitval;
-            } else {
-                int rank = 0;
-                for (int j = s; j < e; ++j) {
-                    const double cj = axis == 2 ? A.z[j] : axis == 1 ? A.y[j] : A.x[j];
-                    rank += (cj < c || (cj == c && j < i)) ? 1 : 0;
-                }
-                left = rank < (mid - s);
-            }
-            move_point(A, i, B, left ? lo++ : hi++);
-        }
-        if (sp + 2 > THREAD_T + 1) { set_err(err, DEV_TASK_OVERFLOW); return; }
-        const int nb = buf ^ 1;
-        stk[sp++] = WTask{mid, e, id, pack_meta(1, intop, nb, mintop - 1, maxtop - 1)};
-        stk[sp++] = WTask{s, mid, id, pack_meta(0, intop, nb, mintop - 1, maxtop - 1)};
     }
 }
 
-__global__ void k_small_subtree(int ntask, const BuildTask* tasks, Points P0, Points P1,
-                                BuildParams BP, Cells C, int* tops, int* ntop, WTask* wstack,
-                                int* err)
+struct SubCentre {
+    double cx, cy, cz, tcx, tcy, tcz, splitval;
+    int axis;
+};
+
+// Centroid, split axis and value of a cell from its sums (src/Cell.cpp:170-200, 481-525).
+template <bool FLATC>
+__device__ __forceinline__ SubCentre sub_centre(const SubPoints& P, int first,
+                                                const BuildParams& BP, const double (&s)[5],
+                                                const long long (&lo)[3], const long long (&hi)[3])
 {
-    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    SubCentre c;
+    if (s[3] != 0.) {
+        const Divisor by(s[3]);
+        c.cx = by(s[0]); c.cy = by(s[1]); c.cz = FLATC ? 0. : by(s[2]);
+        if (!FLATC && BP.coords == SPHERE) normalize3(c.cx, c.cy, c.cz);
+    } else {
+        c.cx = P.x[first]; c.cy = P.y[first]; c.cz = FLATC ? 0. : P.z[first];
+    }
+    double l[3], h[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { l[q] = dunkey(lo[q]); h[q] = dunkey(hi[q]); }
+    c.axis = split_axis(FLATC ? FLAT : BP.coords, h[0] - l[0], h[1] - l[1], h[2] - l[2]);
+    if (BP.split == MIDDLE)
+        c.splitval = c.axis == 2 ? (h[2] + l[2]) / 2. : c.axis == 1 ? (h[1] + l[1]) / 2.
+                                                                     : (h[0] + l[0]) / 2.;
+    else
+        c.splitval = c.axis == 2 ? c.cz : c.axis == 1 ? c.cy : c.cx;
+    c.tcx = c.cx; c.tcy = c.cy; c.tcz = c.cz;
+    if (!FLATC && BP.coords == THREED) normalize3(c.tcx, c.tcy, c.tcz);
+    return c;
+}
+
+// The second pass: size, payload, points left of the split value.
+template <bool FLATC, bool CPLX>
+__device__ __forceinline__ void sub_pass2(const SubPoints& P, const unsigned short* perm, int i0,
+                                          int e, int step, const BuildParams& BP,
+                                          const SubCentre& c, double& sizesq, double& pr,
+                                          double& pi, int& nleft)
+{
+    sizesq = 0.; pr = 0.; pi = 0.;
+    nleft = 0;
+    const double* ax = c.axis == 2 ? P.z : c.axis == 1 ? P.y : P.x;
+    for (int i = i0; i < e; i += step) {
+        const int p = perm[i];
+        const double px = P.x[p], py = P.y[p], pz = FLATC ? 0. : P.z[p];
+        double d = (c.cx - px) * (c.cx - px) + (c.cy - py) * (c.cy - py);
+        if (!FLATC) d += (c.cz - pz) * (c.cz - pz);
+        sizesq = fmax(sizesq, d);
+        nleft += (ax[p] < c.splitval) ? 1 : 0;
+        if (CPLX) {
+            if (FLATC) { pr += P.d1[p]; pi += P.d2[p]; }
+            else transport_near(BP.coords, BP.spin, c.tcx, c.tcy, c.tcz, c.cz, px, py, pz, d,
+                                P.d1[p], P.d2[p], pr, pi);
+        } else if (BP.dkind == DK) {
+            pr += P.d1[p];
+        }
+    }
+}
+
+// Whether point i of [s, e) is among the mid - s smallest by (coordinate, position).
+__device__ __forceinline__ bool sub_rank_left(const double* ax, const unsigned short* perm,
+                                              int s, int e, int mid, int i)
+{
+    const double c = ax[perm[i]];
+    int rank = 0;
+    for (int j = s; j < e; ++j) {
+        const double cj = ax[perm[j]];
+        rank += (cj < c || (cj == c && j < i)) ? 1 : 0;
+    }
+    return rank < (mid - s);
+}
+
+// What follows the two passes of a cell: the decision, the split point and the cell itself
+// (written by the caller's one thread).
+struct SubSplit {
+    bool split, rank;
+    int mid, intop;
+};
+__device__ __forceinline__ SubSplit sub_finish(const BuildParams& BP, const WTask& w, int base,
+                                               const SubCentre& c, float wsum, double sizesq,
+                                               double pr, double pi, int nleft, bool writer,
+                                               const Cells& C, int* tops, int* ntop)
+{
+    const int n = w.e - w.s;
+    SubSplit r;
+    r.intop = (w.meta >> 1) & 1;
+    const int mintop = ((w.meta >> 8) & 0xfff) - 2048;
+    const int maxtop = ((w.meta >> 20) & 0xfff) - 2048;
+    bool is_top;
+    r.split = decide_split(BP, r.intop, mintop, maxtop, sizesq, is_top);
+    r.rank = (BP.split == MEDIAN);
+    r.mid = w.s + nleft;
+    if (r.split && !r.rank && (nleft == 0 || nleft == n)) r.rank = true;
+    if (r.split && r.rank) r.mid = (w.s + w.e) / 2;   // SplitDataCore<Median>, src/Cell.cpp:464-479
+    if (writer) {
+        float d1 = float(pr), d2 = float(pi);
+        if (BP.dkind == DN) { d1 = 0.f; d2 = 0.f; }
+        if (BP.dkind == DK) d2 = 0.f;
+        const int id = r.split ? base + r.mid - 1 : (BP.n - 1) + base + w.s;
+        write_cell(C, id, c.cx, c.cy, c.cz, r.split ? cell_size(BP, sizesq) : 0.f, wsum, d1, d2,
+                   n, base + w.s, w.parent, w.meta & 1);
+        if (is_top) add_top(tops, ntop, id, base + w.s);
+    }
+    return r;
+}
+
+__device__ __forceinline__ WTask sub_child(const WTask& w, const SubSplit& r, int base, int side)
+{
+    const int mintop = ((w.meta >> 8) & 0xfff) - 2048;
+    const int maxtop = ((w.meta >> 20) & 0xfff) - 2048;
+    const int nb = ((w.meta >> 2) & 1) ^ 1;
+    WTask c;
+    c.s = side ? r.mid : w.s;
+    c.e = side ? w.e : r.mid;
+    c.parent = base + r.mid - 1;
+    c.meta = pack_meta(side, r.intop, nb, mintop - 1, maxtop - 1);
+    return c;
+}
+
+// A one-point child is noted at its position; the block writes these leaves together at the
+// end, to consecutive ids.  (Ids of internal cells are below n < 2^30, so the packing holds.)
+__device__ __forceinline__ void sub_single(SubPoints& P, const WTask& w, int base,
+                                           const BuildParams& BP, int* tops, int* ntop)
+{
+    const int s = w.s, buf = (w.meta >> 2) & 1;
+    P.single[s] = ((unsigned)(w.parent + 1) << 2) | (buf << 1) | (w.meta & 1);
+    if ((w.meta >> 1) & 1) add_top(tops, ntop, (BP.n - 1) + base + s, base + s);
+}
+
+// A cell of 2 .. THREAD_T points by one thread.  Positions are relative to base (the block's
+// first point); a finished cell's order ends up in perm[0].  Returns whether it was split,
+// with its children in k.
+template <bool FLATC, bool CPLX>
+__device__ __forceinline__ bool sub_by_thread(const WTask& w, int base, SubPoints& P,
+                                              const BuildParams& BP, const Cells& C, int* tops,
+                                              int* ntop, WTask (&k)[2])
+{
+    const int s = w.s, e = w.e, buf = (w.meta >> 2) & 1;
+    const unsigned short* perm = P.perm[buf];
+    unsigned short* to = P.perm[buf ^ 1];
+    double sum[5];
+    long long lo[3], hi[3];
+    sub_pass1<FLATC>(P, perm, s, e, 1, sum, lo, hi);
+    const SubCentre c = sub_centre<FLATC>(P, perm[s], BP, sum, lo, hi);
+    double sizesq, pr, pi;
+    int nleft;
+    sub_pass2<FLATC, CPLX>(P, perm, s, e, 1, BP, c, sizesq, pr, pi, nleft);
+    const SubSplit r = sub_finish(BP, w, base, c, float(sum[4]), sizesq, pr, pi, nleft, true, C,
+                                  tops, ntop);
+    if (!r.split) {
+        if (buf) for (int i = s; i < e; ++i) P.perm[0][i] = perm[i];
+        return false;
+    }
+    // Stable partition into the other index buffer.
+    const double* ax = c.axis == 2 ? P.z : c.axis == 1 ? P.y : P.x;
+    int l = s, h = r.mid;
+    for (int i = s; i < e; ++i) {
+        const unsigned short p = perm[i];
+        const bool left = r.rank ? sub_rank_left(ax, perm, s, e, r.mid, i) : ax[p] < c.splitval;
+        const int dst = left ? l++ : h++;
+        if (dst < e) to[dst] = p;
+    }
+    k[0] = sub_child(w, r, base, 0);
+    k[1] = sub_child(w, r, base, 1);
+    return true;
+}
+
+// A child of at most THREAD_T points: noted if it is one point, else onto the list.
+__device__ __forceinline__ void sub_small(const WTask& k, int base, SubPoints& P,
+                                          const BuildParams& BP, int* tops, int* ntop,
+                                          WTask* list, int* count)
+{
+    if (k.e - k.s == 1) sub_single(P, k, base, BP, tops, ntop);
+    else list[atomicAdd(count, 1)] = k;
+}
+
+// One warp's share (part of parts) of a cell above THREAD_T points; COOP: several warps of
+// the block work on the cell and meet at block barriers (every warp of the block makes the
+// same calls).  `on` is false for a warp without a cell in a COOP round.
+template <bool FLATC, bool CPLX, bool COOP>
+__device__ __forceinline__ void sub_cell(SubShared& S, bool on, WTask w, int part, int parts,
+                                         int base, const BuildParams& BP, const Cells& C,
+                                         int* tops, int* ntop, int next, WTask* small, int lane,
+                                         int wid)
+{
+    SubPoints& P = S.P;
+    const int n = w.e - w.s, buf = (w.meta >> 2) & 1;
+    const unsigned short* perm = P.perm[buf];
+    unsigned short* to = P.perm[buf ^ 1];
+    const int per = ((n + parts - 1) / parts + 31) & ~31;
+    const int i0 = min(w.e, w.s + part * per), i1 = min(w.e, i0 + per);
+    const int p0 = wid - part;      // the first warp of this cell's group
+    double sum[5];
+    long long lo[3], hi[3];
+    sub_pass1<FLATC>(P, perm, on ? i0 + lane : i1, i1, 32, sum, lo, hi);
+    warp_sums<5>(sum, lane);
+#pragma unroll
+    for (int q = 0; q < (FLATC ? 2 : 3); ++q) { lo[q] = warp_kmin(lo[q]); hi[q] = warp_kmax(hi[q]); }
+    if (COOP) {
+        if (lane == 0) {
+#pragma unroll
+            for (int q = 0; q < 5; ++q) S.part[wid].sum[q] = sum[q];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) { S.part[wid].lo[q] = lo[q]; S.part[wid].hi[q] = hi[q]; }
+        }
+        __syncthreads();
+        for (int t = 0; t < parts; ++t) {
+            const SubPart& o = S.part[p0 + t];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) sum[q] = t ? sum[q] + o.sum[q] : o.sum[q];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) { lo[q] = min(lo[q], o.lo[q]); hi[q] = max(hi[q], o.hi[q]); }
+        }
+    }
+    const SubCentre c = sub_centre<FLATC>(P, on ? perm[w.s] : 0, BP, sum, lo, hi);
+    double sizesq, pp[2];
+    int nleft;
+    sub_pass2<FLATC, CPLX>(P, perm, on ? i0 + lane : i1, i1, 32, BP, c, sizesq, pp[0], pp[1], nleft);
+    sizesq = dunkey(warp_kmax(dkey(sizesq)));
+    if (BP.dkind != DN) warp_sums<2>(pp, lane);
+    nleft = warp_isum(nleft);
+    int before = 0;                 // left points of the parts before this one
+    if (COOP) {
+        if (lane == 0) {
+            SubPart& o = S.part[wid];
+            o.sizesq = sizesq; o.pr = pp[0]; o.pi = pp[1]; o.nleft = nleft;
+        }
+        __syncthreads();
+        nleft = 0;
+        pp[0] = pp[1] = 0.;
+        for (int t = 0; t < parts; ++t) {
+            const SubPart& o = S.part[p0 + t];
+            sizesq = fmax(sizesq, o.sizesq);
+            pp[0] += o.pr; pp[1] += o.pi;
+            if (t < part) before += o.nleft;
+            nleft += o.nleft;
+        }
+    }
+    if (on) {
+        const SubSplit r = sub_finish(BP, w, base, c, float(sum[4]), sizesq, pp[0], pp[1], nleft,
+                                      part == 0 && lane == 0, C, tops, ntop);
+        if (!r.split) {
+            if (buf) for (int i = i0 + lane; i < i1; i += 32) P.perm[0][i] = perm[i];
+        } else {
+            // Stable partition into the other index buffer.
+            const double* ax = c.axis == 2 ? P.z : c.axis == 1 ? P.y : P.x;
+            if (COOP && r.rank) {
+                // By rank the parts before this one are counted anew.
+                before = 0;
+                for (int i = w.s + lane; i < i0; i += 32)
+                    before += sub_rank_left(ax, perm, w.s, w.e, r.mid, i) ? 1 : 0;
+                before = warp_isum(before);
+            }
+            int l = w.s + before, h = r.mid + (i0 - w.s) - before;
+            const unsigned lt = (1u << lane) - 1u;
+            for (int b = i0; b < i1; b += 32) {
+                const int i = b + lane;
+                const bool valid = i < i1;
+                const unsigned short p = valid ? perm[i] : 0;
+                bool left = false;
+                if (valid) left = r.rank ? sub_rank_left(ax, perm, w.s, w.e, r.mid, i)
+                                         : ax[p] < c.splitval;
+                const unsigned bl = __ballot_sync(0xffffffffu, valid && left);
+                const unsigned br = __ballot_sync(0xffffffffu, valid && !left);
+                if (valid) {
+                    const int dst = left ? l + __popc(bl & lt) : h + __popc(br & lt);
+                    if (dst < w.e) to[dst] = p;
+                }
+                l += __popc(bl);
+                h += __popc(br);
+            }
+            if (part == 0 && lane < 2) {
+                const WTask k = sub_child(w, r, base, lane);
+                if (k.e - k.s > THREAD_T) S.cell[next][atomicAdd(&S.ncell[next], 1)] = k;
+                else sub_small(k, base, P, BP, tops, ntop, small, &S.nsmall[0]);
+            }
+        }
+    }
+}
+
+// One block builds the whole subtree of a cell of at most SMALL points.  The points are read
+// once into shared memory.  The cells above THREAD_T points are taken depth by depth, a few
+// warps to a cell near the root, one further down; then the smaller ones in rounds, one
+// thread to a cell and the children onto the next round's list, so that the lanes of a warp
+// work on cells of like size (a thread that walked its own subtree would leave most lanes
+// waiting: its cells of 2 points fall together with another lane's of 20).
+// Bound: the FP64 pipe (2 lanes per clock and SM; ~50 FP64 instructions per point and depth
+// with the parallel transport of a spin-2 field on the sphere, ~100 per cell) once the
+// subtrees fill the chip, the chain of a subtree's depths for small catalogs.
+// Measured, spin-2 field on the sphere, against one warp per subtree with the points in global
+// memory: 10M points 42.8 -> 19.2 ms, 200K 6.8 -> 0.57 ms; 5000 flat points 2.7 -> 0.21 ms.
+// A thread per cell of 32 points with its whole subtree took 34.0, 1.37 and 0.47 ms.
+template <bool FLATC, bool CPLX>
+__global__ void __launch_bounds__(SB, 2) k_subtree(const BuildTask* tasks, Points P0, Points P1,
+                                                   BuildParams BP, Cells C, int* tops, int* ntop,
+                                                   WTask* wstack, int* err)
+{
+    extern __shared__ __align__(16) unsigned char sub_sh[];
+    SubShared& S = *reinterpret_cast<SubShared*>(sub_sh);
+    SubPoints& P = S.P;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const BuildTask root = tasks[blockIdx.x];
+    const int base = root.s, n = root.e - root.s;
+    if (n > SMALL) {                        // (the host sends none)
+        if (tid == 0) set_err(err, DEV_TASK_OVERFLOW);
+        return;
+    }
+    // Lists of cells of 2 .. THREAD_T points, this round's and the next one's: the cells of a
+    // list are disjoint, so n / 2 entries hold them.
+    WTask* list[2] = {wstack + base, wstack + base + n / 2};
+    const Points& A = root.buf ? P1 : P0;
+    for (int i = tid; i < n; i += SB) {
+        P.x[i] = A.x[base + i]; P.y[i] = A.y[base + i]; P.z[i] = A.z[base + i];
+        P.wp[i] = A.wp[base + i];
+        P.w[i] = A.w[base + i]; P.d1[i] = A.d1[base + i]; P.d2[i] = A.d2[base + i];
+        P.perm[0][i] = P.perm[1][i] = (unsigned short)i;
+        P.single[i] = NOT_SINGLE;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const WTask w = {0, n, root.parent, pack_meta(root.side, root.intop, 0, root.mintop, root.maxtop)};
+        S.ncell[0] = S.ncell[1] = S.nsmall[0] = S.nsmall[1] = 0;
+        if (n > THREAD_T) { S.cell[0][0] = w; S.ncell[0] = 1; }
+        else sub_small(w, base, P, BP, tops, ntop, list[0], &S.nsmall[0]);
+    }
+    __syncthreads();
+    // A depth's cells are disjoint and each holds more than THREAD_T points, so a list never
+    // holds more than SBIG - 1 cells, and a cell has fewer points at every depth.
+    for (int cur = 0;; cur ^= 1) {
+        const int m = S.ncell[cur];
+        if (m == 0) break;
+        if (m * 2 <= SW) {
+            const int parts = SW / (m == 1 ? 1 : m == 2 ? 2 : 4);
+            const int ci = wid / parts;
+            const bool on = ci < m;
+            sub_cell<FLATC, CPLX, true>(S, on, S.cell[cur][on ? ci : 0], wid % parts, parts, base,
+                                        BP, C, tops, ntop, cur ^ 1, list[0], lane, wid);
+        } else {
+            for (int ci = wid; ci < m; ci += SW)
+                sub_cell<FLATC, CPLX, false>(S, true, S.cell[cur][ci], 0, 1, base, BP, C, tops,
+                                             ntop, cur ^ 1, list[0], lane, wid);
+        }
+        __syncthreads();
+        if (tid == 0) S.ncell[cur] = 0;
+        __syncthreads();
+    }
+    for (int cur = 0;; cur ^= 1) {
+        const int m = S.nsmall[cur];
+        if (m == 0) break;
+        for (int t = tid; t < m; t += SB) {
+            WTask k[2];
+            if (sub_by_thread<FLATC, CPLX>(list[cur][t], base, P, BP, C, tops, ntop, k)) {
+                sub_small(k[0], base, P, BP, tops, ntop, list[cur ^ 1], &S.nsmall[cur ^ 1]);
+                sub_small(k[1], base, P, BP, tops, ntop, list[cur ^ 1], &S.nsmall[cur ^ 1]);
+            }
+        }
+        __syncthreads();
+        if (tid == 0) S.nsmall[cur] = 0;
+        __syncthreads();
+    }
+    // The points in tree order (the original indices read before any is overwritten) and the
+    // one-point leaves (src/Cell.cpp:564-575).
+    int idx[SMALL / SB], pos[SMALL / SB];
+#pragma unroll
+    for (int u = 0; u < SMALL / SB; ++u) {
+        const int i = tid + u * SB;
+        if (i >= n) continue;
+        const unsigned sg = P.single[i];
+        pos[u] = P.perm[sg != NOT_SINGLE ? (sg >> 1) & 1 : 0][i];
+        idx[u] = A.idx[base + pos[u]];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < SMALL / SB; ++u) {
+        const int i = tid + u * SB;
+        if (i >= n) continue;
+        const int p = pos[u];
+        const double x = P.x[p], y = P.y[p], z = P.z[p];
+        const float w = P.w[p], d1 = P.d1[p], d2 = P.d2[p];
+        P0.x[base + i] = x; P0.y[base + i] = y; P0.z[base + i] = z;
+        P0.wp[base + i] = P.wp[p];
+        P0.w[base + i] = w; P0.d1[base + i] = d1; P0.d2[base + i] = d2;
+        P0.idx[base + i] = idx[u];
+        const unsigned sg = P.single[i];
+        if (sg != NOT_SINGLE)
+            write_cell(C, (BP.n - 1) + base + i, x, y, z, 0.f, w, d1, d2, 1, base + i,
+                       (int)(sg >> 2) - 1, sg & 1);
+    }
+}
+
+// Median splits of cells above SMALL points (rank by a count over the cell, which the
+// cooperative levels have no pass for): one warp walks down from the root and leaves every
+// cell of at most SMALL points to k_subtree.
+__global__ void k_median_levels(BuildTask root, Points P0, Points P1, BuildParams BP, Cells C,
+                                int* tops, int* ntop, WTask* stk, BuildTask* small_out,
+                                int* nsmall_out, int* err)
+{
     const int lane = threadIdx.x & 31;
-    if (t >= ntask) return;
-    const BuildTask root = tasks[t];
-    WTask* stk = wstack + root.s;          // this task owns [root.s, root.e) of the stack
-    // Cells of at most THREAD_T points wait here until each lane can take one.
-    __shared__ WTask deferred[4][32];
-    WTask* dq = deferred[(threadIdx.x >> 5) & 3];
-    int ndq = 0;
     int sp = 0;
     if (lane == 0) {
         WTask w0 = {root.s, root.e, root.parent,
@@ -628,41 +1059,23 @@ __global__ void k_small_subtree(int ntask, const BuildTask* tasks, Points P0, Po
     }
     sp = 1;
     __syncwarp();
-    while (sp > 0 || ndq > 0) {
-        if (sp == 0 || ndq == 32) {
-            __syncwarp();
-            if (lane < ndq) subtree_by_thread(dq[lane], P0, P1, BP, C, tops, ntop, err);
-            ndq = 0;
-            __syncwarp();
-            continue;
-        }
+    while (sp > 0) {
         --sp;
         WTask w = stk[sp];
         __syncwarp();
-        if (w.e - w.s <= THREAD_T) {
-            if (lane == 0) dq[ndq] = w;
-            ++ndq;
-            continue;
-        }
         const int s = w.s, e = w.e, n = e - s;
         const int side = w.meta & 1, buf = (w.meta >> 2) & 1;
         int intop = (w.meta >> 1) & 1;
         const int mintop = ((w.meta >> 8) & 0xfff) - 2048;
         const int maxtop = ((w.meta >> 20) & 0xfff) - 2048;
-        const Points& A = buf ? P1 : P0;
-        const Points& B = buf ? P0 : P1;
-        if (n == 1) {
-            // Single point: a leaf holding the point's own data (src/Cell.cpp:564-575).
-            if (lane == 0) {
-                int id = (BP.n - 1) + s;
-                write_cell(C, id, A.x[s], A.y[s], A.z[s], 0.f, A.w[s], A.d1[s], A.d2[s], 1, s,
-                           w.parent, side);
-                if (intop) add_top(tops, ntop, id, s);
-                if (buf) move_point(A, s, P0, s);
-            }
-            __syncwarp();
+        if (n <= SMALL) {
+            if (lane == 0)
+                small_out[atomicAdd(nsmall_out, 1)] =
+                    BuildTask{s, e, w.parent, side, mintop, maxtop, intop, buf};
             continue;
         }
+        const Points& A = buf ? P1 : P0;
+        const Points& B = buf ? P0 : P1;
         // Pass 1: centroid, weight, bounds (src/Cell.cpp:170-200, 520-525).
         double sx = 0., sy = 0., sz = 0., swp = 0., sw = 0.;
         double xmin = DBL_MAX, ymin = DBL_MAX, zmin = DBL_MAX;
@@ -686,24 +1099,15 @@ __global__ void k_small_subtree(int ntask, const BuildTask* tasks, Points P0, Po
             cx = A.x[s]; cy = A.y[s]; cz = A.z[s];
         }
         const int axis = split_axis(BP.coords, xmax - xmin, ymax - ymin, zmax - zmin);
-        double splitval;
-        if (BP.split == MIDDLE)
-            splitval = axis == 2 ? (zmax + zmin) / 2. : axis == 1 ? (ymax + ymin) / 2.
-                                                                   : (xmax + xmin) / 2.;
-        else
-            splitval = axis == 2 ? cz : axis == 1 ? cy : cx;
-        // Pass 2: size, payload, left count.
+        // Pass 2: size, payload.
         double tcx = cx, tcy = cy, tcz = cz;
         if (BP.coords == THREED) normalize3(tcx, tcy, tcz);
         double sizesq = 0., pr = 0., pi = 0.;
-        int nleft = 0;
         for (int i = s + lane; i < e; i += 32) {
             double px = A.x[i], py = A.y[i], pz = A.z[i];
             double d = (cx - px) * (cx - px) + (cy - py) * (cy - py);
             if (BP.coords != FLAT) d += (cz - pz) * (cz - pz);
             sizesq = fmax(sizesq, d);
-            double c = axis == 2 ? pz : axis == 1 ? py : px;
-            nleft += (c < splitval) ? 1 : 0;
             if (BP.dkind == DK) pr += A.d1[i];
             else if (BP.dkind == DG) {
                 if (BP.coords == FLAT) { pr += A.d1[i]; pi += A.d2[i]; }
@@ -712,13 +1116,9 @@ __global__ void k_small_subtree(int ntask, const BuildTask* tasks, Points P0, Po
             }
         }
         sizesq = warp_max(sizesq); pr = warp_sum(pr); pi = warp_sum(pi);
-        nleft = warp_isum(nleft);
         bool is_top;
-        bool split = decide_split(BP, intop, mintop, maxtop, sizesq, is_top);
-        bool use_rank = (BP.split == MEDIAN);
-        int mid = s + nleft;
-        if (split && !use_rank && (nleft == 0 || nleft == n)) use_rank = true;
-        if (split && use_rank) mid = (s + e) / 2;   // SplitDataCore<Median>, src/Cell.cpp:464-479
+        const bool split = decide_split(BP, intop, mintop, maxtop, sizesq, is_top);
+        const int mid = (s + e) / 2;    // SplitDataCore<Median>, src/Cell.cpp:464-479
         float d1 = float(pr), d2 = float(pi);
         if (BP.dkind == DN) { d1 = 0.f; d2 = 0.f; }
         if (BP.dkind == DK) d2 = 0.f;
@@ -741,24 +1141,20 @@ __global__ void k_small_subtree(int ntask, const BuildTask* tasks, Points P0, Po
             bool valid = i < e;
             bool left = false;
             if (valid) {
+                // Rank of point i by (coordinate, position): the mid - s smallest go left.
                 double c = axis == 2 ? A.z[i] : axis == 1 ? A.y[i] : A.x[i];
-                if (!use_rank) {
-                    left = c < splitval;
-                } else {
-                    // Rank of point i by (coordinate, position): the mid-s smallest go left.
-                    int rank = 0;
-                    for (int j = s; j < e; ++j) {
-                        double cj = axis == 2 ? A.z[j] : axis == 1 ? A.y[j] : A.x[j];
-                        rank += (cj < c || (cj == c && j < i)) ? 1 : 0;
-                    }
-                    left = rank < (mid - s);
+                int rank = 0;
+                for (int j = s; j < e; ++j) {
+                    double cj = axis == 2 ? A.z[j] : axis == 1 ? A.y[j] : A.x[j];
+                    rank += (cj < c || (cj == c && j < i)) ? 1 : 0;
                 }
+                left = rank < (mid - s);
             }
             unsigned bl = __ballot_sync(0xffffffffu, valid && left);
             unsigned br = __ballot_sync(0xffffffffu, valid && !left);
             if (valid) {
                 int dst = left ? lbase + __popc(bl & lt) : rbase + __popc(br & lt);
-                move_point(A, i, B, dst);
+                if (dst < e) move_point(A, i, B, dst);
             }
             lbase += __popc(bl);
             rbase += __popc(br);
@@ -778,6 +1174,29 @@ __global__ void k_small_subtree(int ntask, const BuildTask* tasks, Points P0, Po
     }
 }
 
+template <bool FLATC, bool CPLX>
+static int subtree_launch(int ntask, const BuildTask* tasks, Points P0, Points P1,
+                          const BuildParams& BP, const Cells& C, int* tops, int* ntop,
+                          WTask* wstack, int* err, cudaStream_t st)
+{
+    TC_CU(cudaFuncSetAttribute(k_subtree<FLATC, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(SubShared)));
+    count_launch();
+    k_subtree<FLATC, CPLX><<<ntask, SB, sizeof(SubShared), st>>>(tasks, P0, P1, BP, C, tops, ntop,
+                                                                 wstack, err);
+    TC_CU(cudaGetLastError());
+    return 0;
+}
+
+static int launch_subtrees(int ntask, const BuildTask* tasks, Points P0, Points P1,
+                           const BuildParams& BP, const Cells& C, int* tops, int* ntop,
+                           WTask* wstack, int* err, cudaStream_t st)
+{
+    const bool flat = BP.coords == FLAT, cplx = BP.dkind == DG;
+    auto* f = flat ? (cplx ? subtree_launch<true, true> : subtree_launch<true, false>)
+                   : (cplx ? subtree_launch<false, true> : subtree_launch<false, false>);
+    return f(ntask, tasks, P0, P1, BP, C, tops, ntop, wstack, err, st);
+}
 // ---------------------------------------------------------------------------------------
 // Structural check of the finished tree: every internal cell has two children that split
 // its point range exactly.  This guarantees that the traversal (which only descends into
@@ -850,7 +1269,14 @@ int build_tree(const BuildParams& BP, Points bufs[2], Cells C, int* d_tops, int*
     TC_CU(cudaMemsetAsync(d_ntop, 0, sizeof(int), st));
     TC_CU(cudaMemsetAsync(S.counters, 0, 2 * sizeof(int), st));
     if (n > SMALL && BP.split != MEDIAN) big.push_back(root);
-    else {
+    else if (n > SMALL) {
+        count_launch();
+        k_median_levels<<<1, 32, 0, st>>>(root, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
+                                          S.small, S.counters + 1, d_err);
+        TC_CU(cudaGetLastError());
+        TC_CU(cudaMemcpyAsync(&nsmall, S.counters + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TC_CU(cudaStreamSynchronize(st));
+    } else {
         TC_CU(cudaMemcpyAsync(S.small, &root, sizeof(BuildTask), cudaMemcpyHostToDevice, st));
         nsmall = 1;
         TC_CU(cudaMemcpyAsync(S.counters + 1, &nsmall, sizeof(int), cudaMemcpyHostToDevice, st));
@@ -893,13 +1319,9 @@ int build_tree(const BuildParams& BP, Points bufs[2], Cells C, int* d_tops, int*
             TC_CU(cudaMemcpy(big.data(), S.big_next, cnt[0] * sizeof(BuildTask), cudaMemcpyDeviceToHost));
         nsmall = cnt[1];
     }
-    if (nsmall > 0) {
-        int threads = 128;
-        long long blocks = ((long long)nsmall * 32 + threads - 1) / threads;
-        count_launch(); k_small_subtree<<<(unsigned)blocks, threads, 0, st>>>(nsmall, S.small, bufs[0], bufs[1],
-                                                              BP, C, d_tops, d_ntop, S.wstack, d_err);
-        TC_CU(cudaGetLastError());
-    }
+    if (nsmall > 0)
+        TC_TRY(launch_subtrees(nsmall, S.small, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
+                               d_err, st));
     int ntop = 0;
     TC_CU(cudaMemcpyAsync(&ntop, d_ntop, sizeof(int), cudaMemcpyDeviceToHost, st));
     TC_CU(cudaStreamSynchronize(st));
