@@ -109,7 +109,7 @@ struct tc_corr2 {
     int nwarps_alloc = 0, nq_alloc = 0;
     double* wacc = nullptr;
     unsigned long long* wnp = nullptr;
-    double* tot = nullptr;
+    double* tot = nullptr;               // slices' sums of the rows, then their total
     unsigned long long* totnp = nullptr;
     unsigned long long* ctl = nullptr;   // root_next, nout, counters[3]
     int* idle = nullptr;
@@ -423,6 +423,18 @@ int field_create_impl(int dkind, int coords, const double* x, const double* y, c
 
 double sqr(double x) { return x * x; }
 
+// Device memory of the stream-ordered pool for the length of a call.
+struct PoolBuf {
+    void* p = nullptr;
+    cudaStream_t st = nullptr;
+    ~PoolBuf() { if (p) cudaFreeAsync(p, st); }
+};
+
+// The rows of sums (per warp of the expansion and the tiles, per unit of the walk) are added
+// up in two steps: SUM_SLICES slices of rows, then the slices, each in order.  One thread per
+// column over all rows took 0.5-1.5 ms for the 4256 rows of a full grid.
+constexpr int SUM_SLICES = 128;
+
 // Accumulators of the level-by-level expansion (per-warp FP64 bins, totals, control words).
 int expand_scratch(tc_corr2* c, int nwarps, int nq)
 {
@@ -431,8 +443,8 @@ int expand_scratch(tc_corr2* c, int nwarps, int nq)
         dfree(c->d_err);
         TC_TRY(dalloc(&c->wacc, (size_t)nwarps * nq * c->nbins));
         TC_TRY(dalloc(&c->wnp, (size_t)nwarps * c->nbins));
-        TC_TRY(dalloc(&c->tot, (size_t)nq * c->nbins));
-        TC_TRY(dalloc(&c->totnp, (size_t)c->nbins));
+        TC_TRY(dalloc(&c->tot, (size_t)(SUM_SLICES + 1) * nq * c->nbins));
+        TC_TRY(dalloc(&c->totnp, (size_t)(SUM_SLICES + 1) * c->nbins));
         TC_TRY(dalloc(&c->ctl, 8));
         TC_TRY(dalloc(&c->d_err, 1));
         c->nwarps_alloc = nwarps;
@@ -466,6 +478,15 @@ int pool_alloc_int2(int2** p, size_t count, cudaStream_t st)
                        " bytes failed: " + cudaGetErrorString(e));
         return TC_ERR_NOMEM;
     }
+    return 0;
+}
+
+int pool_alloc(PoolBuf& b, size_t bytes, cudaStream_t st)
+{
+    int2* p = nullptr;
+    TC_TRY(pool_alloc_int2(&p, (bytes + sizeof(int2) - 1) / sizeof(int2), st));
+    b.p = p;
+    b.st = st;
     return 0;
 }
 
@@ -654,6 +675,239 @@ int expand_run(tc_corr2* c, const TravParams& T, int blocks, long long npoints, 
     return TC_OK;
 }
 
+// The total of nrow rows into c->tot, c->totnp.
+int sum_rows(tc_corr2* c, const double* rows, const unsigned long long* rownp, long long nrow,
+             int nq, cudaStream_t st)
+{
+    const int nd = nq * c->nbins, ni = c->nbins;
+    double* part = c->tot + nd;
+    unsigned long long* partnp = c->totnp + ni;
+    TC_TRY(launch_sum_rows(rows, rownp, nrow, nullptr, SUM_SLICES, nd, ni, part, partnp, st));
+    return launch_sum_rows(part, partnp, SUM_SLICES, nullptr, 1, nd, ni, c->tot, c->totnp, st);
+}
+
+// Corr2::finishProcess adds into the caller's arrays (src/Corr2.cpp:527-566).
+void add_outputs(tc_corr2* c, const double* tot, const unsigned long long* totnp, int quick)
+{
+    const int nb = c->nbins;
+    for (int k = 0; k < nb && !c->no_output; ++k) {
+        c->weight[k] += tot[k];
+        if (!quick) {
+            c->meanr[k] += tot[nb + k];
+            c->meanlogr[k] += tot[2 * nb + k];
+            c->npairs[k] += (double)totnp[k];
+        }
+        add_xi(c, tot, nb, k);
+    }
+}
+
+// Stack items per warp of the walk: a pop of 32 items pushes at most 128, so a level of the
+// pair tree holds at most 96 items more than the one above; a pair of trees of depth d is at
+// most 2 d levels deep, and the trees of n points are rarely deeper than log2 n + 8.  (A walk
+// that needs more reports it, and the call takes the expansion instead.)
+int walk_stack_cap(long long npoints)
+{
+    int lg = 1;
+    while ((1LL << lg) < npoints) ++lg;
+    // Test hook: a shorter stack makes the way back to the expansion reachable.
+    if (const char* e = std::getenv("TCGPU_WALK_STACK")) return std::max(128, std::atoi(e));
+    return 96 * 2 * (lg + 8) + 128;
+}
+
+// Rows the walk's units may fill: enough that the last units to finish do not matter
+// (~7 per warp), bounded by 256 MB.
+long long walk_max_units(int nq, int nb)
+{
+    const long long row = 8LL * (nq + 1) * nb;
+    return std::max(4096LL, std::min(32768LL, (256LL << 20) / row));
+}
+
+// The bin_slop traversal of whole fields: the expansion up to a level of enough items, then
+// the walk.  *done = false when the walk ran out of stack (nothing is added then).
+int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cudaStream_t st,
+             int quick, bool* done)
+{
+    const int nb = c->nbins;
+    const long long npoints = n1 + (T.autoc ? 0 : n2);
+    *done = true;
+    int blocks = 0, nwarps = 0, wblocks = 0, wwarps = 0;
+    TC_TRY(walk_grid(T, &wblocks, &wwarps));
+    // Items the walk starts from: 8 per point, 2^17 to 2^21 (or the tuned chunk).
+    const long long want = c->chunk > 0 ? std::min(c->chunk, 1LL << 21)
+                                        : std::max(1LL << 17, std::min(1LL << 21, 8 * npoints));
+    // With few points per top cell a top-level pair is a small subtree already (at 32 x 32
+    // points some 4000 evaluations at most), and the walk starts from those.
+    const double per_pair = ((double)n1 / (double)T.ntop1) * ((double)n2 / (double)T.ntop2);
+    const bool expand = T.ngen < want && (per_pair > 1024. || T.ngen < 4096);
+    if (expand) TC_TRY(expand_grid(nq, nb, &blocks, &nwarps, 0));
+    const long long max_units = walk_max_units(nq, nb);
+    TC_TRY(expand_scratch(c, (int)(nwarps + max_units), nq));
+    T.wacc = c->wacc; T.wnp = c->wnp; T.err = c->d_err;
+    T.counters = c->ctl + 2;
+    T.nsamples = c->ctl + 6;
+    T.in_tasks = nullptr; T.nin = 0;
+    T.wctr = nullptr;
+    T.nwarps = nwarps;
+    TC_CU(cudaMemsetAsync(c->ctl, 0, 8 * sizeof(unsigned long long), st));
+    TC_CU(cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
+    cudaEvent_t e0, e1, e2;
+    TC_CU(cudaEventCreate(&e0)); TC_CU(cudaEventCreate(&e1)); TC_CU(cudaEventCreate(&e2));
+    struct Events { cudaEvent_t a, b, c; ~Events() { cudaEventDestroy(a); cudaEventDestroy(b); cudaEventDestroy(c); } } ev{e0, e1, e2};
+    TC_CU(cudaEventRecord(e0, st));
+    WalkParams W;
+    std::memset(&W, 0, sizeof(W));
+    walk_constants(T, W);
+    int derr = 0;
+    long long launches = 0, n_items = T.ngen;
+    PoolBuf lev[2], dout, dcnt, stacks;
+    if (expand) {
+        // Each launch takes a whole level, so two buffers hold the level and its children.
+        TC_CU(cudaMemsetAsync(c->wacc, 0, sizeof(double) * (size_t)nwarps * nq * nb, st));
+        TC_CU(cudaMemsetAsync(c->wnp, 0, sizeof(unsigned long long) * (size_t)nwarps * nb, st));
+        if (!c->sched) TC_TRY(dalloc(&c->sched, 1));
+        const long long cap = 4 * want;
+        for (auto& b : lev) TC_TRY(pool_alloc(b, sizeof(int2) * (size_t)cap, st));
+        if (g_deterministic.load()) {
+            const long long ipw = det_items_per_warp(want, nwarps);
+            TC_TRY(pool_alloc(dout, sizeof(int2) * (size_t)(4 * ipw * nwarps), st));
+            TC_TRY(pool_alloc(dcnt, sizeof(int) * 2 * (size_t)nwarps, st));
+            // (k_compact reads the tile counts too)
+            TC_CU(cudaMemsetAsync(dcnt.p, 0, sizeof(int) * 2 * (size_t)nwarps, st));
+            T.det = 1; T.det_nw = nwarps;
+            T.det_out = static_cast<int2*>(dout.p);
+            T.det_cnt = static_cast<int*>(dcnt.p);
+            T.det_ccap = 4 * ipw; T.det_tcap = ipw;
+        }
+        ExpandSched hs;
+        std::memset(&hs, 0, sizeof(hs));
+        hs.cnt[0] = T.ngen;
+        hs.cap = cap; hs.chunk_max = want; hs.out_level = -1; hs.nlev = EXP_MAXLEV;
+        hs.walk_min = want;
+        for (int l = 1; l < EXP_MAXLEV; ++l) hs.lev[l] = static_cast<int2*>(lev[l & 1].p);
+        TC_CU(cudaMemcpyAsync(c->sched, &hs, sizeof(hs), cudaMemcpyHostToDevice, st));
+        for (int batch = 0;; ++batch) {
+            TC_TRY(launch_expand_batch(T, blocks, c->sched, 8, st));
+            TC_CU(cudaMemcpyAsync(&hs, c->sched, sizeof(hs), cudaMemcpyDeviceToHost, st));
+            TC_CU(cudaMemcpyAsync(&derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            TC_CU(cudaStreamSynchronize(st));
+            if (derr || hs.done) break;
+            if (hs.need_levels) {
+                set_last_error("the dual-tree expansion is deeper than 512 levels");
+                return TC_ERR_DEVICE;
+            }
+        }
+        launches = hs.launches;
+        n_items = hs.walk_level > 0 ? hs.cnt[hs.walk_level] : 0;
+        W.items = hs.walk_level > 0 ? hs.lev[hs.walk_level] : nullptr;
+    }
+    long long rows = nwarps;
+    if (!derr && n_items > 0xFFFFFFFFLL) { *done = false; return TC_OK; }   // (32-bit items)
+    if (!derr && n_items > 0) {
+        const long long n_units = std::min(max_units, (n_items + 31) / 32);
+        const int cap = walk_stack_cap(npoints);
+        TC_TRY(pool_alloc(stacks, sizeof(int2) * (size_t)cap * wwarps, st));
+        W.n_items = (unsigned)n_items; W.n_units = (unsigned)n_units;
+        W.next = c->ctl;
+        W.stacks = static_cast<int2*>(stacks.p);
+        W.stack_cap = cap;
+        W.rows = c->wacc + (size_t)nwarps * nq * nb;
+        W.rownp = c->wnp + (size_t)nwarps * nb;
+        rows += n_units;
+        TC_CU(cudaMemsetAsync(W.rows, 0, sizeof(double) * (size_t)n_units * nq * nb, st));
+        TC_CU(cudaMemsetAsync(W.rownp, 0, sizeof(unsigned long long) * (size_t)n_units * nb, st));
+        TC_TRY(launch_walk(T, W, wblocks, st));
+        ++launches;
+    }
+    TC_CU(cudaEventRecord(e1, st));
+    TC_TRY(sum_rows(c, c->wacc, c->wnp, rows, nq, st));
+    launches += 2;
+    TC_CU(cudaEventRecord(e2, st));
+    std::vector<double> tot((size_t)nq * nb);
+    std::vector<unsigned long long> totnp(nb);
+    unsigned long long cntr[4] = {0, 0, 0, 0};
+    TC_CU(cudaMemcpyAsync(cntr, c->ctl + 2, sizeof(cntr), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaMemcpyAsync(&derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaMemcpyAsync(tot.data(), c->tot, tot.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaMemcpyAsync(totnp.data(), c->totnp, nb * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaStreamSynchronize(st));
+    if (derr == DEV_STACK_OVERFLOW) { *done = false; return TC_OK; }
+    if (derr) {
+        set_last_error(std::string("device error: ") + dev_err_msg(derr));
+        return TC_ERR_DEVICE;
+    }
+    float ms = 0.f, ms2 = 0.f;
+    TC_CU(cudaEventElapsedTime(&ms, e0, e1));
+    TC_CU(cudaEventElapsedTime(&ms2, e0, e2));
+    c->stats.cell_pairs = (int64_t)cntr[0];
+    c->stats.accepted = (int64_t)cntr[1];
+    c->stats.escalated = (int64_t)cntr[2];
+    c->stats.launches = launches;
+    c->stats.traverse_ms = ms2;
+    c->stats.expand_ms = ms;
+    add_outputs(c, tot.data(), totnp.data(), quick);
+    return TC_OK;
+}
+
+// The patch batch by the walk, straight from the top-level items: every unit belongs to one
+// patch pair, so its row holds that pair's sums only and the pairs' rows are added in order.
+// (The expansion's warps mix pairs, each with atomic adds to its pair's sums.)  *walked =
+// false when it does not apply or ran out of stack.
+int walk_patches(tc_corr2* c, TravParams T, const std::vector<long long>& roff,
+                 const std::vector<int>& P1, const std::vector<int>& P2, long long npoints, int nq,
+                 double* pacc, unsigned long long* pnp, cudaStream_t st, int* derr,
+                 long long* launches, bool* walked)
+{
+    const int nb = c->nbins, npair = (int)P1.size();
+    // Units in proportion to the pairs' items; an item within a patch counts four times (near
+    // pairs, where the traversal goes deep).
+    double weight = 0.;
+    for (int p = 0; p < npair; ++p) {
+        const long long n = roff[p + 1] - roff[p];
+        if (n >= (1LL << 32)) return TC_OK;
+        weight += (double)n * (P1[p] == P2[p] ? 4. : 1.);
+    }
+    const double share = (double)walk_max_units(nq, nb) / std::max(weight, 1.);
+    std::vector<int> uoff(npair + 1, 0);
+    for (int p = 0; p < npair; ++p) {
+        const long long n = roff[p + 1] - roff[p];
+        const long long u = (long long)(share * (double)n * (P1[p] == P2[p] ? 4. : 1.));
+        uoff[p + 1] = uoff[p] + (int)std::max(1LL, std::min(u, (n + 31) / 32));
+    }
+    const int n_units = uoff[npair];
+    int wblocks = 0, wwarps = 0;
+    TC_TRY(walk_grid(T, &wblocks, &wwarps));
+    TC_TRY(expand_scratch(c, n_units, nq));
+    T.err = c->d_err; T.counters = c->ctl + 2;
+    T.wctr = nullptr;
+    WalkParams W;
+    std::memset(&W, 0, sizeof(W));
+    walk_constants(T, W);
+    PoolBuf stacks, off;
+    const int cap = walk_stack_cap(npoints);
+    TC_TRY(pool_alloc(stacks, sizeof(int2) * (size_t)cap * wwarps, st));
+    TC_TRY(pool_alloc(off, sizeof(int) * uoff.size(), st));
+    TC_CU(cudaMemcpyAsync(off.p, uoff.data(), sizeof(int) * uoff.size(), cudaMemcpyHostToDevice, st));
+    TC_CU(cudaMemsetAsync(c->ctl, 0, 8 * sizeof(unsigned long long), st));
+    TC_CU(cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
+    TC_CU(cudaMemsetAsync(c->wacc, 0, sizeof(double) * (size_t)n_units * nq * nb, st));
+    TC_CU(cudaMemsetAsync(c->wnp, 0, sizeof(unsigned long long) * (size_t)n_units * nb, st));
+    W.n_units = (unsigned)n_units;
+    W.unit_off = static_cast<const int*>(off.p);
+    W.next = c->ctl;
+    W.stacks = static_cast<int2*>(stacks.p);
+    W.stack_cap = cap;
+    W.rows = c->wacc;
+    W.rownp = c->wnp;
+    TC_TRY(launch_walk(T, W, wblocks, st));
+    TC_TRY(launch_sum_rows(c->wacc, c->wnp, n_units, W.unit_off, npair, nq * nb, nb, pacc, pnp, st));
+    TC_CU(cudaMemcpyAsync(derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaStreamSynchronize(st));
+    if (*derr == DEV_STACK_OVERFLOW) { *derr = 0; return TC_OK; }
+    *launches = 2;
+    *walked = true;
+    return TC_OK;
+}
+
 // BaseCorr2::process for one or two fields.
 int corr_process(tc_corr2* c, tc_field* f1, tc_field* f2, int quick, int metric)
 {
@@ -713,12 +967,23 @@ int corr_process(tc_corr2* c, tc_field* f1, tc_field* f2, int quick, int metric)
     T.mlp = c->mlp;
     T.samples = c->samples; T.sample_cap = c->sample_cap; T.sample_mod = c->sample_mod;
     int blocks = 0, nwarps = 0;
-    TC_TRY(expand_grid(nq, nb, &blocks, &nwarps, mode));
     // Exact mode: every pair the reference accepts is a pair of leaves (angle_slop 0, or two
     // brute fields), so the leaf pairs below small cell pairs go through k_tiles.
     // TCGPU_TILES=0 turns the tiles off (the traversal then walks down to the leaves).
     bool tiles = mode == 0 && (c->a == 0. || (f1->brute && g->brute));
     if (const char* ev = std::getenv("TCGPU_TILES")) tiles = tiles && std::atoi(ev) != 0;
+    if (mode == 0 && !tiles) {
+        // The bin_slop rule: a short expansion, then the walk.  TCGPU_WALK=0 turns the walk off
+        // (the expansion then goes down to the last level).
+        const char* ev = std::getenv("TCGPU_WALK");
+        if (!ev || std::atoi(ev) != 0) {
+            bool done = false;
+            TravParams T2 = T;
+            TC_TRY(walk_run(c, T2, f1->n, g->n, nq, st, quick, &done));
+            if (done) return TC_OK;
+        }
+    }
+    TC_TRY(expand_grid(nq, nb, &blocks, &nwarps, mode));
     int tblocks = 0, twarps = 0;
     if (tiles) {
         T.tile_leaf = c->tile_leaf > 0 ? c->tile_leaf : TILE_LEAF;   // (tiles_grid picks the
@@ -821,7 +1086,7 @@ int corr_process(tc_corr2* c, tc_field* f1, tc_field* f2, int quick, int metric)
         cudaEventDestroy(e0); cudaEventDestroy(e1);
         return TC_ERR_DEVICE;
     }
-    TC_TRY(launch_reduce(nwarps + twarps, nq, nb, c->wacc, c->wnp, c->tot, c->totnp, st));
+    TC_TRY(sum_rows(c, c->wacc, c->wnp, nwarps + twarps, nq, st));
     TC_CU(cudaEventRecord(e1, st));
     std::vector<double> tot((size_t)nq * nb);
     std::vector<unsigned long long> totnp(nb);
@@ -849,16 +1114,7 @@ int corr_process(tc_corr2* c, tc_field* f1, tc_field* f2, int quick, int metric)
     c->stats.tiles = tiles ? (int64_t)tcnt[2] : 0;
     c->stats.tile_pairs = (int64_t)tcnt[3];
     c->stats.tile_escalated = (int64_t)tcnt[4];
-    // Corr2::finishProcess adds into the caller's arrays (src/Corr2.cpp:527-566).
-    for (int k = 0; k < nb && !c->no_output; ++k) {
-        c->weight[k] += tot[k];
-        if (!quick) {
-            c->meanr[k] += tot[nb + k];
-            c->meanlogr[k] += tot[2 * nb + k];
-            c->npairs[k] += (double)totnp[k];
-        }
-        add_xi(c, tot.data(), nb, k);
-    }
+    add_outputs(c, tot.data(), totnp.data(), quick);
     return TC_OK;
 }
 
@@ -973,7 +1229,7 @@ int corr_process_auto_noalloc(tc_corr2* c, tc_field* f, int quick, int metric)
         set_last_error(std::string("device error: ") + dev_err_msg(derr));
         return TC_ERR_DEVICE;
     }
-    TC_TRY(launch_reduce(nwarps, nq, nb, wacc, wnp, tot, totnp, st));
+    TC_TRY(launch_sum_rows(wacc, wnp, nwarps, nullptr, 1, nq * nb, nb, tot, totnp, st));
     double h_tot[NOALLOC_NQ * NOALLOC_MAXNB];
     unsigned long long h_np[NOALLOC_MAXNB];
     unsigned long long cnt[3];
@@ -1819,9 +2075,7 @@ int tc_corr2_process_patches(tc_corr2* c, tc_field* const* fields, int npatch, i
             cudaMemcpyAsync(d_pairs, hpairs.data(), sizeof(int2) * hpairs.size(), cudaMemcpyHostToDevice, st) ||
             cudaMemcpyAsync(d_top, htop.data(), sizeof(int) * htop.size(), cudaMemcpyHostToDevice, st) ||
             cudaMemcpyAsync(d_topoff, htopoff.data(), sizeof(int) * htopoff.size(), cudaMemcpyHostToDevice, st) ||
-            cudaMemcpyAsync(d_pidx, pidx.data(), sizeof(int) * pidx.size(), cudaMemcpyHostToDevice, st) ||
-            cudaMemsetAsync(pacc, 0, sizeof(double) * (size_t)npair * nq * nb, st) ||
-            cudaMemsetAsync(pnp, 0, sizeof(unsigned long long) * (size_t)npair * nb, st)) {
+            cudaMemcpyAsync(d_pidx, pidx.data(), sizeof(int) * pidx.size(), cudaMemcpyHostToDevice, st)) {
             set_last_error("patch setup copy failed"); rc = TC_ERR_CUDA; break;
         }
         TravParams T;
@@ -1833,18 +2087,27 @@ int tc_corr2_process_patches(tc_corr2* c, tc_field* const* fields, int npatch, i
         T.mode = 3; T.npatch = npatch; T.pair_index = d_pidx; T.pacc = pacc; T.pnp = pnp;
         T.npair = npair; T.proot_off = d_roff; T.ppairs = d_pairs; T.ptop = d_top;
         T.ptop_off = d_topoff;
-        int blocks = 0, nwarps = 0;
-        if ((rc = expand_grid(nq, nb, &blocks, &nwarps, 3))) break;
-        if ((rc = expand_scratch(c, nwarps, nq))) break;
-        T.nwarps = nwarps; T.err = c->d_err; T.counters = c->ctl + 2;
-        cudaMemsetAsync(c->ctl, 0, 8 * sizeof(unsigned long long), st);
-        cudaMemsetAsync(c->d_err, 0, sizeof(int), st);
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0); cudaEventCreate(&e1);
+        struct Events { cudaEvent_t a, b; ~Events() { cudaEventDestroy(a); cudaEventDestroy(b); } } ev{e0, e1};
         cudaEventRecord(e0, st);
         int derr = 0;
         long long launches = 0;
-        rc = expand_run(c, T, blocks, npoints, st, &derr, &launches);
+        bool walked = false;
+        const char* env = std::getenv("TCGPU_WALK");
+        if (!env || std::atoi(env) != 0)
+            rc = walk_patches(c, T, hroff, P1, P2, npoints, nq, pacc, pnp, st, &derr, &launches, &walked);
+        if (!rc && !walked) {
+            int blocks = 0, nwarps = 0;
+            if ((rc = expand_grid(nq, nb, &blocks, &nwarps, 3))) break;
+            if ((rc = expand_scratch(c, nwarps, nq))) break;
+            T.nwarps = nwarps; T.err = c->d_err; T.counters = c->ctl + 2;
+            cudaMemsetAsync(c->ctl, 0, 8 * sizeof(unsigned long long), st);
+            cudaMemsetAsync(c->d_err, 0, sizeof(int), st);
+            cudaMemsetAsync(pacc, 0, sizeof(double) * (size_t)npair * nq * nb, st);
+            cudaMemsetAsync(pnp, 0, sizeof(unsigned long long) * (size_t)npair * nb, st);
+            rc = expand_run(c, T, blocks, npoints, st, &derr, &launches);
+        }
         cudaEventRecord(e1, st);
         if (!rc && derr) { set_last_error(std::string("device error: ") + dev_err_msg(derr)); rc = TC_ERR_DEVICE; }
         std::vector<double> hacc;
@@ -1858,10 +2121,9 @@ int tc_corr2_process_patches(tc_corr2* c, tc_field* const* fields, int npatch, i
                 cudaMemcpyAsync(cntr, c->ctl + 2, sizeof(cntr), cudaMemcpyDeviceToHost, st) ||
                 cudaStreamSynchronize(st)) { set_last_error("result copy failed"); rc = TC_ERR_CUDA; }
         }
+        if (rc) break;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
-        cudaEventDestroy(e0); cudaEventDestroy(e1);
-        if (rc) break;
         // results[p] = weight, meanr, meanlogr, xi0..xi3, npairs (each nb doubles).
         for (int p = 0; p < npair; ++p) {
             double* r = results + (size_t)p * 8 * nb;

@@ -30,6 +30,7 @@
 #include "tc_host.hpp"
 #include "traverse2pt.hpp"
 #include "pair_math.cuh"
+#include "roots.cuh"
 #include "learned.cuh"
 
 namespace tc {
@@ -201,67 +202,6 @@ __device__ __forceinline__ Decision decide32(const TravParams& T, float rsq, flo
     }
     D.act = which == 2 ? ACT_SPLIT12 : (sw ? ACT_SPLIT2 : ACT_SPLIT1);
     return D;
-}
-
-// ---------------------------------------------------------------------------------------
-// Root generation.
-
-// Row i of the upper triangle (self + pairs j > i) of n top cells starts at
-// i*n - i*(i-1)/2; item g of that enumeration.
-__device__ __forceinline__ void tri_index(long long n, long long g, long long& i, long long& j)
-{
-    double b = 2.0 * n + 1.0;
-    i = (long long)((b - sqrt(b * b - 8.0 * (double)g)) * 0.5);
-    if (i < 0) i = 0;
-    if (i > n - 1) i = n - 1;
-    while (i > 0 && i * n - i * (i - 1) / 2 > g) --i;
-    while (i + 1 < n && (i + 1) * n - (i + 1) * i / 2 <= g) ++i;
-    j = g - (i * n - i * (i - 1) / 2) + i;
-}
-
-// Patches: root g of all patch pairs (auto enumeration within a patch, all top pairs
-// across two patches).
-__device__ __forceinline__ int2 make_patch_root(const TravParams& T, long long g)
-{
-    int lo = 0, hi = T.npair;          // proot_off[lo] <= g < proot_off[hi]
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (T.proot_off[mid] <= g) lo = mid; else hi = mid;
-    }
-    const int2 pr = T.ppairs[lo];
-    const long long r = g - T.proot_off[lo];
-    const int* ti = T.ptop + T.ptop_off[pr.x];
-    if (pr.x == pr.y) {
-        const long long n = T.ptop_off[pr.x + 1] - T.ptop_off[pr.x];
-        long long i, j;
-        tri_index(n, r, i, j);
-        return j == i ? make_int2(ti[i], -1) : make_int2(ti[i], ti[j]);
-    }
-    const int* tj = T.ptop + T.ptop_off[pr.y];
-    const long long nj = T.ptop_off[pr.y + 1] - T.ptop_off[pr.y];
-    return make_int2(ti[r / nj], tj[r % nj]);
-}
-
-template <int MODE = 0>
-__device__ __forceinline__ int2 make_root(const TravParams& T, long long g)
-{
-    if constexpr (MODE == 3) return make_patch_root(T, g);
-    if (g >= T.ngen) return T.in_tasks[g - T.ngen];
-    if (T.autoc) {
-        // Row i of the upper triangle (self + pairs j>i) starts at i*n - i*(i-1)/2.
-        long long n = T.ntop1;
-        double b = 2.0 * n + 1.0;
-        long long i = (long long)((b - sqrt(b * b - 8.0 * (double)g)) * 0.5);
-        if (i < 0) i = 0;
-        if (i > n - 1) i = n - 1;
-        while (i > 0 && i * n - i * (i - 1) / 2 > g) --i;
-        while (i + 1 < n && (i + 1) * n - (i + 1) * i / 2 <= g) ++i;
-        long long j = g - (i * n - i * (i - 1) / 2) + i;
-        if (j == i) return make_int2(T.tops1[i], -1);
-        return make_int2(T.tops1[i], T.tops1[j]);
-    }
-    long long i = g / T.ntop2, j = g - i * T.ntop2;
-    return make_int2(T.tops1[i], T.tops2[j]);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -903,9 +843,16 @@ __device__ void sched_step(ExpandSched* S)
     S->n_in = 0;
     S->pending = 0;
     if (S->done || S->need_levels) return;
-    int L = S->nlev - 1;
+    // No level above `top` holds items (a search from the last buffer down took 20-40 us of
+    // one thread's loads per launch with 512 levels).
+    int L = S->top;
     while (L >= 0 && S->cnt[L] == 0) --L;
     if (L < 0) { S->done = 1; return; }
+    if (L > 0 && S->walk_min > 0 && S->cnt[L] >= S->walk_min) {
+        S->walk_level = L;
+        S->done = 1;
+        return;
+    }
     if (L + 1 >= S->nlev) { S->need_levels = 1; return; }
     const long long chunk = S->cnt[L] < S->chunk_max ? S->cnt[L] : S->chunk_max;
     const long long start = S->cnt[L] - chunk;
@@ -916,6 +863,7 @@ __device__ void sched_step(ExpandSched* S)
     S->out = S->lev[L + 1] + S->cnt[L + 1];
     S->out_cap = S->cap - S->cnt[L + 1];
     S->out_level = L + 1;
+    S->top = L + 1;
     S->launches += 1;
     S->pending = 1;
 }
@@ -1034,24 +982,6 @@ long long det_items_per_warp(long long chunk, int nwarps)
     return 32LL * ((chunk + per - 1) / per);
 }
 
-// Sum of the per-warp totals in a fixed order: out[q*nb+k] (double), outnp[k] (u64).
-__global__ void k_reduce_acc(int nwarps, int nq, int nb, const double* wacc,
-                             const unsigned long long* wnp, double* out,
-                             unsigned long long* outnp)
-{
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < nq * nb) {
-        double s = 0.;
-        for (int w = 0; w < nwarps; ++w) s += wacc[(size_t)w * nq * nb + q];
-        out[q] = s;
-    }
-    if (q < nb) {
-        unsigned long long s = 0;
-        for (int w = 0; w < nwarps; ++w) s += wnp[(size_t)w * nb + q];
-        outnp[q] = s;
-    }
-}
-
 // ---------------------------------------------------------------------------------------
 // Host side.
 
@@ -1166,16 +1096,6 @@ int launch_traverse(const TravParams& T, int blocks, cudaStream_t st)
     return 0;
 }
 
-int launch_reduce(int nwarps, int nq, int nb, const double* wacc, const unsigned long long* wnp,
-                  double* out, unsigned long long* outnp, cudaStream_t st)
-{
-    int n = nq * nb > nb ? nq * nb : nb;
-    count_launch(); k_reduce_acc<<<(n + 127) / 128, 128, 0, st>>>(nwarps, nq, nb, wacc, wnp, out, outnp);
-    TC_CU(cudaGetLastError());
-    return 0;
-}
-
-
 // ---------------------------------------------------------------------------------------
 // Fixed traversal scratch for callers that cannot allocate device memory.
 //
@@ -1196,8 +1116,7 @@ int noalloc_preload()
 {
     cudaFuncAttributes at;
     TC_CU(cudaFuncGetAttributes(&at, k_traverse));
-    TC_CU(cudaFuncGetAttributes(&at, k_reduce_acc));
-    return 0;
+    return sum_rows_preload();
 }
 
 int noalloc_scratch(void** base)

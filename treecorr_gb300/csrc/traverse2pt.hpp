@@ -97,6 +97,28 @@ struct TravParams {
     long long det_ccap, det_tcap;
 };
 
+// The depth-first walk (walk.cu): units of items, each with a row of sums of its own.
+struct WalkParams {
+    const int2* items;              // the expansion's items; null: generated roots
+    unsigned n_items, n_units;      // unit u takes items u, u + n_units, ..
+    const int* unit_off;            // patches: pair p's units are unit_off[p] .. [p + 1] - 1
+    unsigned long long* next;       // the next unit
+    int2* stacks;                   // per warp
+    int stack_cap;
+    double* rows;                   // [unit][nqf][nbins]
+    unsigned long long* rownp;      // [unit][nbins]
+    // Constants of the rule with both ends of their FP32 margins (walk_constants).
+    float min_lo, min_hi, max_lo, max_hi, a_lo, a_hi, b_lo, b_hi, h_lo, h_hi, c_lo, c_hi;
+    float per_log2, ek0, ek1, t0, half_min;
+};
+void walk_constants(const TravParams& T, WalkParams& W);
+int walk_grid(const TravParams& T, int* blocks, int* nwarps);
+int launch_walk(const TravParams& T, const WalkParams& W, int blocks, cudaStream_t st);
+int launch_sum_rows(const double* rows, const unsigned long long* rownp, long long nrow,
+                    const int* off, int nseg, int nd, int ni, double* out,
+                    unsigned long long* outnp, cudaStream_t st);
+int sum_rows_preload();
+
 // Fixed traversal scratch of the allocation-free entry point (traverse2pt.cu).
 static constexpr int NOALLOC_MAXW = 1024;           // warps launched at most
 static constexpr int NOALLOC_SCAP = 2048;           // work items per warp stack
@@ -128,6 +150,7 @@ struct ExpandSched {
     long long cap;                 // items per level buffer
     long long chunk_max;
     int nlev;                      // levels with a buffer
+    int top;                       // the deepest level that can hold items
     int done, need_levels, out_level;
     const int2* in;                // current launch
     long long n_in, gen0, out_cap;
@@ -136,6 +159,8 @@ struct ExpandSched {
     long long launches;
     unsigned int warps_done;       // warps of the current expand launch that have finished
     int pending;                   // a picked chunk waits for its expand launch
+    long long walk_min;            // > 0: stop (done) once a level holds this many items,
+    int walk_level;                // which the walk then takes (0: none, the expansion ended)
 };
 
 void launch_pack_cells(int ncap, const Cells& C, TCell* out, cudaStream_t st);
@@ -156,7 +181,6 @@ long long det_items_per_warp(long long chunk, int nwarps);
 static constexpr int TILE_LEAF = 48;
 int tiles_grid(const TravParams& T, int* blocks, int* nwarps);
 int launch_tiles(const TravParams& T, cudaStream_t st);
-int launch_reduce(int nwarps, int nq, int nb, const double* wacc, const unsigned long long* wnp,
-                  double* out, unsigned long long* outnp, cudaStream_t st);
+
 
 }  // namespace tc
