@@ -436,10 +436,10 @@ int tc_get_omp_threads(void);
 int tc_set_deterministic(int on);
 int tc_get_deterministic(void);
 
-/* The 2-point expansion's level buffers (about 1 GB each at 10M points) come from the
- * current device's stream-ordered memory pool, which keeps them after a corr is freed so
- * that the next corr reuses them without driver calls.  tc_trim_memory returns the pool's
- * unused memory to the driver (no reference counterpart). */
+/* The library's device memory comes from a stream-ordered pool of its own, which keeps what
+ * freed objects held (at most an eighth of the device's memory beyond the next
+ * synchronisation) so that the next call reuses it without driver calls.  tc_trim_memory
+ * returns the pool's unused memory to the driver (no reference counterpart). */
 int tc_trim_memory(void);
 
 /* Message of the last failure on the calling thread ("" if none). */

@@ -44,6 +44,70 @@ static int stream_get(cudaStream_t* s)
     return 0;
 }
 
+// The library's memory pool on a device.  A call allocates some 80 arrays and frees them with
+// its objects: through cudaMalloc and cudaFree that is 20 us each way (3 ms of a call on 200K
+// points, 14 of 17 ms of a small three-point call), from the pool about 1 us.  The pool keeps
+// what is freed up to an eighth of the device's memory, so that the rest goes back to the
+// driver at the next synchronisation; tc_trim_memory gives back all of it.  Everything is
+// allocated, used and freed in the order of the library's one stream, so threads share it
+// safely.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[64] = {nullptr};
+
+static int pool_get(cudaMemPool_t* pool)
+{
+    int dev = 0;
+    TC_CU(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) { set_last_error("device index out of range"); return TC_ERR_CUDA; }
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        TC_CU(cudaMemPoolCreate(&p, &props));
+        cudaDeviceProp dp;
+        TC_CU(cudaGetDeviceProperties(&dp, dev));
+        unsigned long long keep = dp.totalGlobalMem / 8;
+        TC_CU(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        g_pool[dev] = p;
+    }
+    *pool = g_pool[dev];
+    return 0;
+}
+
+int dev_alloc(void** p, size_t bytes)
+{
+    *p = nullptr;
+    cudaStream_t st;
+    cudaMemPool_t pool;
+    TC_TRY(stream_get(&st));
+    TC_TRY(pool_get(&pool));
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        // What the pool holds may be in too small pieces: hand it back and try once more.
+        cudaGetLastError();
+        cudaStreamSynchronize(st);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+        set_last_error(std::string("device allocation of ") + std::to_string(bytes) +
+                       " bytes failed: " + cudaGetErrorString(e));
+        return TC_ERR_NOMEM;
+    }
+    return 0;
+}
+
+void dev_free(void* p)
+{
+    if (p) cudaFreeAsync(p, g_stream);
+}
+
 static const char* dev_err_msg(int code)
 {
     switch (code) {
@@ -423,11 +487,10 @@ int field_create_impl(int dkind, int coords, const double* x, const double* y, c
 
 double sqr(double x) { return x * x; }
 
-// Device memory of the stream-ordered pool for the length of a call.
+// Device memory for the length of a call.
 struct PoolBuf {
     void* p = nullptr;
-    cudaStream_t st = nullptr;
-    ~PoolBuf() { if (p) cudaFreeAsync(p, st); }
+    ~PoolBuf() { dev_free(p); }
 };
 
 // The rows of sums (per warp of the expansion and the tiles, per unit of the walk) are added
@@ -453,49 +516,6 @@ int expand_scratch(tc_corr2* c, int nwarps, int nq)
     return 0;
 }
 
-// The expansion's level buffers (up to 1 GB each, ~31 of them at 10M points) come from the
-// device's stream-ordered memory pool, which keeps freed memory for the next corr instead of
-// returning it to the driver: a new corr per step then costs no cudaMalloc / cudaFree of
-// tens of GB (freeing them through the driver took 25 ms per 10M-point correlation).
-int pool_alloc_int2(int2** p, size_t count, cudaStream_t st)
-{
-    static bool configured[64] = {false};
-    int dev = 0;
-    TC_CU(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaMemPool_t pool;
-        TC_CU(cudaDeviceGetDefaultMemPool(&pool, dev));
-        unsigned long long thr = ~0ULL;   // keep freed blocks in the pool
-        TC_CU(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
-        configured[dev] = true;
-    }
-    *p = nullptr;
-    const cudaError_t e = cudaMallocAsync((void**)p, std::max<size_t>(count, 1) * sizeof(int2), st);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        *p = nullptr;
-        set_last_error(std::string("cudaMallocAsync of ") + std::to_string(count * sizeof(int2)) +
-                       " bytes failed: " + cudaGetErrorString(e));
-        return TC_ERR_NOMEM;
-    }
-    return 0;
-}
-
-int pool_alloc(PoolBuf& b, size_t bytes, cudaStream_t st)
-{
-    int2* p = nullptr;
-    TC_TRY(pool_alloc_int2(&p, (bytes + sizeof(int2) - 1) / sizeof(int2), st));
-    b.p = p;
-    b.st = st;
-    return 0;
-}
-
-void pool_free(int2*& p, cudaStream_t st)
-{
-    if (p) cudaFreeAsync(p, st);
-    p = nullptr;
-}
-
 // Makes level L's item buffer hold at least `need` items, keeping its first `keep` items.
 int level_reserve(tc_corr2* c, int L, long long keep, long long need, cudaStream_t st)
 {
@@ -503,11 +523,10 @@ int level_reserve(tc_corr2* c, int L, long long keep, long long need, cudaStream
     if (c->levcap[L] >= need) return 0;
     long long cap = std::max(need, 2 * c->levcap[L]);
     int2* p = nullptr;
-    TC_TRY(pool_alloc_int2(&p, (size_t)cap, st));
+    TC_TRY(dalloc(&p, (size_t)cap));
     if (keep > 0)
         TC_CU(cudaMemcpyAsync(p, c->lev[L], sizeof(int2) * (size_t)keep, cudaMemcpyDeviceToDevice, st));
-    TC_CU(cudaStreamSynchronize(st));
-    pool_free(c->lev[L], st);
+    dfree(c->lev[L]);
     c->lev[L] = p;
     c->levcap[L] = cap;
     return 0;
@@ -766,11 +785,11 @@ int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cud
         TC_CU(cudaMemsetAsync(c->wnp, 0, sizeof(unsigned long long) * (size_t)nwarps * nb, st));
         if (!c->sched) TC_TRY(dalloc(&c->sched, 1));
         const long long cap = 4 * want;
-        for (auto& b : lev) TC_TRY(pool_alloc(b, sizeof(int2) * (size_t)cap, st));
+        for (auto& b : lev) TC_TRY(dev_alloc(&b.p, sizeof(int2) * (size_t)cap));
         if (g_deterministic.load()) {
             const long long ipw = det_items_per_warp(want, nwarps);
-            TC_TRY(pool_alloc(dout, sizeof(int2) * (size_t)(4 * ipw * nwarps), st));
-            TC_TRY(pool_alloc(dcnt, sizeof(int) * 2 * (size_t)nwarps, st));
+            TC_TRY(dev_alloc(&dout.p, sizeof(int2) * (size_t)(4 * ipw * nwarps)));
+            TC_TRY(dev_alloc(&dcnt.p, sizeof(int) * 2 * (size_t)nwarps));
             // (k_compact reads the tile counts too)
             TC_CU(cudaMemsetAsync(dcnt.p, 0, sizeof(int) * 2 * (size_t)nwarps, st));
             T.det = 1; T.det_nw = nwarps;
@@ -805,7 +824,7 @@ int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cud
     if (!derr && n_items > 0) {
         const long long n_units = std::min(max_units, (n_items + 31) / 32);
         const int cap = walk_stack_cap(npoints);
-        TC_TRY(pool_alloc(stacks, sizeof(int2) * (size_t)cap * wwarps, st));
+        TC_TRY(dev_alloc(&stacks.p, sizeof(int2) * (size_t)cap * wwarps));
         W.n_items = (unsigned)n_items; W.n_units = (unsigned)n_units;
         W.next = c->ctl;
         W.stacks = static_cast<int2*>(stacks.p);
@@ -884,8 +903,8 @@ int walk_patches(tc_corr2* c, TravParams T, const std::vector<long long>& roff,
     walk_constants(T, W);
     PoolBuf stacks, off;
     const int cap = walk_stack_cap(npoints);
-    TC_TRY(pool_alloc(stacks, sizeof(int2) * (size_t)cap * wwarps, st));
-    TC_TRY(pool_alloc(off, sizeof(int) * uoff.size(), st));
+    TC_TRY(dev_alloc(&stacks.p, sizeof(int2) * (size_t)cap * wwarps));
+    TC_TRY(dev_alloc(&off.p, sizeof(int) * uoff.size()));
     TC_CU(cudaMemcpyAsync(off.p, uoff.data(), sizeof(int) * uoff.size(), cudaMemcpyHostToDevice, st));
     TC_CU(cudaMemsetAsync(c->ctl, 0, 8 * sizeof(unsigned long long), st));
     TC_CU(cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
@@ -1789,7 +1808,7 @@ void tc_corr2_free(tc_corr2* c)
     {
         cudaStream_t st = nullptr;
         if (stream_get(&st) == 0)
-            for (auto& p : c->lev) pool_free(p, st);
+            for (auto& p : c->lev) dfree(p);
     }
     dfree(c->sched);
     dfree(c->mlp); dfree(c->samples);
@@ -2593,13 +2612,11 @@ int tc_get_omp_threads(void) { return 1; }
 
 int tc_trim_memory(void)
 {
-    int dev = 0;
-    TC_CU(cudaGetDevice(&dev));
     cudaStream_t st;
     TC_TRY(stream_get(&st));
     TC_CU(cudaStreamSynchronize(st));
     cudaMemPool_t pool;
-    TC_CU(cudaDeviceGetDefaultMemPool(&pool, dev));
+    TC_TRY(pool_get(&pool));
     TC_CU(cudaMemPoolTrimTo(pool, 0));
     return TC_OK;
 }

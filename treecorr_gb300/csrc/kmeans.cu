@@ -883,7 +883,7 @@ struct KMScratch {
     }
 };
 
-int scratch_alloc(const KMField& F, int npatch, KMScratch& S)
+int scratch_alloc(const KMField& F, int npatch, KMScratch& S, cudaStream_t st)
 {
     TC_TRY(dalloc(&S.cen, 3 * (size_t)npatch));
     TC_TRY(dalloc(&S.inertia, npatch));
@@ -895,7 +895,7 @@ int scratch_alloc(const KMField& F, int npatch, KMScratch& S)
     S.pool_cap = std::max<long long>(1 << 22, 4LL * npatch + 2LL * F.ntop);
     TC_TRY(dalloc(&S.pool, S.pool_cap));
     TC_TRY(dalloc(&S.assign, F.ncap));
-    TC_CU(cudaMemset(S.assign, 0xff, sizeof(int) * (size_t)F.ncap));
+    TC_CU(cudaMemsetAsync(S.assign, 0xff, sizeof(int) * (size_t)F.ncap, st));
     TC_TRY(dalloc(&S.lvl, 1));
     // Accumulator warps per block: as many as fit (at most 8), each npatch x KM_NQ doubles
     // plus a 32-lane staging row.
@@ -1121,7 +1121,7 @@ int kmeans_run(const KMField& F, double* centers, int npatch, int max_iter, doub
     // KMeansRun1 (src/KMeans.cpp:773-833).
     TC_TRY(check_npatch(F, npatch));
     KMScratch S;
-    TC_TRY(scratch_alloc(F, npatch, S));
+    TC_TRY(scratch_alloc(F, npatch, S, st));
     TC_TRY(upload_centers(centers, npatch, F.coords, S, st));
     const double tolsq = (tol * F.size) * (tol * F.size) * npatch;
     int it = 0;
@@ -1156,7 +1156,7 @@ int kmeans_assign(const KMField& F, const double* centers, int npatch, int64_t* 
     // KMeansAssign1 (src/KMeans.cpp:835-849).
     TC_TRY(check_npatch(F, npatch));
     KMScratch S;
-    TC_TRY(scratch_alloc(F, npatch, S));
+    TC_TRY(scratch_alloc(F, npatch, S, st));
     TC_TRY(upload_centers(centers, npatch, F.coords, S, st));
     TC_TRY(find_cells(F, npatch, nullptr, S, st));
     int64_t* d_out = nullptr;

@@ -32,27 +32,23 @@ void count_launch();
         if (s_ != 0) return s_;                                                            \
     } while (0)
 
-// Device allocation that records a message and returns TC_ERR_NOMEM (5) on failure.
+// Device memory from the library's stream-ordered pool on the current device, usable in the
+// order of the library's stream (capi.cu); freed memory stays in the pool for the next call.
+// Records a message and returns TC_ERR_NOMEM (5) on failure.
+int dev_alloc(void** p, size_t bytes);
+void dev_free(void* p);
+
 template <class T>
 int dalloc(T** p, size_t count)
 {
     *p = nullptr;
-    if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        *p = nullptr;
-        set_last_error(std::string("cudaMalloc of ") + std::to_string(count * sizeof(T)) +
-                       " bytes failed: " + cudaGetErrorString(e));
-        return 5;
-    }
-    return 0;
+    return dev_alloc((void**)p, (count == 0 ? 1 : count) * sizeof(T));
 }
 
 template <class T>
 void dfree(T*& p)
 {
-    if (p) cudaFree(p);
+    if (p) dev_free((void*)p);
     p = nullptr;
 }
 
