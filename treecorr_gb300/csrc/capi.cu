@@ -641,19 +641,22 @@ int expand_run(tc_corr2* c, const TravParams& T, int blocks, long long npoints, 
     int derr = 0;
     long long launches = 0;
     // Device time of the expansion and tile kernels, from events around every launch.
+    // Launches per host check: fewer with tiles, where each iteration has six and a traversal
+    // takes a few tens of iterations.
     constexpr int BATCH = 64;
+    const int iters = T.tile_leaf > 0 ? 16 : BATCH;
     if (c->kev.empty()) {
         c->kev.resize(3 * BATCH);
         for (auto& e : c->kev) TC_CU(cudaEventCreate(&e));
     }
     double expand_ms = 0., tiles_ms = 0.;
     for (int batch = 0;; ++batch) {
-        TC_TRY(launch_expand_batch(T, blocks, c->sched, BATCH, st, c->kev.data()));
+        TC_TRY(launch_expand_batch(T, blocks, c->sched, iters, st, c->kev.data()));
         int flags[3];
         TC_CU(cudaMemcpyAsync(flags, &c->sched->done, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaMemcpyAsync(&derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaStreamSynchronize(st));
-        for (int it = 0; it < BATCH; ++it) {
+        for (int it = 0; it < iters; ++it) {
             float a = 0.f, b = 0.f;
             TC_CU(cudaEventElapsedTime(&a, c->kev[3 * it], c->kev[3 * it + 1]));
             TC_CU(cudaEventElapsedTime(&b, c->kev[3 * it + 1], c->kev[3 * it + 2]));
@@ -1004,17 +1007,30 @@ int corr_process(tc_corr2* c, tc_field* f1, tc_field* f2, int quick, int metric)
     }
     TC_TRY(expand_grid(nq, nb, &blocks, &nwarps, mode));
     int tblocks = 0, twarps = 0;
+    PoolBuf tkeys, terr;
     if (tiles) {
-        T.tile_leaf = c->tile_leaf > 0 ? c->tile_leaf : TILE_LEAF;   // (tiles_grid picks the
-                                                                     // kernel from T's classes)
+        T.brute = f1->brute || g->brute;
+        const bool packed = packed_tiles(T);
+        T.tile_leaf = c->tile_leaf > 0 ? c->tile_leaf : packed ? PACKED_LEAF : TILE_LEAF;
         TC_TRY(tiles_grid(T, &tblocks, &twarps));
-        const long long cap = c->chunk > 0 ? c->chunk : expand_chunk(f1->n + (f2 ? f2->n : 0));
+        // The packed tile kernels work the list off in few large launches: it holds several
+        // chunks' tiles, and is drained when another chunk's would not fit.
+        const long long CH = c->chunk > 0 ? c->chunk : expand_chunk(f1->n + (f2 ? f2->n : 0));
+        const long long cap = packed ? CH + std::max(CH, 1LL << 22) : CH;
         if (c->tile_cap < cap) {
             dfree(c->tiles);
-            c->tiles = nullptr;
             c->tile_cap = 0;
             TC_TRY(dalloc(&c->tiles, (size_t)cap));
             c->tile_cap = cap;
+        }
+        if (packed) {
+            TC_TRY(dev_alloc(&tkeys.p, sizeof(unsigned) * (size_t)c->tile_cap));
+            TC_TRY(dev_alloc(&terr.p, sizeof(float2) * (size_t)c->tile_cap));
+            if (!c->sched) TC_TRY(dalloc(&c->sched, 1));
+            T.tile_keys = static_cast<unsigned*>(tkeys.p);
+            T.tile_err = static_cast<float2*>(terr.p);
+            T.sched = c->sched;
+            T.tile_drain = c->tile_cap - CH;
         }
         if (!c->tctl) TC_TRY(dalloc(&c->tctl, 8));
         if (!c->tedge) TC_TRY(dalloc(&c->tedge, 2 * (size_t)(nb + 1)));
@@ -1027,7 +1043,6 @@ int corr_process(tc_corr2* c, tc_field* f1, tc_field* f2, int quick, int metric)
         TC_CU(cudaMemcpyAsync(c->tedge, te.data(), te.size() * sizeof(float),
                               cudaMemcpyHostToDevice, st));
         TC_CU(cudaMemsetAsync(c->tctl, 0, 8 * sizeof(unsigned long long), st));
-        T.tile_leaf = c->tile_leaf > 0 ? c->tile_leaf : TILE_LEAF;
         T.leaf_base1 = (int)(f1->n - 1);
         T.leaf_base2 = (int)(g->n - 1);
         T.tiles = c->tiles;

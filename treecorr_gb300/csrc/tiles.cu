@@ -47,6 +47,7 @@
 #include "tc_host.hpp"
 #include "traverse2pt.hpp"
 #include "pair_math.cuh"
+#include "tile_common.cuh"
 
 namespace tc {
 
@@ -65,9 +66,6 @@ constexpr int TMINB = TILES_MINB; // resident blocks per SM the registers are si
 constexpr int TCAP = TILE_CAP;    // most leaves per tile side (>= the traversal's tile_leaf)
 static_assert(TCAP * 4 >= 32 * 8, "a tile side's X array doubles as the 32 x 8 staging area");
 
-enum { TG_FLAT = 0, TG_ARC = 1, TG_SPHEUC = 2, TG_3D = 3 };   // geometry
-enum { TK_NN = 0, TK_SC = 1, TK_GEN = 2, TK_GG = 3 };           // class family
-
 // One side of a tile: its valid leaves (n > 0, w != 0) in point order.  Pair loops read P and
 // W of both sides (two 16-byte shared loads per side) and X only where it is needed.
 struct TileLeaves {
@@ -76,16 +74,6 @@ struct TileLeaves {
                       // complex kinds), point count
     float4 X[TCAP];   // (x, y, id bits, 0): FP32 position (sphere projections), leaf cell id
 };
-
-__host__ __device__ inline size_t bins_bytes(int nq, int nb)
-{
-    return ((size_t)nq * nb * 8 + (size_t)nb * 8 + (size_t)nq * nb * 4 + 15) & ~(size_t)15;
-}
-
-__host__ __device__ inline size_t edges_bytes(int nb)
-{
-    return ((size_t)2 * (nb + 1) * 4 + 15) & ~(size_t)15;
-}
 
 __host__ __device__ inline size_t warp_bytes(int nq, int nb)
 {
@@ -138,75 +126,6 @@ __device__ __forceinline__ int stage(const TCell* cells, int base, float4 cc, fl
     }
     single = all1;
     return cnt;
-}
-
-__device__ __forceinline__ float warp_max(float v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// Sums v[0..7] over the warp: after the reduce-scatter each group of 4 lanes holds one value's
-// total; lane 4 q + 0 returns value q's total in *out (q = 0..7) and true.
-__device__ __forceinline__ bool warp_sum8(float (&v)[8], int lane, float& out)
-{
-    // xor 16: keep 4 of 8.
-    const bool h16 = lane & 16;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const float send = h16 ? v[q] : v[q + 4];
-        const float got = __shfl_xor_sync(0xffffffffu, send, 16);
-        v[q] = (h16 ? v[q + 4] : v[q]) + got;
-    }
-    // xor 8: keep 2 of 4.
-    const bool h8 = lane & 8;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const float send = h8 ? v[q] : v[q + 2];
-        const float got = __shfl_xor_sync(0xffffffffu, send, 8);
-        v[q] = (h8 ? v[q + 2] : v[q]) + got;
-    }
-    // xor 4: keep 1 of 2.
-    const bool h4 = lane & 4;
-    {
-        const float send = h4 ? v[0] : v[1];
-        const float got = __shfl_xor_sync(0xffffffffu, send, 4);
-        v[0] = (h4 ? v[1] : v[0]) + got;
-    }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    out = v[0];
-    return (lane & 3) == 0;
-}
-
-// Which value a lane holds after warp_sum8: bit 4 picks the upper half, bit 3 the upper
-// quarter of that, bit 2 the upper one of the last two.
-__device__ __forceinline__ int warp_sum8_index(int lane)
-{
-    return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-}
-
-// A leaf pair decided in FP64 with the reference's formulas: decide64 (the reference's
-// process11 for s1 = s2 = 0) on the FP64 leaf positions.  Out of line: it runs for about one
-// pair in 10^5, and keeping it out of the loop keeps the loop's registers low.
-__device__ __noinline__ int leaf_pair64(const TravParams& T, int ida, int idb, bool self,
-                                        float* r, float* logr)
-{
-    const double* x2 = self ? T.x1 : T.x2;
-    const double* y2 = self ? T.y1 : T.y2;
-    const double* z2 = self ? T.z1 : T.z2;
-    const double dx = T.x1[ida] - x2[idb], dy = T.y1[ida] - y2[idb];
-    double dsq = dx * dx + dy * dy;
-    if (T.coords != FLAT) {
-        const double dz = T.z1[ida] - z2[idb];
-        dsq += dz * dz;
-    }
-    const Decision D = decide64(T, dsq, 0., 0.);
-    if (D.act != ACT_ACCEPT) return -1;
-    *r = D.r;
-    *logr = D.logr;
-    return D.k;
 }
 
 // The generic values of an accepted leaf pair (every class, with the projections of
@@ -282,38 +201,6 @@ __device__ __forceinline__ void pair_products(const TravParams& T, const TileLea
     }
 }
 
-// The great-circle angle from a chord c < 0.25 (the tile checks it): the Maclaurin series
-// of 2 asin(c / 2) to x^7, x = c / 2 (the first omitted term is below 2e-9 of x).
-__device__ __forceinline__ float arc_series(float c)
-{
-    const float x = 0.5f * c, x2 = x * x;
-    return 2.f * x * fmaf(x2, fmaf(x2, fmaf(x2, 5.f / 112.f, 3.f / 40.f), 1.f / 6.f), 1.f);
-}
-
-// Adds a tile's per-lane sums of one bin into the warp's FP32 bins.  acc: weight, sum w w r,
-// sum w w lr (lr = log2(r^2 / edge^2) of the tile's reference edge), products; the bin's
-// meanlogr sum is (ln 2 / 2) sum w w lr + log(edge) sum w w.
-__device__ __forceinline__ void tile_bin_out(float (&acc)[8], unsigned cn, int kb, int nq, int nb,
-                                             float ledge, float* fb, unsigned long long* np,
-                                             bool quick, bool single, int lane)
-{
-    if (!__any_sync(0xffffffffu, cn != 0u) || kb >= nb) return;
-    acc[2] = fmaf(acc[2], 0.5f * 0.69314718f, acc[0] * ledge);
-    float tot;
-    const bool holder = warp_sum8(acc, lane, tot);
-    const int q = warp_sum8_index(lane);
-    if (holder && q < nq) fb[q * nb + kb] += tot;
-    if (!quick) {
-        if (single) {
-            const unsigned ct = __reduce_add_sync(0xffffffffu, cn);
-            if (lane == 0) np[kb] += ct;
-        } else if (cn) {
-            atomicAdd(&np[kb], (unsigned long long)cn);
-        }
-    }
-    __syncwarp();
-}
-
 // Everything a tile's pair loop needs besides its leaves.
 struct TileCtx {
     int na, nbl, kref;
@@ -355,27 +242,6 @@ __device__ __forceinline__ void tile_fast(const TravParams& T, const TileLeaves&
             for (int q = 0; q < NX; ++q) acc[3 + q] = fmaf(x[q], sc, acc[3 + q]);
         }
         cnt += (unsigned)__float_as_int(Wa.w) * (unsigned)__float_as_int(Wb.w);
-    }
-}
-
-// Adds the pairs that lanes hold for the shared bins (kx >= 0, values v) in ascending lane
-// order: lane q < nq adds quantity q of each, so the sums do not depend on the order in which
-// conflicting shared atomics would land.
-__device__ __forceinline__ void shared_bins_in_order(int kx, const float (&v)[8], float* fb,
-                                                     int nq, int nb, int lane)
-{
-    unsigned m = __ballot_sync(0xffffffffu, kx >= 0);
-    while (m) {
-        const int t = __ffs(m) - 1;
-        m &= m - 1u;
-        const int kt = __shfl_sync(0xffffffffu, kx, t);
-        float x = 0.f;
-#pragma unroll
-        for (int q = 0; q < 7; ++q) {
-            const float y = __shfl_sync(0xffffffffu, v[q], t);
-            x = lane == q ? y : x;
-        }
-        if (lane < nq) fb[lane * nb + kt] += x;
     }
 }
 
@@ -809,8 +675,6 @@ __global__ void __launch_bounds__(TPB, TMINB) k_tiles(const __grid_constant__ Tr
     }
 }
 
-using TileKernel = void (*)(TravParams);
-
 template <int GEO>
 TileKernel pick_kind(const TravParams& T)
 {
@@ -835,6 +699,7 @@ int tiles_grid(const TravParams& T, int* blocks, int* nwarps)
         set_last_error("tile leaf size above the tile kernel's staging capacity");
         return 1;
     }
+    if (packed_tiles(T)) return packed_grid(T, blocks, nwarps);
     int dev = 0, nsm = 0, per = 0;
     TC_CU(cudaGetDevice(&dev));
     TC_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -851,6 +716,7 @@ int tiles_grid(const TravParams& T, int* blocks, int* nwarps)
 
 int launch_tiles(const TravParams& T, cudaStream_t st)
 {
+    if (packed_tiles(T)) return launch_packed_tiles(T, st);
     const size_t sm = edges_bytes(T.nbins) + warp_bytes(T.nqf, T.nbins) * TWPB;
     count_launch();
     pick(T)<<<T.tile_blocks, TPB, sm, st>>>(T);

@@ -917,6 +917,8 @@ __global__ void __launch_bounds__(CPB * 32) k_compact(const __grid_constant__ Tr
     const int* cc = T.det_cnt;
     const int* ct = T.det_cnt + nw;
     const int r0 = blockIdx.x * CPB;
+    // Tiles that still wait from earlier launches stay in front (packed tiles).
+    const long long t0 = T.tile_leaf > 0 ? (long long)*(volatile unsigned long long*)&T.tctl[0] : 0;
     // Counts of the regions before this block's, four at a time (nw and r0 are multiples of
     // 4, so both count arrays are 16-byte aligned).
     long long pc = 0, pt = 0;
@@ -931,7 +933,7 @@ __global__ void __launch_bounds__(CPB * 32) k_compact(const __grid_constant__ Tr
     pt = warp_sum_ll(pt);
     if (lane == 0) { red[0][w] = pc; red[1][w] = pt; }
     __syncthreads();
-    long long oc = 0, ot = 0;
+    long long oc = 0, ot = t0;
     for (int q = 0; q < CPB; ++q) { oc += red[0][q]; ot += red[1][q]; }
     const int r = r0 + w;
     if (r < nw) {
@@ -967,7 +969,7 @@ __global__ void __launch_bounds__(CPB * 32) k_compact(const __grid_constant__ Tr
     if (lane == 0) { red[0][w] = tc; red[1][w] = tt; }
     __syncthreads();
     if (tid == 0) {
-        tc = 0; tt = 0;
+        tc = 0; tt = t0;
         for (int q = 0; q < CPB; ++q) { tc += red[0][q]; tt += red[1][q]; }
         S->warps_done = 0;
         S->nout = (unsigned long long)(tc < S->out_cap ? tc : S->out_cap);

@@ -76,6 +76,7 @@ struct TravParams {
     // self tile (c, -2 - c); k_tiles evaluates every leaf pair of a tile.  The leaf starting
     // at point p of field 1 (2) has cell id leaf_base1 (leaf_base2) + p.
     int tile_leaf;                  // 0: no tiles
+    int brute;                      // a field is brute: its cells' sizes are infinite
     int leaf_base1, leaf_base2;
     int2* tiles;
     unsigned long long* tctl;       // [0] tiles waiting, [1] blocks of k_tiles done,
@@ -84,6 +85,12 @@ struct TravParams {
     int tile_blocks, tile_wbase;    // k_tiles grid; its warps' slots start at tile_wbase
     const float* tile_edge;         // [nbins+1]: 1 / (min_sep^2 exp(2 k bin_size))
     const float* tile_ledge;        // [nbins+1]: log(min_sep) + k bin_size
+    // Packed tiles (tile_packed.cu): the list is worked off once it holds more than tile_drain
+    // tiles or the schedule is done; k_tile_class writes a key and the error bounds per tile.
+    const struct ExpandSched* sched;
+    long long tile_drain;
+    unsigned* tile_keys;
+    float2* tile_err;
     // Fixed-order expansion (det != 0; modes 0 and 2): every warp of an expansion launch
     // writes its children and tiles into regions of its own (det_out + gw det_ccap,
     // det_tout + gw det_tcap) and their counts into det_cnt[gw] and det_cnt[det_nw + gw];
@@ -179,6 +186,13 @@ long long det_items_per_warp(long long chunk, int nwarps);
 // Leaf-pair tiles (tiles.cu): the leaf size of a tile side, the k_tiles grid for a traversal
 // (its blocks fill every SM), and one k_tiles launch over the tiles waiting in T.tiles.
 static constexpr int TILE_LEAF = 48;
+// The packed kernels take twice that area in their stride (10^6 points GG 150 ms at 64, 154 at 48;
+// NN 96 and 104; 200,000 points KK 5.8 and 6.9).
+static constexpr int PACKED_LEAF = 64;
+using TileKernel = void (*)(TravParams);
+bool packed_tiles(const TravParams& T);           // tile_packed.cu takes T's classes
+int packed_grid(const TravParams& T, int* blocks, int* nwarps);
+int launch_packed_tiles(const TravParams& T, cudaStream_t st);
 int tiles_grid(const TravParams& T, int* blocks, int* nwarps);
 int launch_tiles(const TravParams& T, cudaStream_t st);
 
