@@ -9,7 +9,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT, "libtcgpu.so")
-SOURCES = ["tree_build.cu", "traverse2pt.cu", "walk.cu", "tiles.cu", "tile_packed.cu", "multipole.cu", "learned.cu",
+SOURCES = ["tree_build.cu", "traverse2pt.cu", "walk.cu", "tiles.cu", "tile_packed.cu", "multipole.cu", "zeta.cu", "learned.cu",
            "tensorcore.cu", "kmeans.cu", "catalog.cu", "capi.cu"]
 NVCC = os.environ.get("NVCC", "nvcc")
 FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a", "-lineinfo", "-O3", "-std=c++17",

@@ -22,8 +22,8 @@
 //     the scratch is copied into a free slot and the right child is pushed, as the
 //     reference's mp.duplicate() does.
 //   * Rows of Zeta that are final become vertex records (FP32 copies of G_n and W_n).  The
-//     contraction over vertices is a sum of outer products per n; k_mp_zeta runs it in
-//     batches (waves) between runs of the finish kernel, FP32 products with FP64 sums.
+//     contraction over vertices is a sum of outer products per n; k_mp_zeta (zeta.cu) runs it
+//     in batches (waves) between runs of the finish kernel, FP32 products with FP64 sums.
 //   * A last kernel sums the per-block outputs, the contraction partials and the diagonal
 //     self-pair corrections in a fixed order.
 //   * A three-field cross keeps vertex 3's pairs in scratch bins [nbd, 2 nbd), so the same
@@ -41,7 +41,6 @@
 #include "tc_internal.cuh"
 #include "tc_host.hpp"
 #include "multipole.hpp"
-#include "tc_mma.cuh"
 
 namespace tc {
 
@@ -1362,349 +1361,8 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
 }
 
 // ---------------------------------------------------------------------------------------
-// Batched Zeta contraction over vertex records.  For one n and a group of records the
-// block computes, for every entry (a, b) of the nbins x nbins tile,
-//   gam0 += (wg1 G_a[n-1]) G_b[-n-1]        gam1 += (conj(wg1) G_a[n+1]) G_b[-n+1]
-//   gam2 += (wg1 G_a[n-1]) conj(G_b[n+1])   gam3 += (wg1 conj(G_a[-n+1])) G_b[-n-1]
-//   weight += (w1 W_a[n]) conj(W_b[n])
-// over the records whose row range [ks, mk) holds min(a, b) -- a sum of outer products over
-// vertices.  Operands are staged in shared memory per chunk of records; products and chunk
-// sums are FP32, the running sums FP64; each group adds its sums to its own partial array.
-// These are GGG's sums (MultipoleHelper<5>).  With shift 0 the G indices are n and -n and
-// wg1 is the real w1 or w1 k1 of an N or K vertex, which makes gam0 and gam2 NGG's / KGG's
-// zeta0 and zeta1 (MultipoleHelper<2>, src/Corr3.cpp:2216-2405).
-
-struct ZParams {
-    const float* rec;
-    long long nrec;
-    int rec_floats, nbins, maxn, chunk, ngroups;
-    int shift;             // 1: G_n at n -+ 1 (a spin-2 vertex); 0: at n (an N or K vertex)
-    int nbd;               // distance bins; a record's rows [ks, mk) hold min(a, b) mod nbd
-    int typo32;            // see MPParams::typo32
-    double* part;          // [group][10][Z]
-    long long Z;
-};
-
-static constexpr int ZB = 256;   // threads per contraction block
+static constexpr int ZB = 256;   // threads per block of the scalar sums
 static constexpr int ZE = 2;     // entries per thread
-
-__global__ void __launch_bounds__(ZB) k_mp_zeta(ZParams Q)
-{
-    extern __shared__ float4 zsh[];    // [chunk][nb][4]: (A0, A1), (A3, AW), (B0, B1), (B2, BW)
-    __shared__ int2 rows_sh[64];
-    const int nb = Q.nbins, M = Q.maxn, nn = 2 * M + 1, gst = 2 * M + 3;
-    const int n = (int)blockIdx.x - M;
-    const int g = blockIdx.y;
-    const int tid = threadIdx.x;
-    int ea[ZE], eb[ZE], em[ZE];     // entry (a, b) and min(a, b) mod nbd (the row mask)
-    bool ev[ZE];
-#pragma unroll
-    for (int j = 0; j < ZE; ++j) {
-        const int e = ((int)blockIdx.z * ZE + j) * ZB + tid;
-        ev[j] = e < nb * nb;
-        ea[j] = ev[j] ? e / nb : 0;
-        eb[j] = ev[j] ? e % nb : 0;
-        em[j] = min(ea[j] % Q.nbd, eb[j] % Q.nbd);
-    }
-    // Sums: FP32 per chunk (F), FP32 over up to 16 chunks (F2), then FP64 (D) -- FP64 work is
-    // kept rare (GB300 runs FP64 at 1/64 of the FP32 rate).
-    double D[ZE][10];
-    float F2[ZE][10];
-#pragma unroll
-    for (int j = 0; j < ZE; ++j)
-#pragma unroll
-        for (int q = 0; q < 10; ++q) { D[j][q] = 0.; F2[j][q] = 0.f; }
-    int nchunk = 0;
-    const long long r0 = Q.nrec * g / Q.ngroups, r1 = Q.nrec * (g + 1) / Q.ngroups;
-    const int nw = (n >= 0) ? n : -n;
-    for (long long c0 = r0; c0 < r1; c0 += Q.chunk) {
-        const int nv = (int)min((long long)Q.chunk, r1 - c0);
-        __syncthreads();
-        for (int idx = tid; idx < nv * nb; idx += ZB) {
-            const int v = idx / nb, a = idx % nb;
-            const float* R = Q.rec + (size_t)(c0 + v) * Q.rec_floats;
-            const float2* RG = reinterpret_cast<const float2*>(R + 8);
-            const float2* RW = RG + (size_t)gst * nb;
-            const float w1 = R[3], wr = R[4], wi = R[5];
-            const int sh = Q.shift;
-            const float2 gm1 = RG[(n - sh + M + 1) * nb + a];     // G[n-1]
-            const float2 gmm1 = RG[(-n - sh + M + 1) * nb + a];   // G[-n-1]
-            const float2 gp1 = RG[(n + sh + M + 1) * nb + a];     // G[n+1]
-            const float2 gmp1 = RG[(-n + sh + M + 1) * nb + a];   // G[-n+1]
-            float2 w = RW[nw * nb + a];
-            if (n < 0) w.y = -w.y;
-            float4 o0, o1, o2, o3;
-            o0.x = wr * gm1.x - wi * gm1.y;  o0.y = wr * gm1.y + wi * gm1.x;     // A0
-            o0.z = wr * gp1.x + wi * gp1.y;  o0.w = wr * gp1.y - wi * gp1.x;     // A1
-            o1.x = wr * gmp1.x + wi * gmp1.y; o1.y = wi * gmp1.x - wr * gmp1.y;  // A3
-            o1.z = w1 * w.x;                 o1.w = w1 * w.y;                    // AW
-            o2 = make_float4(gmm1.x, gmm1.y, gmp1.x, gmp1.y);                   // B0, B1
-            o3 = make_float4(gp1.x, -gp1.y, w.x, -w.y);                         // B2, BW
-            float4* d = zsh + ((size_t)v * nb + a) * 4;
-            d[0] = o0; d[1] = o1; d[2] = o2; d[3] = o3;
-            if (a == 0) rows_sh[v] = make_int2(__float_as_int(R[1]), __float_as_int(R[2]));
-        }
-        __syncthreads();
-        float F[ZE][10];
-#pragma unroll
-        for (int j = 0; j < ZE; ++j)
-#pragma unroll
-            for (int q = 0; q < 10; ++q) F[j][q] = 0.f;
-        for (int v = 0; v < nv; ++v) {
-            const int2 rw = rows_sh[v];
-#pragma unroll
-            for (int j = 0; j < ZE; ++j) {
-                const int m = em[j];
-                if (!ev[j] || m < rw.x || m >= rw.y) continue;
-                const float4* pa = zsh + ((size_t)v * nb + ea[j]) * 4;
-                const float4* pb = zsh + ((size_t)v * nb + eb[j]) * 4;
-                const float4 a01 = pa[0], a3w = pa[1], b01 = pb[2], b2w = pb[3];
-                F[j][0] += a01.x * b01.x - a01.y * b01.y;  F[j][1] += a01.x * b01.y + a01.y * b01.x;
-                F[j][2] += a01.z * b01.z - a01.w * b01.w;  F[j][3] += a01.z * b01.w + a01.w * b01.z;
-                F[j][4] += a01.x * b2w.x - a01.y * b2w.y;  F[j][5] += a01.x * b2w.y + a01.y * b2w.x;
-                F[j][6] += a3w.x * b01.x - a3w.y * b01.y;  F[j][7] += a3w.x * b01.y + a3w.y * b01.x;
-                F[j][8] += a3w.z * b2w.z - a3w.w * b2w.w;  F[j][9] += a3w.z * b2w.w + a3w.w * b2w.z;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < ZE; ++j)
-#pragma unroll
-            for (int q = 0; q < 10; ++q) F2[j][q] += F[j][q];
-        if (++nchunk == 16) {
-            nchunk = 0;
-#pragma unroll
-            for (int j = 0; j < ZE; ++j)
-#pragma unroll
-                for (int q = 0; q < 10; ++q) { D[j][q] += (double)F2[j][q]; F2[j][q] = 0.f; }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < ZE; ++j)
-#pragma unroll
-        for (int q = 0; q < 10; ++q) D[j][q] += (double)F2[j][q];
-#pragma unroll
-    for (int j = 0; j < ZE; ++j) {
-        if (!ev[j]) continue;
-        const size_t i = (size_t)(ea[j] * nb + eb[j]) * nn + M + n;
-        double* p = Q.part + (size_t)g * 10 * Q.Z + i;
-        if (ea[j] == eb[j]) D[j][9] = 0.;   // W_a conj(W_a) is real
-#pragma unroll
-        for (int q = 0; q < 10; ++q) p[(size_t)q * Q.Z] += D[j][q];
-    }
-}
-
-// Tensor-core contraction (tcgen05, nbins <= 32).  Same sums as k_mp_zeta, as two real
-// GEMMs per n over the vertex records (the K dimension):
-//   region 0: rows [Re A0, Im A0, Re A3, Im A3] x cols [Re B0, Im B0, Re B2, Im B2]
-//   region 1: rows [Re A1, Im A1, Re AW, Im AW] x cols [Re B1, Im B1, Re BW, Im BW]
-// (each 4 nbins long, rows padded to M = 128, cols to NC = a multiple of 16), whose blocks
-// combine into the complex gam0, gam3, gam2 (region 0) and gam1, weight (region 1).  The
-// row-range mask min(a, b) in [ks, mk) is {a, b >= ks} minus {a, b >= mk}: every record
-// enters as two K entries, the second with negated A and both masked at mk.  Operands are
-// split into TF32 hi + lo parts and multiplied as hi*hi + hi*lo + lo*hi (FP32-level
-// products); the FP32 accumulators in TMEM are drained to FP64 every TC_DRAIN chunks.
-static constexpr int TCB = 128;        // threads (4 warps = the 128 TMEM lanes)
-static constexpr int TC_REC = 16;      // records per chunk = 32 K entries = 4 K steps
-// Chunks between FP64 drains: the TMEM accumulators add 3 MMAs x 4 K steps x 2 entries per
-// record in FP32, and that error grows with the records per drain (at 20 bins / max_n 30,
-// 1024 records per drain gave 1.6e-5 of max|gam|; 128 records keep it near 2e-6).
-static constexpr int TC_DRAIN = 8;
-
-__device__ __forceinline__ void tf32_split(float x, float& hi, float& lo)
-{
-    hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-    lo = x - hi;
-}
-
-__global__ void __launch_bounds__(TCB) k_mp_zeta_tc(ZParams Q, int* status)
-{
-    extern __shared__ __align__(1024) unsigned char zts[];
-    __shared__ uint64_t mbar;
-    __shared__ uint32_t taddr_sh;
-    const int nb = Q.nbins, M = Q.maxn, nn = 2 * M + 1, gst = 2 * M + 3;
-    const int n = (int)blockIdx.x - M;
-    const int g = blockIdx.y;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int NC = (4 * nb + 15) & ~15;
-    const int aBytes = 4 * 4096, bBytes = 4 * NC * 32, rgBytes = aBytes + bBytes;
-    // Operand tiles: [region][hi, lo][A (4 K steps of 128 rows) | B (4 K steps of NC rows)].
-    auto tileA = [&](int r, int h, int st) { return zts + (r * 2 + h) * rgBytes + st * 4096; };
-    auto tileB = [&](int r, int h, int st) { return zts + (r * 2 + h) * rgBytes + aBytes + st * NC * 32; };
-    for (int q = tid; q < 4 * rgBytes / 16; q += TCB)
-        reinterpret_cast<float4*>(zts)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tid == 0) mbar_init(&mbar, 1);
-    __syncthreads();
-    if (wid == 0) tmem_alloc(&taddr_sh, 256);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tm = taddr_sh;
-    const uint32_t idesc = umma_idesc_tf32(128, NC);
-    const int nw = n >= 0 ? n : -n;
-    const long long r0 = Q.nrec * g / Q.ngroups, r1 = Q.nrec * (g + 1) / Q.ngroups;
-    uint32_t phase = 0;
-    int nchunk = 0;
-    bool fresh = true;     // the next MMA overwrites the accumulators
-    bool failed = false;
-    float* S = reinterpret_cast<float*>(zts);   // drain buffer [128][2 NC], over the tiles
-    const size_t Zs = (size_t)Q.Z;
-    auto drain = [&]() {
-        __syncthreads();
-        for (int r = 0; r < 2; ++r)
-            for (int c0 = 0; c0 < NC; c0 += 8) {
-                float v[8];
-                tmem_ld8(tm + ((uint32_t)(32 * wid) << 16) + (uint32_t)(r * 128 + c0), v);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) S[(32 * wid + lane) * (2 * NC) + r * NC + c0 + q] = v[q];
-            }
-        tc_fence_before();
-        __syncthreads();
-        double* part = Q.part + (size_t)g * 10 * Zs;
-        for (int e = tid; e < nb * nb; e += TCB) {
-            const int a = e / nb, b = e % nb;
-            auto C0 = [&](int row, int col) { return S[row * (2 * NC) + col]; };
-            auto C1 = [&](int row, int col) { return S[row * (2 * NC) + NC + col]; };
-            // (Re X + i Im X)(Re Y + i Im Y) from the four real blocks.
-            const float g0r = C0(a, b) - C0(nb + a, nb + b), g0i = C0(a, nb + b) + C0(nb + a, b);
-            const float g2r = C0(a, 2 * nb + b) - C0(nb + a, 3 * nb + b);
-            const float g2i = C0(a, 3 * nb + b) + C0(nb + a, 2 * nb + b);
-            const float g3r = C0(2 * nb + a, b) - C0(3 * nb + a, nb + b);
-            const float g3i = C0(2 * nb + a, nb + b) + C0(3 * nb + a, b);
-            const float g1r = C1(a, b) - C1(nb + a, nb + b), g1i = C1(a, nb + b) + C1(nb + a, b);
-            const float wr = C1(2 * nb + a, 2 * nb + b) - C1(3 * nb + a, 3 * nb + b);
-            const float wi = a == b ? 0.f : C1(2 * nb + a, 3 * nb + b) + C1(3 * nb + a, 2 * nb + b);
-            const size_t i = (size_t)(a * nb + b) * nn + M + n;
-            // All ten loads first, then the stores: one round trip per entry instead of ten
-            // (the compiler cannot reorder a load past a store to a possibly equal address).
-            const float add[10] = {g0r, g0i, g1r, g1i, g2r, g2i, g3r, g3i, wr, wi};
-            double o[10];
-#pragma unroll
-            for (int q = 0; q < 10; ++q) o[q] = part[q * Zs + i];
-#pragma unroll
-            for (int q = 0; q < 10; ++q) part[q * Zs + i] = o[q] + (double)add[q];
-        }
-        __syncthreads();
-        // The tile area was overwritten: restore the zero padding before the next fill.
-        for (int q = tid; q < 4 * rgBytes / 16; q += TCB)
-            reinterpret_cast<float4*>(zts)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncthreads();
-        fresh = true;
-        nchunk = 0;
-    };
-    // The chunk's record data is loaded into registers one chunk ahead, so the loads of
-    // chunk i+1 overlap the MMAs of chunk i.  A thread holds up to TC_IT fill items.
-    const int nab = (nb + 7) >> 3;
-    constexpr int TC_IT = 4;                 // nab * 8 * TC_REC / TCB <= 4 for nbins <= 32
-    float2 ig[TC_IT][5];
-    float4 ih[TC_IT];                        // w1, Re wg1, Im wg1, (ks, mk) packed
-    auto load_items = [&](long long cb) {
-        const int nvb = (int)min((long long)TC_REC, r1 - cb);
-#pragma unroll
-        for (int j = 0; j < TC_IT; ++j) {
-            const int idx = tid + j * TCB;
-            const int w = idx >> 5, l = idx & 31;
-            const int a = (w % nab) * 8 + (l & 7);
-            const int v = (w / nab) * 4 + (l >> 3);
-            ih[j] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-            if (idx >= nab * 8 * TC_REC || a >= nb || v >= nvb) continue;
-            const float* R = Q.rec + (size_t)(cb + v) * Q.rec_floats;
-            const float2* RG = reinterpret_cast<const float2*>(R + 8);
-            const float2* RW = RG + (size_t)gst * nb;
-            const int sh = Q.shift;
-            ig[j][0] = RG[(n - sh + M + 1) * nb + a];    // G[n-1]
-            ig[j][1] = RG[(-n - sh + M + 1) * nb + a];   // G[-n-1]
-            ig[j][2] = RG[(n + sh + M + 1) * nb + a];    // G[n+1]
-            ig[j][3] = RG[(-n + sh + M + 1) * nb + a];   // G[-n+1]
-            ig[j][4] = RW[nw * nb + a];            // W[|n|]
-            const int ks = __float_as_int(R[1]), mk = __float_as_int(R[2]);
-            ih[j] = make_float4(R[3], R[4], R[5], __int_as_float((ks << 8) | mk));
-        }
-    };
-    if (r0 < r1) load_items(r0);
-    for (long long c0 = r0; c0 < r1 && !failed; c0 += TC_REC) {
-        // Fill the K entries v (rows >= ks) and TC_REC + v (rows >= mk, A negated) of the
-        // chunk.  A warp covers 8 consecutive bins x 4 consecutive records: its stores hit
-        // the 8 rows x 4 k of core matrices, all 32 banks once.
-#pragma unroll
-        for (int j = 0; j < TC_IT; ++j) {
-            const int idx = tid + j * TCB;
-            const int w = idx >> 5, l = idx & 31;
-            const int a = (w % nab) * 8 + (l & 7);
-            const int v = (w / nab) * 4 + (l >> 3);
-            if (idx >= nab * 8 * TC_REC || a >= nb) continue;
-            float A0r = 0.f, A0i = 0.f, A1r = 0.f, A1i = 0.f, A3r = 0.f, A3i = 0.f, AWr = 0.f, AWi = 0.f;
-            float B0r = 0.f, B0i = 0.f, B1r = 0.f, B1i = 0.f, B2r = 0.f, B2i = 0.f, BWr = 0.f, BWi = 0.f;
-            int ks = nb, mk = nb;
-            const int am = a % Q.nbd;    // the row mask's bin
-            const int km = __float_as_int(ih[j].w);
-            if (km >= 0) {
-                const float w1 = ih[j].x, wr = ih[j].y, wi = ih[j].z;
-                ks = km >> 8; mk = km & 255;
-                const float2 gm1 = ig[j][0], gmm1 = ig[j][1], gp1 = ig[j][2], gmp1 = ig[j][3];
-                float2 w = ig[j][4];
-                if (n < 0) w.y = -w.y;
-                A0r = wr * gm1.x - wi * gm1.y;   A0i = wr * gm1.y + wi * gm1.x;
-                A1r = wr * gp1.x + wi * gp1.y;   A1i = wr * gp1.y - wi * gp1.x;
-                A3r = wr * gmp1.x + wi * gmp1.y; A3i = wi * gmp1.x - wr * gmp1.y;
-                AWr = w1 * w.x;                  AWi = w1 * w.y;
-                B0r = gmm1.x; B0i = gmm1.y; B1r = gmp1.x; B1i = gmp1.y;
-                B2r = gp1.x;  B2i = -gp1.y; BWr = w.x;    BWi = -w.y;
-            }
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const int e = t * TC_REC + v, st = e >> 3, kk = e & 7;
-                const bool on = am >= (t == 0 ? ks : mk);
-                const float sg = on ? (t == 0 ? 1.f : -1.f) : 0.f, sb = on ? 1.f : 0.f;
-                const float av[2][4] = {{A0r, A0i, A3r, A3i}, {A1r, A1i, AWr, AWi}};
-                const float bv[2][4] = {{B0r, B0i, B2r, B2i}, {B1r, B1i, BWr, BWi}};
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int row = q * nb + a;
-                        float hi, lo;
-                        tf32_split(sg * av[r][q], hi, lo);
-                        *reinterpret_cast<float*>(tileA(r, 0, st) + umma_tile_off(row, kk)) = hi;
-                        *reinterpret_cast<float*>(tileA(r, 1, st) + umma_tile_off(row, kk)) = lo;
-                        tf32_split(sb * bv[r][q], hi, lo);
-                        *reinterpret_cast<float*>(tileB(r, 0, st) + umma_tile_off(row, kk)) = hi;
-                        *reinterpret_cast<float*>(tileB(r, 1, st) + umma_tile_off(row, kk)) = lo;
-                    }
-            }
-        }
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            for (int r = 0; r < 2; ++r) {
-                const uint32_t d = tm + (uint32_t)(r * 128);
-                for (int st = 0; st < 4; ++st) {
-                    const uint64_t ah = umma_desc(smem_u32(tileA(r, 0, st)), 128, 256);
-                    const uint64_t al = umma_desc(smem_u32(tileA(r, 1, st)), 128, 256);
-                    const uint64_t bh = umma_desc(smem_u32(tileB(r, 0, st)), 128, 256);
-                    const uint64_t bl = umma_desc(smem_u32(tileB(r, 1, st)), 128, 256);
-                    umma_tf32(d, ah, bh, idesc, (fresh && st == 0) ? 0u : 1u);
-                    umma_tf32(d, ah, bl, idesc, 1u);
-                    umma_tf32(d, al, bh, idesc, 1u);
-                }
-            }
-            umma_commit(&mbar);
-        }
-        if (c0 + TC_REC < r1) load_items(c0 + TC_REC);   // overlaps the MMAs
-        const bool ok = mbar_wait(&mbar, phase, 1 << 24);
-        phase ^= 1u;
-        tc_fence_after();
-        failed = __syncthreads_or(!ok) != 0;
-        fresh = false;
-        if (failed) break;
-        if (++nchunk == TC_DRAIN) drain();
-    }
-    if (!failed && !fresh) drain();
-    if (failed && tid == 0) atomicExch(status, 1);
-    tc_fence_before();
-    __syncthreads();
-    if (wid == 0) tmem_dealloc(tm, 256);
-}
 
 // The n = 0 scalar outputs of calculateZeta over vertex records (ntri, meand2/3,
 // meanlogd2/3): for every entry (a, b) whose min(a, b) lies in the record's rows,
@@ -1712,7 +1370,7 @@ __global__ void __launch_bounds__(TCB) k_mp_zeta_tc(ZParams Q, int* status)
 //   a == b: ntri += n1 np_a (np_a - 1), meand2 = meand3 += w1 (sumw_a sumwr_a - sumwwr_a)
 // (meanlogd likewise with sumwlogr).  ntri is an exact 64-bit integer sum; the means are FP32
 // products with FP64 sums.  Block (g, tile) adds its sums to group g's partial arrays.
-__global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, double* spart,
+__global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, int chunk, double* spart,
                                                  unsigned long long* ntp)
 {
     extern __shared__ float4 zsh[];    // [chunk][nb][2]
@@ -1735,8 +1393,8 @@ __global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, double* spart,
 #pragma unroll
     for (int j = 0; j < ZE; ++j) { C[j] = 0ull; for (int q = 0; q < 4; ++q) D[j][q] = 0.; }
     const long long r0 = Q.nrec * g / gridDim.x, r1 = Q.nrec * (g + 1) / gridDim.x;
-    for (long long c0 = r0; c0 < r1; c0 += Q.chunk) {
-        const int nv = (int)min((long long)Q.chunk, r1 - c0);
+    for (long long c0 = r0; c0 < r1; c0 += chunk) {
+        const int nv = (int)min((long long)chunk, r1 - c0);
         __syncthreads();
         for (int idx = tid; idx < nv * nb; idx += ZB) {
             const int v = idx / nb, a = idx % nb;
@@ -1802,7 +1460,7 @@ __global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, double* spart,
 // the diagonal corrections.
 __global__ void k_mp_reduce(int nblk, long long stride, long long Z, int nb, int nn,
                             const double* in, const double* diag, long long diag_stride,
-                            int ngroups, const double* part, int nsg, const double* spart,
+                            const double* part, int nsg, const double* spart,
                             const unsigned long long* ntp, double* out)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1812,10 +1470,17 @@ __global__ void k_mp_reduce(int nblk, long long stride, long long Z, int nb, int
     double s = 0.;
     for (int b = 0; b < nblk; ++b) s += in[(size_t)b * stride + i];
     const int qp = q < 8 ? q : (q == 12 ? 8 : (q == 13 ? 9 : -1));
-    if (qp >= 0)
-        for (int g = 0; g < ngroups; ++g) s += part[((size_t)g * 10 + qp) * Z + r];
     const long long ab = r / nn;
-    const int a = (int)(ab / nb), b = (int)(ab % nb);
+    const int a = (int)(ab / nb), b = (int)(ab % nb), n = (int)(r % nn) - nn / 2;
+    // The contraction's sums (zeta.cu: 4 x 2 tiles, n >= 0); those of (a, b, -n) are those of
+    // (b, a, n) with gam2 and gam3 exchanged.  W_a conj(W_a) is real.
+    if (qp >= 0 && !(a == b && qp == 9)) {
+        const int ea = n < 0 ? b : a, eb = n < 0 ? a : b, an = n < 0 ? -n : n;
+        const int qe = n < 0 && qp >= 4 && qp < 8 ? qp ^ 2 : qp;
+        const int tcols = (nb + 1) >> 1, ntile = ((nb + 3) >> 2) * tcols;
+        const int e = 2 * (ea & 3) + (eb & 1), tile = (ea >> 2) * tcols + (eb >> 1);
+        s += part[((size_t)an * 80 + qe * 8 + e) * ntile + tile];
+    }
     if (r % nn == nn / 2 && ((q >= 8 && q <= 11) || q == 14)) {
         const size_t nb2 = (size_t)nb * nb;
         if (q == 14) {
@@ -1863,20 +1528,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
     const int nblk = nsm * std::min(per, 2);
     P.slot_doubles = (long long)mp_slot_doubles(nb, M);
     P.out_stride = 15 * Z;
-    // Contraction geometry: records per shared-memory chunk, entry tiles, record groups.
-    const int chunk = (int)std::max<long long>(1, std::min<long long>(64, (96 * 1024) / (64LL * nb)));
-    const size_t zsh = (size_t)chunk * nb * 64;
-    TC_CU(cudaFuncSetAttribute(k_mp_zeta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsh));
     const int etiles = (nb * nb + ZE * ZB - 1) / (ZE * ZB);
-    // The tensor-core contraction (tcgen05) for nbins <= 32, unless TCGPU_MP_TENSOR=0.  Its
-    // shared memory keeps at most two blocks on an SM (each holds 256 TMEM columns).
-    bool use_tc = 4 * nb <= 128;
-    if (const char* ev = std::getenv("TCGPU_MP_TENSOR")) use_tc = use_tc && std::atoi(ev) != 0;
-    const int NCt = (4 * nb + 15) & ~15;
-    const size_t tcsm = std::max<size_t>((size_t)4 * (16384 + 128 * NCt), 100 * 1024);
-    if (use_tc)
-        TC_CU(cudaFuncSetAttribute(k_mp_zeta_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcsm));
-    const int ngroups = std::max(1, (4 * nsm + nn * etiles - 1) / (nn * etiles));
     // Scalar outputs: records per chunk and record groups.
     const int chunk2 = (int)std::max<long long>(1, std::min<long long>(64, (48 * 1024) / (32LL * nb)));
     const size_t zsh2 = (size_t)chunk2 * nb * 32;
@@ -1956,14 +1608,23 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             TC_TRY(dalloc(&X.ntp, (size_t)nsg * nb * nb));
             X.nsg = nsg; X.spart_nb2 = (long long)nb * nb;
         }
-        if (X.ngroups < ngroups || X.part_stride < 10 * Z) {
+        const size_t npart = zeta_part_doubles(nb, M);
+        if (X.npart < npart) {
             dfree(X.part);
-            X.ngroups = 0;
-            TC_TRY(dalloc(&X.part, (size_t)ngroups * 10 * Z));
-            X.ngroups = ngroups; X.part_stride = 10 * Z;
+            X.npart = 0;
+            TC_TRY(dalloc(&X.part, npart));
+            X.npart = npart;
+        }
+        const long long nkey = (long long)P.nbd * (P.nbd + 1), nsegs = zeta_segments(X.zcap, P.nbd);
+        if (X.order_cap < X.zcap || X.nkey < nkey || X.nsegs < nsegs) {
+            dfree(X.order); dfree(X.keys); dfree(X.segs);
+            X.order_cap = 0; X.nkey = 0; X.nsegs = 0;
+            TC_TRY(dalloc(&X.order, (size_t)X.zcap));
+            TC_TRY(dalloc(&X.keys, 2 * (size_t)nkey + 1));
+            TC_TRY(dalloc(&X.segs, (size_t)nsegs));
+            X.order_cap = X.zcap; X.nkey = nkey; X.nsegs = nsegs;
         }
         if (!X.ctl) TC_TRY(dalloc(&X.ctl, 4));
-        if (!X.tcstatus) TC_TRY(dalloc(&X.tcstatus, 1));
         if (!X.err) TC_TRY(dalloc(&X.err, 2));
         if (!X.dbg) TC_TRY(dalloc(&X.dbg, 32));
         X.nblk = std::max(X.nblk, nblk);
@@ -1986,12 +1647,11 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
         P.err = X.err;
         P.dbg = X.dbg;
         TC_CU(cudaMemsetAsync(X.ctl, 0, 4 * sizeof(unsigned long long), st));
-        TC_CU(cudaMemsetAsync(X.tcstatus, 0, sizeof(int), st));
         X.overflow = 0; X.records = 0; X.waves = 0;
         TC_CU(cudaMemsetAsync(X.err, 0, 2 * sizeof(int), st));
         TC_CU(cudaMemsetAsync(X.out, 0, sizeof(double) * (size_t)P.out_stride * nblk, st));
         TC_CU(cudaMemsetAsync(X.diag, 0, sizeof(double) * (size_t)9 * nb * nblk, st));
-        TC_CU(cudaMemsetAsync(X.part, 0, sizeof(double) * (size_t)ngroups * 10 * Z, st));
+        TC_CU(cudaMemsetAsync(X.part, 0, sizeof(double) * npart, st));
         TC_CU(cudaMemsetAsync(X.spart, 0, sizeof(double) * (size_t)nsg * 4 * nb * nb, st));
         TC_CU(cudaMemsetAsync(X.ntp, 0, sizeof(unsigned long long) * (size_t)nsg * nb * nb, st));
         count_launch();
@@ -2017,20 +1677,16 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             if (e) break;
             ZParams Q;
             Q.rec = X.zrec; Q.nrec = std::min<long long>((long long)c[2], X.zcap);
-            Q.rec_floats = recf; Q.nbins = nb; Q.maxn = M; Q.chunk = chunk;
-            Q.ngroups = ngroups; Q.part = X.part; Q.Z = Z;
+            Q.rec_floats = recf; Q.nbins = nb; Q.maxn = M;
+            Q.part = X.part; Q.order = X.order; Q.segs = X.segs;
+            Q.count = X.keys; Q.first = X.keys + X.nkey; Q.nseg = X.keys + 2 * X.nkey;
             Q.shift = P.vreal ? 0 : 1;
             Q.nbd = P.nbd; Q.typo32 = P.typo32;
             if (Q.nrec > 0) {
-                count_launch();
-                if (use_tc) k_mp_zeta_tc<<<dim3(nn, ngroups), TCB, tcsm, st>>>(Q, X.tcstatus);
-                else k_mp_zeta<<<dim3(nn, ngroups, etiles), ZB, zsh, st>>>(Q);
-                TC_CU(cudaGetLastError());
+                TC_TRY(launch_zeta(Q, nsm, st));
                 if (!P.quick) {
-                    ZParams Q2 = Q;
-                    Q2.chunk = chunk2;
                     count_launch();
-                    k_mp_zscal<<<dim3(nsg, etiles), ZB, zsh2, st>>>(Q2, X.spart, X.ntp);
+                    k_mp_zscal<<<dim3(nsg, etiles), ZB, zsh2, st>>>(Q, chunk2, X.spart, X.ntp);
                     TC_CU(cudaGetLastError());
                 }
             }
@@ -2066,18 +1722,9 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             set_last_error("multipole: device stack overflow (tree too deep)");
             return 4;
         }
-        {
-            int tcs = 0;
-            TC_CU(cudaMemcpyAsync(&tcs, X.tcstatus, sizeof(int), cudaMemcpyDeviceToHost, st));
-            TC_CU(cudaStreamSynchronize(st));
-            if (tcs) {
-                set_last_error("multipole: a tensor-core contraction did not complete in time");
-                return 4;
-            }
-        }
         count_launch();
         k_mp_reduce<<<(unsigned)((P.out_stride + 255) / 256), 256, 0, st>>>(
-            nblk, P.out_stride, Z, nb, nn, X.out, X.diag, 9LL * nb, ngroups, X.part,
+            nblk, P.out_stride, Z, nb, nn, X.out, X.diag, 9LL * nb, X.part,
             P.quick ? 0 : nsg, X.spart, X.ntp, X.total);
         TC_CU(cudaGetLastError());
         TC_CU(cudaMemcpyAsync(h_out, X.total, sizeof(double) * (size_t)P.out_stride,
@@ -2094,7 +1741,8 @@ void free_mp_scratch(MPScratch& X)
     dfree(X.arena1); dfree(X.jobs); dfree(X.arena2); dfree(X.acc); dfree(X.perm);
     dfree(X.slots); dfree(X.out); dfree(X.diag); dfree(X.total); dfree(X.zrec); dfree(X.part);
     dfree(X.spart); dfree(X.ntp);
-    dfree(X.ctl); dfree(X.err); dfree(X.dbg); dfree(X.tcstatus);
+    dfree(X.ctl); dfree(X.err); dfree(X.dbg);
+    dfree(X.order); dfree(X.keys); dfree(X.segs);
     X = MPScratch();
 }
 

@@ -106,9 +106,12 @@ struct MPScratch {
     float* zrec = nullptr;
     long long zcap = 0;
     int zrec_floats = 0;
-    double* part = nullptr;     // per contraction group: 10 arrays of nbins^2 (2 maxn + 1)
-    long long part_stride = 0;
-    int ngroups = 0;
+    double* part = nullptr;     // the contraction's sums (zeta.cu)
+    size_t npart = 0;
+    int* order = nullptr;       // the records by row range, the ranges' counts and segments
+    int* keys = nullptr;
+    int4* segs = nullptr;
+    long long order_cap = 0, nkey = 0, nsegs = 0;
     double* spart = nullptr;    // per scalar group: 4 arrays of nbins^2 (meand2/3, meanlogd2/3)
     unsigned long long* ntp = nullptr;   // per scalar group: nbins^2 triangle counts
     long long spart_nb2 = 0;
@@ -119,11 +122,29 @@ struct MPScratch {
     unsigned long long* ctl = nullptr;
     int* err = nullptr;
     double* dbg = nullptr;
-    int* tcstatus = nullptr;    // set when a tensor-core contraction timed out
     // Requested minimum capacities, raised after an overflow.
     long long want_a1 = 0, want_jobs = 0, want_a2 = 0;
     int want_slots = 0;
 };
+
+// The contraction over vertex records (zeta.cu) and the scalar sums over them.
+struct ZParams {
+    const float* rec;
+    long long nrec;
+    int rec_floats, nbins, maxn;
+    int shift;             // 1: G_n at n -+ 1 (a spin-2 vertex); 0: at n (an N or K vertex)
+    int nbd;               // distance bins; a record's rows [ks, mk) hold min(a, b) mod nbd
+    int typo32;            // see MPParams::typo32
+    double* part;          // [n >= 0][10][entry of a 4 x 2 tile][tile]
+    int* order;            // record numbers by row range
+    int* count;            // per row range ks (nbd + 1) + mk: records, first place in order
+    int* first;
+    int4* segs;            // (first place, records, ks, mk)
+    int* nseg;
+};
+size_t zeta_part_doubles(int nb, int M);
+long long zeta_segments(long long nrec, int nbd);
+int launch_zeta(const ZParams& Q, int nsm, cudaStream_t st);
 
 int launch_leaf_sums(int ncap, const Cells& C, double* ls, float4* lsf, cudaStream_t st);
 // N / K pair cells as the real payload (w or w k, 0) of GNN, GKK, NKK, KNN.
