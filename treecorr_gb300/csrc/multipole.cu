@@ -44,7 +44,9 @@
 
 namespace tc {
 
-static constexpr int MB = 256;            // threads per multipole block
+static constexpr int MB = 128;            // threads per multipole block (4 blocks per SM: 264 ms
+                                          // for the call below, 5: 272, 256 threads: 267)
+static constexpr int MBLK = 4;            // multipole blocks per SM
 static constexpr int MW = MB / 32;        // warps per block
 static constexpr int MSTACK = 128;        // depth of the block-local stacks
 
@@ -487,216 +489,177 @@ __device__ __forceinline__ double* slot_ptr(const MPParams& P, int blk, int s)
 // Accepted-pair record (MP_REC floats): z (2), wg = g2 * e (2), w2, n2 (int), k (int), pad,
 // then the 14 scalar terms of calculateGn: w2, w2 r, w2 logr, sum w^2, (sum w^2) r,
 // (sum w^2) logr, sumwwgg0 (2), sumwwgg1 (2), sumwwgg2 (2), wg (2).
-static constexpr int REC_K = 6, REC_S = 8, NSCAL = 14;
+static constexpr int REC_K = 6;
+
+// A warp's staged batch of 32 records: powers of z, (wg, w2, bin), scalar terms (14, n2, w2).
+struct AccBatch {
+    float2 pw[32][33];
+    float4 hk[32];
+    float sc[32][17];
+};
+static_assert(sizeof(AccBatch) % 16 == 0, "");
 
 // Bin-ordered G_n / W_n accumulation of the records [0, nrec) of this block into slot S.
-// The records are ranked stably by bin (list order within a bin), then warp w takes the
-// w-th contiguous share of the ranked records.  A warp walks its share one record at a time:
-// lane l forms z^(l+1) (and z^(l+33)) by a multiplicative warp scan and adds the record's
-// W_n, G_{+n}, G_{-n} terms in FP32; lanes 0..13 add the scalar terms, lane 14 counts n2.
-// The FP32 partials go to FP64 registers every 32 records and to the slot (FP64 atomics,
-// since two warps can share a bin) when the bin changes.
+// The records are ranked by bin, then warp w takes the w-th contiguous share of the ranked
+// records, 32 at a time: lane = record writes the powers z, z^2, .. z^32 (z^33 .. in a second
+// round) to shared memory, one complex multiplication each, and the record's other terms; then
+// lane = n walks the records of each bin's run with six FP32 multiply-adds each (the sums of
+// Re wg z^n and Im wg z^n, which make both G_n and G_-n, and w z^n), lanes 0..15 adding
+// the scalar terms as well.  The FP32 sums (F over a batch, F2 over the share: at most 16
+// batches) go to the slot in FP64 when the bin changes (atomics: two warps can share a bin).
+// A record costs the warp 22 instructions; raising every lane to its own power by squaring
+// took 75.
 __device__ void mp_accumulate(const MPParams& P, const float* rec, int* perm, int nrec,
-                              double* S, int* bh, int (*bw)[MP_MAXNB])
+                              double* S, int* bh, AccBatch* batches)
 {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nb = P.nbins, M = P.maxn, gst = 2 * M + 3;
-    // Stable ranking by bin: bh holds the per-bin counts on entry.
-    if (tid == 0) {
-        int s = 0;
-        for (int k = 0; k < nb; ++k) { const int c = bh[k]; bh[k] = s; s += c; }
-        if (s != nrec) mp_check_fail(P.err, 8);   // counts and records disagree
+    // Ranking by bin: bh holds the per-bin counts on entry.
+    if (wid == 0) {
+        int total = 0;
+        for (int k0 = 0; k0 < nb; k0 += 32) {
+            const int c = k0 + lane < nb ? bh[k0 + lane] : 0;
+            int x = c;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (k0 + lane < nb) bh[k0 + lane] = total + x - c;
+            total += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0 && total != nrec) mp_check_fail(P.err, 8);   // counts and records disagree
     }
-    for (int q = tid; q < MW * MP_MAXNB; q += MB) bw[q / MP_MAXNB][q % MP_MAXNB] = 0;
-    for (int a = tid; a < nrec; a += MB) perm[a] = -1;
     __syncthreads();
-    for (int c0 = 0; c0 < nrec; c0 += MB) {
-        const int a = c0 + tid;
-        const int k = a < nrec ? __float_as_int(__ldcg(rec + (size_t)a * MP_REC + REC_K)) : nb;
+    for (int c0 = 32 * wid; c0 < nrec; c0 += MB) {
+        const int a = c0 + lane;
+        const int k = a < nrec ? __float_as_int(__ldcg(rec + (size_t)a * MP_REC + REC_K)) : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, k);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (a < nrec && rank == 0) bw[wid][k] = __popc(peers);
-        __syncthreads();
-        if (a < nrec) {
-            int pos = bh[k] + rank;
-            for (int w = 0; w < wid; ++w) pos += bw[w][k];
-            perm[pos] = a;
-        }
-        __syncthreads();
-        if (tid < nb) {
-            int t = 0;
-            for (int w = 0; w < MW; ++w) { t += bw[w][tid]; bw[w][tid] = 0; }
-            bh[tid] += t;
-        }
-        __syncthreads();
+        const int leader = __ffs(peers) - 1;
+        int pos = 0;
+        if (lane == leader && k >= 0 && k < nb) pos = atomicAdd(&bh[k], __popc(peers));
+        pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+        if (k >= 0 && pos < nrec) perm[pos] = a;
     }
+    __syncthreads();
     for (int k = tid; k < nb; k += MB) bh[k] = 0;   // counts of the next batch
     double* W = S;
     double* G = S + 2 * (size_t)nb * (M + 1);
-    double* GG = G + 2 * (size_t)nb * gst;
-    double* SC = GG + 6 * (size_t)nb;
     const int per = (nrec + MW - 1) / MW;
     const int p0 = wid * per, p1 = min(nrec, p0 + per);
-    constexpr int KNONE = 0x7fffffff;
-    __shared__ float4 bz[MW][32];
-    __shared__ float2 bk[MW][32];
-    // FP32 sums of the current bin: F over one batch, F2 over up to 32 batches; they reach
-    // FP64 (D, then the slot) only every 32 batches and when the bin changes.
-    float F[12], F2[12];
-    double D[12];
+    AccBatch& B = batches[wid];
+    // This lane's scalar sum in the slot: place for bin 0 and step per bin.
+    const int oG = 2 * nb * (M + 1), oGG = oG + 2 * nb * gst, oSC = oGG + 6 * nb;
+    int sc0 = 0, scs = 1;
+    if (lane < 6) sc0 = oSC + (lane + 1) * nb;
+    else if (lane < 12) { sc0 = oGG + ((lane - 6) >> 1) * 2 * nb + (lane & 1); scs = 2; }
+    else if (lane < 14) { sc0 = oG + (int)sG(nb, M, 0, 0) + lane - 12; scs = 2; }
+    else if (lane == 14) sc0 = oSC;
+    else { sc0 = (int)sW(nb, 0, 0); scs = 2; }
+    float F[2][6], F2[2][6], fs = 0.f, fs2 = 0.f;
+    unsigned cn = 0;
+    int curk[2] = {-1, -1};
 #pragma unroll
-    for (int q = 0; q < 12; ++q) { F[q] = 0.f; F2[q] = 0.f; D[q] = 0.; }
-    int curk = -1, nbatch = 0;
-    // Power sums of lane n = lane+1 (and lane+33) to the slot.
-    auto flushp = [&](int k) {
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int q = 0; q < 12; ++q) { D[q] += (double)(F2[q] + F[q]); F[q] = 0.f; F2[q] = 0.f; }
-        nbatch = 0;
-        const int n = lane + 1, n1 = lane + 33;
-        if (n <= M) { double* wp = W + sW(nb, n, k); atomicAdd(wp, D[0]); atomicAdd(wp + 1, D[1]); }
+        for (int q = 0; q < 6; ++q) { F[h][q] = 0.f; F2[h][q] = 0.f; }
+    auto flush = [&](int h, int k) {
+        const int n = lane + 1 + 32 * h;
+        float* f = F[h];
+        float* f2 = F2[h];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) { f2[q] += f[q]; f[q] = 0.f; }
+        if (n <= M) {
+            double* wp = W + sW(nb, n, k);
+            atomicAdd(wp, (double)f2[0]);
+            atomicAdd(wp + 1, (double)f2[1]);
+        }
         if (n <= M + 1) {
-            double* gpp = G + sG(nb, M, n, k);
-            double* gmp = G + sG(nb, M, -n, k);
-            atomicAdd(gpp, D[2]); atomicAdd(gpp + 1, D[3]);
-            atomicAdd(gmp, D[4]); atomicAdd(gmp + 1, D[5]);
-        }
-        if (n1 <= M) { double* wp = W + sW(nb, n1, k); atomicAdd(wp, D[6]); atomicAdd(wp + 1, D[7]); }
-        if (n1 <= M + 1) {
-            double* gpp = G + sG(nb, M, n1, k);
-            double* gmp = G + sG(nb, M, -n1, k);
-            atomicAdd(gpp, D[8]); atomicAdd(gpp + 1, D[9]);
-            atomicAdd(gmp, D[10]); atomicAdd(gmp + 1, D[11]);
+            double* gp = G + sG(nb, M, n, k);
+            double* gm = G + sG(nb, M, -n, k);
+            atomicAdd(gp, (double)(f2[2] - f2[5]));
+            atomicAdd(gp + 1, (double)(f2[3] + f2[4]));
+            atomicAdd(gm, (double)(f2[2] + f2[5]));
+            atomicAdd(gm + 1, (double)(f2[4] - f2[3]));
         }
 #pragma unroll
-        for (int q = 0; q < 12; ++q) D[q] = 0.;
+        for (int q = 0; q < 6; ++q) f2[q] = 0.f;
+        if (h == 0) {
+            if (lane < 16) atomicAdd(S + sc0 + (size_t)scs * k, lane == 14 ? (double)cn : (double)(fs2 + fs));
+            fs = fs2 = 0.f;
+            cn = 0;
+        }
     };
-    // Batches of 32 ranked records: lane l loads record base+l.  The scalar terms are summed
-    // by a segmented warp scan over the lanes of equal bin (the bins ascend along the lanes);
-    // the last lane of each run adds its run to the slot.  The powers walk the batch one
-    // record at a time with the record's values taken from its lane.
-    // Scalar sums of one run of bin kb to the slot.
-    auto flush_scal = [&](int kb, const float* v, long long cnt) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) atomicAdd(&SC[(size_t)(q + 1) * nb + kb], (double)v[q]);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) atomicAdd(&GG[(size_t)(q >> 1) * 2 * nb + 2 * kb + (q & 1)], (double)v[6 + q]);
-        atomicAdd(&G[sG(nb, M, 0, kb)], (double)v[12]);
-        atomicAdd(&G[sG(nb, M, 0, kb) + 1], (double)v[13]);
-        atomicAdd(&W[sW(nb, 0, kb)], (double)v[0]);
-        atomicAdd(&SC[kb], (double)cnt);
-    };
-    float cs[NSCAL];                  // carried run: FP32 scalar sums, count, bin, batches
-    long long cn = 0;
-    int ck = -1, cnum = 0;
-#pragma unroll
-    for (int q = 0; q < NSCAL; ++q) cs[q] = 0.f;
     for (int base = p0; base < p1; base += 32) {
-        const int p = base + lane;
-        bool ok = p < p1;
-        const int pi = ok ? __ldcg(perm + p) : 0;
-        if (ok && (pi < 0 || pi >= nrec)) {          // every rank is filled exactly once
-            mp_check_fail(P.err, 4);
-            ok = false;
-        }
-        const float4* r4 = reinterpret_cast<const float4*>(rec + (size_t)(ok ? pi : 0) * MP_REC);
-        const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 h0 = ok ? __ldcg(r4) : zero4, h1 = ok ? __ldcg(r4 + 1) : zero4;
-        const float4 q0 = ok ? __ldcg(r4 + 2) : zero4, q1 = ok ? __ldcg(r4 + 3) : zero4;
-        const float4 q2 = ok ? __ldcg(r4 + 4) : zero4, q3 = ok ? __ldcg(r4 + 5) : zero4;
-        int k = ok ? __float_as_int(h1.z) : KNONE;
-        if (ok && (k < 0 || k >= nb)) { mp_check_fail(P.err, 5); k = KNONE; ok = false; }
-        float sv[NSCAL] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
-                           q2.x, q2.y, q2.z, q2.w, q3.x, q3.y};
-        long long n2 = ok ? (long long)__float_as_int(h1.y) : 0;
-        if (!ok) {
-#pragma unroll
-            for (int q = 0; q < NSCAL; ++q) sv[q] = 0.f;
-        }
-        // The run carried from the previous batch joins lane 0 when the bin continues, and
-        // goes to the slot when it does not.
-        if (lane == 0 && ck >= 0) {
-            if (k == ck) {
-#pragma unroll
-                for (int q = 0; q < NSCAL; ++q) sv[q] += cs[q];
-                n2 += cn;
-            } else {
-                flush_scal(ck, cs, cn);
-            }
-        }
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int kk = __shfl_up_sync(0xffffffffu, k, o);
-            const bool same = lane >= o && kk == k;
-#pragma unroll
-            for (int q = 0; q < NSCAL; ++q) {
-                const float t = __shfl_up_sync(0xffffffffu, sv[q], o);
-                if (same) sv[q] += t;
-            }
-            const long long tn = __shfl_up_sync(0xffffffffu, n2, o);
-            if (same) n2 += tn;
-        }
-        const int kn = __shfl_down_sync(0xffffffffu, k, 1);
-        // The last run of the batch is carried on while it stays short; runs that end inside
-        // the batch, or at the end of the warp's range, go to the slot.
-        const bool last_batch = base + 32 >= p1;
-        const bool run_end = ok && (lane == 31 || kn != k);
-        const bool carry = run_end && lane == 31 && !last_batch && cnum < 32;
-        if (run_end && !carry) flush_scal(k, sv, n2);
-        {
-            const bool c31 = __shfl_sync(0xffffffffu, carry, 31);
-            const int k31 = __shfl_sync(0xffffffffu, k, 31);
-#pragma unroll
-            for (int q = 0; q < NSCAL; ++q) cs[q] = __shfl_sync(0xffffffffu, sv[q], 31);
-            cn = __shfl_sync(0xffffffffu, n2, 31);
-            ck = c31 ? k31 : -1;
-            cnum = c31 ? cnum + 1 : 0;
-        }
         const int nv = min(32, p1 - base);
-        // The batch's (z, wg) and (w2, k) go through shared memory: lane j's record is read
-        // by the whole warp with broadcast loads.
-        bz[wid][lane] = h0;
-        bk[wid][lane] = make_float2(h1.x, __int_as_float(k));
-        __syncwarp();
-        const int m = lane + 1;
-        for (int j = 0; j < nv; ++j) {
-            const float4 hz = bz[wid][j];
-            const float2 hk = bk[wid][j];
-            const int kj = __float_as_int(hk.y);
-            const float zr = hz.x, zi = hz.y, wgr = hz.z, wgi = hz.w, w2 = hk.x;
-            if (kj == KNONE) continue;
-            if (kj != curk) {
-                if (curk >= 0) flushp(curk);
-                curk = kj;
-            }
-            // z^(lane+1) by binary powering: every lane squares z up to z^32 and multiplies
-            // the powers of the bits of lane+1.
-            float pre = 1.f, pim = 0.f, br = zr, bi = zi;
+        const bool in = lane < nv;
+        const int pi = in ? __ldcg(perm + base + lane) : 0;
+        const bool bad = pi < 0 || pi >= nrec;          // every rank is filled exactly once
+        if (bad) mp_check_fail(P.err, 4);
+        const float4* r4 = reinterpret_cast<const float4*>(rec + (size_t)(bad ? 0 : pi) * MP_REC);
+        const float4 h0 = __ldcg(r4), h1 = __ldcg(r4 + 1), q0 = __ldcg(r4 + 2), q1 = __ldcg(r4 + 3);
+        const float4 q2 = __ldcg(r4 + 4), q3 = __ldcg(r4 + 5);
+        int k = __float_as_int(h1.z);
+        if (k < 0 || k >= nb) { mp_check_fail(P.err, 5); k = 0; }
+        const int kp = __shfl_up_sync(0xffffffffu, k, 1);
+        const unsigned starts = __ballot_sync(0xffffffffu, in && lane > 0 && k != kp);
+        __syncwarp();                                   // the batch before has been read
+        B.hk[lane] = make_float4(h0.z, h0.w, h1.x, __int_as_float(k));
+        {
+            const float sv[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
+                                  q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, h1.y, h1.x};
 #pragma unroll
-            for (int t = 0; t < 6; ++t) {
-                if (m & (1 << t)) { const float u = pre * br - pim * bi; pim = pre * bi + pim * br; pre = u; }
-                if (t < 5) { const float u = br * br - bi * bi; bi = 2.f * br * bi; br = u; }
+            for (int q = 0; q < 16; ++q) B.sc[lane][q] = sv[q];
+        }
+        float pr = 1.f, pi2 = 0.f;                      // z^(32 h), then on
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h == 1 && M + 1 <= 32) break;
+            const int nc = min(32, M + 1 - 32 * h);
+            if (h == 1) __syncwarp();
+#pragma unroll 4
+            for (int n = 0; n < nc; ++n) {
+                const float t = pr * h0.x - pi2 * h0.y;
+                pi2 = pr * h0.y + pi2 * h0.x;
+                pr = t;
+                B.pw[lane][n] = make_float2(pr, pi2);
             }
-            F[0] += w2 * pre; F[1] += w2 * pim;
-            F[2] += wgr * pre - wgi * pim; F[3] += wgr * pim + wgi * pre;
-            F[4] += wgr * pre + wgi * pim; F[5] += wgi * pre - wgr * pim;
-            if (M + 1 > 32) {
-                const float z32r = br, z32i = bi;     // z^32
-                const float qr = z32r * pre - z32i * pim, qi = z32r * pim + z32i * pre;
-                F[6] += w2 * qr; F[7] += w2 * qi;
-                F[8] += wgr * qr - wgi * qi; F[9] += wgr * qi + wgi * qr;
-                F[10] += wgr * qr + wgi * qi; F[11] += wgi * qr - wgr * qi;
+            __syncwarp();
+            for (int js = 0; js < nv;) {
+                const unsigned later = js < 31 ? starts & ~((2u << js) - 1u) : 0u;
+                const int je = later ? __ffs(later) - 1 : nv;
+                const int kj = __float_as_int(B.hk[js].w);
+                if (kj != curk[h]) {
+                    if (curk[h] >= 0) flush(h, curk[h]);
+                    curk[h] = kj;
+                }
+#pragma unroll 4
+                for (int j = js; j < je; ++j) {
+                    const float2 z = B.pw[j][lane];
+                    const float4 hk = B.hk[j];
+                    F[h][0] = fmaf(hk.z, z.x, F[h][0]);
+                    F[h][1] = fmaf(hk.z, z.y, F[h][1]);
+                    F[h][2] = fmaf(hk.x, z.x, F[h][2]);     // Re wg Re z^n
+                    F[h][3] = fmaf(hk.x, z.y, F[h][3]);     // Re wg Im z^n
+                    F[h][4] = fmaf(hk.y, z.x, F[h][4]);     // Im wg Re z^n
+                    F[h][5] = fmaf(hk.y, z.y, F[h][5]);     // Im wg Im z^n
+                    if (h == 0) {
+                        const float v = B.sc[j][lane & 15];
+                        fs += v;
+                        cn += __float_as_uint(v);           // (lane 14: the point count)
+                    }
+                }
+                js = je;
             }
         }
 #pragma unroll
-        for (int q = 0; q < 12; ++q) { F2[q] += F[q]; F[q] = 0.f; }
-        if (++nbatch == 32) {
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int q = 0; q < 12; ++q) { D[q] += (double)F2[q]; F2[q] = 0.f; }
-            nbatch = 0;
-        }
-        __syncwarp();
+            for (int q = 0; q < 6; ++q) { F2[h][q] += F[h][q]; F[h][q] = 0.f; }
+        fs2 += fs;
+        fs = 0.f;
     }
-    if (curk >= 0) flushp(curk);
+    if (curk[0] >= 0) flush(0, curk[0]);
+    if (curk[1] >= 0) flush(1, curk[1]);
     __syncthreads();
 }
 
@@ -757,11 +720,10 @@ __device__ void zeta_diag(const MPParams& P, int c1, const double* S, int ks, in
         const C2 t0 = cmul(wg1, {__ldcg(GG + 2 * a), __ldcg(GG + 2 * a + 1)});
         const C2 t1 = cmul(conj2(wg1), {__ldcg(GG + 2 * nb + 2 * a), __ldcg(GG + 2 * nb + 2 * a + 1)});
         const C2 t2 = cmul(wg1, {__ldcg(GG + 4 * nb + 2 * a), __ldcg(GG + 4 * nb + 2 * a + 1)});
-        diag[0 * nb + a] += t0.re; diag[1 * nb + a] += t0.im;
-        diag[2 * nb + a] += t1.re; diag[3 * nb + a] += t1.im;
-        diag[4 * nb + a] += t2.re; diag[5 * nb + a] += t2.im;
-        diag[6 * nb + a] += t2.re; diag[7 * nb + a] += t2.im;
-        diag[8 * nb + a] += w1 * __ldcg(sumww + a);
+        // (this block's own sums; atomics only so that no thread waits for a load)
+        const double v[9] = {t0.re, t0.im, t1.re, t1.im, t2.re, t2.im, t2.re, t2.im, w1 * __ldcg(sumww + a)};
+#pragma unroll
+        for (int q = 0; q < 9; ++q) atomicAdd(diag + q * nb + a, v[q]);
     }
 }
 
@@ -895,38 +857,60 @@ __device__ void zeta_inplace3(const MPParams& P, int c1, const double* S, int ks
 
 // calculateZeta for vertex c1, rows [ks, mk): the diagonal self-pair corrections now, the
 // rest as one vertex record for the batched contraction kernels (k_mp_zeta, k_mp_zscal).
-// Record (floats): header (c1, ks, mk, w1, Re/Im wg1, n1, pad), then G_n [n = -(M+1) ..
-// M+1][bin] and W_n [n = 0 .. M][bin] complex, then npairs (int), sumw, sumwr, sumwlogr,
-// sumwwr, sumwwlogr [bin].  A record that does not fit the buffer is contracted in place.
+// Record (floats): header (c1, ks, mk, w1, Re/Im wg1, n1, pad), then npairs (int), sumw, sumwr,
+// sumwlogr, sumwwr, sumwwlogr [bin], then G_n [n = -(M+1) .. M+1][bin] and W_n [n = 0 ..
+// M][bin] complex, of the bins from ks on (min(a, b) >= ks; all bins of a three-field cross).
+// A record that does not fit the buffer is contracted in place.
 __device__ void zeta_emit(const MPParams& P, int c1, const double* S, int ks, int mk,
                           double* out, double* diag, double* shG, double* shW,
                           unsigned long long* zidx_sh, int* emits_sh)
 {
     const int nb = P.nbins, M = P.maxn, gst = 2 * M + 3;
-    // (a three-field cross has no self-pair corrections: getMP2 / getMP3 without ww)
-    if (!P.three) zeta_diag(P, c1, S, ks, mk, diag);
-    if (threadIdx.x == 0) {
-        *zidx_sh = atomicAdd(P.zcount, 1ull);
+    // (number, 16-byte offset), in one counter
+    const int c0 = P.three ? 0 : ks, nc = nb - c0, total = (gst + M + 1) * nc;
+    const long long units = (8 + 6 * nb + 2 * total + 3) / 4;
+    if (threadIdx.x == MB - 1) {
+        *zidx_sh = atomicAdd(P.zcount, ZC_ONE + (unsigned long long)units);
         ++*emits_sh;
     }
+    // G's rows, then W's, eight columns per thread in flight.
+    const double2* W = reinterpret_cast<const double2*>(S);
+    const double2* G = W + (size_t)nb * (M + 1);
+    const int dr = MB / nc, dc = MB - dr * nc;
+    int row = threadIdx.x / nc, col = threadIdx.x - row * nc;
+    double2 v[8];
+    auto load8 = [&](int q0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (q0 + u * MB < total)
+                v[u] = __ldcg((row < gst ? G + (size_t)row * nb : W + (size_t)(row - gst) * nb) + c0 + col);
+            row += dr;
+            col += dc;
+            if (col >= nc) { col -= nc; ++row; }
+        }
+    };
+    // (a three-field cross has no self-pair corrections: getMP2 / getMP3 without ww)
+    if (!P.three) zeta_diag(P, c1, S, ks, mk, diag);
     __syncthreads();
-    const unsigned long long zi = *zidx_sh;
-    if ((long long)zi < P.zcap) {
-        float* R = P.zrec + (size_t)zi * P.zrec_floats;
+    const long long zi = (long long)(*zidx_sh / ZC_ONE), off = (long long)(*zidx_sh % ZC_ONE);
+    const bool fits = zi < P.zmax && off + units <= P.zcap;
+    if (threadIdx.x == 0 && zi < P.zmax) P.zoff[zi] = fits ? (unsigned)off : ZOFF_NONE;
+    if (fits) {
+        float* R = P.zrec + 4 * (size_t)off;
         if (threadIdx.x == 0) {
             R[0] = __int_as_float(c1); R[1] = __int_as_float(ks); R[2] = __int_as_float(mk);
             R[3] = P.w[c1]; R[4] = P.d1[c1]; R[5] = P.d2[c1];
             R[6] = __int_as_float(P.n[c1]); R[7] = 0.f;
         }
-        // G then W: the slot's first 2 nb (M+1) + 2 nb gst doubles, reordered G-first.
-        const double* W = S;
-        const double* G = S + 2 * (size_t)nb * (M + 1);
-        float* RG = R + 8;
-        float* RW = RG + 2 * (size_t)gst * nb;
-        for (int q = threadIdx.x; q < 2 * gst * nb; q += MB) RG[q] = (float)__ldcg(G + q);
-        for (int q = threadIdx.x; q < 2 * (M + 1) * nb; q += MB) RW[q] = (float)__ldcg(W + q);
-        const double* SC = G + 2 * (size_t)nb * gst + 6 * (size_t)nb;
-        float* RS = RW + 2 * (size_t)(M + 1) * nb;
+        float2* RG = reinterpret_cast<float2*>(R + 8 + 6 * nb);
+        for (int q0 = threadIdx.x; q0 < total; q0 += 8 * MB) {
+            load8(q0);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (q0 + u * MB < total) RG[q0 + u * MB] = make_float2((float)v[u].x, (float)v[u].y);
+        }
+        const double* SC = S + 2 * (size_t)nb * (M + 1) + 2 * (size_t)nb * gst + 6 * (size_t)nb;
+        float* RS = R + 8;
         for (int q = threadIdx.x; q < nb; q += MB) {
             RS[q] = __int_as_float((int)__ldcg(SC + q));                // npairs
             RS[nb + q] = (float)__ldcg(SC + nb + q);                    // sumw
@@ -944,21 +928,42 @@ __device__ void zeta_emit(const MPParams& P, int c1, const double* S, int ks, in
     __syncthreads();
 }
 
+// No job is started once the buffer holds zstop units or zmaxstop records.
+__device__ __forceinline__ bool zbuffer_full(const MPParams& P)
+{
+    const unsigned long long c = *(volatile unsigned long long*)P.zcount;
+    return (long long)(c % ZC_ONE) >= P.zstop || (long long)(c / ZC_ONE) >= P.zmaxstop;
+}
+
+// Phase 2.  GGG of 500,000 points (20 bins, max_n 30) walks 1.87e6 lists of 908 cells on average,
+// accepts 0.8e9 pairs and emits 1.57e6 vertex records: 373 ms before, 225 ms now, of which some
+// 90 are the lists' decisions, 85 the accumulation and 50 the records.  What counts, as
+// one SM has 16 warps here (registers) and every list is a chain of dependent loads and barriers:
+//   * FP64: an instruction takes 16 cycles of the SM.  The largest r + s, the bin of its
+//     logarithm and the block's maximum took a third of the time on all warps; now only the
+//     threads that can hold the maximum leave FP32.
+//   * one barrier per 128 list entries (places by ballots), none for the running counts;
+//   * G_n, W_n rows copied and converted eight loads at a time, and only the record's columns;
+//   * one buffer for all records: a wave's end costs the blocks' last jobs, 10 ms.
+// Taken back: the next entries loaded ahead (spills: 287 ms for the call against 254),
+// mp_accumulate out of line (295), five blocks of 128 (272) or three of 256 threads (303).
+//
 // THREE: a three-field cross (two pair lists); compiled apart so that the auto and cross12
 // paths carry none of its registers.
 template <bool THREE>
-__global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
+__global__ void __launch_bounds__(MB, MBLK) k_mp_finish(const __grid_constant__ MPParams P)
 {
     extern __shared__ __align__(16) double mp_sh[];
     __shared__ P2Entry stk[MSTACK];
-    __shared__ int sp, free_cnt, free_list[64], scan_sh[MW];
+    __shared__ int sp, free_cnt, free_list[64];
+    __shared__ int2 scan_sh[2][MW];
     __shared__ P2Entry cur;
-    __shared__ unsigned long long job_sh, zidx_sh;
-    __shared__ int acc_n, new_n, anysplit, alloc_ok, have_sh, job_emits;
-    __shared__ double maxr_sh[MW], maxr3_sh[MW];
+    __shared__ unsigned long long job_sh, zidx_sh, max_sh[2];
+    __shared__ int alloc_ok, have_sh, job_emits;
+    __shared__ unsigned best_sh[2][MW];     // warps' largest r + s (float bits); any split: bit 31
     __shared__ long long arena_top;
     __shared__ int bh[MP_MAXNB];
-    __shared__ int bw[MW][MP_MAXNB];
+    AccBatch* batches = reinterpret_cast<AccBatch*>(mp_sh);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int blk = blockIdx.x;
     const int nb = P.nbins, M = P.maxn;
@@ -978,7 +983,7 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
             // After an error the results are discarded and the call is retried: stop early.
             // With the vertex-record buffer nearly full, stop taking jobs until it is drained.
             if (*(volatile int*)P.err ||
-                (long long)*(volatile unsigned long long*)P.zcount >= P.zstop)
+                zbuffer_full(P))
                 job_sh = (unsigned long long)P.njobs_val;
             else
                 job_sh = atomicAdd(P.job_next, 1ull);
@@ -1053,25 +1058,28 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
                 const double s1 = P.size[c1];
                 // oneBinLessThan of each list's previous maximum
                 const double thresh1_2 = (1. - P.binsize) * cur.maxr;
-                const double thresh1_3 = (1. - P.binsize) * cur.maxr3;
+                const double thresh1_3 = THREE ? (1. - P.binsize) * cur.maxr3 : 0.;
                 const int* list = (cur.goff >= 0) ? (arena1 + cur.goff) : nullptr;
                 const int* list2 = (cur.goff < 0) ? (arena + (-cur.goff - 1)) : nullptr;
                 const long long nbase = arena_top;
                 double* S = slot_ptr(P, blk, cur.slot);
-                if (tid == 0) { acc_n = 0; new_n = 0; anysplit = 0; }
+                if (tid < 2) max_sh[tid] = 0ull;
                 double mymax = 0., mymax3 = 0.;
-                float run32 = 0.f, run32_3 = 0.f;
-                int myany = 0;
-                const float4 c1a = __ldg(reinterpret_cast<const float4*>(P.tc + c1));
-                const float4 c1b = __ldg(reinterpret_cast<const float4*>(P.tc + c1) + 1);
+                float best = 0.f, best3 = 0.f;       // this thread's largest FP32 r + s, and its cell
+                int bestc = -1, best3c = -1;
+                int myany = 0, acc_n = 0, n_new = 0, parity = 0;
+                bool full = false;
+                const float4* c1t = reinterpret_cast<const float4*>(P.tc + c1);
+                const float4 c1a = __ldg(c1t), c1b = __ldg(c1t + 1);
+                const int left1 = __float_as_int(__ldg(c1t + 2).w);
                 const float s1f = c1a.w;
                 const float thresh1f_2 = (float)thresh1_2, thresh1f_3 = (float)thresh1_3;
-                __syncthreads();
-                for (int j0 = 0; j0 < cur.len; j0 += MB) {
+                const int len = cur.len;
+                for (int j0 = 0; j0 < len; j0 += MB) {
                     const int j = j0 + tid;
                     int cnt = 0, ca = -1, cb = -1, acc_ok = 0, kacc = -1;
                     double racc = 0., lracc = 0.;
-                    const int c2 = j < cur.len ? __ldcg(list ? list + j : list2 + j) : 0;
+                    const int c2 = j < len ? __ldcg(list ? list + j : list2 + j) : 0;
                     // A vertex-3 cell of a three-field cross: its own threshold, maximum and
                     // bins [nbd, 2 nbd).
                     const bool is3 = THREE && c2 >= P.base3;
@@ -1156,31 +1164,46 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
                         }
                     }
                     // The maximum of r + s over the unaccepted entries is kept exact (it sets
-                    // the next pass's thresholds): the warp's FP32 maximum is compared with its
-                    // running FP32 maximum, and the entries within the FP32 error of the larger
-                    // one get their FP64 value; all other entries are below an evaluated one.
-                    // (per list for a three-field cross)
-                    for (int li = 0; li < (THREE ? 2 : 1); ++li) {
-                        const float rsl = (li == 1) == is3 ? rs32 : 0.f;
-                        float& runl = li ? run32_3 : run32;
-                        float wm = rsl;
-                        for (int o = 16; o > 0; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-                        if (wm > runl * (1.f - 8e-6f)) {
-                            if (rsl > 0.f && rsl > wm * (1.f - 8e-6f)) {
-                                const double rs64 = sqrt(mp_dist_sq(P, c1, c2)) + (s1 + (double)ta.w);
-                                if (li) mymax3 = fmax(mymax3, rs64);
-                                else mymax = fmax(mymax, rs64);
-                            }
-                            runl = fmaxf(runl, wm);
+                    // the next pass's thresholds).  A thread keeps its largest FP32 value; of
+                    // two within the FP32 error of each other both get their FP64 value.  (FP64
+                    // instructions take 16 cycles of the SM each: they are for the few entries
+                    // that can be the maximum.)
+                    if (rs32 > 0.f) {
+                        float& bs = is3 ? best3 : best;
+                        int& bc = is3 ? best3c : bestc;
+                        if (rs32 > bs * (1.f + 1.6e-5f)) {
+                            bs = rs32;
+                            bc = c2;
+                        } else if (rs32 > bs * (1.f - 1.6e-5f)) {
+                            const double rs64 = sqrt(mp_dist_sq(P, c1, c2)) + (s1 + (double)ta.w);
+                            if (is3) mymax3 = fmax(mymax3, rs64);
+                            else mymax = fmax(mymax, rs64);
+                            bs = fmaxf(bs, rs32);
                         }
                     }
                     if (acc_ok && is3) kacc += P.nbd;
-                    int tot_new, tot_acc;
-                    int pos = block_excl_scan(cnt, scan_sh, tot_new);
-                    int apos = block_excl_scan(acc_ok, scan_sh, tot_acc);
-                    const long long wbase = nbase + new_n;
+                    // Places of the new entries and the accepted records (one barrier: the next
+                    // chunk writes the other buffer).
+                    const unsigned lt = (1u << lane) - 1u;
+                    const unsigned b1 = __ballot_sync(0xffffffffu, cnt >= 1);
+                    const unsigned b2 = __ballot_sync(0xffffffffu, cnt == 2);
+                    const unsigned ba = __ballot_sync(0xffffffffu, acc_ok);
+                    if (lane == 0) scan_sh[parity][wid] = make_int2(__popc(b1) + __popc(b2), __popc(ba));
+                    __syncthreads();
+                    int pos = __popc(b1 & lt) + __popc(b2 & lt), apos = __popc(ba & lt);
+                    int tot_new = 0, tot_acc = 0;
+#pragma unroll
+                    for (int w = 0; w < MW; ++w) {
+                        const int2 t = scan_sh[parity][w];
+                        if (w < wid) { pos += t.x; apos += t.y; }
+                        tot_new += t.x;
+                        tot_acc += t.y;
+                    }
+                    parity ^= 1;
+                    const long long wbase = nbase + n_new;
                     if (wbase + tot_new > P.arena2_cap || acc_n + tot_acc > P.acc_cap) {
                         if (tid == 0) set_mp_err(P.err, MP_ERR_ARENA);
+                        full = true;
                     } else {
                         if (cnt >= 1) arena[wbase + pos] = ca;
                         if (cnt == 2) arena[wbase + pos + 1] = cb;
@@ -1188,14 +1211,12 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
                             // calculateGn's per-pair terms in FP32: ExpIPhi z = d / r, the
                             // spin-2 factor e = conj(d^2) / |d|^2, the projected shear wg and
                             // the scalar sums.
-                            const float rr = r32 > 0.f ? r32 : 1.f;
-                            const float zr = dxf / rr, zi = dyf / rr;
-                            float nn2 = dxf * dxf + dyf * dyf;
-                            if (!(nn2 > 0.f)) nn2 = 1.f;
+                            const float inv = __frcp_rn(r32 > 0.f ? r32 : 1.f);
+                            const float zr = dxf * inv, zi = dyf * inv;
                             // (no rotation for the real payload of N / K pairs)
                             const bool rl = (P.pspin0 >> (is3 ? 1 : 0)) & 1;
-                            const float er = rl ? 1.f : (dxf * dxf - dyf * dyf) / nn2;
-                            const float ei = rl ? 0.f : -(2.f * dxf * dyf) / nn2;
+                            const float er = rl ? 1.f : zr * zr - zi * zi;
+                            const float ei = rl ? 0.f : -2.f * zr * zi;
                             const float w2 = tb.w;
                             const float4 lf = __ldg(P.lsf + ca);
                             const float l0 = lf.x, l1 = lf.y, l2 = lf.z, l3 = lf.w;
@@ -1246,56 +1267,77 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
                             atomicAdd(&bh[kacc], 1);
                         }
                     }
-                    __syncthreads();
-                    if (tid == 0) { new_n += tot_new; acc_n += tot_acc; }
-                    __syncthreads();
-                    if (acc_n > P.acc_cap - MB) {      // record buffer full: accumulate now
-                        mp_accumulate(P, acc, perm, acc_n, S, bh, bw);
-                        if (tid == 0) acc_n = 0;
+                    n_new += tot_new;
+                    acc_n += tot_acc;
+                    // (record buffer full, or the pass is over; the barrier also ends this
+                    // chunk's writes to the list)
+                    if (full) break;
+                    const bool last = j0 + MB >= len;
+                    if (last || acc_n > P.acc_cap - MB) {
                         __syncthreads();
+                        if (acc_n > 0) mp_accumulate(P, acc, perm, acc_n, S, bh, batches);
+                        acc_n = 0;
                     }
                 }
                 // An overflow of the arenas leaves the lists incomplete: stop this job (the
                 // call is retried with larger arenas).
-                if (tid == 0) alloc_ok = (*(volatile int*)P.err) ? 0 : 1;
-                __syncthreads();
-                if (!alloc_ok) break;
-                if (acc_n > 0) mp_accumulate(P, acc, perm, acc_n, S, bh, bw);
-                // Block max of the remaining separations and OR of anysplit1.
-                for (int o = 16; o > 0; o >>= 1) {
-                    mymax = fmax(mymax, __shfl_xor_sync(0xffffffffu, mymax, o));
-                    mymax3 = fmax(mymax3, __shfl_xor_sync(0xffffffffu, mymax3, o));
-                    myany |= __shfl_xor_sync(0xffffffffu, myany, o);
-                }
-                if (lane == 0) {
-                    maxr_sh[wid] = mymax; maxr3_sh[wid] = mymax3;
-                    if (myany) atomicOr(&anysplit, 1);
-                }
-                __syncthreads();
-                double maxrem2 = 0., maxrem3 = 0.;
-                for (int k = 0; k < MW; ++k) {
-                    maxrem2 = fmax(maxrem2, maxr_sh[k]);
-                    maxrem3 = fmax(maxrem3, maxr3_sh[k]);
-                }
-                const double maxrem = fmax(maxrem2, maxrem3);
-                const int n_new = new_n;
+                if (full) break;
                 int mink = cur.mink;
                 if (n_new == 0) {
                     zeta_emit(P, c1, S, 0, mink, out, diag, shG, shW, &zidx_sh, &job_emits);
                     break;
                 }
+                // The largest remaining separations: the threads whose FP32 value can be the
+                // block's maximum take it in FP64.
+                {
+                    const unsigned any = __any_sync(0xffffffffu, myany) ? 0x80000000u : 0u;
+                    const unsigned m2 = __reduce_max_sync(0xffffffffu, __float_as_uint(best));
+                    const unsigned m3 = THREE ? __reduce_max_sync(0xffffffffu, __float_as_uint(best3)) : 0u;
+                    if (lane == 0) { best_sh[0][wid] = m2 | any; best_sh[1][wid] = m3; }
+                }
+                __syncthreads();
+                bool anysplit = false;
+                {
+                    unsigned bm2 = 0u, bm3 = 0u;
+#pragma unroll
+                    for (int w = 0; w < MW; ++w) {
+                        const unsigned v = best_sh[0][w];
+                        anysplit = anysplit || (v >> 31);
+                        bm2 = max(bm2, v & 0x7fffffffu);
+                        if (THREE) bm3 = max(bm3, best_sh[1][w]);
+                    }
+                    if (best > 0.f && best >= __uint_as_float(bm2) * (1.f - 8e-6f))
+                        mymax = fmax(mymax, sqrt(mp_dist_sq(P, c1, bestc)) + (s1 + (double)P.size[bestc]));
+                    if (mymax > 0.) atomicMax(&max_sh[0], (unsigned long long)__double_as_longlong(mymax));
+                    if (THREE) {
+                        if (best3 > 0.f && best3 >= __uint_as_float(bm3) * (1.f - 8e-6f))
+                            mymax3 = fmax(mymax3, sqrt(mp_dist_sq(P, c1, best3c)) + (s1 + (double)P.size[best3c]));
+                        if (mymax3 > 0.) atomicMax(&max_sh[1], (unsigned long long)__double_as_longlong(mymax3));
+                    }
+                }
+                __syncthreads();
+                const double maxrem2 = __longlong_as_double((long long)max_sh[0]);
+                const double maxrem3 = THREE ? __longlong_as_double((long long)max_sh[1]) : 0.;
+                const double maxrem = THREE ? fmax(maxrem2, maxrem3) : maxrem2;
                 if (maxrem < P.maxsep) {
                     int k = 0;
-                    if (lane == 0 && !(maxrem < P.minsep))
-                        k = int((log(maxrem) - P.logminsep) / P.binsize) + 1;
-                    k = __shfl_sync(0xffffffffu, k, 0);
+                    if (!(maxrem < P.minsep)) {
+                        // int((log(maxrem) - logminsep) / binsize) + 1, in FP64 only near an
+                        // integer (FP32: 3e-7 of |log| + |logminsep|, over binsize).
+                        const float lr = logf((float)maxrem);
+                        const float kk = (lr - P.f_logminsep) / P.f_binsize;
+                        const float err = 1e-5f * (1.f + fabsf(kk)) +
+                                          1e-6f * (1.f + fabsf(lr) + fabsf(P.f_logminsep)) / P.f_binsize;
+                        const float frac = kk - floorf(kk);
+                        if (frac > err && frac < 1.f - err) k = (int)kk + 1;
+                        else k = int((log(maxrem) - P.logminsep) / P.binsize) + 1;
+                    }
                     if (k < mink) {
                         zeta_emit(P, c1, S, k, mink, out, diag, shG, shW, &zidx_sh, &job_emits);
                         mink = k;
                     }
                 }
-                const bool split1 = anysplit && P.left[c1] >= 0;
-                __syncthreads();
+                const bool split1 = anysplit && left1 >= 0;
                 if (tid == 0) {
                     arena_top = nbase + n_new;
                     alloc_ok = 1;
@@ -1317,11 +1359,17 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
                 if (!alloc_ok) break;
                 if (split1) {
                     // The right child gets a copy of the scratch (mp.duplicate()).
-                    const double* src = S;
-                    double* dst = slot_ptr(P, blk, stk[sp - 1].slot);
-                    for (int q = tid; q < P.slot_doubles; q += MB) dst[q] = __ldcg(src + q);
+                    const double2* src = reinterpret_cast<const double2*>(S);
+                    double2* dst = reinterpret_cast<double2*>(slot_ptr(P, blk, stk[sp - 1].slot));
+                    const int half = (int)(P.slot_doubles / 2);
+                    for (int q0 = tid; q0 < half; q0 += 8 * MB) {
+                        double2 v[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) if (q0 + u * MB < half) v[u] = __ldcg(src + q0 + u * MB);
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) if (q0 + u * MB < half) dst[q0 + u * MB] = v[u];
+                    }
                 }
-                __syncthreads();
                 // Without a split, the old list is dead unless a pushed entry still uses it:
                 // move the new list down onto it, so a chain of passes reuses one region.
                 long long newoff = nbase;
@@ -1341,7 +1389,7 @@ __global__ void __launch_bounds__(MB, 2) k_mp_finish(MPParams P)
                 }
                 __syncthreads();
                 if (tid == 0) {
-                    if (split1) cur.c1 = P.left[c1];
+                    if (split1) cur.c1 = left1;
                     cur.len = n_new;
                     cur.goff = -newoff - 1;
                     cur.mink = mink;
@@ -1375,7 +1423,7 @@ __global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, int chunk, double* s
 {
     extern __shared__ float4 zsh[];    // [chunk][nb][2]
     __shared__ int4 hdr_sh[64];
-    const int nb = Q.nbins, M = Q.maxn, gst = 2 * M + 3;
+    const int nb = Q.nbins;
     const int nb2 = nb * nb;
     const int g = blockIdx.x, tid = threadIdx.x;
     int ea[ZE], eb[ZE], em[ZE];     // entry (a, b) and min(a, b) mod nbd (the row mask)
@@ -1398,8 +1446,13 @@ __global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, int chunk, double* s
         __syncthreads();
         for (int idx = tid; idx < nv * nb; idx += ZB) {
             const int v = idx / nb, a = idx % nb;
-            const float* R = Q.rec + (size_t)(c0 + v) * Q.rec_floats;
-            const float* RS = R + 8 + 2 * (size_t)gst * nb + 2 * (size_t)(M + 1) * nb;
+            const unsigned off = Q.off[c0 + v];
+            if (off == ZOFF_NONE) {      // contracted in place
+                if (a == 0) hdr_sh[v] = make_int4(0, 0, 0, 0);
+                continue;
+            }
+            const float* R = Q.rec + 4 * (size_t)off;
+            const float* RS = R + 8;
             float4* d = zsh + ((size_t)v * nb + a) * 2;
             d[0] = make_float4(RS[a], RS[nb + a], RS[2 * nb + a], RS[3 * nb + a]);
             d[1] = make_float4(RS[4 * nb + a], RS[5 * nb + a], 0.f, 0.f);
@@ -1502,10 +1555,11 @@ __global__ void k_mp_reduce(int nblk, long long stride, long long Z, int nb, int
 // Host orchestration.
 
 size_t mp_slot_doubles(int nb, int M)
-{ return 2 * (size_t)nb * (M + 1) + 2 * (size_t)nb * (2 * M + 3) + 13 * (size_t)nb; }
+{ return (2 * (size_t)nb * (M + 1) + 2 * (size_t)nb * (2 * M + 3) + 13 * (size_t)nb + 1) & ~(size_t)1; }
 
-static int mp_rec_floats(int nb, int M)
-{ return (8 + 2 * nb * (2 * M + 3) + 2 * nb * (M + 1) + 6 * nb + 3) & ~3; }
+// 16-byte units of a vertex record of all bins
+static long long mp_rec_units(int nb, int M)
+{ return (8 + 2 * (long long)nb * (2 * M + 3) + 2 * nb * (M + 1) + 6 * nb + 3) / 4; }
 
 int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* h_out)
 {
@@ -1514,8 +1568,9 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
     int dev = 0, nsm = 0;
     TC_CU(cudaGetDevice(&dev));
     TC_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const size_t shbytes = sizeof(double) * (2 * (size_t)nb * (2 * M + 3) + 2 * (size_t)nb * (M + 1));
-    if (shbytes > 160 * 1024 || M + 1 > 64 || nb > MP_MAXNB) {
+    const size_t inplace = sizeof(double) * (2 * (size_t)nb * (2 * M + 3) + 2 * (size_t)nb * (M + 1));
+    const size_t shbytes = std::max(inplace, sizeof(AccBatch) * MW);
+    if (inplace > 160 * 1024 || M + 1 > 64 || nb > MP_MAXNB) {
         set_last_error("the GPU multipole path needs max_n <= 63, nbins <= 128 and "
                        "nbins * max_n within its shared-memory staging");
         return 3;
@@ -1525,7 +1580,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
     int per = 0;
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfin, MB, shbytes));
     if (per < 1) per = 1;
-    const int nblk = nsm * std::min(per, 2);
+    const int nblk = nsm * std::min(per, MBLK);
     P.slot_doubles = (long long)mp_slot_doubles(nb, M);
     P.out_stride = 15 * Z;
     const int etiles = (nb * nb + ZE * ZB - 1) / (ZE * ZB);
@@ -1535,7 +1590,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
     // (with its static header array this can pass the 48 KB that needs no opt-in)
     TC_CU(cudaFuncSetAttribute(k_mp_zscal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsh2));
     const int nsg = std::max(1, 2 * nsm / etiles);
-    const int recf = mp_rec_floats(nb, M);
+    const long long recu = mp_rec_units(nb, M);
     const long long acc_cap = 4096;
     X.want_a1 = std::max<long long>(X.want_a1, 4LL * std::max(ntop, P.ntop2) + (1 << 16));
     X.want_jobs = std::max<long long>(X.want_jobs, 1 << 18);
@@ -1584,21 +1639,29 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             X.out_stride = P.out_stride; X.diag_stride = 9LL * nb;
         }
         {
-            // The vertex-record buffer: up to 16 GiB and a quarter of the free memory, or the
-            // byte count in TCGPU_MP_RECORD_BYTES (at least 16 records).
-            size_t budget = (size_t)16 << 30;
+            // The vertex-record buffer: up to 32 GiB and a quarter of the free memory, or the
+            // byte count in TCGPU_MP_RECORD_BYTES (at least 16 records of all bins).  With one
+            // buffer for all records there is one wave: each wave ends with the blocks' last
+            // jobs (10 ms of 240 at 500,000 points, 17 GB of records).  A cell leaves three
+            // records or so, and the stop margin below is for the blocks' jobs in flight.
+            size_t budget = (size_t)32 << 30;
             if (const char* ev = std::getenv("TCGPU_MP_RECORD_BYTES"))
-                budget = (size_t)std::max(0LL, std::atoll(ev));
-            const long long cap = std::max<long long>(16, (long long)(budget / (4ULL * recf)));
-            if (!X.zrec || X.zrec_floats != recf || X.zcap != cap) {
-                dfree(X.zrec);
+                budget = std::min<size_t>((size_t)48 << 30, (size_t)std::max(0LL, std::atoll(ev)));   // (32-bit offsets)
+            const long long want = (16LL * P.ncells + (1 << 19)) * recu;
+            const long long cap = std::max<long long>(16 * recu, std::min<long long>((long long)(budget / 16), want));
+            if (!X.zrec || X.zrec_units != recu || X.zcap < cap || (X.zcap > cap && cap < want)) {
+                dfree(X.zrec); dfree(X.zoff); dfree(X.order);
                 X.zcap = 0;
                 size_t fr = 0, tot = 0;
                 TC_CU(cudaMemGetInfo(&fr, &tot));
-                const long long fit = std::max<long long>(16, (long long)(fr / 4 / (4ULL * recf)));
-                const long long c2 = std::min(cap, fit);
-                TC_TRY(dalloc(&X.zrec, (size_t)c2 * recf));
-                X.zcap = c2; X.zrec_floats = recf;
+                X.zcap = 0;
+                const long long c2 = std::min(cap, std::max<long long>(16 * recu, (long long)(fr / 4 / 16)));
+                // (records hold the bins from ks on: room for numbers of half the size)
+                X.zmax = 2 * c2 / recu + 16;
+                TC_TRY(dalloc(&X.zrec, 4 * (size_t)c2));
+                TC_TRY(dalloc(&X.zoff, (size_t)X.zmax));
+                TC_TRY(dalloc(&X.order, (size_t)X.zmax));
+                X.zcap = c2; X.zrec_units = recu;
             }
         }
         if (X.nsg < nsg || X.spart_nb2 < (long long)nb * nb) {
@@ -1615,14 +1678,13 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             TC_TRY(dalloc(&X.part, npart));
             X.npart = npart;
         }
-        const long long nkey = (long long)P.nbd * (P.nbd + 1), nsegs = zeta_segments(X.zcap, P.nbd);
-        if (X.order_cap < X.zcap || X.nkey < nkey || X.nsegs < nsegs) {
-            dfree(X.order); dfree(X.keys); dfree(X.segs);
-            X.order_cap = 0; X.nkey = 0; X.nsegs = 0;
-            TC_TRY(dalloc(&X.order, (size_t)X.zcap));
-            TC_TRY(dalloc(&X.keys, 2 * (size_t)nkey + 1));
+        const long long nkey = (long long)P.nbd * (P.nbd + 1), nsegs = zeta_segments(X.zmax, P.nbd);
+        if (X.nkey < nkey || X.nsegs < nsegs) {
+            dfree(X.keys); dfree(X.segs);
+            X.nkey = 0; X.nsegs = 0;
+            TC_TRY(dalloc(&X.keys, 2 * (size_t)nkey + 2));
             TC_TRY(dalloc(&X.segs, (size_t)nsegs));
-            X.order_cap = X.zcap; X.nkey = nkey; X.nsegs = nsegs;
+            X.nkey = nkey; X.nsegs = nsegs;
         }
         if (!X.ctl) TC_TRY(dalloc(&X.ctl, 4));
         if (!X.err) TC_TRY(dalloc(&X.err, 2));
@@ -1636,12 +1698,13 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
         P.slots = X.slots; P.nslots = X.nslots;
         P.out = X.out;
         P.diag = X.diag;
-        P.zrec = X.zrec; P.zcap = X.zcap; P.zrec_floats = recf;
-        // Jobs are not started once the buffer holds zstop records; the blocks' jobs in
-        // flight then fill at most nblk x (the largest job so far) more.
+        P.zrec = X.zrec; P.zcap = X.zcap; P.zoff = X.zoff; P.zmax = X.zmax;
+        // Jobs are not started once the buffer is nearly full; the blocks' jobs in flight then
+        // add at most nblk x (the largest job so far) records.
         auto set_zstop = [&](long long maxjob) {
             const long long margin = (long long)nblk * std::max<long long>(64, 2 * maxjob);
-            P.zstop = std::max<long long>(X.zcap / 4, X.zcap - margin);
+            P.zstop = std::max<long long>(X.zcap / 4, X.zcap - margin * recu);
+            P.zmaxstop = std::max<long long>(X.zmax / 4, X.zmax - margin);
         };
         set_zstop(512);
         P.err = X.err;
@@ -1676,10 +1739,11 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             TC_CU(cudaStreamSynchronize(st));
             if (e) break;
             ZParams Q;
-            Q.rec = X.zrec; Q.nrec = std::min<long long>((long long)c[2], X.zcap);
-            Q.rec_floats = recf; Q.nbins = nb; Q.maxn = M;
+            const long long emitted = (long long)(c[2] / ZC_ONE);
+            Q.rec = X.zrec; Q.off = X.zoff; Q.nrec = std::min<long long>(emitted, X.zmax);
+            Q.nbins = nb; Q.maxn = M;
             Q.part = X.part; Q.order = X.order; Q.segs = X.segs;
-            Q.count = X.keys; Q.first = X.keys + X.nkey; Q.nseg = X.keys + 2 * X.nkey;
+            Q.count = X.keys; Q.first = X.keys + X.nkey; Q.nseg = X.keys + 2 * X.nkey + 1;
             Q.shift = P.vreal ? 0 : 1;
             Q.nbd = P.nbd; Q.typo32 = P.typo32;
             if (Q.nrec > 0) {
@@ -1690,8 +1754,12 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
                     TC_CU(cudaGetLastError());
                 }
             }
-            X.overflow += std::max<long long>(0, (long long)c[2] - X.zcap);
-            X.records += (long long)c[2];
+            // (contracted in place: those without a number, and those whose units did not fit)
+            int placed = 0;
+            TC_CU(cudaMemcpyAsync(&placed, Q.first + nkey, sizeof(int), cudaMemcpyDeviceToHost, st));
+            TC_CU(cudaStreamSynchronize(st));
+            X.overflow += emitted - (Q.nrec > 0 ? placed : 0);
+            X.records += emitted;
             ++X.waves;
             set_zstop((long long)c[3]);
             if ((long long)c[1] >= P.njobs_val) break;
@@ -1742,7 +1810,7 @@ void free_mp_scratch(MPScratch& X)
     dfree(X.slots); dfree(X.out); dfree(X.diag); dfree(X.total); dfree(X.zrec); dfree(X.part);
     dfree(X.spart); dfree(X.ntp);
     dfree(X.ctl); dfree(X.err); dfree(X.dbg);
-    dfree(X.order); dfree(X.keys); dfree(X.segs);
+    dfree(X.order); dfree(X.keys); dfree(X.segs); dfree(X.zoff);
     X = MPScratch();
 }
 

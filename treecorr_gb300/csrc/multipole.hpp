@@ -21,6 +21,9 @@ enum MPErr : int {
     MP_ERR_CHECK = 15,   // a consistency check failed (err[1] names the site)
 };
 
+constexpr unsigned long long ZC_ONE = 1ull << 36;
+constexpr unsigned ZOFF_NONE = 0xffffffffu;
+
 struct MPParams {
     int coords, metric, quick, nbins, maxn;
     // 0: a spin-2 vertex (GGG: G_n up to n = max_n + 1, self-pair sums with z^2); 1: an N or
@@ -72,11 +75,13 @@ struct MPParams {
     double* out;         // per block: 15 arrays of nbins^2 (2 maxn + 1) doubles
     long long out_stride;
     double* diag;        // per block: 9 x nbins self-pair corrections of the diagonal k2 == k3
-    // Vertex records for the batched contraction: zcount counts them; records at index
-    // >= zcap are contracted in place instead; jobs are not started once zcount >= zstop.
+    // Vertex records for the batched contraction, one after another: zcount holds their number
+    // (times ZC_ONE) and the units of 16 bytes they take; zoff[i] is where record i begins.
+    // Records beyond zmax in number or zcap units are contracted in place instead (ZOFF_NONE);
+    // jobs are not started once zcount is at zstop units or zmaxstop records.
     float* zrec;
-    long long zcap, zstop;
-    int zrec_floats;
+    unsigned* zoff;
+    long long zcap, zstop, zmax, zmaxstop;
     unsigned long long* zcount;
     unsigned long long* zmaxjob;   // largest number of records of one job
     int* err;
@@ -104,14 +109,14 @@ struct MPScratch {
     long long out_stride = 0;
     long long diag_stride = 0;
     float* zrec = nullptr;
-    long long zcap = 0;
-    int zrec_floats = 0;
+    unsigned* zoff = nullptr;
+    long long zcap = 0, zmax = 0, zrec_units = 0;
     double* part = nullptr;     // the contraction's sums (zeta.cu)
     size_t npart = 0;
-    int* order = nullptr;       // the records by row range, the ranges' counts and segments
+    unsigned* order = nullptr;  // the records by row range, the ranges' counts and segments
     int* keys = nullptr;
     int4* segs = nullptr;
-    long long order_cap = 0, nkey = 0, nsegs = 0;
+    long long nkey = 0, nsegs = 0;
     double* spart = nullptr;    // per scalar group: 4 arrays of nbins^2 (meand2/3, meanlogd2/3)
     unsigned long long* ntp = nullptr;   // per scalar group: nbins^2 triangle counts
     long long spart_nb2 = 0;
@@ -130,14 +135,16 @@ struct MPScratch {
 // The contraction over vertex records (zeta.cu) and the scalar sums over them.
 struct ZParams {
     const float* rec;
+    const unsigned* off;   // where record i begins, in units of 16 bytes (ZOFF_NONE: no record)
     long long nrec;
-    int rec_floats, nbins, maxn;
+    int nbins, maxn;
     int shift;             // 1: G_n at n -+ 1 (a spin-2 vertex); 0: at n (an N or K vertex)
     int nbd;               // distance bins; a record's rows [ks, mk) hold min(a, b) mod nbd
     int typo32;            // see MPParams::typo32
     double* part;          // [n >= 0][10][entry of a 4 x 2 tile][tile]
-    int* order;            // record numbers by row range
-    int* count;            // per row range ks (nbd + 1) + mk: records, first place in order
+    unsigned* order;       // the records' offsets by row range
+    int* count;            // per row range ks (nbd + 1) + mk: records, first place in order (and
+                           // the number of records)
     int* first;
     int4* segs;            // (first place, records, ks, mk)
     int* nseg;

@@ -12,7 +12,7 @@
 //
 //   * Only n >= 0 is contracted: exchanging the factors, gam0, gam1 and weight of (a, b, -n) are
 //     those of (b, a, n), and gam2 of (a, b, -n) is gam3 of (b, a, n) (k_mp_reduce reads them so).
-//   * The records are put in the order of their row ranges (a counting sort of their numbers)
+//   * The records are put in the order of their row ranges (a counting sort of their offsets)
 //     and cut into segments of one range each.  Within a segment the set of entries is fixed:
 //     its 4 x 2 tiles are dealt out to the threads, the sums run over the records without any
 //     test, and the range is applied when they are added up.  At 20 bins and 500,000 points a
@@ -23,8 +23,8 @@
 //     the chunk before is contracted from shared memory.
 //
 // Bounds: 98e9 FP32 multiply-adds of needed entries (131e9 with the tiles' edges, 3.5 ms at the
-// FMA rate) and 24 GB of records (3.6 ms of measured copy bandwidth) at 500,000 points, 20 bins,
-// max_n 30; measured 21.2 ms for the contraction and 0.4 ms for the ordering.  Before, a tcgen05
+// FMA rate) and 17 GB of records (2.5 ms of measured copy bandwidth) at 500,000 points, 20 bins,
+// max_n 30; measured 19.8 ms for the contraction and 0.4 ms for the ordering.  Before, a tcgen05
 // kernel took 172 ms: it did every record's full matrix for all n of both signs, twice (the row
 // range as a difference of two), on 3 x TF32 operands whose staging (shared-memory stores)
 // bound it, and its TMEM sums were the least precise of the path: the error of the whole
@@ -46,27 +46,29 @@ constexpr int ZIT = 2;              // (record, bin) items a thread loads per ch
 constexpr int ZPAD = 4;             // bins a ragged tile may read past the last record
 constexpr int SEG_MIN = 256, SEG_MAX = 4096;
 
-__device__ __forceinline__ int record_key(const ZParams& Q, long long i)
+__device__ __forceinline__ int record_key(const ZParams& Q, unsigned off)
 {
-    const float* R = Q.rec + (size_t)i * Q.rec_floats;
+    if (off == ZOFF_NONE) return -1;
+    const float* R = Q.rec + 4 * (size_t)off;
     return __float_as_int(R[1]) * (Q.nbd + 1) + __float_as_int(R[2]);
 }
 
-// Row range counts, then (scatter) the records' numbers in the order of their ranges.
+// Row range counts, then (scatter) the records' offsets in the order of their ranges.
 __global__ void __launch_bounds__(256) k_zrows(ZParams Q, bool scatter)
 {
     const int lane = threadIdx.x & 31;
     for (long long i0 = (long long)blockIdx.x * 256 + threadIdx.x - lane; i0 < Q.nrec;
          i0 += (long long)gridDim.x * 256) {
         const long long i = i0 + lane;
-        const int key = i < Q.nrec ? record_key(Q, i) : -1;
+        const unsigned off = i < Q.nrec ? Q.off[i] : ZOFF_NONE;
+        const int key = record_key(Q, off);
         const unsigned peers = __match_any_sync(0xffffffffu, key);
         const int leader = __ffs(peers) - 1;
         int base = 0;
         if (lane == leader && key >= 0)
             base = atomicAdd((scatter ? Q.first : Q.count) + key, __popc(peers));
         base = __shfl_sync(0xffffffffu, base, leader);
-        if (scatter && key >= 0) Q.order[base + __popc(peers & ((1u << lane) - 1u))] = (int)i;
+        if (scatter && key >= 0) Q.order[base + __popc(peers & ((1u << lane) - 1u))] = off;
     }
 }
 
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(1024) k_zrows_segments(ZParams Q)
         rec0 = tot[0];
         seg0 = tot[1];
     }
-    if (tid == 0) *Q.nseg = seg0;
+    if (tid == 0) { *Q.nseg = seg0; Q.first[nkey] = rec0; }
 }
 
 __global__ void __launch_bounds__(ZT, 2) k_mp_zeta(ZParams Q)
@@ -128,6 +130,7 @@ __global__ void __launch_bounds__(ZT, 2) k_mp_zeta(ZParams Q)
         const int n = rest / ntc, tc = rest - n * ntc;
         const int4 sg = Q.segs[seg];
         const int ks = sg.z, mk = sg.w;
+        const int col0 = nbd == nb ? ks : 0, ncol = nb - col0;      // the record's columns
         // The segment's tiles (those with an entry in the row range), ZT of them from ZT tc.
         int nvalid = 0;
         __syncthreads();
@@ -176,14 +179,14 @@ __global__ void __launch_bounds__(ZT, 2) k_mp_zeta(ZParams Q)
                 const int v = idx / nb, a = idx - v * nb;
                 on[j] = v < chunk && c0 + v < sg.y && (a >= nbd ? a - nbd : a) >= ks;
                 if (!on[j]) continue;
-                const float* R = Q.rec + (size_t)Q.order[sg.x + c0 + v] * Q.rec_floats;
-                const float2* RG = reinterpret_cast<const float2*>(R + 8) + a;
+                const float* R = Q.rec + 4 * (size_t)Q.order[sg.x + c0 + v];
+                const float2* RG = reinterpret_cast<const float2*>(R + 8 + 6 * nb) + a - col0;
                 w1[j] = R[3]; wr[j] = R[4]; wi[j] = R[5];
-                g[j][0] = RG[(n - sh + M + 1) * nb];        // G[n-1]
-                g[j][1] = RG[(-n - sh + M + 1) * nb];       // G[-n-1]
-                g[j][2] = RG[(n + sh + M + 1) * nb];        // G[n+1]
-                g[j][3] = RG[(-n + sh + M + 1) * nb];       // G[-n+1]
-                g[j][4] = RG[(gst + n) * nb];               // W[n]
+                g[j][0] = RG[(n - sh + M + 1) * ncol];      // G[n-1]
+                g[j][1] = RG[(-n - sh + M + 1) * ncol];     // G[-n-1]
+                g[j][2] = RG[(n + sh + M + 1) * ncol];      // G[n+1]
+                g[j][3] = RG[(-n + sh + M + 1) * ncol];     // G[-n+1]
+                g[j][4] = RG[(gst + n) * ncol];             // W[n]
             }
         };
         auto store = [&](float4* T) {
