@@ -6,15 +6,17 @@
 // alternate form first measures each patch's inertia (CalculateInertia, 387-463) and adds it
 // as a penalty to the distances.
 //
-// GPU form.  FindCellsInPatches is a breadth-first pass over the tree: a work item is
+// GPU form.  FindCellsInPatches starts as a breadth-first pass over the tree: a work item is
 // (cell, candidate list); one warp evaluates the cell against its candidates, prunes those
 // that cannot hold any of its points, and either assigns the cell (one candidate left, or a
 // cell of size 0) or hands the survivors to both children.  Children share the list, and a
-// list that lost no candidate is not copied.  The per-patch sums then run over the cells in
-// id order with per-warp accumulators in shared memory, block partials and a fixed-order
-// final sum, so the result does not depend on scheduling.  All distances are FP64 with the
-// reference's association and no contraction, so candidate decisions and nearest-centre
-// choices are the reference's; sums differ from its OpenMP order only by rounding.
+// list that lost no candidate is not copied.  After some levels the lists are short, and one
+// kernel walks the rest of the tree (k_km_walk).  The per-patch sums then run over the cells
+// in id order with per-warp accumulators in shared memory, block partials and a fixed-order
+// final sum, so the result does not depend on scheduling.  Distances are FP32 of float pairs
+// where that decides, else FP64 with the reference's association and no contraction, so
+// candidate decisions and nearest-centre choices are the reference's; sums differ from its
+// OpenMP order only by rounding.
 //
 // The initialisations (KMeansInitTree / Rand / KMPP) draw from the C library's rand()
 // stream exactly as the reference's urand() does, walking the few cells they visit from
@@ -37,11 +39,14 @@ namespace tc {
 
 namespace {
 
-constexpr int KM_NQ = 5;            // per-patch sums: centres w x, w y, w z, w; inertia I, I_size, w
+constexpr int KM_NQ = 4;            // per-patch sums: centres w x, w y, w z, w; inertia I, I_size, w
 constexpr int KM_MAX_PATCH = 5000;  // per-warp shared accumulators must fit one warp at least
-constexpr int KM_NBLK = 1216;       // accumulation blocks (fixed: the sum order depends on it)
+constexpr int KM_NBLK = 304;        // accumulation blocks (fixed: the sum order depends on it)
 constexpr int KM_LTB = 256;         // threads per block of the level kernel
 constexpr int KM_LEVELS_PER_CHECK = 16;
+// Subtrees the walk should have: below, more levels are taken first (9 us each).  2,000,000 points,
+// 64 patches, 200 iterations: 37.0 ms at 512, 39.4 at 256, 37.6 at 1024.
+constexpr long long KM_UNITS = 512;
 // assign[cell] = tag * KM_TAG + patch for the cells assigned by the pass with that tag, so the
 // array needs no clearing between passes (npatch <= KM_MAX_PATCH < KM_TAG).
 constexpr int KM_TAG = 8192;
@@ -61,6 +66,18 @@ struct KMLevel {
     int err;                 // 1: candidate pool full, 2: item array full
     int leaf_multi;          // leaves reached with more than one candidate
     int levels;              // levels that held items
+    int wide;                // items of the current level with long candidate lists
+    int wide_next;           // .. of the next level
+    long long units;         // items the walk started from
+};
+
+// The iterations' control: kernels of a stopped run return at once, so that several iterations
+// can be in the queue before the host looks.
+enum { KM_RUN = 0, KM_CONVERGED = 1, KM_ERR_POOL = 2, KM_ERR_WIDE = 3, KM_ERR_STACK = 4, KM_ERR_ITEMS = 5 };
+struct KMCtl {
+    int stop;
+    int iters;               // iterations run
+    unsigned total_done;     // blocks of k_km_total
 };
 
 __device__ __forceinline__ int km_patch_of(int v, int tag)
@@ -92,65 +109,144 @@ __device__ __forceinline__ bool km_keep(double d, double s, double thresh, const
     return !(d > thresh);
 }
 
+// A candidate list of at most KM_SMALL entries is handled by one thread; longer lists (the
+// top levels) by a whole warp.
+constexpr int KM_SMALL = 16;
+
 __global__ void k_km_start(const int* tops, int ntop, int npatch, KMItem* items, int* pool,
-                           KMLevel* L)
+                           KMLevel* L, const KMCtl* ctl, const double* cen, float4* cen32)
 {
+    if (ctl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < npatch) {                    // the centres as FP32 pairs
+        const double x = cen[3 * i], y = cen[3 * i + 1], z = cen[3 * i + 2];
+        const float hx = (float)x, hy = (float)y, hz = (float)z;
+        cen32[2 * i] = make_float4(hx, hy, hz, fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))));
+        cen32[2 * i + 1] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.f);
+    }
     if (i < ntop) items[i] = KMItem{tops[i], npatch, 0};
     if (i < npatch) pool[i] = i;
     if (i == 0) {
         L->lo = 0; L->hi = ntop; L->total = ntop; L->pool_top = npatch;
         L->blocks_done = 0; L->err = 0; L->leaf_multi = 0; L->levels = 0;
+        L->wide = npatch > KM_SMALL; L->wide_next = 0; L->units = 0;
     }
 }
 
-// A candidate list of at most KM_SMALL entries is handled by one thread; longer lists (the
-// top levels) by a whole warp.
-constexpr int KM_SMALL = 16;
+// The distance squared of a cell and a centre in FP32 from pairs of floats: within 1e-6 of itself
+// where it is beyond 1e-6 of the coordinates (the low parts are good to 4e-15 of them).  A
+// decision within 1e-5 of its limit is left to FP64 (km_close), whose instructions take 16
+// cycles of the SM each.
+struct KMPos {
+    float hx, hy, hz, lx, ly, lz, amax;
+};
+__device__ __forceinline__ KMPos km_pos(double x, double y, double z)
+{
+    KMPos p;
+    p.hx = (float)x; p.hy = (float)y; p.hz = (float)z;
+    p.lx = (float)(x - p.hx); p.ly = (float)(y - p.hy); p.lz = (float)(z - p.hz);
+    p.amax = fmaxf(fabsf(p.hx), fmaxf(fabsf(p.hy), fabsf(p.hz)));
+    return p;
+}
+__device__ __forceinline__ float km_dsq32(const KMPos& a, const float4* cen32, int p, float& far)
+{
+    const float4 h = cen32[2 * p], l = cen32[2 * p + 1];
+    const float dx = (a.hx - h.x) + (a.lx - l.x), dy = (a.hy - h.y) + (a.ly - l.y);
+    const float dz = (a.hz - h.z) + (a.lz - l.z);
+    far = fmaxf(far, h.w);
+    return dx * dx + dy * dy + dz * dz;
+}
+__device__ __forceinline__ bool km_plain(float best, float thresh, float far)
+{ return best > 1e-12f * far * far && best > 1e-30f && thresh < 1e30f; }
+// d is too near the smallest distance or the limit for FP32.
+__device__ __forceinline__ bool km_close(float d, float best, float thresh)
+{ return !(d > best * (1.f + 1e-5f) && fabsf(d - thresh) > 1e-5f * thresh); }
+
+// The closest candidate's place, and how many others can hold points of the cell, in FP32;
+// false: left to FP64.
+__device__ __forceinline__ bool km_item_warp32(const int* lst, int m, int lane, const KMPos& a, float s,
+                                               const float4* cen32, int& bpos, int& nkeep, float& thresh)
+{
+    float best = 0.f, far = a.amax;
+    bpos = INT_MAX;
+    for (int j = lane; j < m; j += 32) {
+        const float d = km_dsq32(a, cen32, lst[j], far);
+        if (bpos == INT_MAX || d < best) { best = d; bpos = j; }
+    }
+    unsigned key = bpos == INT_MAX ? 0xffffffffu : __float_as_uint(best);
+    const unsigned mn = __reduce_min_sync(0xffffffffu, key);
+    bpos = __reduce_min_sync(0xffffffffu, key == mn ? (unsigned)bpos : 0xffffffffu);
+    best = __uint_as_float(mn);
+    far = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(far)));
+    const float t = sqrtf(best) + 2.f * s;
+    thresh = t * t;
+    bool sure = km_plain(best, thresh, far);
+    nkeep = 0;
+    for (int j0 = 0; j0 < m; j0 += 32) {
+        const int j = j0 + lane;
+        bool keep = false;
+        if (j < m && j != bpos) {
+            const float d = km_dsq32(a, cen32, lst[j], far);
+            sure = sure && !km_close(d, best, thresh);
+            keep = !(d > thresh);
+        }
+        nkeep += __popc(__ballot_sync(0xffffffffu, keep));
+    }
+    return __all_sync(0xffffffffu, sure);
+}
 
 // The whole-warp form for one item with a long candidate list.
-__device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* cen,
+__device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* cen, const float4* cen32,
                              const double* inertia, KMItem* items, long long item_cap, int* pool,
                              long long pool_cap, int* assign, int tag, KMLevel* L)
 {
     const int c = it.cell, m = it.len;
     const int* lst = pool + it.off;
     const double px = C.x[c], py = C.y[c], pz = C.z[c];
-    const double s = (double)C.size[c];
-    // The closest centre by the (penalised) distance: the first minimum in list order.
-    double bmod = 0., bdsq = 0.;
-    int bpos = INT_MAX;
-    for (int j = lane; j < m; j += 32) {
-        const int p = lst[j];
-        const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
-        const double mod = inertia ? __dadd_rn(d, inertia[p]) : d;
-        if (bpos == INT_MAX || mod < bmod) { bmod = mod; bdsq = d; bpos = j; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double om = __shfl_xor_sync(0xffffffffu, bmod, o);
-        const double od = __shfl_xor_sync(0xffffffffu, bdsq, o);
-        const int op = __shfl_xor_sync(0xffffffffu, bpos, o);
-        if (op != INT_MAX && (bpos == INT_MAX || om < bmod || (om == bmod && op < bpos))) {
-            bmod = om; bdsq = od; bpos = op;
+    const float sf = C.size[c];
+    const double s = (double)sf;
+    const int left = C.left[c];
+    const KMPos pos = km_pos(px, py, pz);
+    int bpos = INT_MAX, nkeep = 0;
+    float thresh32 = 0.f, unused = 0.f;
+    double thresh = 0.;
+    const bool sure = !inertia && km_item_warp32(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32);
+    if (!sure) {
+        // The closest centre by the (penalised) distance: the first minimum in list order.
+        double bmod = 0., bdsq = 0.;
+        bpos = INT_MAX;
+        for (int j = lane; j < m; j += 32) {
+            const int p = lst[j];
+            const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
+            const double mod = inertia ? __dadd_rn(d, inertia[p]) : d;
+            if (bpos == INT_MAX || mod < bmod) { bmod = mod; bdsq = d; bpos = j; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double om = __shfl_xor_sync(0xffffffffu, bmod, o);
+            const double od = __shfl_xor_sync(0xffffffffu, bdsq, o);
+            const int op = __shfl_xor_sync(0xffffffffu, bpos, o);
+            if (op != INT_MAX && (bpos == INT_MAX || om < bmod || (om == bmod && op < bpos))) {
+                bmod = om; bdsq = od; bpos = op;
+            }
+        }
+        const int cp = lst[bpos];
+        const double min_d = sqrt(bdsq);
+        thresh = inertia ? __dadd_rn(sqd(__dadd_rn(min_d, s)), inertia[cp])
+                         : sqd(__dadd_rn(min_d, __dmul_rn(2., s)));
+        nkeep = 0;
+        for (int j0 = 0; j0 < m; j0 += 32) {
+            const int j = j0 + lane;
+            bool keep = false;
+            if (j < m && j != bpos) {
+                const int p = lst[j];
+                const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
+                keep = km_keep(d, s, thresh, inertia, p);
+            }
+            nkeep += __popc(__ballot_sync(0xffffffffu, keep));
         }
     }
     const int cp = lst[bpos];
-    const double min_d = sqrt(bdsq);
-    const double thresh = inertia ? __dadd_rn(sqd(__dadd_rn(min_d, s)), inertia[cp])
-                                  : sqd(__dadd_rn(min_d, __dmul_rn(2., s)));
-    int nkeep = 0;
-    for (int j0 = 0; j0 < m; j0 += 32) {
-        const int j = j0 + lane;
-        bool keep = false;
-        if (j < m && j != bpos) {
-            const int p = lst[j];
-            const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
-            keep = km_keep(d, s, thresh, inertia, p);
-        }
-        nkeep += __popc(__ballot_sync(0xffffffffu, keep));
-    }
     const int ncand = nkeep + 1;
-    const int left = C.left[c];
     if (ncand == 1 || s == 0. || left < 0) {
         if (lane == 0) {
             assign[c] = tag * KM_TAG + cp;
@@ -177,8 +273,9 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
             int p = 0;
             if (j < m && j != bpos) {
                 p = lst[j];
-                const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
-                keep = km_keep(d, s, thresh, inertia, p);
+                keep = sure ? !(km_dsq32(pos, cen32, p, unused) > thresh32)
+                            : km_keep(dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]), s,
+                                      thresh, inertia, p);
             }
             const unsigned bal = __ballot_sync(0xffffffffu, keep);
             if (keep) pool[off + base + __popc(bal & ((1u << lane) - 1u))] = p;
@@ -192,6 +289,7 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
         if (lane == 0) atomicCAS(&L->err, 0, 2);
         return;
     }
+    if (lane == 0 && ncand > KM_SMALL) atomicAdd(&L->wide_next, 2);
     if (lane == 0) items[t] = KMItem{left, ncand, off};
     if (lane == 1) items[t + 1] = KMItem{C.right[c], ncand, off};
 }
@@ -200,11 +298,13 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
 // lists are processed one per thread; their child items and new lists are reserved with one
 // atomic per warp.
 __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
+                                                     const float4* cen32,
                                                      const double* inertia, KMItem* items,
                                                      long long item_cap, int* pool,
                                                      long long pool_cap, int* assign,
-                                                     int tag, KMLevel* L)
+                                                     int tag, KMLevel* L, const KMCtl* ctl)
 {
+    if (ctl->stop) return;
     const int lane = threadIdx.x & 31;
     const long long lo = *(volatile long long*)&L->lo;
     // After an error the level window may cover unwritten slots: process nothing.
@@ -216,7 +316,7 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
         // A small level (the top of the tree, long lists): one item per warp.
         for (long long i = lo + (long long)blockIdx.x * (KM_LTB / 32) + (threadIdx.x >> 5); i < hi;
              i += nwarps)
-            km_item_warp(items[i], lane, C, cen, inertia, items, item_cap, pool, pool_cap, assign,
+            km_item_warp(items[i], lane, C, cen, cen32, inertia, items, item_cap, pool, pool_cap, assign,
                          tag, L);
     } else
     for (long long base = lo + (long long)blockIdx.x * KM_LTB + (threadIdx.x & ~31); base < hi;
@@ -315,7 +415,7 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
             w.cell = __shfl_sync(0xffffffffu, it.cell, l);
             w.len = __shfl_sync(0xffffffffu, it.len, l);
             w.off = __shfl_sync(0xffffffffu, it.off, l);
-            km_item_warp(w, lane, C, cen, inertia, items, item_cap, pool, pool_cap, assign, tag, L);
+            km_item_warp(w, lane, C, cen, cen32, inertia, items, item_cap, pool, pool_cap, assign, tag, L);
         }
     }
     // The last block to finish moves the level window to the appended items.
@@ -328,14 +428,165 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
             if (hi > lo) L->levels += 1;
             L->lo = hi;
             L->hi = *(volatile long long*)&L->total;
+            L->wide = *(volatile int*)&L->wide_next;
+            L->wide_next = 0;
+        }
+    }
+}
+
+// The rest of the tree below a level whose candidate lists are short: one warp per item of the
+// level, its subtree depth first, up to 32 cells at a time (one per lane) from a stack in
+// shared memory that holds every cell with its list.  The same decisions as k_km_level's (the
+// path from a top cell to a cell is the same), without its launch and its latency for each of the
+// tree's 20 or so levels.  2,000,000 points, 64 patches: 17 us a level and 360 us a pass before,
+// now 54 us for the walk (90 with every distance in FP64) and 9 for each of six levels; what
+// bounds it is the chain of a step (stack, cell, distances, stack) at some 20 steps per subtree.
+// The stack holds KW_CAP cells: when it fills up, fewer are taken at a time (a cell taken
+// leaves one more at most), at last one, with room for KW_DEPTH levels more; a tree too deep for
+// that stops the run (KM_ERR_STACK: the host goes on level by level).
+constexpr int KW_CAP = 192, KW_DEPTH = 32;
+struct KMEntry {
+    int cell, len;
+    unsigned short cand[KM_SMALL];
+};
+static_assert(KM_MAX_PATCH < 65536 && sizeof(KMEntry) == 40, "");
+constexpr int KW_WARPS = KM_LTB / 32;
+constexpr int KW_BLOCKS = 3;        // per SM
+constexpr size_t KW_SMEM = sizeof(KMEntry) * KW_CAP * KW_WARPS;
+
+__global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const double* cen, const float4* cen32, const double* inertia,
+                                                    const KMItem* items, long long item_cap,
+                                                    const int* pool, int* assign, int tag, KMLevel* L,
+                                                    KMCtl* ctl)
+{
+    extern __shared__ __align__(16) double kmsm[];
+    if (ctl->stop) return;
+    const long long lo = L->lo, hi = min(L->hi, item_cap);
+    if (L->err || L->wide) {
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            atomicCAS(&ctl->stop, KM_RUN, L->err == 1 ? KM_ERR_POOL : L->err ? KM_ERR_ITEMS : KM_ERR_WIDE);
+        return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) L->units = hi - lo;
+    const int lane = threadIdx.x & 31;
+    KMEntry* st = reinterpret_cast<KMEntry*>(kmsm) + (threadIdx.x >> 5) * KW_CAP;
+    const long long nwarps = (long long)gridDim.x * KW_WARPS;
+    // (neighbouring subtrees go to different SMs)
+    for (long long u = lo + blockIdx.x + (long long)gridDim.x * (threadIdx.x >> 5); u < hi; u += nwarps) {
+        {
+            const KMItem it = items[u];
+            if (lane == 0) { st[0].cell = it.cell; st[0].len = it.len; }
+            if (lane < it.len) st[0].cand[lane] = (unsigned short)pool[it.off + lane];
+            __syncwarp();
+        }
+        int size = 1;
+        while (size > 0) {
+            const int take = min(min(32, size), max(1, (KW_CAP - KW_DEPTH - size) / 2));
+            if (size + take > KW_CAP) {
+                if (lane == 0) atomicCAS(&ctl->stop, KM_RUN, KM_ERR_STACK);
+                return;
+            }
+            size -= take;
+            const bool on = lane < take;
+            int c = 0, m = 0;
+            unsigned short cand[KM_SMALL];
+            if (on) {
+                const KMEntry& e = st[size + lane];
+                c = e.cell;
+                m = e.len;
+#pragma unroll
+                for (int j = 0; j < KM_SMALL; ++j) cand[j] = j < m ? e.cand[j] : 0;
+            }
+            __syncwarp();
+            unsigned kept = 0;        // bit j: candidate j survives (the closest excluded)
+            int nout = 0, ncand = 0, bpos = 0, left = -1, right = -1;
+            if (on) {
+                const double px = C.x[c], py = C.y[c], pz = C.z[c];
+                const float sf = C.size[c];
+                left = C.left[c];
+                right = C.right[c];
+                int cp = 0;
+                bool sure = inertia == nullptr;
+                if (sure) {
+                    const KMPos pos = km_pos(px, py, pz);
+                    float df[KM_SMALL], bd = 0.f, far = pos.amax;
+#pragma unroll
+                    for (int j = 0; j < KM_SMALL; ++j) {
+                        if (j < m) {
+                            df[j] = km_dsq32(pos, cen32, cand[j], far);
+                            if (j == 0 || df[j] < bd) { bd = df[j]; bpos = j; cp = cand[j]; }
+                        }
+                    }
+                    const float t = sqrtf(bd) + 2.f * sf, thresh = t * t;
+                    sure = km_plain(bd, thresh, far);
+#pragma unroll
+                    for (int j = 0; j < KM_SMALL; ++j) {
+                        if (j < m && j != bpos) {
+                            sure = sure && !km_close(df[j], bd, thresh);
+                            if (!(df[j] > thresh)) kept |= 1u << j;
+                        }
+                    }
+                }
+                if (!sure) {
+                    const double s = (double)sf;
+                    double bmod = 0., bdsq = 0.;
+                    kept = 0;
+#pragma unroll
+                    for (int j = 0; j < KM_SMALL; ++j) {
+                        if (j < m) {
+                            const int p = cand[j];
+                            const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
+                            const double mod = inertia ? __dadd_rn(d, inertia[p]) : d;
+                            if (j == 0 || mod < bmod) { bmod = mod; bdsq = d; bpos = j; cp = p; }
+                        }
+                    }
+                    const double min_d = sqrt(bdsq);
+                    const double thresh = inertia ? __dadd_rn(sqd(__dadd_rn(min_d, s)), inertia[cp])
+                                                  : sqd(__dadd_rn(min_d, __dmul_rn(2., s)));
+#pragma unroll
+                    for (int j = 0; j < KM_SMALL; ++j) {
+                        if (j < m && j != bpos) {
+                            const int p = cand[j];
+                            const double d = dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]);
+                            if (km_keep(d, s, thresh, inertia, p)) kept |= 1u << j;
+                        }
+                    }
+                }
+                ncand = 1 + __popc(kept);
+                if (ncand == 1 || sf == 0.f || left < 0) {
+                    assign[c] = tag * KM_TAG + cp;
+                    if (ncand > 1 && sf != 0.f) atomicAdd(&L->leaf_multi, 1);
+                } else {
+                    nout = 2;
+                }
+            }
+            const unsigned outs = __ballot_sync(0xffffffffu, nout);
+            if (nout) {
+                KMEntry* e = st + size + 2 * __popc(outs & ((1u << lane) - 1u));
+                e[0].cell = left;
+                e[1].cell = right;
+                e[0].len = e[1].len = ncand;
+                // The closest first, then the rest in list order; an unpruned list as it was.
+                int q = 0;
+                if (ncand < m) {
+#pragma unroll
+                    for (int j = 0; j < KM_SMALL; ++j)
+                        if (j == bpos) e[0].cand[0] = e[1].cand[0] = cand[j];
+                    q = 1;
+                }
+#pragma unroll
+                for (int j = 0; j < KM_SMALL; ++j)
+                    if (ncand < m ? (kept >> j) & 1u : j < m) { e[0].cand[q] = e[1].cand[q] = cand[j]; ++q; }
+            }
+            size += 2 * __popc(outs);
+            __syncwarp();
         }
     }
 }
 
 enum { KM_SUM_CENTERS = 0, KM_SUM_INERTIA = 1 };
 
-// Per-patch sums over the assigned cells, in cell id order: block b takes a contiguous id
-// range, each warp its own accumulators; lanes of one patch are combined in lane order.
+// An assigned cell's terms of its patch's sums:
 //   centres: (w x, w y, w z, w)          (UpdateCenters::run, src/KMeans.cpp:355-359)
 //   inertia: (|x - c|^2 w, 0.75 s^2 w, w) (CalculateInertia::run, 397-417)
 __device__ __forceinline__ void km_cell_values(Cells C, long long id, int p, const double* cen,
@@ -345,108 +596,102 @@ __device__ __forceinline__ void km_cell_values(Cells C, long long id, int p, con
     const double x = C.x[id], y = C.y[id], z = C.z[id];
     if (mode == KM_SUM_CENTERS) {
         v[0] = __dmul_rn(x, w); v[1] = __dmul_rn(y, w); v[2] = __dmul_rn(z, w);
-        v[3] = w; v[4] = 0.;
+        v[3] = w;
     } else {
         const double s = (double)C.size[id], ssq = __dmul_rn(s, s);
         v[0] = __dmul_rn(dsq3(x, y, z, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]), w);
         v[1] = ssq > 0. ? __dmul_rn(__dmul_rn(0.75, ssq), w) : 0.;
-        v[2] = w; v[3] = 0.; v[4] = 0.;
+        v[2] = w; v[3] = 0.;
     }
 }
 
-// Per-patch sums over the cells assigned by pass `tag`, in cell id order: block b takes a
-// contiguous id range (a multiple of 16 ids; each thread reads 16 consecutive assignments with
-// four 16-byte loads in flight), each warp its own accumulators; lanes of one patch are
-// combined in lane order.
-//   centres: (w x, w y, w z, w)          (UpdateCenters::run, src/KMeans.cpp:355-359)
-//   inertia: (|x - c|^2 w, 0.75 s^2 w, w) (CalculateInertia::run, 397-417)
+// Per-patch sums over the cells assigned by pass `tag`, in a fixed order: warp w of all takes the
+// w-th contiguous range of ids and its own accumulators.  It collects the assigned ids (one
+// in forty or so) and adds them up 32 at a time, the lanes of one patch in lane order: an FP64
+// instruction takes 16 cycles of the SM however few lanes it has, and adding the ids up in the
+// 16 slots they were read in took 61 us for 4,000,000 cells, this 30.
+constexpr int KM_STEP = 512;        // ids a warp reads at once
 __global__ void k_km_accum(Cells C, int ncap, const int* assign, int tag, const double* cen,
-                           int npatch, int mode, double* partial)
+                           int npatch, int mode, double* partial, const KMCtl* ctl)
 {
+    if (ctl->stop) return;
     extern __shared__ __align__(16) double kmsm[];
     const int nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double* my = kmsm + (size_t)wib * npatch * KM_NQ;
     double* stage = kmsm + (size_t)nw * npatch * KM_NQ + (size_t)wib * 32 * KM_NQ;
+    int* ids = reinterpret_cast<int*>(kmsm + (size_t)nw * (npatch + 32) * KM_NQ) + wib * (KM_STEP + 32);
     for (int q = lane; q < npatch * KM_NQ; q += 32) my[q] = 0.;
     __syncwarp();
-    long long per = ((long long)ncap + gridDim.x - 1) / gridDim.x;
-    per = (per + 15) & ~15LL;
-    const long long b0 = (long long)blockIdx.x * per;
+    const long long nwarps = (long long)gridDim.x * nw;
+    long long per = ((long long)ncap + nwarps - 1) / nwarps;
+    per = (per + 3) & ~3LL;
+    const long long b0 = ((long long)blockIdx.x * nw + wib) * per;
     const long long b1 = min(b0 + per, (long long)ncap);
-    for (long long base = b0; base < b1; base += 16LL * blockDim.x) {
-        const long long id0 = base + 16LL * threadIdx.x;
-        int a[16];
-        if (id0 + 15 < b1) {
-            const int4* a4 = reinterpret_cast<const int4*>(assign + id0);
-            int4 q[4];
+    // The ids in ids[at .. at + n), at most 32 of them.
+    auto add = [&](int at, int n) {
+        const bool on = lane < n;
+        const int id = on ? ids[at + lane] : 0;
+        const int p = on ? km_patch_of(assign[id], tag) : -1;
+        double v[KM_NQ] = {0., 0., 0., 0.};
+        if (on) km_cell_values(C, id, p, cen, mode, v);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) q[r] = a4[r];
+        for (int q = 0; q < KM_NQ; ++q) stage[lane * KM_NQ + q] = v[q];
+        __syncwarp();
+        const unsigned grp = __match_any_sync(0xffffffffu, p);
+        if (on && lane == __ffs(grp) - 1) {
+            double sum[KM_NQ];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                a[4 * r] = q[r].x; a[4 * r + 1] = q[r].y; a[4 * r + 2] = q[r].z; a[4 * r + 3] = q[r].w;
+            for (int q = 0; q < KM_NQ; ++q) sum[q] = my[p * KM_NQ + q];
+            for (unsigned g = grp; g; g &= g - 1) {
+                const int l = __ffs(g) - 1;
+#pragma unroll
+                for (int q = 0; q < KM_NQ; ++q) sum[q] = __dadd_rn(sum[q], stage[l * KM_NQ + q]);
             }
-        } else {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) a[k] = id0 + k < b1 ? assign[id0 + k] : -1;
+            for (int q = 0; q < KM_NQ; ++q) my[p * KM_NQ + q] = sum[q];
         }
-        unsigned mine = 0;   // bit k: id0 + k is assigned in this pass
+        __syncwarp();
+    };
+    int pending = 0;
+    for (long long base = b0; base < b1; base += KM_STEP) {
+        // Lane l reads ids base + 4 (l + 32 r) .. + 3 (b0 and base are multiples of four).
+        int4 a[4];
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-            if (km_patch_of(a[k], tag) >= 0) mine |= 1u << k;
-        if (!__ballot_sync(0xffffffffu, mine != 0)) continue;
-        for (int k0 = 0; k0 < 16; k0 += 4) {
-            if (!__ballot_sync(0xffffffffu, (mine >> k0) & 0xfu)) continue;
-            // The cell values of four slots, loaded together.
-            int pp[4];
-            double vv[4][KM_NQ];
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                pp[kk] = ((mine >> (k0 + kk)) & 1u) ? km_patch_of(assign[id0 + k0 + kk], tag) : -1;
-#pragma unroll
-                for (int q = 0; q < KM_NQ; ++q) vv[kk][q] = 0.;
-                if (pp[kk] >= 0) km_cell_values(C, id0 + k0 + kk, pp[kk], cen, mode, vv[kk]);
+        for (int r = 0; r < 4; ++r) {
+            const long long id = base + 4 * (lane + 32 * r);
+            a[r] = make_int4(-1, -1, -1, -1);
+            if (id + 3 < b1) a[r] = *reinterpret_cast<const int4*>(assign + id);
+            else if (id < b1) {
+                a[r].x = assign[id];
+                if (id + 1 < b1) a[r].y = assign[id + 1];
+                if (id + 2 < b1) a[r].z = assign[id + 2];
             }
+        }
+        const int lo = tag * KM_TAG, hi = lo + KM_TAG;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-            const int p = pp[kk];
-            if (!__ballot_sync(0xffffffffu, p >= 0)) continue;
+        for (int r = 0; r < 4; ++r) {
+            const int av[4] = {a[r].x, a[r].y, a[r].z, a[r].w};
 #pragma unroll
-            for (int q = 0; q < KM_NQ; ++q) stage[lane * KM_NQ + q] = vv[kk][q];
-            __syncwarp();
-            const unsigned grp = __match_any_sync(0xffffffffu, p);
-            if (p >= 0 && lane == __ffs(grp) - 1) {
-                double sum[KM_NQ] = {0., 0., 0., 0., 0.};
-                for (unsigned g = grp; g; g &= g - 1) {
-                    const int l = __ffs(g) - 1;
-#pragma unroll
-                    for (int q = 0; q < KM_NQ; ++q) sum[q] = __dadd_rn(sum[q], stage[l * KM_NQ + q]);
-                }
-#pragma unroll
-                for (int q = 0; q < KM_NQ; ++q) my[p * KM_NQ + q] = __dadd_rn(my[p * KM_NQ + q], sum[q]);
+            for (int k = 0; k < 4; ++k) {
+                const bool mine = av[k] >= lo && av[k] < hi;
+                const unsigned bal = __ballot_sync(0xffffffffu, mine);
+                if (mine) ids[pending + __popc(bal & ((1u << lane) - 1u))] = (int)(base + 4 * (lane + 32 * r)) + k;
+                pending += __popc(bal);
             }
-            __syncwarp();
-            }
+        }
+        __syncwarp();
+        while (pending >= 32) {
+            pending -= 32;
+            add(pending, 32);
         }
     }
+    if (pending > 0) add(0, pending);
     __syncthreads();
     for (int q = threadIdx.x; q < npatch * KM_NQ; q += blockDim.x) {
         double s = 0.;
         for (int w = 0; w < nw; ++w) s = __dadd_rn(s, kmsm[(size_t)w * npatch * KM_NQ + q]);
         partial[(size_t)blockIdx.x * npatch * KM_NQ + q] = s;
     }
-}
-
-// Block partials -> totals: one warp per summed quantity, lanes over the blocks, then a
-// fixed-shape warp reduction (deterministic).
-__global__ void k_km_total(int nq, int nblk, const double* partial, double* tot)
-{
-    const int q = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (q >= nq) return;
-    double s = 0.;
-    for (int b = lane; b < nblk; b += 32) s = __dadd_rn(s, partial[(size_t)b * nq + q]);
-    for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
-    if (lane == 0) tot[q] = s;
 }
 
 // Fixed-shape block sum (the same tree of additions on every run).
@@ -462,19 +707,40 @@ __device__ double block_sum(double v, double* red)
     return t;
 }
 
-// The finalize step of the sums, one thread per patch.
-__global__ void __launch_bounds__(1024) k_km_finish(int npatch, const double* tot, int mode,
-                                                    int coords, double* cen, double* inertia,
-                                                    double* shift)
+// Block partials -> totals: one warp per summed quantity, lanes over the blocks, then a
+// fixed-shape warp reduction (deterministic).  The last block to finish takes the finalize step
+// of the sums, one thread per patch, and ends the run when the centres have settled.
+__global__ void __launch_bounds__(256) k_km_total(int npatch, int nblk, const double* partial,
+                                                  double* tot, int mode, int coords, double* cen,
+                                                  double* inertia, double tolsq, KMCtl* ctl)
 {
     __shared__ double red[32];
+    __shared__ int last;
+    if (ctl->stop) return;
+    const int nq = npatch * KM_NQ;
+    const int q = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (q < nq) {
+        double s = 0.;
+        for (int b = lane; b < nblk; b += 32) s = __dadd_rn(s, partial[(size_t)b * nq + q]);
+        for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (lane == 0) tot[q] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&ctl->total_done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
     if (mode == KM_SUM_CENTERS) {
         // UpdateCenters::finalize (src/KMeans.cpp:370-380), CalculateShiftSq (689-706).
         double sh = 0.;
         for (int p = threadIdx.x; p < npatch; p += blockDim.x) {
             const double* t = tot + p * KM_NQ;
-            double x = t[0], y = t[1], z = t[2];
-            const double w = t[3];
+            double x = __ldcg(t), y = __ldcg(t + 1), z = __ldcg(t + 2);
+            const double w = __ldcg(t + 3);
             if (w > 0.) {
                 x = __ddiv_rn(x, w); y = __ddiv_rn(y, w); z = __ddiv_rn(z, w);
                 if (coords == SPHERE) {
@@ -487,16 +753,20 @@ __global__ void __launch_bounds__(1024) k_km_finish(int npatch, const double* to
             cen[3 * p] = x; cen[3 * p + 1] = y; cen[3 * p + 2] = z;
         }
         sh = block_sum(sh, red);
-        if (threadIdx.x == 0) *shift = sh;
+        if (threadIdx.x == 0) {
+            ctl->iters += 1;
+            if (sh < tolsq) ctl->stop = KM_CONVERGED;
+        }
     } else {
         // CalculateInertia::finalize (src/KMeans.cpp:419-446): I_i / (sum w / npatch / 3).
         double sw = 0.;
-        for (int p = threadIdx.x; p < npatch; p += blockDim.x) sw = __dadd_rn(sw, tot[p * KM_NQ + 2]);
+        for (int p = threadIdx.x; p < npatch; p += blockDim.x) sw = __dadd_rn(sw, __ldcg(tot + p * KM_NQ + 2));
         const double sumw = block_sum(sw, red);
         const double meanw = __ddiv_rn(__ddiv_rn(sumw, (double)npatch), 3.);
         for (int p = threadIdx.x; p < npatch; p += blockDim.x)
-            inertia[p] = __ddiv_rn(__dadd_rn(tot[p * KM_NQ], tot[p * KM_NQ + 1]), meanw);
+            inertia[p] = __ddiv_rn(__dadd_rn(__ldcg(tot + p * KM_NQ), __ldcg(tot + p * KM_NQ + 1)), meanw);
     }
+    if (threadIdx.x == 0) ctl->total_done = 0u;
 }
 
 // AssignPatches::run (src/KMeans.cpp:482-510): every point of an assigned cell gets its
@@ -866,7 +1136,9 @@ int kmpp_rec(CellCache& cc, int id, const std::vector<V3>& cen, long ncen, V3& o
 
 // Device scratch of one KMeansRun / KMeansAssign call.
 struct KMScratch {
-    double *cen = nullptr, *inertia = nullptr, *partial = nullptr, *tot = nullptr, *shift = nullptr;
+    double *cen = nullptr, *inertia = nullptr, *partial = nullptr, *tot = nullptr;
+    KMCtl* ctl = nullptr;
+    float4* cen32 = nullptr;
     KMItem* items = nullptr;
     int* pool = nullptr;
     int* assign = nullptr;
@@ -876,9 +1148,11 @@ struct KMScratch {
     size_t acc_smem = 0;
     int tag = 0;           // tag of the last tree pass (assignments of older passes are stale)
     int levels = 0;        // levels with items in the last tree pass
+    int pre = 1;           // levels before the walk
+    bool walk = true;      // the walk takes the rest (else all levels one by one)
     ~KMScratch()
     {
-        dfree(cen); dfree(inertia); dfree(partial); dfree(tot); dfree(shift); dfree(items);
+        dfree(cen); dfree(inertia); dfree(partial); dfree(tot); dfree(ctl); dfree(cen32); dfree(items);
         dfree(pool); dfree(assign); dfree(lvl);
     }
 };
@@ -889,7 +1163,9 @@ int scratch_alloc(const KMField& F, int npatch, KMScratch& S, cudaStream_t st)
     TC_TRY(dalloc(&S.inertia, npatch));
     TC_TRY(dalloc(&S.partial, (size_t)KM_NBLK * npatch * KM_NQ));
     TC_TRY(dalloc(&S.tot, (size_t)npatch * KM_NQ));
-    TC_TRY(dalloc(&S.shift, 1));
+    TC_TRY(dalloc(&S.cen32, 2 * (size_t)npatch));
+    TC_TRY(dalloc(&S.ctl, 1));
+    TC_CU(cudaMemsetAsync(S.ctl, 0, sizeof(KMCtl), st));
     S.item_cap = std::max<long long>(F.ncap, F.ntop);
     TC_TRY(dalloc(&S.items, S.item_cap));
     S.pool_cap = std::max<long long>(1 << 22, 4LL * npatch + 2LL * F.ntop);
@@ -899,11 +1175,12 @@ int scratch_alloc(const KMField& F, int npatch, KMScratch& S, cudaStream_t st)
     TC_TRY(dalloc(&S.lvl, 1));
     // Accumulator warps per block: as many as fit (at most 8), each npatch x KM_NQ doubles
     // plus a 32-lane staging row.
-    const size_t per_warp = ((size_t)npatch * KM_NQ + 32 * KM_NQ) * sizeof(double);
+    const size_t per_warp = ((size_t)npatch * KM_NQ + 32 * KM_NQ) * sizeof(double) + (KM_STEP + 32) * sizeof(int);
     int nw = (int)std::min<size_t>(8, (200 * 1024) / per_warp);
     if (nw < 1) { set_last_error("k-means: too many patches for the accumulators"); return TC_ERR_UNSUPPORTED; }
     S.acc_threads = 32 * nw;
     S.acc_smem = per_warp * nw;
+    TC_CU(cudaFuncSetAttribute(k_km_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KW_SMEM));
     if (S.acc_smem > 48 * 1024)
         TC_CU(cudaFuncSetAttribute(k_km_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.acc_smem));
     return 0;
@@ -923,25 +1200,89 @@ int upload_centers(const double* centers, int npatch, int coords, KMScratch& S, 
     return 0;
 }
 
-// FindCellsInPatches over the whole field: assign[cell] = patch for the cells that lie in
-// one patch.
+int sm_count(int* nsm)
+{
+    int dev = 0;
+    TC_CU(cudaGetDevice(&dev));
+    TC_CU(cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev));
+    return 0;
+}
+
+int next_tag(const KMField& F, KMScratch& S, cudaStream_t st)
+{
+    if (++S.tag >= KM_TAG_MAX) {
+        TC_CU(cudaMemsetAsync(S.assign, 0xff, sizeof(int) * (size_t)F.ncap, st));
+        S.tag = 1;
+    }
+    return 0;
+}
+
+// FindCellsInPatches over the whole field: assign[cell] = patch for the cells that lie in one
+// patch.  Enqueues the first S.pre levels and the walk; what stops it is in S.ctl.
+int enqueue_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S, cudaStream_t st)
+{
+    int nsm = 0;
+    TC_TRY(sm_count(&nsm));
+    TC_TRY(next_tag(F, S, st));
+    const int nstart = std::max(F.ntop, npatch);
+    count_launch();
+    k_km_start<<<(nstart + 255) / 256, 256, 0, st>>>(F.d_tops, F.ntop, npatch, S.items, S.pool, S.lvl, S.ctl,
+                                                     S.cen, S.cen32);
+    for (int k = 0; k < S.pre; ++k) {
+        count_launch();
+        k_km_level<<<nsm, KM_LTB, 0, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap, S.pool,
+                                               S.pool_cap, S.assign, S.tag, S.lvl, S.ctl);
+    }
+    count_launch();
+    k_km_walk<<<KW_BLOCKS * nsm, KM_LTB, KW_SMEM, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap, S.pool, S.assign,
+                                          S.tag, S.lvl, S.ctl);
+    TC_CU(cudaGetLastError());
+    return 0;
+}
+
+int grow_pool(KMScratch& S)
+{
+    if (S.pool_cap > (1LL << 36)) { set_last_error("k-means: candidate pool could not be sized"); return TC_ERR_NOMEM; }
+    dfree(S.pool);
+    S.pool_cap *= 4;
+    TC_TRY(dalloc(&S.pool, S.pool_cap));
+    return 0;
+}
+
+// After a stop other than convergence: makes room, another level before the walk, or no walk.
+// The centres are those before the pass that stopped.
+int mend_stop(KMScratch& S, int stop, cudaStream_t st)
+{
+    switch (stop) {
+      case KM_ERR_POOL: TC_TRY(grow_pool(S)); break;
+      case KM_ERR_WIDE: if (++S.pre > 24) S.walk = false; break;
+      case KM_ERR_STACK: S.walk = false; break;
+      default: set_last_error("k-means: work item array full (inconsistent tree)"); return TC_ERR_DEVICE;
+    }
+    TC_CU(cudaMemsetAsync(&S.ctl->stop, 0, sizeof(int), st));
+    TC_CU(cudaMemsetAsync(&S.ctl->total_done, 0, sizeof(unsigned), st));
+    return 0;
+}
+
+// The same, completed: with the walk, or level by level where it cannot be used.
 int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S, cudaStream_t st)
 {
-    static int nblocks = 0;
-    if (!nblocks) {
-        int dev = 0, sms = 0;
-        TC_CU(cudaGetDevice(&dev));
-        TC_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        nblocks = 4 * std::max(sms, 1);
+    while (S.walk) {
+        TC_TRY(enqueue_cells(F, npatch, inertia, S, st));
+        KMCtl c{};
+        TC_CU(cudaMemcpyAsync(&c, S.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
+        TC_CU(cudaStreamSynchronize(st));
+        if (!c.stop) return 0;
+        TC_TRY(mend_stop(S, c.stop, st));
     }
+    int nsm = 0;
+    TC_TRY(sm_count(&nsm));
     for (int attempt = 0; attempt < 6; ++attempt) {
-        if (++S.tag >= KM_TAG_MAX) {
-            TC_CU(cudaMemsetAsync(S.assign, 0xff, sizeof(int) * (size_t)F.ncap, st));
-            S.tag = 1;
-        }
+        TC_TRY(next_tag(F, S, st));
         const int nstart = std::max(F.ntop, npatch);
         count_launch();
-        k_km_start<<<(nstart + 255) / 256, 256, 0, st>>>(F.d_tops, F.ntop, npatch, S.items, S.pool, S.lvl);
+        k_km_start<<<(nstart + 255) / 256, 256, 0, st>>>(F.d_tops, F.ntop, npatch, S.items, S.pool, S.lvl, S.ctl,
+                                                     S.cen, S.cen32);
         TC_CU(cudaGetLastError());
         KMLevel h{};
         bool done = false;
@@ -950,8 +1291,8 @@ int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S
         for (int lev = 0; lev < F.ncap + 2 && !done; lev += batch, batch = KM_LEVELS_PER_CHECK) {
             for (int k = 0; k < batch; ++k) {
                 count_launch();
-                k_km_level<<<nblocks, KM_LTB, 0, st>>>(F.cells, S.cen, inertia, S.items, S.item_cap,
-                                                       S.pool, S.pool_cap, S.assign, S.tag, S.lvl);
+                k_km_level<<<4 * nsm, KM_LTB, 0, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap,
+                                                       S.pool, S.pool_cap, S.assign, S.tag, S.lvl, S.ctl);
             }
             TC_CU(cudaGetLastError());
             TC_CU(cudaMemcpyAsync(&h, S.lvl, sizeof(KMLevel), cudaMemcpyDeviceToHost, st));
@@ -962,26 +1303,20 @@ int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S
         if (!done) { set_last_error("k-means: tree pass did not end"); return TC_ERR_DEVICE; }
         if (h.err == 2) { set_last_error("k-means: work item array full (inconsistent tree)"); return TC_ERR_DEVICE; }
         if (h.err == 0) return 0;
-        // Candidate pool full: grow it and repeat the pass.
-        dfree(S.pool);
-        S.pool_cap *= 4;
-        TC_TRY(dalloc(&S.pool, S.pool_cap));
+        TC_TRY(grow_pool(S));       // and repeat the pass
     }
     set_last_error("k-means: candidate pool could not be sized");
     return TC_ERR_NOMEM;
 }
 
-int sum_cells(const KMField& F, int npatch, int mode, KMScratch& S, cudaStream_t st)
+int sum_cells(const KMField& F, int npatch, int mode, double tolsq, KMScratch& S, cudaStream_t st)
 {
     count_launch();
     k_km_accum<<<KM_NBLK, S.acc_threads, S.acc_smem, st>>>(F.cells, F.ncap, S.assign, S.tag, S.cen,
-                                                           npatch, mode, S.partial);
-    TC_CU(cudaGetLastError());
-    const int nq = npatch * KM_NQ;
+                                                           npatch, mode, S.partial, S.ctl);
     count_launch();
-    k_km_total<<<(nq + 7) / 8, 256, 0, st>>>(nq, KM_NBLK, S.partial, S.tot);
-    count_launch();
-    k_km_finish<<<1, 1024, 0, st>>>(npatch, S.tot, mode, F.coords, S.cen, S.inertia, S.shift);
+    k_km_total<<<(npatch * KM_NQ + 7) / 8, 256, 0, st>>>(npatch, KM_NBLK, S.partial, S.tot, mode, F.coords,
+                                                         S.cen, S.inertia, tolsq, S.ctl);
     TC_CU(cudaGetLastError());
     return 0;
 }
@@ -1124,18 +1459,31 @@ int kmeans_run(const KMField& F, double* centers, int npatch, int max_iter, doub
     TC_TRY(scratch_alloc(F, npatch, S, st));
     TC_TRY(upload_centers(centers, npatch, F.coords, S, st));
     const double tolsq = (tol * F.size) * (tol * F.size) * npatch;
-    int it = 0;
-    for (; it < max_iter; ++it) {
-        if (alt) {
-            TC_TRY(find_cells(F, npatch, nullptr, S, st));
-            TC_TRY(sum_cells(F, npatch, KM_SUM_INERTIA, S, st));
+    // Iterations are enqueued in batches (the first alone: it may have to be mended); those
+    // after the last one return at once.
+    int it = 0, batch = 1;
+    while (it < max_iter) {
+        const bool queued = S.walk;
+        const int m = queued ? std::min(batch, max_iter - it) : 1;
+        for (int k = 0; k < m; ++k) {
+            if (alt) {
+                TC_TRY((queued ? enqueue_cells : find_cells)(F, npatch, nullptr, S, st));
+                TC_TRY(sum_cells(F, npatch, KM_SUM_INERTIA, tolsq, S, st));
+            }
+            TC_TRY((queued ? enqueue_cells : find_cells)(F, npatch, alt ? S.inertia : nullptr, S, st));
+            TC_TRY(sum_cells(F, npatch, KM_SUM_CENTERS, tolsq, S, st));
         }
-        TC_TRY(find_cells(F, npatch, alt ? S.inertia : nullptr, S, st));
-        TC_TRY(sum_cells(F, npatch, KM_SUM_CENTERS, S, st));
-        double shift = 0.;
-        TC_CU(cudaMemcpyAsync(&shift, S.shift, sizeof(double), cudaMemcpyDeviceToHost, st));
+        KMCtl c{};
+        KMLevel h{};
+        TC_CU(cudaMemcpyAsync(&c, S.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
+        TC_CU(cudaMemcpyAsync(&h, S.lvl, sizeof(h), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaStreamSynchronize(st));
-        if (shift < tolsq) { ++it; break; }
+        it = c.iters;
+        if (c.stop == KM_CONVERGED) break;
+        if (c.stop) { TC_TRY(mend_stop(S, c.stop, st)); batch = 1; continue; }
+        // Enough subtrees for the warps, if another level gives them.
+        if (queued && h.units > 0 && h.units < KM_UNITS && S.pre < 12) ++S.pre;
+        batch = std::min(2 * batch, 16);
     }
     if (iters_out) *iters_out = it;
     std::vector<double> h(3 * (size_t)npatch);
@@ -1174,6 +1522,10 @@ int kmeans_assign(const KMField& F, const double* centers, int npatch, int64_t* 
         count_launch();
         k_km_paint_big<<<1216, 256, 0, st>>>(F.cells, S.assign, S.tag, F.idx, big, nbig, d_out);
         if (cudaGetLastError() != cudaSuccess) { set_last_error("k-means assign launch failed"); rc = TC_ERR_CUDA; break; }
+        // The caller's array may have no pages yet: the copy takes 16 ms for 16 MB where the device
+        // has to fault them in one by one, 1 ms where they are there.
+        for (int64_t i = 0; i < F.n; i += 4096 / (int64_t)sizeof(int64_t))
+            *const_cast<volatile int64_t*>(patches + i) = -1;
         if (cudaMemcpyAsync(patches, d_out, sizeof(int64_t) * F.n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             set_last_error("k-means assign copy failed"); rc = TC_ERR_CUDA; break;
