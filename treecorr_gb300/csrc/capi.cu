@@ -305,9 +305,9 @@ int alloc_cells(Cells& C, int64_t m)
 
 void free_scratch(BuildScratch& S)
 {
-    dfree(S.tasks); dfree(S.chunk0); dfree(S.chunks); dfree(S.part1); dfree(S.part2);
-    dfree(S.stats); dfree(S.big_next); dfree(S.small); dfree(S.counters); dfree(S.wstack);
-    S.cap_tasks = S.cap_chunks = 0;
+    dfree(S.L.small); dfree(S.wstack);
+    dev_free(S.level_mem);
+    S = BuildScratch();
 }
 
 void field_release(tc_field* f)
@@ -344,9 +344,8 @@ int field_build(tc_field* f)
     TC_TRY(dalloc(&f->tcells, ncap));
     TC_TRY(dalloc(&f->d_tops_raw, 2 * n));
     TC_TRY(dalloc(&f->d_ntop, 1));
-    TC_TRY(dalloc(&f->S.small, n));
+    TC_TRY(dalloc(&f->S.L.small, n));
     TC_TRY(dalloc(&f->S.wstack, n));
-    TC_TRY(dalloc(&f->S.counters, 2));
     TC_TRY(alloc_points(f->buf[1], n));
     // Unused ids (inside list leaves) keep harmless contents: no children, no points.
     TC_CU(cudaMemsetAsync(f->cells.left, 0xff, ncap * sizeof(int), st));
@@ -365,21 +364,19 @@ int field_build(tc_field* f)
     BP.minsizesq = f->minsize * f->minsize;
     BP.maxsizesq = f->maxsize * f->maxsize;
     BP.n = (int)n;
-    TC_TRY(build_tree(BP, f->buf, f->cells, f->d_tops_raw, f->d_ntop, f->S, st, f->tops, f->d_err,
+    TC_TRY(build_tree(BP, f->buf, f->cells, f->tcells, f->d_tops_raw, f->d_ntop, f->S, st, f->tops, f->d_err,
                       f->mintop, f->maxtop));
-    launch_pack_cells((int)ncap, f->cells, f->tcells, st);
-    TC_CU(cudaGetLastError());
     TC_TRY(dalloc(&f->d_tops, f->tops.size()));
     TC_CU(cudaMemcpyAsync(f->d_tops, f->tops.data(), f->tops.size() * sizeof(int),
                           cudaMemcpyHostToDevice, st));
     launch_validate_tree((int)ncap, f->cells, f->d_tops, (int)f->tops.size(), f->d_err, st);
     TC_CU(cudaGetLastError());
     TC_CU(cudaEventRecord(e1, st));
-    TC_CU(cudaEventSynchronize(e1));
-    TC_CU(cudaEventElapsedTime(&f->build_ms, e0, e1));
+    const int rc = check_dev_err(f->d_err, st);     // (waits for the stream)
+    if (!rc) cudaEventElapsedTime(&f->build_ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    TC_TRY(check_dev_err(f->d_err, st));
+    if (rc) return rc;
     // The second point buffer and the build scratch are no longer needed.
     free_points(f->buf[1]);
     free_scratch(f->S);

@@ -53,7 +53,7 @@ void dfree(T*& p)
 }
 
 // Tree build (tree_build.cu).
-int build_tree(const BuildParams& BP, Points bufs[2], Cells C, int* d_tops, int* d_ntop,
+int build_tree(const BuildParams& BP, Points bufs[2], Cells C, TCell* tcells, int* d_tops, int* d_ntop,
                BuildScratch& S, cudaStream_t st, std::vector<int>& tops_out, int* d_err,
                int mintop, int maxtop);
 int field_center(const BuildParams& BP, Points P, BuildScratch& S, cudaStream_t st,
@@ -61,7 +61,6 @@ int field_center(const BuildParams& BP, Points P, BuildScratch& S, cudaStream_t 
 void launch_prepare(int n, int coords, int dkind, const double* x, const double* y,
                     const double* z, const double* d1, const double* d2, const double* w,
                     const double* wpos, Points P, cudaStream_t st);
-int scratch_ensure_level(BuildScratch& S, int nt, int nc);
 int tcgen05_selftest(const float* A, const float* B, float* C, int N, int K, cudaStream_t st);
 void launch_validate_tree(int ncap, const Cells& C, const int* tops, int ntop, int* err,
                           cudaStream_t st);

@@ -85,7 +85,7 @@ struct BuildParams {
 };
 
 
-static constexpr int CH = 4096;        // points per chunk in the cooperative levels
+static constexpr int CH = 4096;        // most points per chunk in the cooperative levels
 static constexpr int CB = 256;         // threads per chunk block
 static constexpr int SMALL = 2048;     // cells at most this big are finished by one block
 
@@ -99,7 +99,7 @@ struct Part2 {   // chunk partial of pass 2
 };
 struct TaskStats {  // per cooperative task, filled by combine1 / combine2
     double cx, cy, cz;
-    double splitval;
+    double splitval, sizesq;
     int axis;
     float w;
     int mid;        // split point, or -1 for a leaf
@@ -114,19 +114,28 @@ struct Chunk {
 
 struct WTask { int s, e, parent, meta; };   // meta: side | intop<<1 | buf<<2 | mintop<<8 | maxtop<<20
 
+// The cooperative levels of the build, all on the device: a level's tasks and their chunks are
+// appended by the level before (arrays [level & 1]); cnt[level] counts them.
+struct LevelBufs {
+    BuildTask* tasks[2];
+    int2* tchunk[2];        // first chunk of a task, number of chunks
+    Chunk* chunks[2];
+    Part1* part1;
+    Part2* part2;
+    TaskStats* stats;
+    int* done;              // per task: chunks that have finished (zero between kernels)
+    int2* cnt;              // per level: tasks, chunks
+    BuildTask* small;       // cells left to k_subtree (capacity n) and their number
+    int* nsmall;
+    int cap_tasks, cap_chunks;
+    int ch, sub;            // points per chunk; most points of a cell left to k_subtree
+};
+
 // Device scratch of the build, grown on demand and kept by the field.
 struct BuildScratch {
-    BuildTask* tasks = nullptr;     // cooperative tasks of the current level
-    int* chunk0 = nullptr;          // first chunk of each task (+1 sentinel)
-    Chunk* chunks = nullptr;
-    Part1* part1 = nullptr;
-    Part2* part2 = nullptr;
-    TaskStats* stats = nullptr;
-    BuildTask* big_next = nullptr;  // cooperative tasks of the next level
-    BuildTask* small = nullptr;     // warp tasks (capacity n)
-    int* counters = nullptr;        // [0] next cooperative count, [1] warp task count
-    WTask* wstack = nullptr;        // per-warp-task stacks (capacity n)
-    int cap_tasks = 0, cap_chunks = 0;
+    LevelBufs L = {};
+    void* level_mem = nullptr;      // the arrays of L but small
+    WTask* wstack = nullptr;        // lists of k_subtree, stack of k_median_levels (capacity n)
 };
 
 

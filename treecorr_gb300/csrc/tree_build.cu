@@ -10,9 +10,10 @@
 // levels are done, or max_top levels are reached.
 //
 // GB300 layout: the build is level-synchronous.  Cells with more than SMALL points are
-// processed cooperatively by many blocks (fixed chunks of CH points, deterministic two-stage
-// FP64 reductions, a stable scatter into the other of two point buffers).  Cells with at
-// most SMALL points are finished by one block each, which keeps the points in shared memory
+// processed cooperatively by many blocks (chunks of CH points, deterministic two-stage FP64
+// reductions, a stable scatter into the other of two point buffers); a level's tasks are
+// written by the level before, so that no level waits for the host.  Cells with at most SMALL
+// points (fewer for small catalogs) are finished by one block each, which keeps the points in shared memory
 // and builds the whole subtree on them.
 // Cell ids are positional, so no allocation counter is needed: an internal cell that
 // splits [s,e) at m gets id m-1, a leaf starting at point s gets id (n-1)+s.
@@ -25,6 +26,7 @@
 
 #include "tc_internal.cuh"
 #include "tc_host.hpp"
+#include "traverse2pt.hpp"
 
 namespace tc {
 
@@ -303,19 +305,107 @@ __device__ __forceinline__ void transport_near(int coords, int spin, double cx, 
 // ---------------------------------------------------------------------------------------
 // Cooperative levels (cells with more than SMALL points).
 
-__global__ void __launch_bounds__(CB) k_chunk_pass1(const Chunk* chunks, const BuildTask* tasks,
-                                                     Points P0, Points P1, int coords, Part1* out)
+// The root [0, n) as level 0's task.
+__global__ void k_level_root(LevelBufs L, BuildTask root)
+{
+    const int n = root.e - root.s, nc = (n + L.ch - 1) / L.ch;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c == 0) {
+        L.tasks[0][0] = root;
+        L.tchunk[0][0] = make_int2(0, nc);
+        L.cnt[0] = make_int2(1, nc);
+    }
+    if (c < nc) {
+        Chunk k;
+        k.task = 0; k.cs = root.s + c * L.ch; k.ce = min(k.cs + L.ch, root.e);
+        k.leftoff = k.rightoff = 0;
+        L.chunks[0][c] = k;
+    }
+}
+
+// Counts a chunk of task t as done; true for the whole block of the task's last one, whose
+// first warp then reads all its chunks' partials (with __ldcg: other blocks wrote them).
+__device__ __forceinline__ bool task_complete(const LevelBufs& L, int t, int nchunk, int* flag)
+{
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const int k = atomicAdd(&L.done[t], 1);
+        *flag = k == nchunk - 1;
+        if (*flag) L.done[t] = 0;
+    }
+    __syncthreads();
+    const bool last = *flag != 0;
+    if (last) __threadfence();
+    return last;
+}
+
+__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
+
+// One warp: centroid, weight, split axis and value of task t.
+__device__ void task_combine1(const LevelBufs& L, int lev, int t, Points P0, Points P1, const BuildParams& BP)
+{
+    const int lane = threadIdx.x & 31;
+    const int2 tc = L.tchunk[lev & 1][t];
+    const int c0 = tc.x, c1 = tc.x + tc.y;
+    double s[5] = {0., 0., 0., 0., 0.};
+    double xmin = DBL_MAX, ymin = DBL_MAX, zmin = DBL_MAX;
+    double xmax = -DBL_MAX, ymax = -DBL_MAX, zmax = -DBL_MAX;
+    for (int c = c0 + lane; c < c1; c += 32) {
+        const Part1* p = L.part1 + c;
+        s[0] += ldcg(&p->sx); s[1] += ldcg(&p->sy); s[2] += ldcg(&p->sz);
+        s[3] += ldcg(&p->swp); s[4] += ldcg(&p->sw);
+        xmin = fmin(xmin, ldcg(&p->xmin)); xmax = fmax(xmax, ldcg(&p->xmax));
+        ymin = fmin(ymin, ldcg(&p->ymin)); ymax = fmax(ymax, ldcg(&p->ymax));
+        zmin = fmin(zmin, ldcg(&p->zmin)); zmax = fmax(zmax, ldcg(&p->zmax));
+    }
+    warp_sums<5>(s, lane);
+    xmin = dunkey(warp_kmin(dkey(xmin))); xmax = dunkey(warp_kmax(dkey(xmax)));
+    ymin = dunkey(warp_kmin(dkey(ymin))); ymax = dunkey(warp_kmax(dkey(ymax)));
+    zmin = dunkey(warp_kmin(dkey(zmin))); zmax = dunkey(warp_kmax(dkey(zmax)));
+    if (lane) return;
+    const BuildTask tk = L.tasks[lev & 1][t];
+    const Points& P = tk.buf ? P1 : P0;
+    TaskStats r;
+    // BuildCellData, src/Cell.cpp:170-200.
+    if (s[3] != 0.) {
+        r.cx = s[0] / s[3]; r.cy = s[1] / s[3]; r.cz = s[2] / s[3];
+        if (BP.coords == SPHERE) normalize3(r.cx, r.cy, r.cz);
+    } else {
+        r.cx = P.x[tk.s]; r.cy = P.y[tk.s]; r.cz = P.z[tk.s];
+    }
+    r.w = float(s[4]);
+    r.axis = split_axis(BP.coords, xmax - xmin, ymax - ymin, zmax - zmin);
+    if (BP.split == MIDDLE) {   // Bounds::getMiddle, include/Bounds.h:67-68
+        r.splitval = r.axis == 2 ? (zmax + zmin) / 2. : r.axis == 1 ? (ymax + ymin) / 2.
+                                                                     : (xmax + xmin) / 2.;
+    } else {                    // Mean: the centroid, src/Cell.cpp:481-495
+        r.splitval = r.axis == 2 ? r.cz : r.axis == 1 ? r.cy : r.cx;
+    }
+    // Remember whether all points share the split coordinate (needed by the fallback).
+    double lo = r.axis == 2 ? zmin : r.axis == 1 ? ymin : xmin;
+    double hi = r.axis == 2 ? zmax : r.axis == 1 ? ymax : xmax;
+    r.allsame = (lo == hi) ? 1 : 0;
+    r.mid = -1;
+    r.copy = 0;
+    r.byindex = 0;
+    r.sizesq = 0.;
+    L.stats[t] = r;
+}
+
+__global__ void __launch_bounds__(CB) k_chunk_pass1(LevelBufs L, int lev, Points P0, Points P1, BuildParams BP)
 {
     __shared__ double sh[CB / 32][5];
     __shared__ long long shk[CB / 32][6];
-    const Chunk ch = chunks[blockIdx.x];
-    const Points& P = tasks[ch.task].buf ? P1 : P0;
+    __shared__ int flag;
+    if ((int)blockIdx.x >= L.cnt[lev].y) return;
+    const Chunk ch = L.chunks[lev & 1][blockIdx.x];
+    const Points& P = L.tasks[lev & 1][ch.task].buf ? P1 : P0;
     double s[5] = {0., 0., 0., 0., 0.};
     long long k[6];                       // minima and, negated, maxima
     const long long big = dkey(DBL_MAX);
 #pragma unroll
     for (int q = 0; q < 3; ++q) { k[2 * q] = big; k[2 * q + 1] = ~dkey(-DBL_MAX); }
-    const bool flat = coords == FLAT;
+    const bool flat = BP.coords == FLAT;
     if (flat) { k[4] = 0; k[5] = ~0ll; }
 #pragma unroll 4
     for (int i = ch.cs + threadIdx.x; i < ch.ce; i += CB) {
@@ -359,82 +449,160 @@ __global__ void __launch_bounds__(CB) k_chunk_pass1(const Chunk* chunks, const B
         r.xmin = dunkey(shk[0][0]); r.xmax = dunkey(~shk[0][1]);
         r.ymin = dunkey(shk[0][2]); r.ymax = dunkey(~shk[0][3]);
         r.zmin = dunkey(shk[0][4]); r.zmax = dunkey(~shk[0][5]);
-        out[blockIdx.x] = r;
+        L.part1[blockIdx.x] = r;
     }
+    if (task_complete(L, ch.task, L.tchunk[lev & 1][ch.task].y, &flag) && threadIdx.x < 32)
+        task_combine1(L, lev, ch.task, P0, P1, BP);
 }
 
-// One warp per cooperative task: centroid, weight, split axis and value.
-__global__ void k_task_combine1(int ntask, const BuildTask* tasks, const int* chunk0,
-                                const Part1* part, Points P0, Points P1, BuildParams BP,
-                                TaskStats* st)
+// One warp: finishes task t's cell, decides, sets the scatter offsets of its chunks and appends
+// the children to the next level or to the small cells.
+__device__ void task_combine2(const LevelBufs& L, int lev, int t, const BuildParams& BP, const Cells& C,
+                              int* tops, int* ntop, int* err)
 {
-    int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (t >= ntask) return;
-    int c0 = chunk0[t], c1 = chunk0[t + 1];
-    double sx = 0., sy = 0., sz = 0., swp = 0., sw = 0.;
-    double xmin = DBL_MAX, ymin = DBL_MAX, zmin = DBL_MAX;
-    double xmax = -DBL_MAX, ymax = -DBL_MAX, zmax = -DBL_MAX;
-    for (int c = c0 + lane; c < c1; c += 32) {
-        const Part1& p = part[c];
-        sx += p.sx; sy += p.sy; sz += p.sz; swp += p.swp; sw += p.sw;
-        xmin = fmin(xmin, p.xmin); xmax = fmax(xmax, p.xmax);
-        ymin = fmin(ymin, p.ymin); ymax = fmax(ymax, p.ymax);
-        zmin = fmin(zmin, p.zmin); zmax = fmax(zmax, p.zmax);
+    const int lane = threadIdx.x & 31;
+    const BuildTask tk = L.tasks[lev & 1][t];
+    const int2 tc = L.tchunk[lev & 1][t];
+    TaskStats s = L.stats[t];
+    Chunk* chunks = L.chunks[lev & 1] + tc.x;
+    const Part2* part = L.part2 + tc.x;
+    long long ks = dkey(0.);
+    double pp[2] = {0., 0.};
+    int nleft = 0;
+    for (int c = lane; c < tc.y; c += 32) {
+        ks = max(ks, dkey(ldcg(&part[c].sizesq)));
+        pp[0] += ldcg(&part[c].pr); pp[1] += ldcg(&part[c].pi);
+        nleft += __ldcg(&part[c].nleft);
     }
-    sx = warp_sum(sx); sy = warp_sum(sy); sz = warp_sum(sz); swp = warp_sum(swp); sw = warp_sum(sw);
-    xmin = warp_min(xmin); ymin = warp_min(ymin); zmin = warp_min(zmin);
-    xmax = warp_max(xmax); ymax = warp_max(ymax); zmax = warp_max(zmax);
-    if (lane) return;
-    const BuildTask tk = tasks[t];
-    const Points& P = tk.buf ? P1 : P0;
-    TaskStats s;
-    // BuildCellData, src/Cell.cpp:170-200.
-    if (swp != 0.) {
-        s.cx = sx / swp; s.cy = sy / swp; s.cz = sz / swp;
-        if (BP.coords == SPHERE) normalize3(s.cx, s.cy, s.cz);
-    } else {
-        s.cx = P.x[tk.s]; s.cy = P.y[tk.s]; s.cz = P.z[tk.s];
+    const double sizesq = dunkey(warp_kmax(ks));
+    warp_sums<2>(pp, lane);
+    nleft = warp_isum(nleft);
+    const int n = tk.e - tk.s;
+    bool is_top;
+    int intop = tk.intop;
+    bool split = decide_split(BP, intop, tk.mintop, tk.maxtop, sizesq, is_top);
+    int mid = tk.s + nleft;
+    int byindex = 0;
+    bool handed = false;
+    if (split && (nleft == 0 || nleft == n)) {
+        // SplitData falls back to Median when the mean puts everything on one side
+        // (src/Cell.cpp:526-551).  On a cooperative level this is only done when every
+        // point shares the split coordinate, where any order is a valid nth_element; other
+        // cells of at most SMALL points go to k_subtree as they are, which ranks the points.
+        if (s.allsame) { mid = (tk.s + tk.e) / 2; byindex = 1; }
+        else if (n <= SMALL) { handed = true; split = false; }
+        else { if (lane == 0) set_err(err, DEV_DEGENERATE_SPLIT); split = false; }
     }
-    s.w = float(sw);
-    s.axis = split_axis(BP.coords, xmax - xmin, ymax - ymin, zmax - zmin);
-    if (BP.split == MIDDLE) {   // Bounds::getMiddle, include/Bounds.h:67-68
-        s.splitval = s.axis == 2 ? (zmax + zmin) / 2. : s.axis == 1 ? (ymax + ymin) / 2.
-                                                                     : (xmax + xmin) / 2.;
-    } else {                    // Mean: the centroid, src/Cell.cpp:481-495
-        s.splitval = s.axis == 2 ? s.cz : s.axis == 1 ? s.cy : s.cx;
+    float d1 = float(pp[0]), d2 = float(pp[1]);
+    if (BP.dkind == DN) { d1 = 0.f; d2 = 0.f; }
+    if (BP.dkind == DK) d2 = 0.f;
+    const int id = split ? mid - 1 : (BP.n - 1) + tk.s;
+    if (lane == 0) {
+        if (handed) {
+            L.small[atomicAdd(L.nsmall, 1)] = tk;
+        } else {
+            write_cell(C, id, s.cx, s.cy, s.cz, split ? cell_size(BP, sizesq) : 0.f, s.w, d1, d2, n,
+                       tk.s, tk.parent, tk.side);
+            if (is_top) add_top(tops, ntop, id, tk.s);
+        }
+        s.mid = split ? mid : -1;
+        s.copy = (!split && !handed && tk.buf == 1) ? 1 : 0;
+        s.byindex = byindex;
+        L.stats[t] = s;
     }
-    // Remember whether all points share the split coordinate (needed by the fallback).
-    double lo = s.axis == 2 ? zmin : s.axis == 1 ? ymin : xmin;
-    double hi = s.axis == 2 ? zmax : s.axis == 1 ? ymax : xmax;
-    s.allsame = (lo == hi) ? 1 : 0;
-    s.mid = -1;
-    s.copy = 0;
-    s.byindex = 0;
-    st[t] = s;
+    if (!split) return;
+    // Chunk offsets for the stable scatter.
+    int loff = 0, roff = 0;
+    for (int b = 0; b < tc.y; b += 32) {
+        const int c = b + lane;
+        int nl = 0, len = 0;
+        if (c < tc.y) {
+            const int cs = chunks[c].cs, ce = chunks[c].ce;
+            nl = byindex ? max(0, min(ce, mid) - cs) : __ldcg(&part[c].nleft);
+            len = ce - cs;
+        }
+        int xl = nl, xa = len;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, xl, o), e = __shfl_up_sync(0xffffffffu, xa, o);
+            if (lane >= o) { xl += a; xa += e; }
+        }
+        if (c < tc.y) {
+            chunks[c].leftoff = loff + xl - nl;
+            chunks[c].rightoff = roff + (xa - xl) - (len - nl);
+        }
+        const int tl = __shfl_sync(0xffffffffu, xl, 31), ta = __shfl_sync(0xffffffffu, xa, 31);
+        loff += tl;
+        roff += ta - tl;
+    }
+    for (int k = 0; k < 2; ++k) {
+        BuildTask c = tk;
+        if (k == 0) c.e = mid;
+        else c.s = mid;
+        c.parent = id;
+        c.side = k;
+        c.intop = intop;
+        c.mintop = tk.mintop - 1;
+        c.maxtop = tk.maxtop - 1;
+        c.buf = tk.buf ^ 1;
+        const int m = c.e - c.s;
+        if (m <= L.sub) {
+            if (lane == 0) L.small[atomicAdd(L.nsmall, 1)] = c;
+            continue;
+        }
+        const int nc = (m + L.ch - 1) / L.ch;
+        int at = 0, first = 0;
+        if (lane == 0) {
+            at = atomicAdd(&L.cnt[lev + 1].x, 1);
+            first = atomicAdd(&L.cnt[lev + 1].y, nc);
+        }
+        at = __shfl_sync(0xffffffffu, at, 0);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (at >= L.cap_tasks || first + nc > L.cap_chunks) {      // (sized for any split)
+            if (lane == 0) set_err(err, DEV_TASK_OVERFLOW);
+            return;
+        }
+        if (lane == 0) {
+            L.tasks[(lev + 1) & 1][at] = c;
+            L.tchunk[(lev + 1) & 1][at] = make_int2(first, nc);
+        }
+        for (int q = lane; q < nc; q += 32) {
+            Chunk w;
+            w.task = at; w.cs = c.s + q * L.ch; w.ce = min(w.cs + L.ch, c.e);
+            w.leftoff = w.rightoff = 0;
+            L.chunks[(lev + 1) & 1][first + q] = w;
+        }
+    }
 }
 
-__global__ void __launch_bounds__(CB) k_chunk_pass2(const Chunk* chunks, const BuildTask* tasks,
-                                                     const TaskStats* st, Points P0, Points P1,
-                                                     int coords, int dkind, int spin, Part2* out)
+// center != 0: only the largest distance from the centroid, into stats (field_center).
+__global__ void __launch_bounds__(CB) k_chunk_pass2(LevelBufs L, int lev, Points P0, Points P1,
+                                                     BuildParams BP, Cells C, int* tops, int* ntop,
+                                                     int* err, int center)
 {
     __shared__ double sh[CB / 32][3];
     __shared__ int shi[CB / 32];
-    const Chunk ch = chunks[blockIdx.x];
-    const TaskStats s = st[ch.task];
-    const Points& P = tasks[ch.task].buf ? P1 : P0;
+    __shared__ int flag;
+    if ((int)blockIdx.x >= L.cnt[lev].y) return;
+    const Chunk ch = L.chunks[lev & 1][blockIdx.x];
+    const TaskStats s = L.stats[ch.task];
+    const Points& P = L.tasks[lev & 1][ch.task].buf ? P1 : P0;
+    const int coords = BP.coords, dkind = center ? DN : BP.dkind, spin = BP.spin;
     double cx = s.cx, cy = s.cy, cz = s.cz;
     double tcx = cx, tcy = cy, tcz = cz;
     if (coords == THREED) normalize3(tcx, tcy, tcz);
-    double sizesq = 0., pr = 0., pi = 0.;
+    long long ks = dkey(0.);
+    const long long ksplit = dkey(s.splitval);
+    const bool splits0 = 0. < s.splitval;
+    double pr = 0., pi = 0.;
     int nleft = 0;
     for (int i = ch.cs + threadIdx.x; i < ch.ce; i += CB) {
         double px = P.x[i], py = P.y[i], pz = P.z[i];
         double d = (cx - px) * (cx - px) + (cy - py) * (cy - py);
         if (coords != FLAT) d += (cz - pz) * (cz - pz);
-        sizesq = fmax(sizesq, d);
+        ks = max(ks, dkey(d));
         double c = s.axis == 2 ? pz : s.axis == 1 ? py : px;
-        nleft += (c < s.splitval) ? 1 : 0;
+        // (0 and -0 are equal, their keys are not)
+        nleft += ((__double_as_longlong(c) << 1) == 0 ? splits0 : dkey(c) < ksplit) ? 1 : 0;
         if (dkind == DK) {
             pr += P.d1[i];
         } else if (dkind == DG) {
@@ -443,7 +611,7 @@ __global__ void __launch_bounds__(CB) k_chunk_pass2(const Chunk* chunks, const B
         }
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    sizesq = dunkey(warp_kmax(dkey(sizesq)));
+    const double sizesq = dunkey(warp_kmax(ks));
     double pp[2] = {pr, pi};
     if (dkind != DN) warp_sums<2>(pp, lane);
     nleft = warp_isum(nleft);
@@ -458,90 +626,29 @@ __global__ void __launch_bounds__(CB) k_chunk_pass2(const Chunk* chunks, const B
             r.pr += sh[w][1]; r.pi += sh[w][2];
             r.nleft += shi[w];
         }
-        out[blockIdx.x] = r;
+        L.part2[blockIdx.x] = r;
     }
-}
-
-// One thread per cooperative task: finish the cell, decide, emit children, and set the
-// scatter offsets of its chunks.
-__global__ void k_task_combine2(int ntask, BuildTask* tasks, const int* chunk0, Chunk* chunks,
-                                const Part2* part, TaskStats* st, BuildParams BP, Cells C,
-                                int* tops, int* ntop, BuildTask* big_out, int* nbig_out,
-                                BuildTask* small_out, int* nsmall_out, int* err)
-{
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntask) return;
-    BuildTask tk = tasks[t];
-    TaskStats s = st[t];
-    int c0 = chunk0[t], c1 = chunk0[t + 1];
-    double sizesq = 0., pr = 0., pi = 0.;
-    int nleft = 0;
-    for (int c = c0; c < c1; ++c) {
-        sizesq = fmax(sizesq, part[c].sizesq);
-        pr += part[c].pr; pi += part[c].pi;
-        nleft += part[c].nleft;
+    const int2 tc = L.tchunk[lev & 1][ch.task];
+    if (!task_complete(L, ch.task, tc.y, &flag) || threadIdx.x >= 32) return;
+    if (!center) {
+        task_combine2(L, lev, ch.task, BP, C, tops, ntop, err);
+        return;
     }
-    const int n = tk.e - tk.s;
-    bool is_top;
-    int intop = tk.intop;
-    bool split = decide_split(BP, intop, tk.mintop, tk.maxtop, sizesq, is_top);
-    int mid = tk.s + nleft;
-    int byindex = 0;
-    if (split && (nleft == 0 || nleft == n)) {
-        // SplitData falls back to Median when the mean puts everything on one side
-        // (src/Cell.cpp:526-551).  On a cooperative level this is only done when every
-        // point shares the split coordinate, where any order is a valid nth_element.
-        if (s.allsame) { mid = (tk.s + tk.e) / 2; byindex = 1; }
-        else { set_err(err, DEV_DEGENERATE_SPLIT); split = false; }
-    }
-    float d1 = float(pr), d2 = float(pi);
-    if (BP.dkind == DN) { d1 = 0.f; d2 = 0.f; }
-    if (BP.dkind == DK) d2 = 0.f;
-    int id = split ? mid - 1 : (BP.n - 1) + tk.s;
-    write_cell(C, id, s.cx, s.cy, s.cz, split ? cell_size(BP, sizesq) : 0.f, s.w, d1, d2, n,
-               tk.s, tk.parent, tk.side);
-    if (is_top) add_top(tops, ntop, id, tk.s);
-    s.mid = split ? mid : -1;
-    s.copy = (!split && tk.buf == 1) ? 1 : 0;
-    s.byindex = byindex;
-    st[t] = s;
-    // Chunk offsets for the stable scatter.
-    if (split) {
-        int loff = 0, roff = 0;
-        for (int c = c0; c < c1; ++c) {
-            chunks[c].leftoff = loff;
-            chunks[c].rightoff = roff;
-            int cs = chunks[c].cs, ce = chunks[c].ce;
-            int nl = byindex ? max(0, min(ce, mid) - cs) : part[c].nleft;
-            loff += nl;
-            roff += (ce - cs) - nl;
-        }
-        BuildTask L = tk, R = tk;
-        L.e = mid; R.s = mid;
-        L.parent = R.parent = id;
-        L.side = 0; R.side = 1;
-        L.intop = R.intop = intop;
-        L.mintop = R.mintop = tk.mintop - 1;
-        L.maxtop = R.maxtop = tk.maxtop - 1;
-        L.buf = R.buf = tk.buf ^ 1;
-        BuildTask* kids[2] = {&L, &R};
-        for (int k = 0; k < 2; ++k) {
-            BuildTask& c = *kids[k];
-            if (c.e - c.s > SMALL && BP.split != MEDIAN) big_out[atomicAdd(nbig_out, 1)] = c;
-            else small_out[atomicAdd(nsmall_out, 1)] = c;
-        }
-    }
+    long long m = dkey(0.);
+    for (int c = lane; c < tc.y; c += 32) m = max(m, dkey(ldcg(&L.part2[tc.x + c].sizesq)));
+    m = warp_kmax(m);
+    if (lane == 0) L.stats[ch.task].sizesq = dunkey(m);
 }
 
 // Stable partition of each split chunk into the other buffer (or a copy of a leaf's
 // points into buffer 0).
-__global__ void __launch_bounds__(CB) k_chunk_scatter(const Chunk* chunks, const BuildTask* tasks,
-                                                       const TaskStats* st, Points P0, Points P1)
+__global__ void __launch_bounds__(CB) k_chunk_scatter(LevelBufs L, int lev, Points P0, Points P1)
 {
     __shared__ int wsum[2][CB / 32];
-    const Chunk ch = chunks[blockIdx.x];
-    const BuildTask tk = tasks[ch.task];
-    const TaskStats s = st[ch.task];
+    if ((int)blockIdx.x >= L.cnt[lev].y) return;
+    const Chunk ch = L.chunks[lev & 1][blockIdx.x];
+    const BuildTask tk = L.tasks[lev & 1][ch.task];
+    const TaskStats s = L.stats[ch.task];
     const Points& A = tk.buf ? P1 : P0;
     const Points& B = tk.buf ? P0 : P1;
     if (s.mid < 0) {
@@ -1233,101 +1340,141 @@ void launch_validate_tree(int ncap, const Cells& C, const int* tops, int ntop, i
 // ---------------------------------------------------------------------------------------
 // Host orchestration.
 
-int scratch_ensure_level(BuildScratch& S, int nt, int nc)
+// Points per chunk and most points of a cell left to one block: the largest up to CH and SMALL,
+// and for fewer than 300 SMALL points as much smaller as gives two blocks to every SM (FP64 runs at
+// 2 lanes per clock and SM, so that the work has to be spread).
+// Whole builds of a spin-2 field on the sphere, against chunks of 4096 and cells of 2048 points with
+// the host in every level: 25,000 points 1.63 -> 0.93 ms, 200,000 2.0 -> 1.55, 10M 43.9 -> 40.5.
+constexpr int BUILD_LEVELS = 64;    // levels counted before the host looks again at the latest
+
+static int spread(int n, int least, int most)
 {
-    if (nt > S.cap_tasks) {
-        int cap = std::max(nt, 2 * S.cap_tasks);
-        dfree(S.tasks); dfree(S.chunk0); dfree(S.stats); dfree(S.big_next);
-        TC_TRY(dalloc(&S.tasks, cap));
-        TC_TRY(dalloc(&S.chunk0, cap + 1));
-        TC_TRY(dalloc(&S.stats, cap));
-        TC_TRY(dalloc(&S.big_next, 2 * (size_t)cap + 2));
-        S.cap_tasks = cap;
-    }
-    if (nc > S.cap_chunks) {
-        int cap = std::max(nc, 2 * S.cap_chunks);
-        dfree(S.chunks); dfree(S.part1); dfree(S.part2);
-        TC_TRY(dalloc(&S.chunks, cap));
-        TC_TRY(dalloc(&S.part1, cap));
-        TC_TRY(dalloc(&S.part2, cap));
-        S.cap_chunks = cap;
-    }
+    const int want = n / 304;
+    int v = least;
+    while (v < want && v < most) v <<= 1;
+    return std::min(v, most);
+}
+
+// Arrays for the cooperative levels of n points (a level's cells are disjoint, each above L.sub
+// points).
+static int scratch_levels(int n, BuildScratch& S, cudaStream_t st)
+{
+    if (S.level_mem) return 0;
+    LevelBufs& L = S.L;
+    L.ch = spread(n, 512, CH);
+    L.sub = spread(n, 256, SMALL);
+    L.cap_tasks = n / L.sub + 2;
+    L.cap_chunks = n / L.ch + L.cap_tasks + 1;
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
+    const size_t nt = L.cap_tasks, nc = L.cap_chunks;
+    const size_t o_cnt = take(sizeof(int2) * (BUILD_LEVELS + 1)), o_small = take(sizeof(int)), o_done = take(sizeof(int) * nt);
+    const size_t zeroed = off;
+    const size_t o_t0 = take(sizeof(BuildTask) * nt), o_t1 = take(sizeof(BuildTask) * nt);
+    const size_t o_k0 = take(sizeof(int2) * nt), o_k1 = take(sizeof(int2) * nt);
+    const size_t o_c0 = take(sizeof(Chunk) * nc), o_c1 = take(sizeof(Chunk) * nc);
+    const size_t o_p1 = take(sizeof(Part1) * nc), o_p2 = take(sizeof(Part2) * nc);
+    const size_t o_st = take(sizeof(TaskStats) * nt);
+    unsigned char* m = nullptr;
+    TC_TRY(dalloc(&m, off));
+    S.level_mem = m;
+    L.cnt = reinterpret_cast<int2*>(m + o_cnt);
+    L.nsmall = reinterpret_cast<int*>(m + o_small);
+    L.done = reinterpret_cast<int*>(m + o_done);
+    L.tasks[0] = reinterpret_cast<BuildTask*>(m + o_t0);
+    L.tasks[1] = reinterpret_cast<BuildTask*>(m + o_t1);
+    L.tchunk[0] = reinterpret_cast<int2*>(m + o_k0);
+    L.tchunk[1] = reinterpret_cast<int2*>(m + o_k1);
+    L.chunks[0] = reinterpret_cast<Chunk*>(m + o_c0);
+    L.chunks[1] = reinterpret_cast<Chunk*>(m + o_c1);
+    L.part1 = reinterpret_cast<Part1*>(m + o_p1);
+    L.part2 = reinterpret_cast<Part2*>(m + o_p2);
+    L.stats = reinterpret_cast<TaskStats*>(m + o_st);
+    TC_CU(cudaMemsetAsync(m, 0, zeroed, st));
     return 0;
 }
 
-int build_tree(const BuildParams& BP, Points bufs[2], Cells C, int* d_tops, int* d_ntop,
+static int launch_root(const BuildTask& root, const LevelBufs& L, cudaStream_t st)
+{
+    const int nc = (root.e - root.s + L.ch - 1) / L.ch;
+    count_launch();
+    k_level_root<<<(nc + 255) / 256, 256, 0, st>>>(L, root);
+    TC_CU(cudaGetLastError());
+    return nc;
+}
+
+int build_tree(const BuildParams& BP, Points bufs[2], Cells C, TCell* tcells, int* d_tops, int* d_ntop,
                BuildScratch& S, cudaStream_t st, std::vector<int>& tops_out, int* d_err,
                int mintop, int maxtop)
 {
     const int n = BP.n;
-    std::vector<BuildTask> big;
     BuildTask root;
     root.s = 0; root.e = n; root.parent = -1; root.side = 0;
     root.mintop = mintop; root.maxtop = maxtop; root.intop = 1; root.buf = 0;
-    std::vector<BuildTask> small_host;
+    TC_TRY(scratch_levels(n, S, st));
+    LevelBufs& L = S.L;
     int nsmall = 0;
     TC_CU(cudaMemsetAsync(d_ntop, 0, sizeof(int), st));
-    TC_CU(cudaMemsetAsync(S.counters, 0, 2 * sizeof(int), st));
-    if (n > SMALL && BP.split != MEDIAN) big.push_back(root);
-    else if (n > SMALL) {
+    TC_CU(cudaMemsetAsync(L.cnt, 0, sizeof(int2) * (BUILD_LEVELS + 1), st));   // (field_center's)
+    TC_CU(cudaMemsetAsync(L.nsmall, 0, sizeof(int), st));
+    if (n > SMALL && BP.split == MEDIAN) {
         count_launch();
         k_median_levels<<<1, 32, 0, st>>>(root, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
-                                          S.small, S.counters + 1, d_err);
+                                          L.small, L.nsmall, d_err);
         TC_CU(cudaGetLastError());
-        TC_CU(cudaMemcpyAsync(&nsmall, S.counters + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TC_CU(cudaMemcpyAsync(&nsmall, L.nsmall, sizeof(int), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaStreamSynchronize(st));
-    } else {
-        TC_CU(cudaMemcpyAsync(S.small, &root, sizeof(BuildTask), cudaMemcpyHostToDevice, st));
+    } else if (n <= L.sub || BP.split == MEDIAN) {
+        TC_CU(cudaMemcpyAsync(L.small, &root, sizeof(BuildTask), cudaMemcpyHostToDevice, st));
         nsmall = 1;
-        TC_CU(cudaMemcpyAsync(S.counters + 1, &nsmall, sizeof(int), cudaMemcpyHostToDevice, st));
-    }
-    while (!big.empty()) {
-        int nt = (int)big.size();
-        std::vector<int> c0(nt + 1);
-        std::vector<Chunk> chunks;
-        for (int t = 0; t < nt; ++t) {
-            c0[t] = (int)chunks.size();
-            for (int cs = big[t].s; cs < big[t].e; cs += CH) {
-                Chunk c; c.task = t; c.cs = cs; c.ce = std::min(cs + CH, big[t].e);
-                c.leftoff = c.rightoff = 0;
-                chunks.push_back(c);
+    } else {
+        // All the levels that even splits need, and a few more, are in the queue before the
+        // host looks; the kernels of levels without tasks return at once.
+        launch_root(root, L, st);
+        int batch = 2;
+        for (int m = L.sub; m < n; m = m > (1 << 29) ? n : 2 * m) ++batch;
+        for (int lev = 0, total = 0;; batch = 8) {
+            const int end = std::min(lev + batch, BUILD_LEVELS);
+            for (; lev < end; ++lev, ++total) {
+                // No more than 2^level tasks: most chunks of a level, so the grid.
+                const int tasks = total < 30 ? std::min(1 << total, L.cap_tasks) : L.cap_tasks;
+                const int nc = std::min(n / L.ch + tasks, L.cap_chunks);
+                count_launch(); k_chunk_pass1<<<nc, CB, 0, st>>>(L, lev, bufs[0], bufs[1], BP);
+                count_launch(); k_chunk_pass2<<<nc, CB, 0, st>>>(L, lev, bufs[0], bufs[1], BP, C, d_tops,
+                                                                 d_ntop, d_err, 0);
+                count_launch(); k_chunk_scatter<<<nc, CB, 0, st>>>(L, lev, bufs[0], bufs[1]);
+            }
+            TC_CU(cudaGetLastError());
+            int2 left = make_int2(0, 0);
+            TC_CU(cudaMemcpyAsync(&left, L.cnt + lev, sizeof(int2), cudaMemcpyDeviceToHost, st));
+            TC_CU(cudaMemcpyAsync(&nsmall, L.nsmall, sizeof(int), cudaMemcpyDeviceToHost, st));
+            TC_CU(cudaStreamSynchronize(st));
+            if (left.x == 0) break;
+            if (lev == BUILD_LEVELS) {
+                // (an even number of levels: the arrays' turns go on)
+                TC_CU(cudaMemsetAsync(L.cnt, 0, sizeof(int2) * (BUILD_LEVELS + 1), st));
+                TC_CU(cudaMemcpyAsync(L.cnt, &left, sizeof(int2), cudaMemcpyHostToDevice, st));
+                TC_CU(cudaStreamSynchronize(st));
+                lev = 0;
             }
         }
-        c0[nt] = (int)chunks.size();
-        int nc = (int)chunks.size();
-        TC_TRY(scratch_ensure_level(S, nt, nc));
-        TC_CU(cudaMemcpyAsync(S.tasks, big.data(), nt * sizeof(BuildTask), cudaMemcpyHostToDevice, st));
-        TC_CU(cudaMemcpyAsync(S.chunk0, c0.data(), (nt + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-        TC_CU(cudaMemcpyAsync(S.chunks, chunks.data(), nc * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-        TC_CU(cudaMemsetAsync(S.counters, 0, sizeof(int), st));   // next big count
-        count_launch(); k_chunk_pass1<<<nc, CB, 0, st>>>(S.chunks, S.tasks, bufs[0], bufs[1], BP.coords, S.part1);
-        count_launch(); k_task_combine1<<<(nt * 32 + 255) / 256, 256, 0, st>>>(nt, S.tasks, S.chunk0, S.part1,
-                                                                bufs[0], bufs[1], BP, S.stats);
-        count_launch(); k_chunk_pass2<<<nc, CB, 0, st>>>(S.chunks, S.tasks, S.stats, bufs[0], bufs[1], BP.coords,
-                                         BP.dkind, BP.spin, S.part2);
-        count_launch(); k_task_combine2<<<(nt + 127) / 128, 128, 0, st>>>(nt, S.tasks, S.chunk0, S.chunks, S.part2,
-                                                          S.stats, BP, C, d_tops, d_ntop, S.big_next,
-                                                          S.counters, S.small + 0, S.counters + 1,
-                                                          d_err);
-        count_launch(); k_chunk_scatter<<<nc, CB, 0, st>>>(S.chunks, S.tasks, S.stats, bufs[0], bufs[1]);
-        TC_CU(cudaGetLastError());
-        int cnt[2];
-        TC_CU(cudaMemcpyAsync(cnt, S.counters, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-        TC_CU(cudaStreamSynchronize(st));
-        big.resize(cnt[0]);
-        if (cnt[0] > 0)
-            TC_CU(cudaMemcpy(big.data(), S.big_next, cnt[0] * sizeof(BuildTask), cudaMemcpyDeviceToHost));
-        nsmall = cnt[1];
     }
     if (nsmall > 0)
-        TC_TRY(launch_subtrees(nsmall, S.small, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
+        TC_TRY(launch_subtrees(nsmall, L.small, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
                                d_err, st));
+    launch_pack_cells(2 * n - 1, C, tcells, st);
+    TC_CU(cudaGetLastError());
     int ntop = 0;
+    constexpr int FIRST = 1024;     // tops read along with their number
+    std::vector<int> pairs(2 * (size_t)std::min(n, FIRST));
     TC_CU(cudaMemcpyAsync(&ntop, d_ntop, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaMemcpyAsync(pairs.data(), d_tops, sizeof(int) * pairs.size(), cudaMemcpyDeviceToHost, st));
     TC_CU(cudaStreamSynchronize(st));
-    std::vector<int> pairs(2 * (size_t)ntop);
-    if (ntop > 0)
-        TC_CU(cudaMemcpy(pairs.data(), d_tops, 2 * sizeof(int) * ntop, cudaMemcpyDeviceToHost));
+    if (ntop > FIRST) {
+        pairs.resize(2 * (size_t)ntop);
+        TC_CU(cudaMemcpyAsync(pairs.data(), d_tops, 2 * sizeof(int) * ntop, cudaMemcpyDeviceToHost, st));
+        TC_CU(cudaStreamSynchronize(st));
+    }
     // Tops in the reference's depth-first order = increasing first point (left before right).
     std::vector<std::pair<int, int>> v(ntop);
     for (int k = 0; k < ntop; ++k) v[k] = {pairs[2 * k], pairs[2 * k + 1]};
@@ -1354,33 +1501,17 @@ int field_center(const BuildParams& BP, Points P, BuildScratch& S, cudaStream_t 
     BuildTask root;
     root.s = 0; root.e = n; root.parent = -1; root.side = 0;
     root.mintop = 0; root.maxtop = 0; root.intop = 0; root.buf = 0;
-    std::vector<int> c0(2);
-    std::vector<Chunk> chunks;
-    for (int cs = 0; cs < n; cs += CH) {
-        Chunk c; c.task = 0; c.cs = cs; c.ce = std::min(cs + CH, n); c.leftoff = c.rightoff = 0;
-        chunks.push_back(c);
-    }
-    c0[0] = 0; c0[1] = (int)chunks.size();
-    int nc = (int)chunks.size();
-    TC_TRY(scratch_ensure_level(S, 1, nc));
-    Points Pn = P;
-    TC_CU(cudaMemcpyAsync(S.tasks, &root, sizeof(BuildTask), cudaMemcpyHostToDevice, st));
-    TC_CU(cudaMemcpyAsync(S.chunk0, c0.data(), 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-    TC_CU(cudaMemcpyAsync(S.chunks, chunks.data(), nc * sizeof(Chunk), cudaMemcpyHostToDevice, st));
+    TC_TRY(scratch_levels(n, S, st));
     BuildParams B2 = BP;
     B2.split = MEAN;
-    count_launch(); k_chunk_pass1<<<nc, CB, 0, st>>>(S.chunks, S.tasks, Pn, Pn, BP.coords, S.part1);
-    count_launch(); k_task_combine1<<<1, 32, 0, st>>>(1, S.tasks, S.chunk0, S.part1, Pn, Pn, B2, S.stats);
-    count_launch(); k_chunk_pass2<<<nc, CB, 0, st>>>(S.chunks, S.tasks, S.stats, Pn, Pn, BP.coords, DN, 0, S.part2);
+    const int nc = launch_root(root, S.L, st);
+    count_launch(); k_chunk_pass1<<<nc, CB, 0, st>>>(S.L, 0, P, P, B2);
+    count_launch(); k_chunk_pass2<<<nc, CB, 0, st>>>(S.L, 0, P, P, B2, Cells{}, nullptr, nullptr, nullptr, 1);
     TC_CU(cudaGetLastError());
-    std::vector<Part2> p2(nc);
     TaskStats ts;
-    TC_CU(cudaMemcpyAsync(p2.data(), S.part2, nc * sizeof(Part2), cudaMemcpyDeviceToHost, st));
-    TC_CU(cudaMemcpyAsync(&ts, S.stats, sizeof(TaskStats), cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaMemcpyAsync(&ts, S.L.stats, sizeof(TaskStats), cudaMemcpyDeviceToHost, st));
     TC_CU(cudaStreamSynchronize(st));
-    double sizesq = 0.;
-    for (int c = 0; c < nc; ++c) sizesq = std::max(sizesq, p2[c].sizesq);
-    out[0] = ts.cx; out[1] = ts.cy; out[2] = ts.cz; out[3] = sizesq;
+    out[0] = ts.cx; out[1] = ts.cy; out[2] = ts.cz; out[3] = ts.sizesq;
     return 0;
 }
 
