@@ -37,25 +37,36 @@ namespace {
 
 constexpr int KB = 128;             // threads of a walk block
 constexpr int KW = KB / 32;
-// Resident blocks per SM the registers are sized for, measured per class family: 72 registers
-// for the families with their own products, 96 for the generic projections.
-constexpr int walk_minb(int kind) { return kind == 3 ? 5 : 7; }
+// Resident blocks per SM the registers are sized for, measured per class family.  7: 72 registers
+// (KK 300K 3-d 9.9 ms; 10.4 with 6).  NN 6: 2M clumped 18.2 ms; 19.0 with 7.  GG 7: 10M 530 ms; 530 with
+// 6, 540 with 5, 592 with 4.  The generic projections 5: 96 registers.
+constexpr int walk_minb(int kind) { return kind == 3 ? 5 : kind == 0 ? 6 : 7; }
 constexpr double W_PER_LN = 2.8853900817779268;    // 2 / ln 2
 constexpr int WFLUSH = 32;          // iterations between flushes of the register bins
 constexpr int WDRAINS = 8;        // lists added to the FP32 sums between their flushes
-constexpr int MCAP = 32;            // entries of the list of other bins
+// Entries of the list of other bins (at least the 32 that an iteration can add).  64 for the kinds
+// of few sums; what GG would gain, its records lose in L1 (10M: 530 ms at 32, 545 at 64).
+constexpr int walk_mcap(int kind) { return kind <= 1 ? 64 : 32; }
 constexpr int UCAP = 64;            // pairs waiting for the FP64 decision
 constexpr int MST = 9;              // words per entry (odd: no bank conflicts)
 constexpr unsigned NSMALL = 1u << 21;  // n1 n2 below this is counted in 32 bits between flushes:
-                                       // 32 iterations x 32 lanes, or 8 lists of 32, hold it
+                                       // 32 iterations x 32 lanes, or 8 lists of 64, hold it
 
 enum { WG_FLAT = 0, WG_ARC = 1, WG_EUC = 2 };                // geometry (EUC: 3 coordinates)
 enum { WK_NN = 0, WK_SC = 1, WK_GG = 2, WK_GEN = 3 };        // class family
 
-__host__ __device__ inline size_t walk_warp_bytes(int nq, int nb)
+// Copies of the FP32 sums of other bins: so many entries of the list are added at once, by 8
+// lanes each (an entry is a chain of a load, an addition and a store; one at a time they took a
+// sixth of the kernel's instructions).  As many as keep a warp's sums small, and one for GG:
+// the shared memory of four is missed as L1 (10M 590 ms, with one 530; KK 300K 3-d 10.7 -> 10.1, NN
+// 2M clumped 19.3 -> 18.6).
+__host__ __device__ inline int walk_copies(int kind, int nq, int nb)
+{ return kind == WK_GG ? 1 : nq * nb <= 128 ? 4 : nq * nb <= 256 ? 2 : 1; }
+
+__host__ __device__ inline size_t walk_warp_bytes(int kind, int nq, int nb)
 {
-    return ((size_t)nq * nb * 8 + (size_t)nb * 8 + (size_t)nq * nb * 4 + (size_t)nb * 4 +
-            MCAP * MST * 4 + UCAP * 8 + 15) & ~(size_t)15;
+    return ((size_t)nq * nb * 8 + (size_t)nb * 8 + (size_t)walk_copies(kind, nq, nb) * nq * nb * 4 +
+            (size_t)nb * 4 + walk_mcap(kind) * MST * 4 + UCAP * 8 + 15) & ~(size_t)15;
 }
 
 // The FP64 decision (out of line: about one pair in 3000 takes it).  Returns the action, the
@@ -187,6 +198,15 @@ __device__ __forceinline__ void add_if(bool on, float (&acc)[8], unsigned& c, fl
             : "r"((unsigned)on), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]));
 }
 
+// Half a record (32 bytes, so one sector) in one load: the lanes' records lie in different
+// lines, and a load costs the L1 a cycle or so per line whatever it takes from it.
+__device__ __forceinline__ void load_half(const float4* p, float4& u, float4& v)
+{
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(p));
+}
+
 __device__ __forceinline__ void df_accumulate(float2* fd, float x)
 {
     float2 f = *fd;
@@ -214,14 +234,17 @@ __global__ void __launch_bounds__(KB, walk_minb(KIND)) k_walk(const __grid_const
 {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NQ = KIND == WK_NN ? 3 : KIND == WK_SC ? 4 : 7;   // values kept per bin
+    constexpr int MCAP = walk_mcap(KIND);
+    static_assert(MCAP >= 32, "");
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int nq = T.nqf, nb = T.nbins;      // nq <= NQ
-    unsigned char* wb = smem + wib * walk_warp_bytes(nq, nb);
+    unsigned char* wb = smem + wib * walk_warp_bytes(KIND, nq, nb);
     int2* ub = reinterpret_cast<int2*>(wb);                     // pairs for the FP64 decision
     float2* fd = reinterpret_cast<float2*>(ub + UCAP);          // the unit's sums
     unsigned long long* np = reinterpret_cast<unsigned long long*>(fd + nq * nb);
     float* fb = reinterpret_cast<float*>(np + nb);              // FP32 sums of other bins
-    unsigned* nb32 = reinterpret_cast<unsigned*>(fb + nq * nb); // their pairs, in 32 bits
+    const int copies = walk_copies(KIND, nq, nb), fbs = nq * nb;      // (their copies, fbs apart)
+    unsigned* nb32 = reinterpret_cast<unsigned*>(fb + copies * fbs); // their pairs, in 32 bits
     float* ml = reinterpret_cast<float*>(nb32 + nb);            // list of other bins' pairs
     int2* stk = W.stacks + (size_t)(blockIdx.x * KW + wib) * W.stack_cap;
     const unsigned lt = (1u << lane) - 1u;
@@ -249,9 +272,11 @@ __global__ void __launch_bounds__(KB, walk_minb(KIND)) k_walk(const __grid_const
         c0 = 0; c1 = 0; since = 0;
     };
     auto flush_fb = [&]() {
-        for (int q = lane; q < nq * nb; q += 32) {
-            const float x = fb[q];
-            if (x != 0.f) { df_accumulate(fd + q, x); fb[q] = 0.f; }
+        for (int q = lane; q < fbs; q += 32) {
+            float x = fb[q];
+            fb[q] = 0.f;
+            for (int c = 1; c < copies; ++c) { x += fb[c * fbs + q]; fb[c * fbs + q] = 0.f; }
+            if (x != 0.f) df_accumulate(fd + q, x);
         }
         for (int q = lane; q < nb; q += 32) { np[q] += nb32[q]; nb32[q] = 0u; }
         __syncwarp();
@@ -259,12 +284,13 @@ __global__ void __launch_bounds__(KB, walk_minb(KIND)) k_walk(const __grid_const
     };
     auto drain = [&]() {
         __syncwarp();
-        if (lane < nq) {
-            float* my = fb + lane * nb;
-#pragma unroll 4
-            for (int t = 0; t < mcount; ++t) {
+        const int q = lane & 7, g = lane >> 3;
+        if (q < nq && g < copies) {
+            float* my = fb + g * fbs + q * nb;
+#pragma unroll 2
+            for (int t = g; t < mcount; t += copies) {
                 const float* e = ml + t * MST;
-                my[__float_as_int(e[7])] += e[lane];
+                my[__float_as_int(e[7])] += e[q];
             }
         }
         mcount = 0;
@@ -291,7 +317,8 @@ __global__ void __launch_bounds__(KB, walk_minb(KIND)) k_walk(const __grid_const
             step = W.unit_off[lo + 1] - W.unit_off[lo];
             count = (unsigned)(T.proot_off[lo + 1] - T.proot_off[lo]);
         }
-        for (int q = lane; q < nq * nb; q += 32) { fd[q] = make_float2(0.f, 0.f); fb[q] = 0.f; }
+        for (int q = lane; q < nq * nb; q += 32) fd[q] = make_float2(0.f, 0.f);
+        for (int q = lane; q < copies * fbs; q += 32) fb[q] = 0.f;
         for (int q = lane; q < nb; q += 32) { np[q] = 0ull; nb32[q] = 0u; }
         __syncwarp();
         unsigned n_eval = 0, n_acc = 0, n_esc = 0;   // of the unit
@@ -343,7 +370,11 @@ __global__ void __launch_bounds__(KB, walk_minb(KIND)) k_walk(const __grid_const
             const bool self = j < 0;
             const TCell* A = T.c1 + i;
             const TCell* B = self ? A : T.c2 + j;
-            const float4 Aa = A->a, Ba = B->a, Ab = A->b, Bb = B->b, Ac = A->c, Bc = B->c;
+            float4 Aa, Ab, Ac, Ad, Ba, Bb, Bc, Bd;
+            load_half(&A->a, Aa, Ab);
+            load_half(&B->a, Ba, Bb);
+            load_half(&A->c, Ac, Ad);
+            load_half(&B->c, Bc, Bd);
             const bool live = has && Ab.w != 0.f && Bb.w != 0.f;
             const float dx = (Aa.x - Ba.x) + (Ab.x - Bb.x);
             const float dy = (Aa.y - Ba.y) + (Ab.y - Bb.y);
@@ -496,9 +527,9 @@ __global__ void __launch_bounds__(KB, walk_minb(KIND)) k_walk(const __grid_const
                 const unsigned m4 = __ballot_sync(0xffffffffu, split && both);
                 if (split || down) {
                     const int l1 = s1st ? __float_as_int(Ac.w) : i;
-                    const int r1 = s1st ? __float_as_int(A->d.x) : i;
+                    const int r1 = s1st ? __float_as_int(Ad.x) : i;
                     const int l2 = s2nd ? __float_as_int(Bc.w) : j;
-                    const int r2 = s2nd ? __float_as_int(B->d.x) : j;
+                    const int r2 = s2nd ? __float_as_int(Bd.x) : j;
                     int2* o = stk + sp + 2 * __popc(m2 & lt) + __popc(m3 & lt) + 2 * __popc(m4 & lt);
                     o[0] = make_int2(l1, down ? -1 : l2);
                     o[1] = make_int2(r1, down ? -1 : r2);
@@ -575,14 +606,23 @@ namespace {
 
 using WalkKernel = void (*)(TravParams, WalkParams);
 
+int walk_kind(const TravParams& T)
+{
+    if (T.k1 == DN && T.k2 == DN) return WK_NN;
+    if (T.k2 != DG) return WK_SC;
+    const bool euc = T.coords != FLAT && T.metric != ARC;
+    return !euc && T.k1 == DG && T.s1 == 2 && T.s2 == 2 ? WK_GG : WK_GEN;
+}
+
 template <int GEO, bool PATCH>
 WalkKernel pick_kind(const TravParams& T)
 {
-    if (T.k1 == DN && T.k2 == DN) return k_walk<GEO, WK_NN, PATCH>;
-    if (T.k2 != DG) return k_walk<GEO, WK_SC, PATCH>;
-    if (GEO != WG_EUC && T.k1 == DG && T.s1 == 2 && T.s2 == 2)
-        return k_walk<GEO, GEO == WG_EUC ? WK_GEN : WK_GG, PATCH>;
-    return k_walk<GEO, WK_GEN, PATCH>;
+    switch (walk_kind(T)) {
+      case WK_NN: return k_walk<GEO, WK_NN, PATCH>;
+      case WK_SC: return k_walk<GEO, WK_SC, PATCH>;
+      case WK_GG: return k_walk<GEO, GEO == WG_EUC ? WK_GEN : WK_GG, PATCH>;
+      default: return k_walk<GEO, WK_GEN, PATCH>;
+    }
 }
 
 template <bool PATCH>
@@ -626,7 +666,7 @@ int walk_grid(const TravParams& T, int* blocks, int* nwarps)
     int dev = 0, nsm = 0, per = 0;
     TC_CU(cudaGetDevice(&dev));
     TC_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const size_t sm = walk_warp_bytes(T.nqf, T.nbins) * KW;
+    const size_t sm = walk_warp_bytes(walk_kind(T), T.nqf, T.nbins) * KW;
     const WalkKernel k = pick(T);
     if (sm > 48 * 1024)
         TC_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -639,7 +679,7 @@ int walk_grid(const TravParams& T, int* blocks, int* nwarps)
 
 int launch_walk(const TravParams& T, const WalkParams& W, int blocks, cudaStream_t st)
 {
-    const size_t sm = walk_warp_bytes(T.nqf, T.nbins) * KW;
+    const size_t sm = walk_warp_bytes(walk_kind(T), T.nqf, T.nbins) * KW;
     count_launch();
     pick(T)<<<blocks, KB, sm, st>>>(T, W);
     TC_CU(cudaGetLastError());
