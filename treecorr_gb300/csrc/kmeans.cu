@@ -44,9 +44,10 @@ constexpr int KM_MAX_PATCH = 5000;  // per-warp shared accumulators must fit one
 constexpr int KM_NBLK = 304;        // accumulation blocks (fixed: the sum order depends on it)
 constexpr int KM_LTB = 256;         // threads per block of the level kernel
 constexpr int KM_LEVELS_PER_CHECK = 16;
-// Subtrees the walk should have: below, more levels are taken first (9 us each).  2,000,000 points,
-// 64 patches, 200 iterations: 37.0 ms at 512, 39.4 at 256, 37.6 at 1024.
-constexpr long long KM_UNITS = 512;
+// Subtrees the walk should have: fewer items are dealt out to 2 .. 32 warps each (9 us for a level
+// more, 2 for a step down a path).  2,000,000 points, 64 patches, 200 iterations: 32.2 ms at 2048,
+// 32.9 at 1024, 37.3 at 4096; with levels until there were 512 items 37.0.
+constexpr long long KM_UNITS = 2048;
 // assign[cell] = tag * KM_TAG + patch for the cells assigned by the pass with that tag, so the
 // array needs no clearing between passes (npatch <= KM_MAX_PATCH < KM_TAG).
 constexpr int KM_TAG = 8192;
@@ -68,7 +69,6 @@ struct KMLevel {
     int levels;              // levels that held items
     int wide;                // items of the current level with long candidate lists
     int wide_next;           // .. of the next level
-    long long units;         // items the walk started from
 };
 
 // The iterations' control: kernels of a stopped run return at once, so that several iterations
@@ -129,7 +129,7 @@ __global__ void k_km_start(const int* tops, int ntop, int npatch, KMItem* items,
     if (i == 0) {
         L->lo = 0; L->hi = ntop; L->total = ntop; L->pool_top = npatch;
         L->blocks_done = 0; L->err = 0; L->leaf_multi = 0; L->levels = 0;
-        L->wide = npatch > KM_SMALL; L->wide_next = 0; L->units = 0;
+        L->wide = npatch > KM_SMALL; L->wide_next = 0;
     }
 }
 
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
 // shared memory that holds every cell with its list.  The same decisions as k_km_level's (the
 // path from a top cell to a cell is the same), without its launch and its latency for each of the
 // tree's 20 or so levels.  2,000,000 points, 64 patches: 17 us a level and 360 us a pass before,
-// now 54 us for the walk (90 with every distance in FP64) and 9 for each of six levels; what
+// now 54 us for the walk (90 with every distance in FP64) and 9 for each of three levels; what
 // bounds it is the chain of a step (stack, cell, distances, stack) at some 20 steps per subtree.
 // The stack holds KW_CAP cells: when it fills up, fewer are taken at a time (a cell taken
 // leaves one more at most), at last one, with room for KW_DEPTH levels more; a tree too deep for
@@ -467,14 +467,20 @@ __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const do
             atomicCAS(&ctl->stop, KM_RUN, L->err == 1 ? KM_ERR_POOL : L->err ? KM_ERR_ITEMS : KM_ERR_WIDE);
         return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) L->units = hi - lo;
     const int lane = threadIdx.x & 31;
     KMEntry* st = reinterpret_cast<KMEntry*>(kmsm) + (threadIdx.x >> 5) * KW_CAP;
     const long long nwarps = (long long)gridDim.x * KW_WARPS;
+    // Few items are dealt out by their subtrees' halves, quarters, ..: a warp goes down its own path
+    // for `bits` cells, as the other warps of the item do, and then has the subtree there.
+    const long long m0 = hi - lo;
+    int bits = 0;
+    while (bits < 5 && (m0 << bits) < KM_UNITS) ++bits;
     // (neighbouring subtrees go to different SMs)
-    for (long long u = lo + blockIdx.x + (long long)gridDim.x * (threadIdx.x >> 5); u < hi; u += nwarps) {
+    for (long long u = blockIdx.x + (long long)gridDim.x * (threadIdx.x >> 5); u < (m0 << bits); u += nwarps) {
+        const unsigned path = (unsigned)u & ((1u << bits) - 1u);
+        int down = 0;               // cells of the path behind
         {
-            const KMItem it = items[u];
+            const KMItem it = items[lo + (u >> bits)];
             if (lane == 0) { st[0].cell = it.cell; st[0].len = it.len; }
             if (lane < it.len) st[0].cand[lane] = (unsigned short)pool[it.off + lane];
             __syncwarp();
@@ -554,16 +560,20 @@ __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const do
                 }
                 ncand = 1 + __popc(kept);
                 if (ncand == 1 || sf == 0.f || left < 0) {
-                    assign[c] = tag * KM_TAG + cp;
-                    if (ncand > 1 && sf != 0.f) atomicAdd(&L->leaf_multi, 1);
+                    // (a cell of the path: by the first of the warps that share it)
+                    if (down >= bits || (path >> down) == 0u) {
+                        assign[c] = tag * KM_TAG + cp;
+                        if (ncand > 1 && sf != 0.f) atomicAdd(&L->leaf_multi, 1);
+                    }
                 } else {
                     nout = 2;
                 }
             }
             const unsigned outs = __ballot_sync(0xffffffffu, nout);
+            const bool on_path = down < bits;
             if (nout) {
                 KMEntry* e = st + size + 2 * __popc(outs & ((1u << lane) - 1u));
-                e[0].cell = left;
+                e[0].cell = on_path && ((path >> down) & 1u) ? right : left;
                 e[1].cell = right;
                 e[0].len = e[1].len = ncand;
                 // The closest first, then the rest in list order; an unpruned list as it was.
@@ -578,7 +588,8 @@ __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const do
                 for (int j = 0; j < KM_SMALL; ++j)
                     if (ncand < m ? (kept >> j) & 1u : j < m) { e[0].cand[q] = e[1].cand[q] = cand[j]; ++q; }
             }
-            size += 2 * __popc(outs);
+            size += on_path ? __popc(outs) : 2 * __popc(outs);      // (one cell on the path)
+            ++down;
             __syncwarp();
         }
     }
@@ -1474,15 +1485,11 @@ int kmeans_run(const KMField& F, double* centers, int npatch, int max_iter, doub
             TC_TRY(sum_cells(F, npatch, KM_SUM_CENTERS, tolsq, S, st));
         }
         KMCtl c{};
-        KMLevel h{};
         TC_CU(cudaMemcpyAsync(&c, S.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
-        TC_CU(cudaMemcpyAsync(&h, S.lvl, sizeof(h), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaStreamSynchronize(st));
         it = c.iters;
         if (c.stop == KM_CONVERGED) break;
         if (c.stop) { TC_TRY(mend_stop(S, c.stop, st)); batch = 1; continue; }
-        // Enough subtrees for the warps, if another level gives them.
-        if (queued && h.units > 0 && h.units < KM_UNITS && S.pre < 12) ++S.pre;
         batch = std::min(2 * batch, 16);
     }
     if (iters_out) *iters_out = it;
