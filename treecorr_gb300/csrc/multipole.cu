@@ -24,7 +24,7 @@
 //   * Rows of Zeta that are final become vertex records (FP32 copies of G_n and W_n).  The
 //     contraction over vertices is a sum of outer products per n; k_mp_zeta (zeta.cu) runs it
 //     in batches (waves) between runs of the finish kernel, FP32 products with FP64 sums.
-//   * A last kernel sums the per-block outputs, the contraction partials and the diagonal
+//   * A last kernel sums what was contracted in place, the contraction's sums and the diagonal
 //     self-pair corrections in a fixed order.
 //   * A three-field cross keeps vertex 3's pairs in scratch bins [nbd, 2 nbd), so the same
 //     kernels produce both cross blocks of a (2 nbd)^2 matrix (MPParams::three).
@@ -44,9 +44,9 @@
 
 namespace tc {
 
-static constexpr int MB = 128;            // threads per multipole block (4 blocks per SM: 264 ms
-                                          // for the call below, 5: 272, 256 threads: 267)
-static constexpr int MBLK = 4;            // multipole blocks per SM
+static constexpr int MB = 128;            // threads per multipole block
+static constexpr int MBLK = 5;            // multipole blocks per SM (96 registers): 221 ms for the call
+                                          // at k_mp_finish, 4: 232, 6: 289 (spills)
 static constexpr int MW = MB / 32;        // warps per block
 static constexpr int MSTACK = 128;        // depth of the block-local stacks
 
@@ -491,9 +491,10 @@ __device__ __forceinline__ double* slot_ptr(const MPParams& P, int blk, int s)
 // (sum w^2) logr, sumwwgg0 (2), sumwwgg1 (2), sumwwgg2 (2), wg (2).
 static constexpr int REC_K = 6;
 
-// A warp's staged batch of 32 records: powers of z, (wg, w2, bin), scalar terms (14, n2, w2).
+// A warp's staged batch of 32 records: powers of z (16 records at a time), (wg, w2, bin), scalar
+// terms (14, n2, w2).
 struct AccBatch {
-    float2 pw[32][33];
+    float2 pw[16][33];
     float4 hk[32];
     float sc[32][17];
 };
@@ -501,15 +502,16 @@ static_assert(sizeof(AccBatch) % 16 == 0, "");
 
 // Bin-ordered G_n / W_n accumulation of the records [0, nrec) of this block into slot S.
 // The records are ranked by bin, then warp w takes the w-th contiguous share of the ranked
-// records, 32 at a time: lane = record writes the powers z, z^2, .. z^32 (z^33 .. in a second
-// round) to shared memory, one complex multiplication each, and the record's other terms; then
-// lane = n walks the records of each bin's run with six FP32 multiply-adds each (the sums of
+// records, 32 at a time: two lanes write a record's powers z .. z^16 and z^17 .. z^32 (z^33 .. in
+// a second round, H = 2) to shared memory, one complex multiplication each, and the record's
+// other terms, 16 records at a time; then lane = n walks the records of each bin's run with six FP32 multiply-adds each (the sums of
 // Re wg z^n and Im wg z^n, which make both G_n and G_-n, and w z^n), lanes 0..15 adding
 // the scalar terms as well.  The FP32 sums (F over a batch, F2 over the share: at most 16
 // batches) go to the slot in FP64 when the bin changes (atomics: two warps can share a bin).
 // A record costs the warp 22 instructions; raising every lane to its own power by squaring
 // took 75.
-__device__ void mp_accumulate(const MPParams& P, const float* rec, int* perm, int nrec,
+template <int H>
+__device__ __forceinline__ void mp_accumulate(const MPParams& P, const float* rec, int* perm, int nrec,
                               double* S, int* bh, AccBatch* batches)
 {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -555,13 +557,15 @@ __device__ void mp_accumulate(const MPParams& P, const float* rec, int* perm, in
     else if (lane < 14) { sc0 = oG + (int)sG(nb, M, 0, 0) + lane - 12; scs = 2; }
     else if (lane == 14) sc0 = oSC;
     else { sc0 = (int)sW(nb, 0, 0); scs = 2; }
-    float F[2][6], F2[2][6], fs = 0.f, fs2 = 0.f;
+    float F[H][6], F2[H][6], fs = 0.f, fs2 = 0.f;
     unsigned cn = 0;
-    int curk[2] = {-1, -1};
+    int curk[H];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < H; ++h) {
+        curk[h] = -1;
 #pragma unroll
         for (int q = 0; q < 6; ++q) { F[h][q] = 0.f; F2[h][q] = 0.f; }
+    }
     auto flush = [&](int h, int k) {
         const int n = lane + 1 + 32 * h;
         float* f = F[h];
@@ -610,61 +614,79 @@ __device__ void mp_accumulate(const MPParams& P, const float* rec, int* perm, in
 #pragma unroll
             for (int q = 0; q < 16; ++q) B.sc[lane][q] = sv[q];
         }
-        float pr = 1.f, pi2 = 0.f;                      // z^(32 h), then on
+        // Records 0..15, then 16..31; two lanes to a record, for the lower and the upper 16 powers.
+        for (int r0 = 0; r0 < nv; r0 += 16) {
+            const int rec16 = lane & 15, up = lane >> 4, jend = min(nv, r0 + 16);
+            const float zr = __shfl_sync(0xffffffffu, h0.x, r0 + rec16);
+            const float zi = __shfl_sync(0xffffffffu, h0.y, r0 + rec16);
+            float sr = zr, si = zi;                     // z^16
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 1 && M + 1 <= 32) break;
-            const int nc = min(32, M + 1 - 32 * h);
-            if (h == 1) __syncwarp();
-#pragma unroll 4
-            for (int n = 0; n < nc; ++n) {
-                const float t = pr * h0.x - pi2 * h0.y;
-                pi2 = pr * h0.y + pi2 * h0.x;
-                pr = t;
-                B.pw[lane][n] = make_float2(pr, pi2);
+            for (int t = 0; t < 4; ++t) {
+                const float u = sr * sr - si * si;
+                si = 2.f * sr * si;
+                sr = u;
             }
-            __syncwarp();
-            for (int js = 0; js < nv;) {
-                const unsigned later = js < 31 ? starts & ~((2u << js) - 1u) : 0u;
-                const int je = later ? __ffs(later) - 1 : nv;
-                const int kj = __float_as_int(B.hk[js].w);
-                if (kj != curk[h]) {
-                    if (curk[h] >= 0) flush(h, curk[h]);
-                    curk[h] = kj;
+            float pr = up ? sr : 1.f, pi2 = up ? si : 0.f;
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                if (h == 1) {                           // from z^16 on: another z^16
+                    const float t = pr * sr - pi2 * si;
+                    pi2 = pr * si + pi2 * sr;
+                    pr = t;
                 }
+                const int nc = min(16, M + 1 - 32 * h - 16 * up);
+                if (r0 + h > 0) __syncwarp();
 #pragma unroll 4
-                for (int j = js; j < je; ++j) {
-                    const float2 z = B.pw[j][lane];
-                    const float4 hk = B.hk[j];
-                    F[h][0] = fmaf(hk.z, z.x, F[h][0]);
-                    F[h][1] = fmaf(hk.z, z.y, F[h][1]);
-                    F[h][2] = fmaf(hk.x, z.x, F[h][2]);     // Re wg Re z^n
-                    F[h][3] = fmaf(hk.x, z.y, F[h][3]);     // Re wg Im z^n
-                    F[h][4] = fmaf(hk.y, z.x, F[h][4]);     // Im wg Re z^n
-                    F[h][5] = fmaf(hk.y, z.y, F[h][5]);     // Im wg Im z^n
-                    if (h == 0) {
-                        const float v = B.sc[j][lane & 15];
-                        fs += v;
-                        cn += __float_as_uint(v);           // (lane 14: the point count)
-                    }
+                for (int n = 0; n < nc; ++n) {
+                    const float t = pr * zr - pi2 * zi;
+                    pi2 = pr * zi + pi2 * zr;
+                    pr = t;
+                    B.pw[rec16][16 * up + n] = make_float2(pr, pi2);
                 }
-                js = je;
+                __syncwarp();
+                for (int js = r0; js < jend;) {
+                    const unsigned later = js < 31 ? starts & ~((2u << js) - 1u) : 0u;
+                    const int je = min(later ? __ffs(later) - 1 : nv, jend);
+                    const int kj = __float_as_int(B.hk[js].w);
+                    if (kj != curk[h]) {
+                        if (curk[h] >= 0) flush(h, curk[h]);
+                        curk[h] = kj;
+                    }
+#pragma unroll 4
+                    for (int j = js; j < je; ++j) {
+                        const float2 z = B.pw[j & 15][lane];
+                        const float4 hk = B.hk[j];
+                        F[h][0] = fmaf(hk.z, z.x, F[h][0]);
+                        F[h][1] = fmaf(hk.z, z.y, F[h][1]);
+                        F[h][2] = fmaf(hk.x, z.x, F[h][2]);     // Re wg Re z^n
+                        F[h][3] = fmaf(hk.x, z.y, F[h][3]);     // Re wg Im z^n
+                        F[h][4] = fmaf(hk.y, z.x, F[h][4]);     // Im wg Re z^n
+                        F[h][5] = fmaf(hk.y, z.y, F[h][5]);     // Im wg Im z^n
+                        if (h == 0) {
+                            const float v = B.sc[j][lane & 15];
+                            fs += v;
+                            cn += __float_as_uint(v);           // (lane 14: the point count)
+                        }
+                    }
+                    js = je;
+                }
             }
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < H; ++h)
 #pragma unroll
             for (int q = 0; q < 6; ++q) { F2[h][q] += F[h][q]; F[h][q] = 0.f; }
         fs2 += fs;
         fs = 0.f;
     }
-    if (curk[0] >= 0) flush(0, curk[0]);
-    if (curk[1] >= 0) flush(1, curk[1]);
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+        if (curk[h] >= 0) flush(h, curk[h]);
     __syncthreads();
 }
 
 // The n = 0 scalar outputs of calculateZeta for rows k2 in [ks, mk): ntri, meand2/3,
-// meanlogd2/3 (FP64, into the block's outputs).
+// meanlogd2/3 (FP64 atomics into the outputs).
 __device__ void zeta_scalars(const MPParams& P, int c1, const double* S, int ks, int mk,
                              double* out)
 {
@@ -687,20 +709,20 @@ __device__ void zeta_scalars(const MPParams& P, int c1, const double* S, int ks,
         if (k3 < k2) continue;
         const int i23 = (k2 * nb + k3) * nn + M;
         if (k3 == k2) {
-            out[14 * Z + i23] += n1 * npairs(k2) * (npairs(k2) - 1);
+            atomicAdd(&out[14 * Z + i23], n1 * npairs(k2) * (npairs(k2) - 1));
             double md = w1 * (sumw(k2) * sumwr(k2) - sumwwr(k2));
             double ml = w1 * (sumw(k2) * sumwlogr(k2) - sumwwlogr(k2));
-            out[8 * Z + i23] += md; out[9 * Z + i23] += ml;
-            out[10 * Z + i23] += md; out[11 * Z + i23] += ml;
+            atomicAdd(&out[8 * Z + i23], md); atomicAdd(&out[9 * Z + i23], ml);
+            atomicAdd(&out[10 * Z + i23], md); atomicAdd(&out[11 * Z + i23], ml);
         } else {
             const int i32 = (k3 * nb + k2) * nn + M;
             double nnn = n1 * npairs(k2) * npairs(k3);
-            out[14 * Z + i23] += nnn; out[14 * Z + i32] += nnn;
+            atomicAdd(&out[14 * Z + i23], nnn); atomicAdd(&out[14 * Z + i32], nnn);
             double ww12 = w1 * sumw(k2), ww13 = w1 * sumw(k3);
-            out[8 * Z + i23] += ww13 * sumwr(k2);  out[10 * Z + i32] += ww13 * sumwr(k2);
-            out[9 * Z + i23] += ww13 * sumwlogr(k2); out[11 * Z + i32] += ww13 * sumwlogr(k2);
-            out[10 * Z + i23] += ww12 * sumwr(k3); out[8 * Z + i32] += ww12 * sumwr(k3);
-            out[11 * Z + i23] += ww12 * sumwlogr(k3); out[9 * Z + i32] += ww12 * sumwlogr(k3);
+            atomicAdd(&out[8 * Z + i23], ww13 * sumwr(k2));  atomicAdd(&out[10 * Z + i32], ww13 * sumwr(k2));
+            atomicAdd(&out[9 * Z + i23], ww13 * sumwlogr(k2)); atomicAdd(&out[11 * Z + i32], ww13 * sumwlogr(k2));
+            atomicAdd(&out[10 * Z + i23], ww12 * sumwr(k3)); atomicAdd(&out[8 * Z + i32], ww12 * sumwr(k3));
+            atomicAdd(&out[11 * Z + i23], ww12 * sumwlogr(k3)); atomicAdd(&out[9 * Z + i32], ww12 * sumwlogr(k3));
         }
     }
 }
@@ -728,7 +750,7 @@ __device__ void zeta_diag(const MPParams& P, int c1, const double* S, int ks, in
 }
 
 // The product terms of calculateZeta for the entries (a, b, n) with min(a, b) in [ks, mk),
-// in FP64 directly into the block's outputs: the path for a vertex record that does not fit
+// in FP64 directly into the outputs (atomics): the path for a vertex record that does not fit
 // the record buffer.
 __device__ void zeta_products(const MPParams& P, int c1, const double* S, int ks, int mk,
                               double* out, double* shG, double* shW)
@@ -768,21 +790,21 @@ __device__ void zeta_products(const MPParams& P, int c1, const double* S, int ks
         // weight (Porth et al. eq. 27)
         if (a == b) {
             C2 wv = Wv(a, n);
-            out[12 * Z + i] += w1 * (wv.re * wv.re + wv.im * wv.im);
+            atomicAdd(&out[12 * Z + i], w1 * (wv.re * wv.re + wv.im * wv.im));
         } else {
             C2 p = cmul(Wv(a, n), conj2(Wv(b, n)));
-            out[12 * Z + i] += w1 * p.re;
-            out[13 * Z + i] += w1 * p.im;
+            atomicAdd(&out[12 * Z + i], w1 * p.re);
+            atomicAdd(&out[13 * Z + i], w1 * p.im);
         }
         // gam0..3 (eqs. 21, 23-25)
         C2 g0 = cmul(cmul(wg1, Gv(a, n - 1)), Gv(b, -n - 1));
         C2 g1 = cmul(cmul(wg1c, Gv(a, n + 1)), Gv(b, -n + 1));
         C2 g2 = cmul(cmul(wg1, Gv(a, n - 1)), conj2(Gv(b, n + 1)));
         C2 g3 = cmul(cmul(wg1, conj2(Gv(a, -n + 1))), Gv(b, -n - 1));
-        out[0 * Z + i] += g0.re; out[1 * Z + i] += g0.im;
-        out[2 * Z + i] += g1.re; out[3 * Z + i] += g1.im;
-        out[4 * Z + i] += g2.re; out[5 * Z + i] += g2.im;
-        out[6 * Z + i] += g3.re; out[7 * Z + i] += g3.im;
+        atomicAdd(&out[0 * Z + i], g0.re); atomicAdd(&out[1 * Z + i], g0.im);
+        atomicAdd(&out[2 * Z + i], g1.re); atomicAdd(&out[3 * Z + i], g1.im);
+        atomicAdd(&out[4 * Z + i], g2.re); atomicAdd(&out[5 * Z + i], g2.im);
+        atomicAdd(&out[6 * Z + i], g3.re); atomicAdd(&out[7 * Z + i], g3.im);
     }
     __syncthreads();
 }
@@ -826,16 +848,16 @@ __device__ void zeta_inplace3(const MPParams& P, int c1, const double* S, int ks
         if (m < ks || m >= mk) continue;
         const size_t i = (size_t)(a * nb + b) * nn + M + n;
         const C2 p = cmul(Wv(a, n), conj2(Wv(b, n)));
-        out[12 * Z + i] += w1 * p.re;
-        out[13 * Z + i] += w1 * p.im;
+        atomicAdd(&out[12 * Z + i], w1 * p.re);
+        atomicAdd(&out[13 * Z + i], w1 * p.im);
         const C2 g0 = cmul(cmul(wg1, Gv(a, n - sh)), Gv(b, -n - sh));
         const C2 g1 = cmul(cmul(wg1c, Gv(a, n + sh)), Gv(b, -n + sh));
         const C2 g2 = cmul(cmul(wg1, Gv(a, n - sh)), conj2(Gv(b, n + sh)));
         const C2 g3 = cmul(cmul(wg1, conj2(Gv(a, -n + sh))), Gv(b, -n - sh));
-        out[0 * Z + i] += g0.re; out[1 * Z + i] += g0.im;
-        out[2 * Z + i] += g1.re; out[3 * Z + i] += g1.im;
-        out[4 * Z + i] += g2.re; out[5 * Z + i] += g2.im;
-        out[6 * Z + i] += g3.re; out[7 * Z + i] += g3.im;
+        atomicAdd(&out[0 * Z + i], g0.re); atomicAdd(&out[1 * Z + i], g0.im);
+        atomicAdd(&out[2 * Z + i], g1.re); atomicAdd(&out[3 * Z + i], g1.im);
+        atomicAdd(&out[4 * Z + i], g2.re); atomicAdd(&out[5 * Z + i], g2.im);
+        atomicAdd(&out[6 * Z + i], g3.re); atomicAdd(&out[7 * Z + i], g3.im);
         if (n == 0 && !P.quick) {
             const size_t i0 = (size_t)(a * nb + b) * nn + M;
             const double npa = __ldcg(SC + a), npb = __ldcg(SC + b);
@@ -845,11 +867,11 @@ __device__ void zeta_inplace3(const MPParams& P, int c1, const double* S, int ks
             // meanlogd3 of the vertex-3 x vertex-2 block for ordered = 1 as the reference
             // writes it: mp3.sumw at the column's bin.
             const double swl = (P.typo32 && a >= nbd) ? __ldcg(SC + nb + (b % nbd) + nbd) : swa;
-            out[14 * Z + i0] += n1 * npa * npb;
-            out[8 * Z + i0] += w1 * swb * sra;
-            out[9 * Z + i0] += w1 * swb * sla;
-            out[10 * Z + i0] += w1 * swa * srb;
-            out[11 * Z + i0] += w1 * swl * slb;
+            atomicAdd(&out[14 * Z + i0], n1 * npa * npb);
+            atomicAdd(&out[8 * Z + i0], w1 * swb * sra);
+            atomicAdd(&out[9 * Z + i0], w1 * swb * sla);
+            atomicAdd(&out[10 * Z + i0], w1 * swa * srb);
+            atomicAdd(&out[11 * Z + i0], w1 * swl * slb);
         }
     }
     __syncthreads();
@@ -936,21 +958,24 @@ __device__ __forceinline__ bool zbuffer_full(const MPParams& P)
 }
 
 // Phase 2.  GGG of 500,000 points (20 bins, max_n 30) walks 1.87e6 lists of 908 cells on average,
-// accepts 0.8e9 pairs and emits 1.57e6 vertex records: 373 ms before, 225 ms now, of which some
-// 90 are the lists' decisions, 85 the accumulation and 50 the records.  What counts, as
-// one SM has 16 warps here (registers) and every list is a chain of dependent loads and barriers:
+// accepts 0.8e9 pairs and emits 1.57e6 vertex records: 373 ms before, 188 ms now (225 with 4 blocks
+// an SM and 32 records' powers staged: 90 of it the lists' decisions, 85 the accumulation and 50
+// the records).  What counts, as one SM has 20 warps here and every list is a chain of
+// dependent loads and barriers:
 //   * FP64: an instruction takes 16 cycles of the SM.  The largest r + s, the bin of its
 //     logarithm and the block's maximum took a third of the time on all warps; now only the
 //     threads that can hold the maximum leave FP32.
 //   * one barrier per 128 list entries (places by ballots), none for the running counts;
 //   * G_n, W_n rows copied and converted eight loads at a time, and only the record's columns;
 //   * one buffer for all records: a wave's end costs the blocks' last jobs, 10 ms.
+//   * shared memory and registers for 5 blocks of 128 threads (4: 232 ms for the call against 221);
+//   * one array of outputs for what is contracted in place, not one per block to clear and sum.
 // Taken back: the next entries loaded ahead (spills: 287 ms for the call against 254),
-// mp_accumulate out of line (295), five blocks of 128 (272) or three of 256 threads (303).
+// mp_accumulate out of line (295), blocks of 256 threads (267 with two, 303 with three).
 //
 // THREE: a three-field cross (two pair lists); compiled apart so that the auto and cross12
 // paths carry none of its registers.
-template <bool THREE>
+template <bool THREE, int H>
 __global__ void __launch_bounds__(MB, MBLK) k_mp_finish(const __grid_constant__ MPParams P)
 {
     extern __shared__ __align__(16) double mp_sh[];
@@ -973,7 +998,7 @@ __global__ void __launch_bounds__(MB, MBLK) k_mp_finish(const __grid_constant__ 
     int* arena = P.arena2 + (size_t)blk * P.arena2_cap;
     float* acc = P.acc + (size_t)blk * P.acc_cap * MP_REC;
     int* perm = P.perm + (size_t)blk * P.acc_cap;
-    double* out = P.out + (size_t)blk * P.out_stride;
+    double* out = P.out;
     double* diag = P.diag + (size_t)blk * 9 * nb;
     const int* arena1 = P.arena1;
     for (int k = tid; k < MP_MAXNB; k += MB) bh[k] = 0;
@@ -1275,7 +1300,7 @@ __global__ void __launch_bounds__(MB, MBLK) k_mp_finish(const __grid_constant__ 
                     const bool last = j0 + MB >= len;
                     if (last || acc_n > P.acc_cap - MB) {
                         __syncthreads();
-                        if (acc_n > 0) mp_accumulate(P, acc, perm, acc_n, S, bh, batches);
+                        if (acc_n > 0) mp_accumulate<H>(P, acc, perm, acc_n, S, bh, batches);
                         acc_n = 0;
                     }
                 }
@@ -1509,9 +1534,9 @@ __global__ void __launch_bounds__(ZB) k_mp_zscal(ZParams Q, int chunk, double* s
     }
 }
 
-// Final sums, in a fixed order: the per-block outputs, the contraction groups' partials and
-// the diagonal corrections.
-__global__ void k_mp_reduce(int nblk, long long stride, long long Z, int nb, int nn,
+// Final sums: what was contracted in place, the contraction's sums and the diagonal
+// corrections.
+__global__ void k_mp_reduce(int nblk, long long Z, int nb, int nn,
                             const double* in, const double* diag, long long diag_stride,
                             const double* part, int nsg, const double* spart,
                             const unsigned long long* ntp, double* out)
@@ -1520,8 +1545,7 @@ __global__ void k_mp_reduce(int nblk, long long stride, long long Z, int nb, int
     if (i >= 15 * Z) return;
     const int q = (int)(i / Z);
     const long long r = i % Z;
-    double s = 0.;
-    for (int b = 0; b < nblk; ++b) s += in[(size_t)b * stride + i];
+    double s = in[i];
     const int qp = q < 8 ? q : (q == 12 ? 8 : (q == 13 ? 9 : -1));
     const long long ab = r / nn;
     const int a = (int)(ab / nb), b = (int)(ab % nb), n = (int)(r % nn) - nn / 2;
@@ -1575,7 +1599,9 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
                        "nbins * max_n within its shared-memory staging");
         return 3;
     }
-    auto* kfin = P.three ? k_mp_finish<true> : k_mp_finish<false>;
+    // (powers up to 32, or up to 64 in two rounds)
+    auto* kfin = M + 1 <= 32 ? (P.three ? k_mp_finish<true, 1> : k_mp_finish<false, 1>)
+                             : (P.three ? k_mp_finish<true, 2> : k_mp_finish<false, 2>);
     TC_CU(cudaFuncSetAttribute(kfin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shbytes));
     int per = 0;
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfin, MB, shbytes));
@@ -1633,7 +1659,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
         if (grow_blk || P.out_stride > X.out_stride || 9LL * nb > X.diag_stride) {
             dfree(X.out); dfree(X.total); dfree(X.diag);
             X.out_stride = 0; X.diag_stride = 0;
-            TC_TRY(dalloc(&X.out, (size_t)P.out_stride * nblk));
+            TC_TRY(dalloc(&X.out, (size_t)P.out_stride));
             TC_TRY(dalloc(&X.total, (size_t)P.out_stride));
             TC_TRY(dalloc(&X.diag, (size_t)9 * nb * nblk));
             X.out_stride = P.out_stride; X.diag_stride = 9LL * nb;
@@ -1712,7 +1738,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
         TC_CU(cudaMemsetAsync(X.ctl, 0, 4 * sizeof(unsigned long long), st));
         X.overflow = 0; X.records = 0; X.waves = 0;
         TC_CU(cudaMemsetAsync(X.err, 0, 2 * sizeof(int), st));
-        TC_CU(cudaMemsetAsync(X.out, 0, sizeof(double) * (size_t)P.out_stride * nblk, st));
+        TC_CU(cudaMemsetAsync(X.out, 0, sizeof(double) * (size_t)P.out_stride, st));
         TC_CU(cudaMemsetAsync(X.diag, 0, sizeof(double) * (size_t)9 * nb * nblk, st));
         TC_CU(cudaMemsetAsync(X.part, 0, sizeof(double) * npart, st));
         TC_CU(cudaMemsetAsync(X.spart, 0, sizeof(double) * (size_t)nsg * 4 * nb * nb, st));
@@ -1792,7 +1818,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
         }
         count_launch();
         k_mp_reduce<<<(unsigned)((P.out_stride + 255) / 256), 256, 0, st>>>(
-            nblk, P.out_stride, Z, nb, nn, X.out, X.diag, 9LL * nb, X.part,
+            nblk, Z, nb, nn, X.out, X.diag, 9LL * nb, X.part,
             P.quick ? 0 : nsg, X.spart, X.ntp, X.total);
         TC_CU(cudaGetLastError());
         TC_CU(cudaMemcpyAsync(h_out, X.total, sizeof(double) * (size_t)P.out_stride,

@@ -72,7 +72,7 @@ struct MPParams {
     double* slots;
     int nslots;
     long long slot_doubles;
-    double* out;         // per block: 15 arrays of nbins^2 (2 maxn + 1) doubles
+    double* out;         // 15 arrays of nbins^2 (2 maxn + 1) doubles: what is contracted in place
     long long out_stride;
     double* diag;        // per block: 9 x nbins self-pair corrections of the diagonal k2 == k3
     // Vertex records for the batched contraction, one after another: zcount holds their number
