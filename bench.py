@@ -32,7 +32,7 @@ a few percent of max|xi+|.  The line therefore carries
   * xi_err: the headline's max over bins of |d xi+-| / max|xi+| against the exact result
     (bin_slop 0, angle_slop 0) on the same catalog;
   * accurate: that exact configuration timed the same way (every pair in range counted at
-    its own separation, the leaf-pair tiles), with its own e2e, its k_tiles roofline (FP32
+    its own separation, the leaf-pair tiles), with its own e2e, the tile kernel's roofline (FP32
     issue), its error against the FP64 oracle on a 200,000-point random subsample
     (xi_err_fp64) and the oracle's CPU rate there (cpu_baseline, vs_cpu).
 
@@ -297,11 +297,11 @@ def run_gpu(args, rank, world):
     ms_e2e = allreduce_max(ms_e2e, world)
     e2e = world * res_e2e[-1][1]["accepted"] * args.steps / (ms_e2e / 1e3)
     out, st = res[-1]
-    # Roofline of the dominant kernel (k_expand, the breadth-first traversal): algorithmic
-    # bytes = cell pairs evaluated x two 48-byte node reads (centre, size, weight, payload and
-    # children of both cells), over k_expand's own device time, measured by the library with
-    # CUDA events around every expansion launch on its stream (per launch: both divided by
-    # the number of expansion launches).
+    # Roofline of the dominant kernel (k_walk, the depth-first traversal after a short
+    # breadth-first expansion): algorithmic bytes = cell pairs evaluated x two 48-byte node reads
+    # (centre, size, weight, payload and children of both cells), over the traversal's device
+    # time, measured by the library with CUDA events around its launches on its stream (per
+    # launch: both divided by the number of launches).
     tr_ms = st["traverse_ms"]
     bytes_per_launch = st["cell_pairs"] * (2 * 48) / max(st["launches"], 1)
     per_launch_ms = st["expand_ms"] / max(st["launches"], 1)
@@ -314,15 +314,16 @@ def run_gpu(args, rank, world):
     achieved = bytes_per_launch / (per_launch_ms / 1e3) / 1e9
     traffic = args.traffic
     if traffic is None and args.n == 10_000_000 and abs(args.bin_slop - 0.1) < 1e-12:
-        # DRAM bytes per launch: 25.3 bytes per evaluated cell pair measured with ncu over a
-        # whole 1M-point traversal, times the cell pairs per launch of this workload.
-        traffic = round(25.3 * st["cell_pairs"] / max(st["launches"], 1))
+        # DRAM bytes per launch: 7.9 bytes per evaluated cell pair measured with ncu over the
+        # walk of a 3M-point catalog (records larger than L2), times the cell pairs per launch
+        # of this workload.
+        traffic = round(7.9 * st["cell_pairs"] / max(st["launches"], 1))
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(achieved / hbm, 4), "traffic": traffic,
-                "traffic_source": "ncu DRAM bytes per cell pair at 1M points, scaled"
+                "traffic_source": "ncu DRAM bytes per cell pair at 3M points, scaled"
                                   if args.traffic is None and traffic is not None else
                                   ("--traffic" if traffic is not None else None),
-                "kernel": "k_expand",
+                "kernel": "k_walk",
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}
     h2d = sum(cat[k].nbytes for k in cols)
     d2h = 8 * nb * 8
@@ -446,10 +447,10 @@ def exact_entry(args, T, dcols, hcols, timed, world):
     ms_e2e, res_e2e, _ = timed(step_host, 1)
     ms_e2e = allreduce_max(ms_e2e, world)
     e2e = world * res_e2e[-1][1]["accepted"] / (ms_e2e / 1e3)
-    # Roofline of k_tiles: FP32 issue (the pair math; no HBM traffic to speak of).
+    # Roofline of k_tiles_packed: FP32 issue (the pair math; no HBM traffic to speak of).
     # Algorithmic work = leaf pairs evaluated x 80 FLOP (a curved-sky GG pair: separation,
     # chord-to-arc, log, two spin-2 directions and rotations, both products, 8 sums), over
-    # k_tiles' own device time (events around every tile launch), per launch.
+    # the tile kernels' own device time (events around every tile launch), per launch.
     props = torch.cuda.get_device_properties(torch.cuda.current_device())
     tl = max(st["launches"], 1)
     achieved = st["tile_pairs"] * 80.0 / tl / (st["tiles_ms"] / tl / 1e3) / 1e12
@@ -461,7 +462,7 @@ def exact_entry(args, T, dcols, hcols, timed, world):
         "e2e": {"value": e2e, "unit": UNIT, "ms_per_step": ms_e2e,
                 "h2d_bytes_per_step": sum(v.numel() * 8 for v in hcols.values()),
                 "d2h_bytes_per_step": 8 * nb * 8, "steps": 1},
-        "roofline": {"bound": "fp32", "kernel": "k_tiles", "achieved": round(achieved, 2),
+        "roofline": {"bound": "fp32", "kernel": "k_tiles_packed", "achieved": round(achieved, 2),
                      "peak": None, "unit": "TFLOP/s", "frac": None,
                      "sms": props.multi_processor_count, "flop_per_pair": 80, "traffic": None,
                      "peak_source": "SMs x 128 FP32 lanes x 2 flop x the median SM clock "
