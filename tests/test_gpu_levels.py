@@ -37,6 +37,19 @@ def test_levels_by_size(gpu_lib, dtype, coords, split, n):
     _compare(gpu_lib, dtype, coords, cat, split)
 
 
+@pytest.mark.parametrize("n", [2, 12, 13, 14, 25, 26, 32, 33, 104])
+@pytest.mark.parametrize("dtype,coords,split", [("G", "spherical", "mean"), ("G", "flat", "median"),
+                                                ("K", "3d", "middle")])
+def test_one_block(gpu_lib, dtype, coords, split, n):
+    # Around the cells that one thread finishes (12 points in small catalogs) and the rounds that
+    # several warps share a cell in.
+    rng = np.random.default_rng(n + 1000)
+    x, y, z = (rng.normal(0, 10., n) for _ in range(3))
+    cat = dict(x=x, y=y, z=None if coords == "flat" else z + 40., w=rng.uniform(0.5, 1.5, n),
+               g1=rng.normal(0, 0.3, n), g2=rng.normal(0, 0.3, n), k=rng.normal(0, 1., n))
+    _compare(gpu_lib, dtype, coords, cat, split)
+
+
 def test_more_levels_than_counted(gpu_lib):
     """Weights that fall by 0.55 from point to point: every split leaves all but two."""
     n = 1000

@@ -32,9 +32,12 @@
 //     at the end, like the traversal's.
 // The kernel is compiled per geometry (flat, sphere with Arc, sphere or 3-d with Euclidean)
 // and per class family (NN; NK and KK; GG; the others through the generic projection code).
-// Measured on the 10M-point curved-sky catalog (bin_slop 0, angle_slop 0): the single-bin
+// tile_packed.cu takes NN, N x scalar and GG over whole ranges of bins that fit; the kernels here
+// take the other classes and forms.
+// Measured with GG on the 10M-point curved-sky catalog (bin_slop 0, angle_slop 0; 15.3 s, which
+// tile_packed.cu's do in 10.8): the single-bin
 // loop runs at ~3.6e11 leaf pairs/s, the two-bin loop at ~2.4e11; tiles of up to 48 points
-// per side (TILE_LEAF; 64 with the autotuner on that catalog) balance the pair loops against
+// per side (TILE_LEAF) balance the pair loops against
 // the per-tile work (staging, bounds, the final butterfly): 32-point tiles took 22.5 s, 48
 // 17.5 s before the two-pass loops, 15.3 s after.  A variant that staged the next tile's
 // leaves with bulk copies (cp.async.bulk + mbarrier) while the current one ran was 6% slower:

@@ -700,14 +700,21 @@ __device__ __forceinline__ int pack_meta(int side, int intop, int buf, int minto
     return side | (intop << 1) | (buf << 2) | (mintop << 8) | (maxtop << 20);
 }
 
-// Cells of at most THREAD_T points are finished by one thread, sums in point order.  Small
-// cells are ~94% of a subtree's cells, and a warp spends the same reductions on a 2-point
-// cell as on a 2048-point one.
+// Cells of at most thread_t points (THREAD_T or THREAD_FEW) are finished by one thread, sums in
+// point order.  Small cells are ~94% of a subtree's cells, and a warp spends the same
+// reductions on a 2-point cell as on a 2048-point one.
 constexpr int THREAD_T = 32;
+// Catalogs whose subtrees hold at most FEW_SUB points leave each SM one or two of them, and the
+// chain of one thread's points is what a block waits for: there warps go on down to THREAD_FEW
+// points.  Whole builds of spin-2 points on the sphere, 32 -> 12: 5000 points 0.67 -> 0.62 ms, 25,000
+// 0.75 -> 0.71 (8 and 16 within 2% of 12); at 100,000 points, with FEW_SUB 512, 8 took 1.09
+// against 1.03, so the line lies below.  Blocks above FEW_N points keep THREAD_T.
+constexpr int THREAD_FEW = 12, FEW_N = 512, FEW_SUB = 256;
 constexpr int SB = 256;             // threads of a subtree block
 constexpr int SW = SB / 32;
 constexpr unsigned NOT_SINGLE = ~0u;
 constexpr int SBIG = SMALL / (THREAD_T + 1) + 1;   // cells above THREAD_T points at one depth
+static_assert(FEW_N / (THREAD_FEW + 1) < SBIG, "a depth's cells fit its list");
 
 // One subtree's points, in shared memory for the whole build of the subtree: the points stay
 // where they are and the cells permute 16-bit indices, so a level moves 2 bytes per point
@@ -725,11 +732,16 @@ struct SubPart {                    // one warp's share of a cell that several w
     double sizesq, pr, pi;
     int nleft;
 };
+struct SubCentre {
+    double cx, cy, cz, tcx, tcy, tcz, splitval;
+    int axis;
+};
 struct SubShared {
     SubPoints P;
-    WTask cell[2][SBIG];            // cells above THREAD_T points of this and the next depth
+    WTask cell[2][SBIG];            // cells above thread_t points of this and the next depth
     int ncell[2], nsmall[2];
     SubPart part[SW];
+    SubCentre centre[SW];
 };
 
 // The first pass over the points i0, i0 + step, .. < e of a cell: sums and bounds.
@@ -758,11 +770,6 @@ __device__ __forceinline__ void sub_pass1(const SubPoints& P, const unsigned sho
         }
     }
 }
-
-struct SubCentre {
-    double cx, cy, cz, tcx, tcy, tcz, splitval;
-    int axis;
-};
 
 // Centroid, split axis and value of a cell from its sums (src/Cell.cpp:170-200, 481-525).
 template <bool FLATC>
@@ -889,7 +896,7 @@ __device__ __forceinline__ void sub_single(SubPoints& P, const WTask& w, int bas
     if ((w.meta >> 1) & 1) add_top(tops, ntop, (BP.n - 1) + base + s, base + s);
 }
 
-// A cell of 2 .. THREAD_T points by one thread.  Positions are relative to base (the block's
+// A cell of 2 .. thread_t points by one thread.  Positions are relative to base (the block's
 // first point); a finished cell's order ends up in perm[0].  Returns whether it was split,
 // with its children in k.
 template <bool FLATC, bool CPLX>
@@ -927,7 +934,7 @@ __device__ __forceinline__ bool sub_by_thread(const WTask& w, int base, SubPoint
     return true;
 }
 
-// A child of at most THREAD_T points: noted if it is one point, else onto the list.
+// A child of at most thread_t points: noted if it is one point, else onto the list.
 __device__ __forceinline__ void sub_small(const WTask& k, int base, SubPoints& P,
                                           const BuildParams& BP, int* tops, int* ntop,
                                           WTask* list, int* count)
@@ -936,14 +943,14 @@ __device__ __forceinline__ void sub_small(const WTask& k, int base, SubPoints& P
     else list[atomicAdd(count, 1)] = k;
 }
 
-// One warp's share (part of parts) of a cell above THREAD_T points; COOP: several warps of
+// One warp's share (part of parts) of a cell above thread_t points; COOP: several warps of
 // the block work on the cell and meet at block barriers (every warp of the block makes the
 // same calls).  `on` is false for a warp without a cell in a COOP round.
 template <bool FLATC, bool CPLX, bool COOP>
 __device__ __forceinline__ void sub_cell(SubShared& S, bool on, WTask w, int part, int parts,
                                          int base, const BuildParams& BP, const Cells& C,
                                          int* tops, int* ntop, int next, WTask* small, int lane,
-                                         int wid)
+                                         int wid, int thread_t)
 {
     SubPoints& P = S.P;
     const int n = w.e - w.s, buf = (w.meta >> 2) & 1;
@@ -974,7 +981,19 @@ __device__ __forceinline__ void sub_cell(SubShared& S, bool on, WTask w, int par
             for (int q = 0; q < 3; ++q) { lo[q] = min(lo[q], o.lo[q]); hi[q] = max(hi[q], o.hi[q]); }
         }
     }
-    const SubCentre c = sub_centre<FLATC>(P, on ? perm[w.s] : 0, BP, sum, lo, hi);
+    // One warp of the group: the FP64 pipe takes a warp's instruction in 16 cycles of the SM
+    // (all warps computing it: 200,000 points 1.43 ms for the whole build, so 1.40).
+    SubCentre c;
+    if (COOP) {
+        if (part == 0) {
+            c = sub_centre<FLATC>(P, on ? perm[w.s] : 0, BP, sum, lo, hi);
+            if (lane == 0) S.centre[wid] = c;
+        }
+        __syncthreads();
+        c = S.centre[p0];
+    } else {
+        c = sub_centre<FLATC>(P, on ? perm[w.s] : 0, BP, sum, lo, hi);
+    }
     double sizesq, pp[2];
     int nleft;
     sub_pass2<FLATC, CPLX>(P, perm, on ? i0 + lane : i1, i1, 32, BP, c, sizesq, pp[0], pp[1], nleft);
@@ -1033,7 +1052,7 @@ __device__ __forceinline__ void sub_cell(SubShared& S, bool on, WTask w, int par
             }
             if (part == 0 && lane < 2) {
                 const WTask k = sub_child(w, r, base, lane);
-                if (k.e - k.s > THREAD_T) S.cell[next][atomicAdd(&S.ncell[next], 1)] = k;
+                if (k.e - k.s > thread_t) S.cell[next][atomicAdd(&S.ncell[next], 1)] = k;
                 else sub_small(k, base, P, BP, tops, ntop, small, &S.nsmall[0]);
             }
         }
@@ -1041,7 +1060,7 @@ __device__ __forceinline__ void sub_cell(SubShared& S, bool on, WTask w, int par
 }
 
 // One block builds the whole subtree of a cell of at most SMALL points.  The points are read
-// once into shared memory.  The cells above THREAD_T points are taken depth by depth, a few
+// once into shared memory.  The cells above thread_t points are taken depth by depth, a few
 // warps to a cell near the root, one further down; then the smaller ones in rounds, one
 // thread to a cell and the children onto the next round's list, so that the lanes of a warp
 // work on cells of like size (a thread that walked its own subtree would leave most lanes
@@ -1055,7 +1074,7 @@ __device__ __forceinline__ void sub_cell(SubShared& S, bool on, WTask w, int par
 template <bool FLATC, bool CPLX>
 __global__ void __launch_bounds__(SB, 2) k_subtree(const BuildTask* tasks, Points P0, Points P1,
                                                    BuildParams BP, Cells C, int* tops, int* ntop,
-                                                   WTask* wstack, int* err)
+                                                   WTask* wstack, int thread_t, int* err)
 {
     extern __shared__ __align__(16) unsigned char sub_sh[];
     SubShared& S = *reinterpret_cast<SubShared*>(sub_sh);
@@ -1067,7 +1086,8 @@ __global__ void __launch_bounds__(SB, 2) k_subtree(const BuildTask* tasks, Point
         if (tid == 0) set_err(err, DEV_TASK_OVERFLOW);
         return;
     }
-    // Lists of cells of 2 .. THREAD_T points, this round's and the next one's: the cells of a
+    if (n > FEW_N) thread_t = THREAD_T;
+    // Lists of cells of 2 .. thread_t points, this round's and the next one's: the cells of a
     // list are disjoint, so n / 2 entries hold them.
     WTask* list[2] = {wstack + base, wstack + base + n / 2};
     const Points& A = root.buf ? P1 : P0;
@@ -1082,11 +1102,11 @@ __global__ void __launch_bounds__(SB, 2) k_subtree(const BuildTask* tasks, Point
     if (tid == 0) {
         const WTask w = {0, n, root.parent, pack_meta(root.side, root.intop, 0, root.mintop, root.maxtop)};
         S.ncell[0] = S.ncell[1] = S.nsmall[0] = S.nsmall[1] = 0;
-        if (n > THREAD_T) { S.cell[0][0] = w; S.ncell[0] = 1; }
+        if (n > thread_t) { S.cell[0][0] = w; S.ncell[0] = 1; }
         else sub_small(w, base, P, BP, tops, ntop, list[0], &S.nsmall[0]);
     }
     __syncthreads();
-    // A depth's cells are disjoint and each holds more than THREAD_T points, so a list never
+    // A depth's cells are disjoint and each holds more than thread_t points, so a list never
     // holds more than SBIG - 1 cells, and a cell has fewer points at every depth.
     for (int cur = 0;; cur ^= 1) {
         const int m = S.ncell[cur];
@@ -1096,11 +1116,11 @@ __global__ void __launch_bounds__(SB, 2) k_subtree(const BuildTask* tasks, Point
             const int ci = wid / parts;
             const bool on = ci < m;
             sub_cell<FLATC, CPLX, true>(S, on, S.cell[cur][on ? ci : 0], wid % parts, parts, base,
-                                        BP, C, tops, ntop, cur ^ 1, list[0], lane, wid);
+                                        BP, C, tops, ntop, cur ^ 1, list[0], lane, wid, thread_t);
         } else {
             for (int ci = wid; ci < m; ci += SW)
                 sub_cell<FLATC, CPLX, false>(S, true, S.cell[cur][ci], 0, 1, base, BP, C, tops,
-                                             ntop, cur ^ 1, list[0], lane, wid);
+                                             ntop, cur ^ 1, list[0], lane, wid, thread_t);
         }
         __syncthreads();
         if (tid == 0) S.ncell[cur] = 0;
@@ -1284,25 +1304,25 @@ __global__ void k_median_levels(BuildTask root, Points P0, Points P1, BuildParam
 template <bool FLATC, bool CPLX>
 static int subtree_launch(int ntask, const BuildTask* tasks, Points P0, Points P1,
                           const BuildParams& BP, const Cells& C, int* tops, int* ntop,
-                          WTask* wstack, int* err, cudaStream_t st)
+                          WTask* wstack, int thread_t, int* err, cudaStream_t st)
 {
     TC_CU(cudaFuncSetAttribute(k_subtree<FLATC, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(SubShared)));
     count_launch();
     k_subtree<FLATC, CPLX><<<ntask, SB, sizeof(SubShared), st>>>(tasks, P0, P1, BP, C, tops, ntop,
-                                                                 wstack, err);
+                                                                 wstack, thread_t, err);
     TC_CU(cudaGetLastError());
     return 0;
 }
 
 static int launch_subtrees(int ntask, const BuildTask* tasks, Points P0, Points P1,
                            const BuildParams& BP, const Cells& C, int* tops, int* ntop,
-                           WTask* wstack, int* err, cudaStream_t st)
+                           WTask* wstack, int thread_t, int* err, cudaStream_t st)
 {
     const bool flat = BP.coords == FLAT, cplx = BP.dkind == DG;
     auto* f = flat ? (cplx ? subtree_launch<true, true> : subtree_launch<true, false>)
                    : (cplx ? subtree_launch<false, true> : subtree_launch<false, false>);
-    return f(ntask, tasks, P0, P1, BP, C, tops, ntop, wstack, err, st);
+    return f(ntask, tasks, P0, P1, BP, C, tops, ntop, wstack, thread_t, err, st);
 }
 // ---------------------------------------------------------------------------------------
 // Structural check of the finished tree: every internal cell has two children that split
@@ -1345,6 +1365,7 @@ void launch_validate_tree(int ncap, const Cells& C, const int* tops, int ntop, i
 // 2 lanes per clock and SM, so that the work has to be spread).
 // Whole builds of a spin-2 field on the sphere, against chunks of 4096 and cells of 2048 points with
 // the host in every level: 25,000 points 1.63 -> 0.93 ms, 200,000 2.0 -> 1.55, 10M 43.9 -> 40.5.
+// Chunks from 256 points instead of 512: 25,000 points another 0.04 ms less.
 constexpr int BUILD_LEVELS = 64;    // levels counted before the host looks again at the latest
 
 static int spread(int n, int least, int most)
@@ -1361,7 +1382,7 @@ static int scratch_levels(int n, BuildScratch& S, cudaStream_t st)
 {
     if (S.level_mem) return 0;
     LevelBufs& L = S.L;
-    L.ch = spread(n, 512, CH);
+    L.ch = spread(n, 256, CH);
     L.sub = spread(n, 256, SMALL);
     L.cap_tasks = n / L.sub + 2;
     L.cap_chunks = n / L.ch + L.cap_tasks + 1;
@@ -1461,7 +1482,7 @@ int build_tree(const BuildParams& BP, Points bufs[2], Cells C, TCell* tcells, in
     }
     if (nsmall > 0)
         TC_TRY(launch_subtrees(nsmall, L.small, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
-                               d_err, st));
+                               L.sub <= FEW_SUB ? THREAD_FEW : THREAD_T, d_err, st));
     launch_pack_cells(2 * n - 1, C, tcells, st);
     TC_CU(cudaGetLastError());
     int ntop = 0;

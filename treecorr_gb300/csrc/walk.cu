@@ -220,11 +220,11 @@ __device__ __forceinline__ void df_accumulate(float2* fd, float x)
 }  // namespace
 
 // Bound: instruction issue (the records of a subtree's cells stay in L1 and L2).
-// 560 instructions per 32 evaluations of GG on the sphere, where the expansion kernel, with one
+// 557 instructions per 32 evaluations of GG on the sphere, where the expansion kernel, with one
 // code path for all classes and interval arithmetic around every comparison, takes 1030.
 // Measured, traversal of whole calls, expansion alone -> with the walk: GG 10M points on the
-// sphere, bin_slop 0.1, 1058 -> 500 ms; GG 200K flat, bin_slop 1, 15 -> 2.2; KK 300K 3-d
-// 72 -> 9.6; NN 2M clumped 46 -> 15; NG 100K x 2M 11.6 -> 6.0; 40 patches of 1M 58 -> 16.5.
+// sphere, bin_slop 0.1, 1058 -> 490 ms; GG 200K flat, bin_slop 1, 15 -> 1.7; KK 300K 3-d
+// 72 -> 8.3; NN 2M clumped 46 -> 14; NG 100K x 2M 11.6 -> 5.3; 40 patches of 1M 58 -> 16.5.
 // Variants: popping the next 32 items early with a prefetch of their records (+8%, two
 // interleaved subtrees share their bins less well); the FP64 decision inside the loop (+10%,
 // its call spills the loop's registers); sums under if / else (+5%, see add_if).
