@@ -53,9 +53,34 @@ void dfree(T*& p)
 }
 
 // Tree build (tree_build.cu).
-int build_tree(const BuildParams& BP, Points bufs[2], Cells C, TCell* tcells, int* d_tops, int* d_ntop,
-               BuildScratch& S, cudaStream_t st, std::vector<int>& tops_out, int* d_err,
-               int mintop, int maxtop);
+
+struct TreeBuild {                  // what a build works on
+    BuildParams BP;
+    Points bufs[2];
+    Cells C;
+    TCell* tcells;
+    int *d_tops, *d_ntop, *d_err;
+    int mintop, maxtop;
+    BuildScratch* S;
+};
+struct BuildRun {                   // how far a build has come
+    int lev = 0, total = 0, batch = 0;
+    bool whole = false;             // one block builds the whole tree
+};
+struct BuildRead {                  // what the host reads of a build
+    static constexpr int FIRST = 1024;
+    int2 left;                      // tasks and chunks of the level after the queued ones
+    int nsmall;                     // cells for k_subtree
+    int ntop;
+    int2 tops[FIRST];               // (first point, id)
+};
+// The build in three parts, so that several can run side by side: each of the first two
+// queues its kernels on st and copies (kind) what the next part reads into *to, which has to
+// be there before that one is called.
+int tree_begin(const TreeBuild& B, BuildRun& R, BuildRead* to, cudaMemcpyKind kind, cudaStream_t st);
+int tree_subtrees(const TreeBuild& B, BuildRun& R, const BuildRead& read, BuildRead* to,
+                  cudaMemcpyKind kind, cudaStream_t st);
+int tree_tops(const TreeBuild& B, const BuildRead& read, cudaStream_t st, std::vector<int>& tops_out);
 int field_center(const BuildParams& BP, Points P, BuildScratch& S, cudaStream_t st,
                  double out[4]);
 void launch_prepare(int n, int coords, int dkind, const double* x, const double* y,

@@ -1424,81 +1424,101 @@ static int launch_root(const BuildTask& root, const LevelBufs& L, cudaStream_t s
     return nc;
 }
 
-int build_tree(const BuildParams& BP, Points bufs[2], Cells C, TCell* tcells, int* d_tops, int* d_ntop,
-               BuildScratch& S, cudaStream_t st, std::vector<int>& tops_out, int* d_err,
-               int mintop, int maxtop)
+// The levels that even splits need, and a few more, go into the queue before the host looks;
+// the kernels of levels without tasks return at once.
+static int queue_levels(const TreeBuild& B, BuildRun& R, cudaStream_t st)
 {
-    const int n = BP.n;
+    const LevelBufs& L = B.S->L;
+    const int n = B.BP.n;
+    for (const int end = std::min(R.lev + R.batch, BUILD_LEVELS); R.lev < end; ++R.lev, ++R.total) {
+        // No more than 2^level tasks: most chunks of a level, so the grid.
+        const int tasks = R.total < 30 ? std::min(1 << R.total, L.cap_tasks) : L.cap_tasks;
+        const int nc = std::min(n / L.ch + tasks, L.cap_chunks);
+        count_launch(); k_chunk_pass1<<<nc, CB, 0, st>>>(L, R.lev, B.bufs[0], B.bufs[1], B.BP);
+        count_launch(); k_chunk_pass2<<<nc, CB, 0, st>>>(L, R.lev, B.bufs[0], B.bufs[1], B.BP, B.C,
+                                                         B.d_tops, B.d_ntop, B.d_err, 0);
+        count_launch(); k_chunk_scatter<<<nc, CB, 0, st>>>(L, R.lev, B.bufs[0], B.bufs[1]);
+    }
+    R.batch = 8;
+    TC_CU(cudaGetLastError());
+    return 0;
+}
+
+int tree_begin(const TreeBuild& B, BuildRun& R, BuildRead* to, cudaMemcpyKind kind, cudaStream_t st)
+{
+    const int n = B.BP.n;
     BuildTask root;
     root.s = 0; root.e = n; root.parent = -1; root.side = 0;
-    root.mintop = mintop; root.maxtop = maxtop; root.intop = 1; root.buf = 0;
-    TC_TRY(scratch_levels(n, S, st));
-    LevelBufs& L = S.L;
-    int nsmall = 0;
-    TC_CU(cudaMemsetAsync(d_ntop, 0, sizeof(int), st));
+    root.mintop = B.mintop; root.maxtop = B.maxtop; root.intop = 1; root.buf = 0;
+    TC_TRY(scratch_levels(n, *B.S, st));
+    const LevelBufs& L = B.S->L;
+    TC_CU(cudaMemsetAsync(B.d_ntop, 0, sizeof(int), st));
     TC_CU(cudaMemsetAsync(L.cnt, 0, sizeof(int2) * (BUILD_LEVELS + 1), st));   // (field_center's)
     TC_CU(cudaMemsetAsync(L.nsmall, 0, sizeof(int), st));
-    if (n > SMALL && BP.split == MEDIAN) {
+    if (n > SMALL && B.BP.split == MEDIAN) {
         count_launch();
-        k_median_levels<<<1, 32, 0, st>>>(root, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
-                                          L.small, L.nsmall, d_err);
+        k_median_levels<<<1, 32, 0, st>>>(root, B.bufs[0], B.bufs[1], B.BP, B.C, B.d_tops, B.d_ntop,
+                                          B.S->wstack, L.small, L.nsmall, B.d_err);
         TC_CU(cudaGetLastError());
+    } else if (n <= L.sub || B.BP.split == MEDIAN) {
+        TC_CU(cudaMemcpyAsync(L.small, &root, sizeof(BuildTask), cudaMemcpyHostToDevice, st));
+        R.whole = true;
+        return 0;
+    } else {
+        launch_root(root, L, st);
+        R.batch = 2;
+        for (int m = L.sub; m < n; m = m > (1 << 29) ? n : 2 * m) ++R.batch;
+        TC_TRY(queue_levels(B, R, st));
+    }
+    TC_CU(cudaMemcpyAsync(&to->left, L.cnt + R.lev, sizeof(int2), kind, st));
+    TC_CU(cudaMemcpyAsync(&to->nsmall, L.nsmall, sizeof(int), kind, st));
+    return 0;
+}
+
+int tree_subtrees(const TreeBuild& B, BuildRun& R, const BuildRead& read, BuildRead* to,
+                  cudaMemcpyKind kind, cudaStream_t st)
+{
+    const LevelBufs& L = B.S->L;
+    const int n = B.BP.n;
+    int2 left = read.left;
+    int nsmall = read.nsmall;
+    if (R.whole) { left = make_int2(0, 0); nsmall = 1; }
+    while (left.x != 0) {
+        if (R.lev == BUILD_LEVELS) {
+            // (an even number of levels: the arrays' turns go on)
+            TC_CU(cudaMemsetAsync(L.cnt, 0, sizeof(int2) * (BUILD_LEVELS + 1), st));
+            TC_CU(cudaMemcpyAsync(L.cnt, &left, sizeof(int2), cudaMemcpyHostToDevice, st));
+            TC_CU(cudaStreamSynchronize(st));
+            R.lev = 0;
+        }
+        TC_TRY(queue_levels(B, R, st));
+        TC_CU(cudaMemcpyAsync(&left, L.cnt + R.lev, sizeof(int2), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaMemcpyAsync(&nsmall, L.nsmall, sizeof(int), cudaMemcpyDeviceToHost, st));
         TC_CU(cudaStreamSynchronize(st));
-    } else if (n <= L.sub || BP.split == MEDIAN) {
-        TC_CU(cudaMemcpyAsync(L.small, &root, sizeof(BuildTask), cudaMemcpyHostToDevice, st));
-        nsmall = 1;
-    } else {
-        // All the levels that even splits need, and a few more, are in the queue before the
-        // host looks; the kernels of levels without tasks return at once.
-        launch_root(root, L, st);
-        int batch = 2;
-        for (int m = L.sub; m < n; m = m > (1 << 29) ? n : 2 * m) ++batch;
-        for (int lev = 0, total = 0;; batch = 8) {
-            const int end = std::min(lev + batch, BUILD_LEVELS);
-            for (; lev < end; ++lev, ++total) {
-                // No more than 2^level tasks: most chunks of a level, so the grid.
-                const int tasks = total < 30 ? std::min(1 << total, L.cap_tasks) : L.cap_tasks;
-                const int nc = std::min(n / L.ch + tasks, L.cap_chunks);
-                count_launch(); k_chunk_pass1<<<nc, CB, 0, st>>>(L, lev, bufs[0], bufs[1], BP);
-                count_launch(); k_chunk_pass2<<<nc, CB, 0, st>>>(L, lev, bufs[0], bufs[1], BP, C, d_tops,
-                                                                 d_ntop, d_err, 0);
-                count_launch(); k_chunk_scatter<<<nc, CB, 0, st>>>(L, lev, bufs[0], bufs[1]);
-            }
-            TC_CU(cudaGetLastError());
-            int2 left = make_int2(0, 0);
-            TC_CU(cudaMemcpyAsync(&left, L.cnt + lev, sizeof(int2), cudaMemcpyDeviceToHost, st));
-            TC_CU(cudaMemcpyAsync(&nsmall, L.nsmall, sizeof(int), cudaMemcpyDeviceToHost, st));
-            TC_CU(cudaStreamSynchronize(st));
-            if (left.x == 0) break;
-            if (lev == BUILD_LEVELS) {
-                // (an even number of levels: the arrays' turns go on)
-                TC_CU(cudaMemsetAsync(L.cnt, 0, sizeof(int2) * (BUILD_LEVELS + 1), st));
-                TC_CU(cudaMemcpyAsync(L.cnt, &left, sizeof(int2), cudaMemcpyHostToDevice, st));
-                TC_CU(cudaStreamSynchronize(st));
-                lev = 0;
-            }
-        }
     }
     if (nsmall > 0)
-        TC_TRY(launch_subtrees(nsmall, L.small, bufs[0], bufs[1], BP, C, d_tops, d_ntop, S.wstack,
-                               L.sub <= FEW_SUB ? THREAD_FEW : THREAD_T, d_err, st));
-    launch_pack_cells(2 * n - 1, C, tcells, st);
+        TC_TRY(launch_subtrees(nsmall, L.small, B.bufs[0], B.bufs[1], B.BP, B.C, B.d_tops, B.d_ntop,
+                               B.S->wstack, L.sub <= FEW_SUB ? THREAD_FEW : THREAD_T, B.d_err, st));
+    launch_pack_cells(2 * n - 1, B.C, B.tcells, st);
     TC_CU(cudaGetLastError());
-    int ntop = 0;
-    constexpr int FIRST = 1024;     // tops read along with their number
-    std::vector<int> pairs(2 * (size_t)std::min(n, FIRST));
-    TC_CU(cudaMemcpyAsync(&ntop, d_ntop, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TC_CU(cudaMemcpyAsync(pairs.data(), d_tops, sizeof(int) * pairs.size(), cudaMemcpyDeviceToHost, st));
-    TC_CU(cudaStreamSynchronize(st));
-    if (ntop > FIRST) {
-        pairs.resize(2 * (size_t)ntop);
-        TC_CU(cudaMemcpyAsync(pairs.data(), d_tops, 2 * sizeof(int) * ntop, cudaMemcpyDeviceToHost, st));
+    TC_CU(cudaMemcpyAsync(&to->ntop, B.d_ntop, sizeof(int), kind, st));
+    TC_CU(cudaMemcpyAsync(to->tops, B.d_tops, sizeof(int2) * std::min(n, BuildRead::FIRST), kind, st));
+    return 0;
+}
+
+int tree_tops(const TreeBuild& B, const BuildRead& read, cudaStream_t st, std::vector<int>& tops_out)
+{
+    const int ntop = read.ntop;
+    std::vector<std::pair<int, int>> v(ntop);
+    std::vector<int2> more;
+    if (ntop > BuildRead::FIRST) {
+        more.resize(ntop);
+        TC_CU(cudaMemcpyAsync(more.data(), B.d_tops, sizeof(int2) * ntop, cudaMemcpyDeviceToHost, st));
         TC_CU(cudaStreamSynchronize(st));
     }
+    const int2* pairs = ntop > BuildRead::FIRST ? more.data() : read.tops;
     // Tops in the reference's depth-first order = increasing first point (left before right).
-    std::vector<std::pair<int, int>> v(ntop);
-    for (int k = 0; k < ntop; ++k) v[k] = {pairs[2 * k], pairs[2 * k + 1]};
+    for (int k = 0; k < ntop; ++k) v[k] = {pairs[k].x, pairs[k].y};
     std::sort(v.begin(), v.end());
     tops_out.resize(ntop);
     for (int k = 0; k < ntop; ++k) tops_out[k] = v[k].second;
