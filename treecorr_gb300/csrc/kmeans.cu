@@ -116,6 +116,7 @@ constexpr int KM_SMALL = 16;
 __global__ void k_km_start(const int* tops, int ntop, int npatch, KMItem* items, int* pool,
                            KMLevel* L, const KMCtl* ctl, const double* cen, float4* cen32)
 {
+    after_previous();
     if (ctl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < npatch) {                    // the centres as FP32 pairs
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
                                                      long long pool_cap, int* assign,
                                                      int tag, KMLevel* L, const KMCtl* ctl)
 {
+    after_previous();
     if (ctl->stop) return;
     const int lane = threadIdx.x & 31;
     const long long lo = *(volatile long long*)&L->lo;
@@ -459,6 +461,7 @@ __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const do
                                                     const int* pool, int* assign, int tag, KMLevel* L,
                                                     KMCtl* ctl)
 {
+    after_previous();
     extern __shared__ __align__(16) double kmsm[];
     if (ctl->stop) return;
     const long long lo = L->lo, hi = min(L->hi, item_cap);
@@ -625,6 +628,7 @@ constexpr int KM_STEP = 512;        // ids a warp reads at once
 __global__ void k_km_accum(Cells C, int ncap, const int* assign, int tag, const double* cen,
                            int npatch, int mode, double* partial, const KMCtl* ctl)
 {
+    after_previous();
     if (ctl->stop) return;
     extern __shared__ __align__(16) double kmsm[];
     const int nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -725,6 +729,7 @@ __global__ void __launch_bounds__(256) k_km_total(int npatch, int nblk, const do
                                                   double* tot, int mode, int coords, double* cen,
                                                   double* inertia, double tolsq, KMCtl* ctl)
 {
+    after_previous();
     __shared__ double red[32];
     __shared__ int last;
     if (ctl->stop) return;
@@ -1236,17 +1241,16 @@ int enqueue_cells(const KMField& F, int npatch, const double* inertia, KMScratch
     TC_TRY(sm_count(&nsm));
     TC_TRY(next_tag(F, S, st));
     const int nstart = std::max(F.ntop, npatch);
-    count_launch();
-    k_km_start<<<(nstart + 255) / 256, 256, 0, st>>>(F.d_tops, F.ntop, npatch, S.items, S.pool, S.lvl, S.ctl,
-                                                     S.cen, S.cen32);
+    TC_TRY(launch_chained(k_km_start, (nstart + 255) / 256, 256, 0, st, F.d_tops, F.ntop, npatch,
+                          S.items, S.pool, S.lvl, S.ctl, S.cen, S.cen32));
     for (int k = 0; k < S.pre; ++k) {
-        count_launch();
-        k_km_level<<<nsm, KM_LTB, 0, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap, S.pool,
-                                               S.pool_cap, S.assign, S.tag, S.lvl, S.ctl);
+        TC_TRY(launch_chained(k_km_level, nsm, KM_LTB, 0, st, F.cells, S.cen, S.cen32, inertia,
+                              S.items, S.item_cap, S.pool, S.pool_cap, S.assign, S.tag, S.lvl,
+                              S.ctl));
     }
-    count_launch();
-    k_km_walk<<<KW_BLOCKS * nsm, KM_LTB, KW_SMEM, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap, S.pool, S.assign,
-                                          S.tag, S.lvl, S.ctl);
+    TC_TRY(launch_chained(k_km_walk, KW_BLOCKS * nsm, KM_LTB, KW_SMEM, st, F.cells, S.cen,
+                          S.cen32, inertia, S.items, S.item_cap, S.pool, S.assign, S.tag, S.lvl,
+                          S.ctl));
     TC_CU(cudaGetLastError());
     return 0;
 }
@@ -1322,12 +1326,10 @@ int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S
 
 int sum_cells(const KMField& F, int npatch, int mode, double tolsq, KMScratch& S, cudaStream_t st)
 {
-    count_launch();
-    k_km_accum<<<KM_NBLK, S.acc_threads, S.acc_smem, st>>>(F.cells, F.ncap, S.assign, S.tag, S.cen,
-                                                           npatch, mode, S.partial, S.ctl);
-    count_launch();
-    k_km_total<<<(npatch * KM_NQ + 7) / 8, 256, 0, st>>>(npatch, KM_NBLK, S.partial, S.tot, mode, F.coords,
-                                                         S.cen, S.inertia, tolsq, S.ctl);
+    TC_TRY(launch_chained(k_km_accum, KM_NBLK, S.acc_threads, S.acc_smem, st, F.cells, F.ncap,
+                          S.assign, S.tag, S.cen, npatch, mode, S.partial, S.ctl));
+    TC_TRY(launch_chained(k_km_total, (npatch * KM_NQ + 7) / 8, 256, 0, st, npatch, KM_NBLK,
+                          S.partial, S.tot, mode, F.coords, S.cen, S.inertia, tolsq, S.ctl));
     TC_CU(cudaGetLastError());
     return 0;
 }

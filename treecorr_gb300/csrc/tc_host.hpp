@@ -52,6 +52,34 @@ void dfree(T*& p)
     p = nullptr;
 }
 
+#ifdef __CUDACC__
+// A kernel launched with launch_chained has its blocks set up as those of the kernel before
+// end; in after_previous, its first statement, they wait until all of that kernel's writes are
+// visible.  (The kernel before gives no earlier sign: blocks set up while it still runs go where it
+// has left room, not evenly over the SMs.  With one, builds of 400,000 points took 2.26 ms
+// instead of 2.12, without chaining 2.16, and k-means of 2M points 32.8 instead of 28.9 and 32.0.)
+__device__ __forceinline__ void after_previous() { cudaGridDependencySynchronize(); }
+
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t st,
+                   A... args)
+{
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    count_launch();
+    TC_CU(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return 0;
+}
+#endif
+
 // Tree build (tree_build.cu).
 
 struct TreeBuild {                  // what a build works on

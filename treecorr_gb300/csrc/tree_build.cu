@@ -305,39 +305,6 @@ __device__ __forceinline__ void transport_near(int coords, int spin, double cx, 
 // ---------------------------------------------------------------------------------------
 // Cooperative levels (cells with more than SMALL points).
 
-// With launch_chained on, a kernel's blocks are set up while the kernel before still runs, and
-// wait here for it to end and its writes to be visible: 27 small kernels follow each other in a
-// build of 25,000 points, 2 us apart otherwise.  On for up to CHAIN_N points.  Above, a block runs
-// long enough for it to matter that the early blocks go where the kernel before has left
-// room, not evenly over the SMs.  Whole builds of spin-2 points on the sphere, off -> on: 1000 flat
-// points 0.39 -> 0.36 ms, 5000 0.59 -> 0.53, 25,000 0.67 -> 0.63, 200,000 1.40 -> 1.39 (flat 0.92 -> 0.88),
-// but 300,000 1.85 -> 1.86, 400,000 2.16 -> 2.26, 10^6 4.55 -> 5.15.
-constexpr int CHAIN_N = 1 << 18;
-
-__device__ __forceinline__ void after_previous()
-{
-    cudaGridDependencySynchronize();
-    cudaTriggerProgrammaticLaunchCompletion();
-}
-
-template <class... P, class... A>
-static int launch_chained(bool on, void (*kernel)(P...), int blocks, int threads, cudaStream_t st,
-                          A... args)
-{
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = on ? 1 : 0;
-    count_launch();
-    TC_CU(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
-    return 0;
-}
-
 // The root [0, n) as level 0's task.
 __global__ void k_level_root(LevelBufs L, BuildTask root)
 {
@@ -1460,21 +1427,23 @@ static int launch_root(const BuildTask& root, const LevelBufs& L, cudaStream_t s
     return nc;
 }
 
+// 27 small kernels follow each other in a build of 25,000 points, 2 us apart: launch_chained takes
+// whole builds of spin-2 points on the sphere from 0.67 to 0.60 ms there, 5000 from 0.59 to 0.52, 200,000
+// from 1.40 to 1.32 and 10^6 from 4.51 to 4.46.
 // The levels that even splits need, and a few more, go into the queue before the host looks;
 // the kernels of levels without tasks return at once.
 static int queue_levels(const TreeBuild& B, BuildRun& R, cudaStream_t st)
 {
     const LevelBufs& L = B.S->L;
     const int n = B.BP.n;
-    const bool chain = n <= CHAIN_N;
     for (const int end = std::min(R.lev + R.batch, BUILD_LEVELS); R.lev < end; ++R.lev, ++R.total) {
         // No more than 2^level tasks: most chunks of a level, so the grid.
         const int tasks = R.total < 30 ? std::min(1 << R.total, L.cap_tasks) : L.cap_tasks;
         const int nc = std::min(n / L.ch + tasks, L.cap_chunks);
-        TC_TRY(launch_chained(chain, k_chunk_pass1, nc, CB, st, L, R.lev, B.bufs[0], B.bufs[1], B.BP));
-        TC_TRY(launch_chained(chain, k_chunk_pass2, nc, CB, st, L, R.lev, B.bufs[0], B.bufs[1], B.BP, B.C,
+        TC_TRY(launch_chained(k_chunk_pass1, nc, CB, 0, st, L, R.lev, B.bufs[0], B.bufs[1], B.BP));
+        TC_TRY(launch_chained(k_chunk_pass2, nc, CB, 0, st, L, R.lev, B.bufs[0], B.bufs[1], B.BP, B.C,
                               B.d_tops, B.d_ntop, B.d_err, 0));
-        TC_TRY(launch_chained(chain, k_chunk_scatter, nc, CB, st, L, R.lev, B.bufs[0], B.bufs[1]));
+        TC_TRY(launch_chained(k_chunk_scatter, nc, CB, 0, st, L, R.lev, B.bufs[0], B.bufs[1]));
     }
     R.batch = 8;
     TC_CU(cudaGetLastError());
@@ -1583,9 +1552,8 @@ int field_center(const BuildParams& BP, Points P, BuildScratch& S, cudaStream_t 
     BuildParams B2 = BP;
     B2.split = MEAN;
     const int nc = launch_root(root, S.L, st);
-    const bool chain = n <= CHAIN_N;
-    TC_TRY(launch_chained(chain, k_chunk_pass1, nc, CB, st, S.L, 0, P, P, B2));
-    TC_TRY(launch_chained(chain, k_chunk_pass2, nc, CB, st, S.L, 0, P, P, B2, Cells{}, nullptr, nullptr,
+    TC_TRY(launch_chained(k_chunk_pass1, nc, CB, 0, st, S.L, 0, P, P, B2));
+    TC_TRY(launch_chained(k_chunk_pass2, nc, CB, 0, st, S.L, 0, P, P, B2, Cells{}, nullptr, nullptr,
                           nullptr, 1));
     TC_CU(cudaGetLastError());
     TaskStats ts;
