@@ -86,6 +86,22 @@ __device__ __forceinline__ void expm2i(float rx, float ry, float& er, float& ei)
     ei = -2.f * rx * ry * inv;
 }
 
+// On the sphere a direction is (s, c) = (sin, cos) of a position angle times |sep| cos(dec), from
+// differences of positions; for a point on a pole FP32 cancels c to 0, and s is 0 or a product with the
+// 6e-17 that cos(90 deg) is in FP64.  The phase then has to stay finite, and as near the FP64 formula's
+// as may be, where c is rounding of some 1e-17 and by far the larger: POLE_SQ counts as c^2.  It is
+// below half an ulp of s^2 + c^2 from |sep| cos(dec) = 4e-12 on, so no other phase changes.
+constexpr float POLE_SQ = 1e-30f;
+
+// expm2i of the direction (s, c) on the sphere.
+__device__ __forceinline__ void expm2i_sphere(float s, float c, float& er, float& ei)
+{
+    const float c2 = fmaf(c, c, POLE_SQ);
+    const float inv = __fdividef(1.f, fmaf(s, s, c2));
+    er = (s * s - c2) * inv;
+    ei = -2.f * s * c * inv;
+}
+
 __device__ __forceinline__ void cmul(float ar, float ai, float br, float bi, float& cr, float& ci)
 {
     cr = ar * br - ai * bi;
@@ -218,12 +234,14 @@ __device__ __forceinline__ void accept_values(const TravParams& T, const TCell& 
         const float sinA = x1 * dy - y1 * dx;
         const float cosA = dz + 0.5f * z2 * dsq;
         float e2r, e2i;
-        expmsi(T.s2, sinA, -cosA, e2r, e2i);
+        if (T.s2 == 2) expm2i_sphere(sinA, -cosA, e2r, e2i);
+        else expmsi(T.s2, sinA, -cosA, e2r, e2i);
         cmul(g2r, g2i, e2r, e2i, g2r, g2i);
         if (both) {
             const float cosB = -dz + 0.5f * z1 * dsq;
             float e1r, e1i;
-            expmsi(T.s1, -sinA, -cosB, e1r, e1i);
+            if (T.s1 == 2) expm2i_sphere(-sinA, -cosB, e1r, e1i);
+            else expmsi(T.s1, -sinA, -cosB, e1r, e1i);
             if (T.s1 & 1) { e1r = -e1r; e1i = -e1i; }
             cmul(g1r, g1i, e1r, e1i, g1r, g1i);
         }

@@ -114,7 +114,7 @@ static_assert(sizeof(PackedSide) % 16 == 0, "");
 struct PTile {
     int na, nj, kref, idA, idB;             // id*: leaf cell ids of the cells' first points
     float inv_edge, emax, band_e, band_0, chx, chy, chz, clx, cly, clz;
-    bool self, small_chord;
+    bool self, special;
 };
 
 // Listed pairs (or, all = true, every pair of the tile), decided and added in FP64 / FP32 as
@@ -218,7 +218,8 @@ __device__ __forceinline__ BPair load_pair(const PackedSide& S, int jp)
 // x, or for GG on the sphere their factors (products<>()).
 struct PVals { f2 r, lr, ic, ww, x[4]; };
 
-template <int GEO, int KIND, bool BIG>
+// SPECIAL: chords of 0.25 and more, or a pole in reach (k_tile_class).
+template <int GEO, int KIND, bool SPECIAL>
 __device__ __forceinline__ void pair_vals(const PTile& C, const PRow& A, const BPair& B, PVals& V)
 {
     const f2 one = mk2(1.f), mone = mk2(-1.f);
@@ -237,8 +238,7 @@ __device__ __forceinline__ void pair_vals(const PTile& C, const PRow& A, const B
         f2 p = fma2(dsq, mk2(5.f / 7168.f), mk2(3.f / 640.f));
         p = fma2(dsq, p, mk2(1.f / 24.f));
         r = mul2(r, fma2(dsq, p, one));
-        if (BIG && !C.small_chord)
-            r = mk2(arc_from_chord_sq(lo2(dsq)), arc_from_chord_sq(hi2(dsq)));
+        if (SPECIAL) r = mk2(arc_from_chord_sq(lo2(dsq)), arc_from_chord_sq(hi2(dsq)));
     }
     V.r = r;
     V.lr = log2_2(mul2(GEO == TG_ARC ? mul2(r, r) : dsq, mk2(C.inv_edge)));
@@ -263,7 +263,8 @@ __device__ __forceinline__ void pair_vals(const PTile& C, const PRow& A, const B
         const f2 cosA = fma2(B.zh, dsq, dz);
         const f2 cosB = fma2(A.nazh, dsq, dz);
         const f2 s2 = mul2(sinA, sinA), tS = mul2(sinA, mk2(-2.f));
-        const f2 m2 = fma2(cosA, cosA, s2), m1 = fma2(cosB, cosB, s2);
+        f2 m2 = fma2(cosA, cosA, s2), m1 = fma2(cosB, cosB, s2);
+        if (SPECIAL) { m2 = add2(m2, mk2(POLE_SQ)); m1 = add2(m1, mk2(POLE_SQ)); }
         const f2 E2r = fma2(s2, mk2(-2.f), m2), E2i = mul2(tS, cosA);
         const f2 E1r = fma2(s2, mk2(-2.f), m1), E1i = mul2(tS, cosB);
         const f2 i2 = rcp2(m2), i1 = rcp2(m1);
@@ -389,7 +390,7 @@ template <int KIND> __host__ __device__ constexpr int hist_words()
 template <int KIND> __host__ __device__ constexpr size_t hist_bytes()
 { return sizeof(float) * 32 * hist_words<KIND>() * (hist_rows<KIND>() + 1); }
 
-template <int GEO, int KIND>
+template <int GEO, int KIND, bool SPECIAL>
 __device__ __forceinline__ void packed_hist(const TravParams& T, PackedSide& S, const PTile& C,
                                             float* hist, int lane, int w0, int& ecount,
                                             unsigned& n_acc)
@@ -415,7 +416,7 @@ __device__ __forceinline__ void packed_hist(const TravParams& T, PackedSide& S, 
             const int jp = t0 + A.grp;
             const BPair B = load_pair<KIND>(S, jp);
             PVals V;
-            pair_vals<GEO, KIND, true>(C, A, B, V);
+            pair_vals<GEO, KIND, SPECIAL>(C, A, B, V);
             const uint2 n2 = *reinterpret_cast<const uint2*>(&S.nbl[2 * jp]);
             // floor(k) (adding 1.5 2^23 rounds to an integer); the distance to the nearer bin
             // edge is 0.5 - |g|.
@@ -464,10 +465,10 @@ template <int KIND> __host__ __device__ inline size_t packed_warp_bytes(int nq, 
 { return bins_bytes(nq, nb) + sizeof(PackedSide) + hist_bytes<KIND>(); }
 
 // What k_tile_class found for a tile, in 32 bits: the kernel that takes it (its NB, 0: no pair
-// in range; 1, 2: bins; 3: the histogram), whether its chords are below 0.25, the lowest bin and
+// in range; 1, 2: bins; 3: the histogram), whether it is special (pair_vals), the lowest bin and
 // how many bins above it the bounds reach.
-__host__ __device__ inline unsigned tile_key(int cls, bool small, int klo, int span)
-{ return (unsigned)cls | (small ? 16u : 0u) | ((unsigned)klo << 5) | ((unsigned)span << 18); }
+__host__ __device__ inline unsigned tile_key(int cls, bool special, int klo, int span)
+{ return (unsigned)cls | (special ? 16u : 0u) | ((unsigned)klo << 5) | ((unsigned)span << 18); }
 constexpr int KEY_MAXNB = 8191;
 
 // A drain of the tile list: the launch after the expansion that left no room for another
@@ -507,6 +508,15 @@ __global__ void __launch_bounds__(256) k_tile_class(const __grid_constant__ Trav
         const float slack = emax + 2e-6f * (Dn + rAB);
         float lo = fmaxf(Dn - rAB - slack, 0.f), hi = Dn + rAB + slack;
         const bool small = hi < 0.25f;
+        // Special tiles: chords of 0.25 and more (Arc), or for GG a direction that FP32 can cancel
+        // to nothing.  That is |p1 - p2| cos(dec) sin(..), and its FP32 error some 2e-7 of
+        // |p1 - p2| (cos(dec) + |p1 - p2|) at most: it is well above the error where every point is 1e-4
+        // from the poles' axis and no pair near antipodal, and its square a normal number
+        // from a min_sep of 1e-13 on (pick).
+        const bool gg = (GEO == TG_ARC || GEO == TG_SPHEUC) && T.k2 == DG;
+        const bool pole = gg && (sqrtf(Aa.x * Aa.x + Aa.y * Aa.y) - Aa.w <= 1e-4f ||
+                                 sqrtf(Ba.x * Ba.x + Ba.y * Ba.y) - Ba.w <= 1e-4f || hi > 1.999f);
+        const bool special = pole || (GEO == TG_ARC && !small);
         if (GEO == TG_ARC) {
             if (small) { lo = arc_series(lo); hi = arc_series(hi); }
             else { lo = arc_from_chord_sq(lo * lo); hi = arc_from_chord_sq(hi * hi); }
@@ -527,9 +537,9 @@ __global__ void __launch_bounds__(256) k_tile_class(const __grid_constant__ Trav
             // |log2| <= lmax here), the roundings of its argument and of kk.
             const float lmax = fmaxf(fabsf(__log2f(hi * hi * T.tile_edge[klo])), 1.f);
             band_0 = 4e-7f * T.finvbinsize + (5e-7f + 4.2e-7f * lmax) * ckk + 2e-7f;
-            const bool plain = interior && !self && (GEO != TG_ARC || small);
+            const bool plain = interior && !self && !special;
             const int span = khi - klo;
-            key = tile_key(plain && span < 2 ? span + 1 : 3, small, klo, span);
+            key = tile_key(plain && span < 2 ? span + 1 : 3, special, klo, span);
         }
         T.tile_keys[t] = key;
         T.tile_err[t] = make_float2(emax, band_0);
@@ -581,7 +591,7 @@ __global__ void __launch_bounds__(PB, PMINB) k_tiles_packed(const __grid_constan
             const float4 Ba = cB[ib].a, Bb = cB[ib].b;
             const int nB = __float_as_int(cB[ib].c.z), sB = __float_as_int(cB[ib].d.z);
             const int cls = key & 7u;
-            C.small_chord = (key & 16u) != 0u;
+            C.special = (key & 16u) != 0u;
             C.kref = (key >> 5) & 8191u;
             const int span = (int)(key >> 18);
             C.inv_edge = T.tile_edge[C.kref];         // 1 / (lower edge of kref)^2
@@ -698,7 +708,12 @@ __global__ void __launch_bounds__(PB, PMINB) k_tiles_packed(const __grid_constan
                     float4* h4 = reinterpret_cast<float4*>(hist);
                     for (int z = lane; z < nr * (RF / 4); z += 32) h4[z] = make_float4(0.f, 0.f, 0.f, 0.f);
                     __syncwarp();
-                    packed_hist<GEO, KIND>(T, S, C, hist, lane, w0, ecount, n_acc);
+                    // (one form with the special steps as a branch in the loop: GG of 10^6 points
+                    // 159 ms, two forms 155)
+                    if ((GEO == TG_ARC || (GEO == TG_SPHEUC && KIND == TK_GG)) && C.special)
+                        packed_hist<GEO, KIND, true>(T, S, C, hist, lane, w0, ecount, n_acc);
+                    else
+                        packed_hist<GEO, KIND, false>(T, S, C, hist, lane, w0, ecount, n_acc);
                     if (ecount > PESC) { n_acc = before; break; }
                     for (int b = 0; b < nr; ++b) {
                         const float* h = hist + b * RF;
@@ -808,6 +823,7 @@ bool pick(const TravParams& T, PackedSet& K)
     // Squared separations are normal FP32 numbers, and max_sep is the last bin's edge.
     if (!(T.fminsep >= 1e-15f && T.fmaxsep <= 1e15f)) return false;
     if (!(std::fabs(0.5 * std::log(T.maxsepsq / T.minsepsq) - T.nbins * T.binsize) <= 1e-9 * T.binsize)) return false;
+    if (T.coords == SPHERE && T.k2 == DG && T.fminsep < 1e-13f) return false;    // (k_tile_class)
     bool found;
     if (T.coords == FLAT) found = pick_kind<TG_FLAT>(T, K);
     else if (T.coords == SPHERE) found = T.metric == ARC ? pick_kind<TG_ARC>(T, K) : pick_kind<TG_SPHEUC>(T, K);

@@ -181,18 +181,19 @@ __device__ __forceinline__ void pair_products(const TravParams& T, const TileLea
     } else if constexpr (KIND == TK_GG && (GEO == TG_ARC || GEO == TG_SPHEUC)) {
         // ProjectHelper<Sphere>, include/ProjectHelper.h:272-388: directions at p2
         // (sinA, -cosA) and at p1 (-sinA, -cosB) on accurate differences (d = p1 - p2):
-        // y1 x2 - x1 y2 = x1 dy - y1 dx.  Spin 2: exp(-2i a) = conj(u)^2 / |u|^2; the two
-        // normalisations are one reciprocal, applied as the scale sc.
+        // y1 x2 - x1 y2 = x1 dy - y1 dx.  Spin 2: exp(-2i a) = conj(u)^2 / |u|^2; that at p1 is
+        // applied as the scale sc.  (One reciprocal of both, n1 n2, could be of 0: near a pole n1
+        // is POLE_SQ.)
         const float4 Xa = LA.X[i];
         const float sinA = fmaf(Xa.x, dy, -Xa.y * dx);
         const float cosA = fmaf(Pb.w, dsq, dz);
         const float cosB = fmaf(Pa.w, dsq, -dz);
-        const float s2 = sinA * sinA;
-        const float n2 = fmaf(cosA, cosA, s2), n1 = fmaf(cosB, cosB, s2);
-        const float e2r = fmaf(-cosA, cosA, s2), e2i = 2.f * sinA * cosA;
-        const float e1r = fmaf(-cosB, cosB, s2), e1i = -2.f * sinA * cosB;
-        sc = __fdividef(1.f, n1 * n2);
-        const float a2r = fmaf(Wb.y, e2r, -Wb.z * e2i), a2i = fmaf(Wb.y, e2i, Wb.z * e2r);
+        const float s2 = sinA * sinA, sp = s2 + POLE_SQ, sm = s2 - POLE_SQ;
+        const float i2 = __fdividef(1.f, fmaf(cosA, cosA, sp));
+        const float e2r = fmaf(-cosA, cosA, sm), e2i = 2.f * sinA * cosA;
+        const float e1r = fmaf(-cosB, cosB, sm), e1i = -2.f * sinA * cosB;
+        sc = __fdividef(1.f, fmaf(cosB, cosB, sp));
+        const float a2r = fmaf(Wb.y, e2r, -Wb.z * e2i) * i2, a2i = fmaf(Wb.y, e2i, Wb.z * e2r) * i2;
         const float a1r = fmaf(Wa.y, e1r, -Wa.z * e1i), a1i = fmaf(Wa.y, e1i, Wa.z * e1r);
         // both_complex_prod(g2, g1), include/ProjectHelper.h:84-101.
         x[0] = fmaf(a2r, a1r, a2i * a1i);     // xi+

@@ -123,12 +123,11 @@ __device__ __forceinline__ void walk_products(const TravParams& T, float4 Aa, fl
         const float sinA = Aa.x * dy - Aa.y * dx;
         const float cosA = fmaf(0.5f * Ba.z, dsq, dz);
         const float cosB = fmaf(0.5f * Aa.z, dsq, -dz);
-        const float s2 = sinA * sinA;
-        const float n2 = fmaf(cosA, cosA, s2), n1 = fmaf(cosB, cosB, s2);
-        const float i2 = n2 > 0.f ? __fdividef(1.f, n2) : 1.f;
-        const float i1 = n1 > 0.f ? __fdividef(1.f, n1) : 1.f;
-        const float e2r = fmaf(-cosA, cosA, s2), e2i = 2.f * sinA * cosA;
-        const float e1r = fmaf(-cosB, cosB, s2), e1i = -2.f * sinA * cosB;
+        const float s2 = sinA * sinA, sp = s2 + POLE_SQ, sm = s2 - POLE_SQ;   // (see POLE_SQ)
+        const float i2 = __fdividef(1.f, fmaf(cosA, cosA, sp));
+        const float i1 = __fdividef(1.f, fmaf(cosB, cosB, sp));
+        const float e2r = fmaf(-cosA, cosA, sm), e2i = 2.f * sinA * cosA;
+        const float e1r = fmaf(-cosB, cosB, sm), e1i = -2.f * sinA * cosB;
         const float a2r = (Bc.x * e2r - Bc.y * e2i) * i2, a2i = (Bc.x * e2i + Bc.y * e2r) * i2;
         const float a1r = (Ac.x * e1r - Ac.y * e1i) * i1, a1i = (Ac.x * e1i + Ac.y * e1r) * i1;
         const float rr = a2r * a1r, ri = a2r * a1i, ir = a2i * a1r, ii = a2i * a1i;
