@@ -701,6 +701,7 @@ int expand_scratch(tc_corr2* c, int nwarps, int nq)
     if (nwarps > c->nwarps_alloc || nq > c->nq_alloc || !c->ctl) {
         dfree(c->wacc); dfree(c->wnp); dfree(c->tot); dfree(c->totnp); dfree(c->ctl);
         dfree(c->d_err);
+        c->nwarps_alloc = 0;            // (until all of them are there)
         TC_TRY(dalloc(&c->wacc, (size_t)nwarps * nq * c->nbins));
         TC_TRY(dalloc(&c->wnp, (size_t)nwarps * c->nbins));
         TC_TRY(dalloc(&c->tot, (size_t)(SUM_SLICES + 1) * nq * c->nbins));
@@ -933,13 +934,11 @@ int walk_stack_cap(long long npoints)
     return 96 * 2 * (lg + 8) + 128;
 }
 
-// Rows the walk's units may fill: enough that the last units to finish do not matter
-// (~7 per warp), bounded by 256 MB.
-long long walk_max_units(int nq, int nb)
-{
-    const long long row = 8LL * (nq + 1) * nb;
-    return std::max(4096LL, std::min(32768LL, (256LL << 20) / row));
-}
+// Rows of one launch of the walk: 256 MB of them, or 4096 (one per warp of the grid).
+long long walk_rows(int nq, int nb) { return std::max(4096LL, (256LL << 20) / (8LL * (nq + 1) * nb)); }
+
+// Units of a traversal: enough that the last ones to finish do not matter (~7 per warp).
+long long walk_max_units(int nq, int nb) { return std::min(32768LL, walk_rows(nq, nb)); }
 
 // The bin_slop traversal of whole fields: the expansion up to a level of enough items, then
 // the walk.  *done = false when the walk ran out of stack (nothing is added then).
@@ -1069,8 +1068,9 @@ int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cud
 
 // The patch batch by the walk, straight from the top-level items: every unit belongs to one
 // patch pair, so its row holds that pair's sums only and the pairs' rows are added in order.
-// (The expansion's warps mix pairs, each with atomic adds to its pair's sums.)  *walked =
-// false when it does not apply or ran out of stack.
+// (The expansion's warps mix pairs, each with atomic adds to its pair's sums.)  A pair has one
+// unit at least, so many pairs take several launches of walk_rows units.  *walked = false when it
+// does not apply or ran out of stack.
 int walk_patches(tc_corr2* c, TravParams T, const std::vector<long long>& roff,
                  const std::vector<int>& P1, const std::vector<int>& P2, long long npoints, int nq,
                  double* pacc, unsigned long long* pnp, cudaStream_t st, int* derr,
@@ -1086,16 +1086,27 @@ int walk_patches(tc_corr2* c, TravParams T, const std::vector<long long>& roff,
         weight += (double)n * (P1[p] == P2[p] ? 4. : 1.);
     }
     const double share = (double)walk_max_units(nq, nb) / std::max(weight, 1.);
-    std::vector<int> uoff(npair + 1, 0);
+    // Launches: pairs p0 .. p1 - 1, whose units' offsets begin at uoff[at].
+    struct Launch { int p0, p1, at; };
+    std::vector<Launch> launch;
+    std::vector<int> uoff;
+    const long long max_rows = walk_rows(nq, nb);
+    int most = 0;
     for (int p = 0; p < npair; ++p) {
         const long long n = roff[p + 1] - roff[p];
-        const long long u = (long long)(share * (double)n * (P1[p] == P2[p] ? 4. : 1.));
-        uoff[p + 1] = uoff[p] + (int)std::max(1LL, std::min(u, (n + 31) / 32));
+        const long long share_u = (long long)(share * (double)n * (P1[p] == P2[p] ? 4. : 1.));
+        const long long u = std::max(1LL, std::min(share_u, (n + 31) / 32));
+        if (launch.empty() || uoff.back() + u > max_rows) {
+            launch.push_back(Launch{p, p, (int)uoff.size()});
+            uoff.push_back(0);
+        }
+        uoff.push_back(uoff.back() + (int)u);
+        launch.back().p1 = p + 1;
+        most = std::max(most, uoff.back());
     }
-    const int n_units = uoff[npair];
     int wblocks = 0, wwarps = 0;
     TC_TRY(walk_grid(T, &wblocks, &wwarps));
-    TC_TRY(expand_scratch(c, n_units, nq));
+    TC_TRY(expand_scratch(c, most, nq));
     T.err = c->d_err; T.counters = c->ctl + 2;
     T.wctr = nullptr;
     WalkParams W;
@@ -1108,21 +1119,29 @@ int walk_patches(tc_corr2* c, TravParams T, const std::vector<long long>& roff,
     TC_CU(cudaMemcpyAsync(off.p, uoff.data(), sizeof(int) * uoff.size(), cudaMemcpyHostToDevice, st));
     TC_CU(cudaMemsetAsync(c->ctl, 0, 8 * sizeof(unsigned long long), st));
     TC_CU(cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
-    TC_CU(cudaMemsetAsync(c->wacc, 0, sizeof(double) * (size_t)n_units * nq * nb, st));
-    TC_CU(cudaMemsetAsync(c->wnp, 0, sizeof(unsigned long long) * (size_t)n_units * nb, st));
-    W.n_units = (unsigned)n_units;
-    W.unit_off = static_cast<const int*>(off.p);
     W.next = c->ctl;
     W.stacks = static_cast<int2*>(stacks.p);
     W.stack_cap = cap;
     W.rows = c->wacc;
     W.rownp = c->wnp;
-    TC_TRY(launch_walk(T, W, wblocks, st));
-    TC_TRY(launch_sum_rows(c->wacc, c->wnp, n_units, W.unit_off, npair, nq * nb, nb, pacc, pnp, st));
+    const long long* const proot_off = T.proot_off;
+    const int2* const ppairs = T.ppairs;
+    for (const Launch& l : launch) {
+        const int np = l.p1 - l.p0, n_units = uoff[l.at + np];
+        T.npair = np; T.proot_off = proot_off + l.p0; T.ppairs = ppairs + l.p0;
+        W.n_units = (unsigned)n_units;
+        W.unit_off = static_cast<const int*>(off.p) + l.at;
+        TC_CU(cudaMemsetAsync(c->ctl, 0, sizeof(unsigned long long), st));
+        TC_CU(cudaMemsetAsync(c->wacc, 0, sizeof(double) * (size_t)n_units * nq * nb, st));
+        TC_CU(cudaMemsetAsync(c->wnp, 0, sizeof(unsigned long long) * (size_t)n_units * nb, st));
+        TC_TRY(launch_walk(T, W, wblocks, st));
+        TC_TRY(launch_sum_rows(c->wacc, c->wnp, n_units, W.unit_off, np, nq * nb, nb,
+                               pacc + (size_t)l.p0 * nq * nb, pnp + (size_t)l.p0 * nb, st));
+    }
     TC_CU(cudaMemcpyAsync(derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     TC_CU(cudaStreamSynchronize(st));
     if (*derr == DEV_STACK_OVERFLOW) { *derr = 0; return TC_OK; }
-    *launches = 2;
+    *launches = 2 * (long long)launch.size();
     *walked = true;
     return TC_OK;
 }
