@@ -1418,13 +1418,14 @@ static int scratch_levels(int n, BuildScratch& S, cudaStream_t st)
     return 0;
 }
 
-static int launch_root(const BuildTask& root, const LevelBufs& L, cudaStream_t st)
+// *nc: the root's chunks.
+static int launch_root(const BuildTask& root, const LevelBufs& L, int* nc, cudaStream_t st)
 {
-    const int nc = (root.e - root.s + L.ch - 1) / L.ch;
+    *nc = (root.e - root.s + L.ch - 1) / L.ch;
     count_launch();
-    k_level_root<<<(nc + 255) / 256, 256, 0, st>>>(L, root);
+    k_level_root<<<(*nc + 255) / 256, 256, 0, st>>>(L, root);
     TC_CU(cudaGetLastError());
-    return nc;
+    return 0;
 }
 
 // 27 small kernels follow each other in a build of 25,000 points, 2 us apart: launch_chained takes
@@ -1471,7 +1472,8 @@ int tree_begin(const TreeBuild& B, BuildRun& R, BuildRead* to, cudaMemcpyKind ki
         R.whole = true;
         return 0;
     } else {
-        launch_root(root, L, st);
+        int nc = 0;
+        TC_TRY(launch_root(root, L, &nc, st));
         R.batch = 2;
         for (int m = L.sub; m < n; m = m > (1 << 29) ? n : 2 * m) ++R.batch;
         TC_TRY(queue_levels(B, R, st));
@@ -1551,7 +1553,8 @@ int field_center(const BuildParams& BP, Points P, BuildScratch& S, cudaStream_t 
     TC_TRY(scratch_levels(n, S, st));
     BuildParams B2 = BP;
     B2.split = MEAN;
-    const int nc = launch_root(root, S.L, st);
+    int nc = 0;
+    TC_TRY(launch_root(root, S.L, &nc, st));
     TC_TRY(launch_chained(k_chunk_pass1, nc, CB, 0, st, S.L, 0, P, P, B2));
     TC_TRY(launch_chained(k_chunk_pass2, nc, CB, 0, st, S.L, 0, P, P, B2, Cells{}, nullptr, nullptr,
                           nullptr, 1));
