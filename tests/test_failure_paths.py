@@ -3,6 +3,7 @@ copy: its object files linked with a runtime that can be made to (fake_cuda.cpp)
 import ctypes
 import os
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -74,3 +75,24 @@ def test_build_reports_its_first_launch(lib):
     assert lib.fake_launches() == at + 1, "launches after the one that failed"
     lib.tc_field_free(h)
     lib.fake_reset()
+
+
+def test_one_stream_for_all_threads(lib):
+    """Allocations and kernels are ordered by the library's one stream: first calls from several
+    threads must not each make one.  (A process of its own: the first call comes once.)"""
+    code = """
+import ctypes, sys, threading
+L = ctypes.CDLL(sys.argv[1])
+L.fake_streams.restype = ctypes.c_longlong
+L.fake_slow_streams(200)
+go = threading.Barrier(8)
+def call():
+    go.wait()
+    L.tc_trim_memory()
+t = [threading.Thread(target=call) for _ in range(8)]
+[x.start() for x in t]
+[x.join() for x in t]
+print(L.fake_streams())
+"""
+    r = subprocess.run([sys.executable, "-c", code, lib.path], capture_output=True, text=True, check=True)
+    assert r.stdout.split() == ["1"]

@@ -37,11 +37,18 @@ static std::atomic<long long> g_launches{0};
 static std::atomic<int> g_deterministic{1};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
-static cudaStream_t g_stream = nullptr;
+// The library's one stream, made by the first call that needs it, whichever thread that is on.
+static std::atomic<cudaStream_t> g_stream{nullptr};
 static int stream_get(cudaStream_t* s)
 {
-    if (!g_stream) TC_CU(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
-    *s = g_stream;
+    static std::mutex mu;
+    *s = g_stream.load(std::memory_order_acquire);
+    if (*s) return 0;
+    std::lock_guard<std::mutex> lk(mu);
+    *s = g_stream.load(std::memory_order_relaxed);
+    if (*s) return 0;
+    TC_CU(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+    g_stream.store(*s, std::memory_order_release);
     return 0;
 }
 
@@ -106,7 +113,7 @@ int dev_alloc(void** p, size_t bytes)
 
 void dev_free(void* p)
 {
-    if (p) cudaFreeAsync(p, g_stream);
+    if (p) cudaFreeAsync(p, g_stream.load(std::memory_order_acquire));
 }
 
 static const char* dev_err_msg(int code)
