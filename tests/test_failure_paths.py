@@ -32,7 +32,7 @@ def lib(tmp_path_factory):
     L.tc_last_error.restype = ctypes.c_char_p
     L.tc_field_ntop.restype = ctypes.c_int64
     L.tc_field_ntop.argtypes = [ctypes.c_void_p]
-    L.tc_field_free.argtypes = [ctypes.c_void_p]
+    L.tc_field_free.argtypes = L.tc_corr2_free.argtypes = [ctypes.c_void_p]
     L.fake_reset()
     L.path = out
     return L
@@ -75,6 +75,91 @@ def test_build_reports_its_first_launch(lib):
     assert lib.fake_launches() == at + 1, "launches after the one that failed"
     lib.tc_field_free(h)
     lib.fake_reset()
+
+
+def _patches(L, *fields):
+    nb, n = 3, len(fields)
+    o = [np.zeros(nb) for _ in range(8)]
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    d, big = ctypes.c_double, sys.float_info.max
+    c = ctypes.c_void_p()
+    assert L.tc_corr2_create(0, 0, 0, d(1.), d(10.), nb, d(np.log(10.) / nb), d(0.1), d(0.1), d(-big), d(big),
+                             d(0.), d(0.), d(0.), *map(p, o), ctypes.byref(c)) == 0
+    i, j, res, got = np.zeros(3, np.int32), np.zeros(3, np.int32), np.zeros((3, 8, nb)), ctypes.c_int(0)
+    rc = L.tc_corr2_process_patches(c, (ctypes.c_void_p * n)(*fields), n, 1, 0, 3, p(i), p(j), p(res),
+                                    ctypes.byref(got))
+    L.tc_corr2_free(c)
+    return rc
+
+
+# fields built alone and side by side (as patches)
+BUILDS = {1: lambda L, f: L.tc_field_ntop(f[0]) < 0, 2: lambda L, f: _patches(L, *f) != 0}
+
+
+@pytest.mark.parametrize("n", [200, 3000])
+@pytest.mark.parametrize("fields", [1, 2])
+def test_build_without_memory_keeps_nothing_and_can_be_repeated(lib, fields, n):
+    lib.fake_reset()
+    f = [_create(lib, n)[1] for _ in range(fields)]
+    before, at = lib.fake_bytes(), lib.fake_allocs()
+    assert lib.tc_field_ntop(_create(lib, n)[1]) >= 0
+    most = lib.fake_allocs() - at                    # (of a field's creation and its build)
+    for k in range(most):
+        lib.fake_reset()
+        lib.fake_fail_allocs_from(k)
+        other = lib.fake_bytes()
+        if fields == 1 and lib.tc_field_ntop(f[0]) >= 0:
+            assert k > 8                             # (enough for a build)
+            break
+        if fields == 2:
+            assert k > 16 or BUILDS[2](lib, f)
+        assert lib.fake_bytes() == other, k
+    lib.fake_reset()
+    for h in f:
+        assert lib.tc_field_ntop(h) >= 0             # (there was memory again)
+        lib.tc_field_free(h)
+
+
+@pytest.mark.parametrize("n", [200, 3000])
+@pytest.mark.parametrize("fields", [1, 2])
+def test_build_that_failed_keeps_nothing_and_is_not_repeated(lib, fields, n):
+    """A build that stopped on its way has moved the points: another on them would not be this
+    catalog's tree."""
+    lib.fake_reset()
+    h = _create(lib, n)[1]
+    at = lib.fake_launches()
+    assert lib.tc_field_ntop(h) >= 0
+    launches = lib.fake_launches() - at              # of a build
+    lib.tc_field_free(h)
+    for k in range(launches):
+        lib.fake_reset()
+        f = [_create(lib, n)[1] for _ in range(fields)]
+        before = lib.fake_bytes()
+        lib.fake_fail_launch(lib.fake_launches() + k)
+        assert BUILDS[fields](lib, f), k
+        assert lib.fake_bytes() <= before, k
+        why = lib.tc_last_error()
+        lib.fake_reset()
+        for q in f:
+            assert lib.tc_field_ntop(q) < 0 and lib.tc_last_error() == why
+            lib.tc_field_free(q)
+    # an error that the kernels report: of the two fields of a group the one it is for
+    lib.fake_reset()
+    f = [_create(lib, n)[1]]
+    word = lib.fake_word()                           # (the field's error word is the first cleared)
+    before = lib.fake_bytes()
+    f += [_create(lib, n)[1] for _ in range(fields - 1)]
+    one = lib.fake_bytes() - before
+    word[0] = 5
+    assert BUILDS[fields](lib, f) and b"device error" in lib.tc_last_error()
+    why = lib.tc_last_error()
+    lib.fake_reset()
+    for q in f[1:]:
+        assert lib.tc_field_ntop(q) >= 0
+        lib.tc_field_free(q)
+    assert lib.fake_bytes() <= before
+    assert lib.tc_field_ntop(f[0]) < 0 and lib.tc_last_error() == why
+    lib.tc_field_free(f[0])
 
 
 def test_one_stream_for_all_threads(lib):

@@ -142,6 +142,8 @@ struct tc_field {
     int64_t n = 0;
     double minsize = 0., maxsize = 0.;
     bool built = false;
+    int broken = 0;              // the error of a build that stopped on its way, and its message
+    std::string broken_why;
     Points buf[2] = {};
     Cells cells = {};
     TCell* tcells = nullptr;
@@ -353,13 +355,29 @@ int build_arrays(tc_field* f)
     return 0;
 }
 
-// Takes back build_arrays.
+// Takes back build_arrays (all or some of it).
 void drop_build_arrays(tc_field* f)
 {
     free_cells(f->cells);
-    dfree(f->tcells); dfree(f->d_tops_raw); dfree(f->d_ntop);
+    dfree(f->tcells); dfree(f->d_tops_raw); dfree(f->d_ntop); dfree(f->d_tops);
     dfree(f->S.L.small); dfree(f->S.wstack);
     free_points(f->buf[1]);
+}
+
+// A build that stopped on its way has moved points between its two buffers: another one would
+// build some other catalog's tree.  The field keeps nothing of it, and its error.
+int build_broke(tc_field* f, int rc)
+{
+    drop_build_arrays(f);
+    f->broken = rc;
+    f->broken_why = g_last_error;
+    return rc;
+}
+
+int check_broken(const tc_field* f)
+{
+    if (f->broken) set_last_error(f->broken_why);
+    return f->broken;
 }
 
 // Unused ids (inside list leaves) keep harmless contents: no children, no points.
@@ -390,10 +408,11 @@ TreeBuild tree_of(tc_field* f)
     return B;
 }
 
-// The ordered tops onto the device, and the check of the finished tree.
+// The ordered tops onto the device, in place of the pairs they were made from (the host has
+// read those), and the check of the finished tree.
 int finish_tops(tc_field* f, cudaStream_t st)
 {
-    TC_TRY(dalloc(&f->d_tops, f->tops.size()));
+    std::swap(f->d_tops, f->d_tops_raw);
     TC_CU(cudaMemcpyAsync(f->d_tops, f->tops.data(), f->tops.size() * sizeof(int),
                           cudaMemcpyHostToDevice, st));
     launch_validate_tree((int)(2 * f->n - 1), f->cells, f->d_tops, (int)f->tops.size(), f->d_err, st);
@@ -409,19 +428,27 @@ void set_built(tc_field* f)
     f->built = true;
 }
 
-// BaseField::BuildCells (src/Field.cpp:206-277) on the device.
-int field_build(tc_field* f)
+// Events that end with a call.
+struct Events {
+    cudaEvent_t a = nullptr, b = nullptr;
+    int make()
+    {
+        TC_CU(cudaEventCreate(&a));
+        TC_CU(cudaEventCreate(&b));
+        return 0;
+    }
+    ~Events()
+    {
+        if (a) cudaEventDestroy(a);
+        if (b) cudaEventDestroy(b);
+    }
+};
+
+// field_build with its arrays there.
+int build_one(tc_field* f, const Events& ev, cudaStream_t st)
 {
-    if (f->built) return 0;
-    cudaStream_t st;
-    TC_TRY(stream_get(&st));
-    if (f->n == 0) { f->built = true; return 0; }
-    TC_TRY(build_arrays(f));
     TC_TRY(clear_cells(f->cells, 2 * f->n - 1, st));
-    cudaEvent_t e0, e1;
-    TC_CU(cudaEventCreate(&e0));
-    TC_CU(cudaEventCreate(&e1));
-    TC_CU(cudaEventRecord(e0, st));
+    TC_CU(cudaEventRecord(ev.a, st));
     const TreeBuild B = tree_of(f);
     BuildRun R;
     std::unique_ptr<BuildRead> read(new BuildRead());
@@ -431,12 +458,26 @@ int field_build(tc_field* f)
     TC_CU(cudaStreamSynchronize(st));
     TC_TRY(tree_tops(B, *read, st, f->tops));
     TC_TRY(finish_tops(f, st));
-    TC_CU(cudaEventRecord(e1, st));
-    const int rc = check_dev_err(f->d_err, st);     // (waits for the stream)
-    if (!rc) cudaEventElapsedTime(&f->build_ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (rc) return rc;
+    TC_CU(cudaEventRecord(ev.b, st));
+    TC_TRY(check_dev_err(f->d_err, st));            // (waits for the stream)
+    cudaEventElapsedTime(&f->build_ms, ev.a, ev.b);
+    return 0;
+}
+
+// BaseField::BuildCells (src/Field.cpp:206-277) on the device.
+int field_build(tc_field* f)
+{
+    if (f->built) return 0;
+    TC_TRY(check_broken(f));
+    cudaStream_t st;
+    TC_TRY(stream_get(&st));
+    if (f->n == 0) { f->built = true; return 0; }
+    Events ev;
+    TC_TRY(ev.make());
+    int rc = build_arrays(f);
+    if (rc) { drop_build_arrays(f); return rc; }    // (no kernel has run: it can be tried again)
+    rc = build_one(f, ev, st);
+    if (rc) return build_broke(f, rc);
     set_built(f);
     return 0;
 }
@@ -473,14 +514,13 @@ struct GroupBuild {
     std::vector<int> err;
     BuildRead* d_read = nullptr;
     int* d_errs = nullptr;
-    cudaEvent_t ev = nullptr, e0 = nullptr, e1 = nullptr;
+    cudaEvent_t ev = nullptr;
+    Events time;
     cudaStream_t side[SIDES] = {nullptr};
     ~GroupBuild()
     {
         dfree(d_read); dfree(d_errs);
         if (ev) cudaEventDestroy(ev);
-        if (e0) cudaEventDestroy(e0);
-        if (e1) cudaEventDestroy(e1);
     }
     // The library's stream after the sides, and what they have written on the host.
     int join(cudaStream_t st)
@@ -500,6 +540,9 @@ struct GroupBuild {
 
 int GroupBuild::run(cudaStream_t st)
 {
+    TC_CU(cudaMemsetAsync(d_read, 0, sizeof(BuildRead) * f.size(), st));
+    TC_CU(cudaEventRecord(time.a, st));
+    for (int k = 0; k < SIDES; ++k) TC_CU(cudaStreamWaitEvent(side[k], time.a, 0));
     for (size_t i = 0; i < f.size(); ++i) {
         cudaStream_t s = side[i % SIDES];
         B.push_back(tree_of(f[i]));
@@ -515,7 +558,7 @@ int GroupBuild::run(cudaStream_t st)
         TC_TRY(finish_tops(f[i], st));
         TC_CU(cudaMemcpyAsync(d_errs + i, f[i]->d_err, sizeof(int), cudaMemcpyDeviceToDevice, st));
     }
-    TC_CU(cudaEventRecord(e1, st));
+    TC_CU(cudaEventRecord(time.b, st));
     TC_CU(cudaMemcpyAsync(err.data(), d_errs, sizeof(int) * f.size(), cudaMemcpyDeviceToHost, st));
     TC_CU(cudaStreamSynchronize(st));
     return 0;
@@ -527,6 +570,8 @@ int build_group(const std::vector<tc_field*>& fields, size_t* taken)
     TC_TRY(stream_get(&st));
     GroupBuild G;
     TC_TRY(side_streams(G.side));
+    TC_CU(cudaEventCreateWithFlags(&G.ev, cudaEventDisableTiming));
+    TC_TRY(G.time.make());
     int64_t points = 0;
     for (tc_field* f : fields) {
         if (build_arrays(f)) { drop_build_arrays(f); break; }
@@ -544,23 +589,24 @@ int build_group(const std::vector<tc_field*>& fields, size_t* taken)
         return 0;
     }
     G.R.resize(m); G.host.resize(m); G.err.assign(m, 0); G.B.reserve(m);
-    TC_CU(cudaMemsetAsync(G.d_read, 0, sizeof(BuildRead) * m, st));
-    TC_CU(cudaEventCreateWithFlags(&G.ev, cudaEventDisableTiming));
-    TC_CU(cudaEventCreate(&G.e0));
-    TC_CU(cudaEventCreate(&G.e1));
-    TC_CU(cudaEventRecord(G.e0, st));
-    for (int k = 0; k < SIDES; ++k) TC_CU(cudaStreamWaitEvent(G.side[k], G.e0, 0));
     rc = G.run(st);
     if (rc) {
-        // Nothing of the group is in flight when the caller frees its fields.
+        // Nothing of the group is in flight when its arrays are freed.
         for (int k = 0; k < SIDES; ++k) cudaStreamSynchronize(G.side[k]);
+        for (tc_field* f : G.f) build_broke(f, rc);
         return rc;
     }
     float ms = 0.f;
-    cudaEventElapsedTime(&ms, G.e0, G.e1);
+    cudaEventElapsedTime(&ms, G.time.a, G.time.b);
     for (size_t i = 0; i < m; ++i) {
         tc_field* f = G.f[i];
-        if (G.err[i]) { const int e = check_dev_err(f->d_err, st); if (!rc) rc = e; continue; }
+        if (G.err[i]) {
+            int e = check_dev_err(f->d_err, st);
+            if (!e) e = TC_ERR_DEVICE;
+            build_broke(f, e);
+            rc = e;
+            continue;
+        }
         f->build_ms = ms * (float)f->n / (float)points;
         set_built(f);
     }
@@ -572,8 +618,10 @@ int build_fields(tc_field* const* fields, int nf)
 {
     std::vector<tc_field*> todo;
     for (int i = 0; i < nf; ++i)
-        if (fields[i] && !fields[i]->built && std::find(todo.begin(), todo.end(), fields[i]) == todo.end())
+        if (fields[i] && !fields[i]->built && std::find(todo.begin(), todo.end(), fields[i]) == todo.end()) {
+            TC_TRY(check_broken(fields[i]));
             todo.push_back(fields[i]);
+        }
     for (size_t at = 0; at < todo.size();) {
         std::vector<tc_field*> g;
         int64_t points = 0;
@@ -977,7 +1025,7 @@ int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cud
     TC_CU(cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
     cudaEvent_t e0, e1, e2;
     TC_CU(cudaEventCreate(&e0)); TC_CU(cudaEventCreate(&e1)); TC_CU(cudaEventCreate(&e2));
-    struct Events { cudaEvent_t a, b, c; ~Events() { cudaEventDestroy(a); cudaEventDestroy(b); cudaEventDestroy(c); } } ev{e0, e1, e2};
+    struct Destroy { cudaEvent_t a, b, c; ~Destroy() { cudaEventDestroy(a); cudaEventDestroy(b); cudaEventDestroy(c); } } ev{e0, e1, e2};
     TC_CU(cudaEventRecord(e0, st));
     WalkParams W;
     std::memset(&W, 0, sizeof(W));
@@ -2346,7 +2394,7 @@ int tc_corr2_process_patches(tc_corr2* c, tc_field* const* fields, int npatch, i
         T.ptop_off = d_topoff;
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0); cudaEventCreate(&e1);
-        struct Events { cudaEvent_t a, b; ~Events() { cudaEventDestroy(a); cudaEventDestroy(b); } } ev{e0, e1};
+        struct Destroy { cudaEvent_t a, b; ~Destroy() { cudaEventDestroy(a); cudaEventDestroy(b); } } ev{e0, e1};
         cudaEventRecord(e0, st);
         int derr = 0;
         long long launches = 0;
