@@ -17,6 +17,9 @@ std::map<void*, size_t> live;
 long long bytes = 0, launches = 0, allocs = 0, streams = 0;
 long long fail_launch = -1, fail_alloc = -1;    // the launch or allocation (counted from 0) that fails
 const void* fail_copy = nullptr;                // a copy to this address fails
+long long answer_at = -1;                       // the 4-byte copy that brings `answer`
+long long copies4 = 0;
+int answer = 0;
 void* word = nullptr;                           // the first 4-byte memset since fake_reset
 cudaError_t last = cudaSuccess;
 int slow_stream_ms = 0;
@@ -47,11 +50,14 @@ void fake_reset()
     fail_launch = fail_alloc = -1;
     fail_copy = nullptr;
     word = nullptr;
+    answer_at = -1;
+    copies4 = 0;
     last = cudaSuccess;
 }
 void fake_fail_launch(long long k) { fail_launch = k; }
 void fake_fail_allocs_from(long long k) { fail_alloc = k; }
 void fake_fail_copy_to(const void* p) { fail_copy = p; }
+void fake_answer(long long k, int v) { answer_at = k; answer = v; }
 void fake_slow_streams(int ms) { slow_stream_ms = ms; }
 long long fake_launches() { return launches; }
 long long fake_allocs() { return allocs; }
@@ -84,6 +90,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 {
     if (d == fail_copy) return last = cudaErrorUnknown;
     std::memcpy(d, s, n);
+    if (n == 4 && copies4++ == answer_at) *static_cast<int*>(d) = answer;
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, s, n, k, nullptr); }

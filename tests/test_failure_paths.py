@@ -181,3 +181,20 @@ print(L.fake_streams())
 """
     r = subprocess.run([sys.executable, "-c", code, lib.path], capture_output=True, text=True, check=True)
     assert r.stdout.split() == ["1"]
+
+
+def test_assign_that_failed_leaves_the_callers_array(lib):
+    """KMeansAssign fills an array that may have no pages yet; without a result it stays as it was."""
+    lib.fake_reset()
+    n, k = 200, 3
+    h = _create(lib, n)[1]
+    lib.fake_answer(ctypes.c_longlong(0), 1)         # (the first of a small build's: its top-level cells)
+    assert lib.tc_field_ntop(h) == 1
+    cen, out = np.arange(2. * k), np.arange(n, dtype=np.int64) + 7
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    lib.fake_fail_copy_to(p(out))
+    rc = lib.tc_kmeans_assign(h, p(cen), k, p(out), ctypes.c_int64(n))
+    assert rc != 0
+    np.testing.assert_array_equal(out, np.arange(n) + 7)
+    lib.fake_reset()
+    lib.tc_field_free(h)

@@ -1532,9 +1532,12 @@ int kmeans_assign(const KMField& F, const double* centers, int npatch, int64_t* 
         k_km_paint_big<<<1216, 256, 0, st>>>(F.cells, S.assign, S.tag, F.idx, big, nbig, d_out);
         if (cudaGetLastError() != cudaSuccess) { set_last_error("k-means assign launch failed"); rc = TC_ERR_CUDA; break; }
         // The caller's array may have no pages yet: the copy takes 16 ms for 16 MB where the device
-        // has to fault them in one by one, 1 ms where they are there.
-        for (int64_t i = 0; i < F.n; i += 4096 / (int64_t)sizeof(int64_t))
-            *const_cast<volatile int64_t*>(patches + i) = -1;
+        // has to fault them in one by one, 1 ms where they are there.  (A store of what is there
+        // makes a page, and a call that fails leaves the array as it was.)
+        for (int64_t i = 0; i < F.n; i += 4096 / (int64_t)sizeof(int64_t)) {
+            volatile int64_t* q = patches + i;
+            *q = *q;
+        }
         if (cudaMemcpyAsync(patches, d_out, sizeof(int64_t) * F.n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             set_last_error("k-means assign copy failed"); rc = TC_ERR_CUDA; break;
