@@ -31,6 +31,9 @@
 #include <unordered_map>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "../../include/tcgpu.h"
 #include "tc_host.hpp"
 #include "kmeans.hpp"
@@ -1507,6 +1510,23 @@ int kmeans_run(const KMField& F, double* centers, int npatch, int max_iter, doub
     return 0;
 }
 
+// A caller's array may have no pages yet: a copy from the device takes 16 ms for 16 MB where the
+// device has to fault them in one by one, 1 ms where they are there.  The contents stay, so that a
+// call that fails leaves the array as it was.
+static void make_pages(void* p, size_t bytes)
+{
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), at = (uintptr_t)p & ~(page - 1);
+    const size_t len = (uintptr_t)p + bytes - at;
+#ifdef MADV_POPULATE_WRITE
+    if (madvise((void*)at, len, MADV_POPULATE_WRITE) == 0) return;
+#endif
+    // (Linux before 5.14; two faults a page.)
+    for (size_t i = 0; i < bytes; i += 4096) {
+        volatile char* q = static_cast<char*>(p) + i;
+        *q = *q;
+    }
+}
+
 int kmeans_assign(const KMField& F, const double* centers, int npatch, int64_t* patches,
                   cudaStream_t st)
 {
@@ -1531,13 +1551,7 @@ int kmeans_assign(const KMField& F, const double* centers, int npatch, int64_t* 
         count_launch();
         k_km_paint_big<<<1216, 256, 0, st>>>(F.cells, S.assign, S.tag, F.idx, big, nbig, d_out);
         if (cudaGetLastError() != cudaSuccess) { set_last_error("k-means assign launch failed"); rc = TC_ERR_CUDA; break; }
-        // The caller's array may have no pages yet: the copy takes 16 ms for 16 MB where the device
-        // has to fault them in one by one, 1 ms where they are there.  (A store of what is there
-        // makes a page, and a call that fails leaves the array as it was.)
-        for (int64_t i = 0; i < F.n; i += 4096 / (int64_t)sizeof(int64_t)) {
-            volatile int64_t* q = patches + i;
-            *q = *q;
-        }
+        make_pages(patches, sizeof(int64_t) * (size_t)F.n);
         if (cudaMemcpyAsync(patches, d_out, sizeof(int64_t) * F.n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             set_last_error("k-means assign copy failed"); rc = TC_ERR_CUDA; break;
