@@ -233,8 +233,9 @@ int tc_corr2_set_tuning(tc_corr2* c, int tile_leaf, int64_t chunk);
 
 /* The autotuner: times this correlation of f1 (and f2, NULL for an auto-correlation) on its
  * first frac of top-level cell pairs for tile leaf sizes 24..64 (exact mode only), then for
- * expansion chunks down to 1/8 of the default, keeps the fastest in c (as
- * tc_corr2_set_tuning) and in a per-process cache keyed by the classes, coordinates, metric,
+ * the powers of two below the default chunk, down to 1/8 of it, that make other launches (none
+ * where the walk starts from the top-level pairs anyway); keeps the fastest, the default unless
+ * another chunk is 2% faster, in c (as tc_corr2_set_tuning) and in a per-process cache keyed by the classes, coordinates, metric,
  * binning, slops, brute flags and catalog sizes (to a factor of 2), so a later call with the
  * same key returns at once.  The corr's output arrays are not touched.  Outputs: the chosen
  * values (0 = default) and the best sample's device time in ms (0 from the cache).  No

@@ -23,6 +23,7 @@
 #include "tc_host.hpp"
 #include "traverse2pt.hpp"
 #include "multipole.hpp"
+#include "tuning.hpp"
 #include "learned.hpp"
 #include "kmeans.hpp"
 #include "catalog.hpp"
@@ -853,15 +854,6 @@ void trav_setup(const tc_corr2* c, TravParams& T, int coords, int metric, int qu
 
 // Runs the breadth-first expansion of T to completion (device-side schedule, batches of
 // launches, more level buffers on demand).  *derr: the device error word afterwards.
-// Items per expansion launch: up to 32M, less for small catalogs (level buffers hold 4
-// chunks each: 1 GB per level at the largest size).
-long long expand_chunk(long long npoints)
-{
-    long long CH = 1LL << 16;
-    while (CH < (1LL << 25) && CH < 2 * npoints) CH <<= 1;
-    return CH;
-}
-
 int expand_run(tc_corr2* c, const TravParams& T, int blocks, long long npoints, cudaStream_t st,
                int* derr_out, long long* launches_out)
 {
@@ -995,6 +987,12 @@ long long walk_rows(int nq, int nb) { return std::max(4096LL, (256LL << 20) / (8
 // Units of a traversal: enough that the last ones to finish do not matter (~7 per warp).
 long long walk_max_units(int nq, int nb) { return std::min(32768LL, walk_rows(nq, nb)); }
 
+// Top-level pairs of a traversal, and pairs of points to each.
+long long root_pairs(const TravParams& T)
+{ return T.autoc ? (long long)T.ntop1 * (T.ntop1 + 1) / 2 : (long long)T.ntop1 * T.ntop2; }
+double pairs_per_root(const TravParams& T, long long n1, long long n2)
+{ return ((double)n1 / (double)T.ntop1) * ((double)n2 / (double)T.ntop2); }
+
 // The bin_slop traversal of whole fields: the expansion up to a level of enough items, then
 // the walk.  *done = false when the walk ran out of stack (nothing is added then).
 int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cudaStream_t st,
@@ -1005,13 +1003,12 @@ int walk_run(tc_corr2* c, TravParams& T, long long n1, long long n2, int nq, cud
     *done = true;
     int blocks = 0, nwarps = 0, wblocks = 0, wwarps = 0;
     TC_TRY(walk_grid(T, &wblocks, &wwarps));
-    // Items the walk starts from: 8 per point, 2^17 to 2^21 (or the tuned chunk).
-    const long long want = c->chunk > 0 ? std::min(c->chunk, 1LL << 21)
-                                        : std::max(1LL << 17, std::min(1LL << 21, 8 * npoints));
-    // With few points per top cell a top-level pair is a small subtree already (at 32 x 32
-    // points some 4000 evaluations at most), and the walk starts from those.
-    const double per_pair = ((double)n1 / (double)T.ntop1) * ((double)n2 / (double)T.ntop2);
-    const bool expand = T.ngen < want && (per_pair > 1024. || T.ngen < 4096);
+    // Items the walk starts from.  (A sample of the autotuner starts at the same depth as the
+    // whole: at its share of the items.)
+    const long long ngen = root_pairs(T);
+    long long want = walk_start(c->chunk, npoints, ngen, pairs_per_root(T, n1, n2));
+    if (T.ngen < ngen) want = (long long)((double)want * (double)T.ngen / (double)ngen);
+    const bool expand = want > 0;
     if (expand) TC_TRY(expand_grid(nq, nb, &blocks, &nwarps, 0));
     const long long max_units = walk_max_units(nq, nb);
     TC_TRY(expand_scratch(c, (int)(nwarps + max_units), nq));
@@ -2634,9 +2631,10 @@ int ilog2(long long n) { int l = 0; while (n > 1) { n >>= 1; ++l; } return l; }
 }  // namespace
 
 // Times the correlation of f1 (and f2) on its first `frac` of top-level pairs for tile leaf
-// sizes 24..64 (exact mode) and then for expansion chunks of 1/2, 1/4 and 1/8 of the default
-// (down to 2^21 items): a coordinate search on event-timed device time.  Keeps the fastest
-// in c and in a per-process cache, and leaves the caller's outputs untouched.
+// sizes 24..64 (exact mode) and then for chunks below the default (tune_chunks: the expansion's in
+// the exact mode, the start of the walk under the bin_slop rule): a coordinate search on event-timed
+// device time.  Keeps the fastest in c and in a per-process cache, and leaves the caller's
+// outputs untouched.
 int tc_corr2_autotune(tc_corr2* c, tc_field* f1, tc_field* f2, int metric, double frac,
                       int* tile_leaf_out, int64_t* chunk_out, double* ms_out)
 {
@@ -2660,10 +2658,12 @@ int tc_corr2_autotune(tc_corr2* c, tc_field* f1, tc_field* f2, int metric, doubl
     TC_TRY(field_build(f1));
     if (f2) TC_TRY(field_build(f2));
     const long long ntop1 = (long long)f1->tops.size();
-    const long long ngen = f2 ? ntop1 * (long long)f2->tops.size() : ntop1 * (ntop1 + 1) / 2;
+    const long long ntop2 = f2 ? (long long)f2->tops.size() : ntop1;
+    const long long ngen = f2 ? ntop1 * ntop2 : ntop1 * (ntop1 + 1) / 2;
     const bool exact = c->a == 0. || (f1->brute && (f2 ? f2->brute : f1->brute));
     const long long npoints = f1->n + (f2 ? f2->n : 0);
-    const long long ch0 = expand_chunk(npoints);
+    const double per_pair = ((double)f1->n / (double)std::max(1LL, ntop1)) *
+                            ((double)(f2 ? f2->n : f1->n) / (double)std::max(1LL, ntop2));
     c->root_limit = std::max<long long>(1, (long long)(frac * (double)ngen));
     c->no_output = true;
     auto trial = [&](int leaf, long long ch, double* ms) {
@@ -2676,27 +2676,29 @@ int tc_corr2_autotune(tc_corr2* c, tc_field* f1, tc_field* f2, int metric, doubl
     int best_leaf = 0;
     long long best_ch = 0;
     double best = 0., ms = 0.;
-    int rc = trial(exact ? TILE_LEAF : 0, ch0, &ms);   // allocations, first launches
-    if (!rc) rc = trial(exact ? TILE_LEAF : 0, ch0, &best);
+    int rc = trial(exact ? TILE_LEAF : 0, 0, &ms);     // allocations, first launches
+    if (!rc) rc = trial(exact ? TILE_LEAF : 0, 0, &best);
     best_leaf = exact ? TILE_LEAF : 0;
-    best_ch = ch0;
     if (!rc && exact) {
         for (int leaf = 24; leaf <= 64 && !rc; leaf += 8) {
             if (leaf == TILE_LEAF) continue;
-            rc = trial(leaf, ch0, &ms);
+            rc = trial(leaf, 0, &ms);
             if (!rc && ms < best) { best = ms; best_leaf = leaf; }
         }
     }
-    for (long long ch = ch0 >> 1; ch >= std::max<long long>(1LL << 21, ch0 >> 3) && !rc; ch >>= 1) {
+    // (Another chunk than the default has to win by more than two runs of one setting differ.)
+    const double to_beat = 0.98 * best;
+    for (long long ch : tune_chunks(!exact, npoints, ngen, per_pair)) {
+        if (rc) break;
         rc = trial(best_leaf, ch, &ms);
-        if (!rc && ms < best) { best = ms; best_ch = ch; }
+        if (!rc && ms < std::min(best, to_beat)) { best = ms; best_ch = ch; }
     }
     c->root_limit = 0;
     c->no_output = false;
     c->stats = tc_stats();
     if (rc) { c->tile_leaf = 0; c->chunk = 0; return rc; }
     c->tile_leaf = best_leaf;
-    c->chunk = best_ch == ch0 ? 0 : best_ch;
+    c->chunk = best_ch;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tuned[key] = {c->tile_leaf, c->chunk};
