@@ -1704,7 +1704,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
             TC_TRY(dalloc(&X.part, npart));
             X.npart = npart;
         }
-        const long long nkey = (long long)P.nbd * (P.nbd + 1), nsegs = zeta_segments(X.zmax, P.nbd);
+        const long long nkey = (long long)P.nbd * (P.nbd + 1), nsegs = zeta_segments(X.zmax, nb, P.nbd);
         if (X.nkey < nkey || X.nsegs < nsegs) {
             dfree(X.keys); dfree(X.segs);
             X.nkey = 0; X.nsegs = 0;

@@ -150,7 +150,7 @@ struct ZParams {
     int* nseg;
 };
 size_t zeta_part_doubles(int nb, int M);
-long long zeta_segments(long long nrec, int nbd);
+long long zeta_segments(long long nrec, int nb, int nbd);
 int launch_zeta(const ZParams& Q, int nsm, cudaStream_t st);
 
 int launch_leaf_sums(int ncap, const Cells& C, double* ls, float4* lsf, cudaStream_t st);

@@ -44,7 +44,12 @@ namespace {
 constexpr int ZT = 192;             // threads per contraction block
 constexpr int ZIT = 2;              // (record, bin) items a thread loads per chunk
 constexpr int ZPAD = 4;             // bins a ragged tile may read past the last record
-constexpr int SEG_MIN = 256, SEG_MAX = 4096;
+// Records of a segment.  Up to 32 bins a stream adds up 64 to 256 of them in FP32 (256 is a segment of
+// one stream); with more bins every segment is of one or two streams, and runs of 256 were less
+// precise than the two levels of some 30 and 16 records that were summed there before:
+// against FP64, 5000 points, 40 bins 8.4e-7 and 6.6e-7, 64 bins 1.6e-6 and 1.1e-6 of zeta's
+// largest value.  Runs of 40: see RUN_MANY.
+constexpr int SEG_MIN = 256, SEG_MAX = 4096, RUN = 64, RUN_MANY = 40, MANY_BINS = 32;
 
 __device__ __forceinline__ int record_key(const ZParams& Q, unsigned off)
 {
@@ -73,7 +78,7 @@ __global__ void __launch_bounds__(256) k_zrows(ZParams Q, bool scatter)
 }
 
 // first[key]: the place of the key's first record; the segments of all keys.  A segment gives
-// each stream of its tiles some 64 records, so that adding up 80 sums per thread stays small.
+// each stream of its tiles RUN or RUN_MANY records, so that adding up 80 sums per thread stays small.
 __global__ void __launch_bounds__(1024) k_zrows_segments(ZParams Q)
 {
     __shared__ int wsum[2][32];
@@ -88,7 +93,8 @@ __global__ void __launch_bounds__(1024) k_zrows_segments(ZParams Q)
         const int f = Q.nbins / Q.nbd;      // 2 for a three-field cross, else 1
         const int ent = f * f * ((Q.nbd - ks) * (Q.nbd - ks) - (Q.nbd - mk) * (Q.nbd - mk));
         const int streams = max(1, ZT * 6 / max(ent, 6));
-        const int len = min(max(64 * streams, SEG_MIN), SEG_MAX);
+        const int len = Q.nbins > MANY_BINS ? min(RUN_MANY * streams, SEG_MAX)
+                                            : min(max(RUN * streams, SEG_MIN), SEG_MAX);
         const int ns = (c + len - 1) / len;
         int x = c, y = ns;
         for (int o = 1; o < 32; o <<= 1) {
@@ -259,8 +265,8 @@ __global__ void __launch_bounds__(ZT, 2) k_mp_zeta(ZParams Q)
 size_t zeta_part_doubles(int nb, int M)
 { return (size_t)(M + 1) * 80 * (((nb + 3) >> 2) * ((nb + 1) >> 1)); }
 
-long long zeta_segments(long long nrec, int nbd)
-{ return nrec / SEG_MIN + (long long)nbd * (nbd + 1) + 1; }
+long long zeta_segments(long long nrec, int nb, int nbd)
+{ return nrec / (nb > MANY_BINS ? RUN_MANY : SEG_MIN) + (long long)nbd * (nbd + 1) + 1; }
 
 int launch_zeta(const ZParams& Q, int nsm, cudaStream_t st)
 {
