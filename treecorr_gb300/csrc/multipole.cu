@@ -1237,7 +1237,13 @@ __global__ void __launch_bounds__(MB, MBLK) k_mp_finish(const __grid_constant__ 
                             // spin-2 factor e = conj(d^2) / |d|^2, the projected shear wg and
                             // the scalar sums.
                             const float inv = __frcp_rn(r32 > 0.f ? r32 : 1.f);
-                            const float zr = dxf * inv, zi = dyf * inv;
+                            float zr = dxf * inv, zi = dyf * inv;
+                            // |z| = 1 again: r's rounding and its reciprocal's would come n-fold
+                            // into z^n (rms error of z^12 9.0 u, with a division 7.7, so 5.2;
+                            // u = 2^-24).
+                            const float h = -0.5f * fmaf(zr, zr, fmaf(zi, zi, -1.f));
+                            zr = fmaf(zr, h, zr);
+                            zi = fmaf(zi, h, zi);
                             // (no rotation for the real payload of N / K pairs)
                             const bool rl = (P.pspin0 >> (is3 ? 1 : 0)) & 1;
                             const float er = rl ? 1.f : zr * zr - zi * zi;
