@@ -506,8 +506,8 @@ static_assert(sizeof(AccBatch) % 16 == 0, "");
 // a second round, H = 2) to shared memory, one complex multiplication each, and the record's
 // other terms, 16 records at a time; then lane = n walks the records of each bin's run with six FP32 multiply-adds each (the sums of
 // Re wg z^n and Im wg z^n, which make both G_n and G_-n, and w z^n), lanes 0..15 adding
-// the scalar terms as well.  The FP32 sums (F over a batch, F2 over the share: at most 16
-// batches) go to the slot in FP64 when the bin changes (atomics: two warps can share a bin).
+// the scalar terms as well.  The FP32 sums (F over a batch, F2 over the share: at most 1024
+// records, so 32 batches) go to the slot in FP64 when the bin changes (atomics: two warps can share a bin).
 // A record costs the warp 22 instructions; raising every lane to its own power by squaring
 // took 75.
 template <int H>

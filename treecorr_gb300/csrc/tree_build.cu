@@ -33,9 +33,6 @@ namespace tc {
 // ---------------------------------------------------------------------------------------
 // device helpers
 
-__device__ __forceinline__ double coord3(const Points& P, int i, int axis)
-{ return axis == 2 ? P.z[i] : axis == 1 ? P.y[i] : P.x[i]; }
-
 __device__ __forceinline__ void set_err(int* err, int code)
 { atomicCAS(err, 0, code); }
 

@@ -638,7 +638,12 @@ WalkKernel pick(const TravParams& T) { return T.mode == 3 ? pick<true>(T) : pick
 
 void walk_constants(const TravParams& T, WalkParams& W)
 {
-    // Margins on each constant; the sums in decide_fast's comment stay below 6e-6.
+    // Margins on each constant: both sides' errors and the constant's own rounding (6e-8) stay below
+    // 6e-6.  dsq is within 5e-7 of itself (two roundings per coordinate difference, the squares and
+    // their sum; the records' low parts add 4e-15 of the coordinates), r within 6e-7 (the Heron
+    // step 1.2e-7, an arc's series or asinf 3e-7): 2.5e-6 is allowed.  S = s1 + s2 is one rounding
+    // of exact sizes, S / r and the smaller size / r a reciprocal (2 ulps) and a product more: 3.2e-6
+    // is allowed.
     const double m = 6e-6;
     const double a = T.a, b = T.b, h = 0.5 * (T.binsize + T.b);
     const double c = std::sqrt(0.3422) * std::fmin(std::fabs(a), std::fabs(b));
