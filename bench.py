@@ -324,6 +324,8 @@ def run_gpu(args, rank, world):
                                   if args.traffic is None and traffic is not None else
                                   ("--traffic" if traffic is not None else None),
                 "kernel": "k_walk",
+                # (the copy rate is a yardstick: the kernel reads its records from L1 and L2)
+                "limiter": "L1 wavefronts 70% and instruction issue 72% busy (ncu)",
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}
     h2d = sum(cat[k].nbytes for k in cols)
     d2h = 8 * nb * 8

@@ -19,7 +19,7 @@
 // k_tiles.
 //
 // Measured against k_tiles, tile kernels of GG on the full sphere, 30 bins, 1' to 300', bin_slop
-// 0: 10^6 points 278.7 -> 150.2 ms, 200,000 points 27.5 -> 9.2 ms; with 10 bins 189.2 -> 119.3 and
+// 0: 10^6 points 278.7 -> 148.3 ms, 200,000 points 27.5 -> 9.0 ms; with 10 bins 189.2 -> 119.3 and
 // 14.9 -> 7.0 ms, with 100 bins 1308 -> 300 and 86.2 -> 25.3 ms; NN of 10^6 points 233.7 -> 96.1,
 // KK of 200,000 25.5 -> 5.8 ms.  In the histogram form a step of 64 pairs takes 48 packed FP32
 // instructions (two FMA-pipe cycles each), 8 reciprocals, roots and logarithms and 32 + 6

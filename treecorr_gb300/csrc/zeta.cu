@@ -17,8 +17,8 @@
 //     its 4 x 2 tiles are dealt out to the threads, the sums run over the records without any
 //     test, and the range is applied when they are added up.  At 20 bins and 500,000 points a
 //     record has 101 of the 400 entries on average, 134 with the ragged tiles.
-//   * A thread keeps its tile's 80 sums in registers, over a few hundred records at most (FP32);
-//     then they go to FP64.  A block's threads are S streams of the segment's tiles, each with
+//   * A thread keeps its tile's 80 sums in registers, over 256 records at most, 40 with more than 32 bins
+//     (FP32); then they go to FP64.  A block's threads are S streams of the segment's tiles, each with
 //     every S-th record.  The five columns of a chunk of records are loaded into registers while
 //     the chunk before is contracted from shared memory.
 //
