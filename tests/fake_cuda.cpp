@@ -17,6 +17,8 @@ std::map<void*, size_t> live;
 long long bytes = 0, launches = 0, allocs = 0, streams = 0;
 long long fail_launch = -1, fail_alloc = -1;    // the launch or allocation (counted from 0) that fails
 const void* fail_copy = nullptr;                // a copy to this address fails
+std::map<const void*, int> smem;                // a kernel's opt-in
+long long lowered = 0;
 long long answer_at = -1;                       // the 4-byte copy that brings `answer`
 long long copies4 = 0;
 int answer = 0;
@@ -63,6 +65,7 @@ long long fake_launches() { return launches; }
 long long fake_allocs() { return allocs; }
 long long fake_bytes() { return bytes; }
 long long fake_streams() { return streams; }
+long long fake_lowered() { return lowered; }
 int* fake_word() { return static_cast<int*>(word); }
 
 // ---- memory
@@ -91,6 +94,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
     if (d == fail_copy) return last = cudaErrorUnknown;
     std::memcpy(d, s, n);
     if (n == 4 && copies4++ == answer_at) *static_cast<int*>(d) = answer;
+    if (n == 12) *static_cast<int*>(d) = 1;     // (an expansion's flags: done)
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, s, n, k, nullptr); }
@@ -137,7 +141,14 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 
 // ---- kernels
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) { std::memset(a, 0, sizeof(*a)); return cudaSuccess; }
-cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v)
+{
+    std::lock_guard<std::mutex> lk(mu);
+    int& have = smem[f];
+    if (v < have) ++lowered;
+    have = v;
+    return cudaSuccess;
+}
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 4; return cudaSuccess; }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return launch(); }
 cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return launch(); }

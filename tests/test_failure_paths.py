@@ -23,7 +23,7 @@ def lib(tmp_path_factory):
                     os.path.join(HERE, "fake_cuda.cpp"), *objs, "-o", out, "-Wl,-Bsymbolic", "-pthread"],
                    check=True)
     L = ctypes.CDLL(out)
-    for f in ("launches", "allocs", "bytes", "streams"):
+    for f in ("launches", "allocs", "bytes", "streams", "lowered"):
         getattr(L, "fake_" + f).restype = ctypes.c_longlong
     for f in ("fail_launch", "fail_allocs_from"):
         getattr(L, "fake_" + f).argtypes = [ctypes.c_longlong]
@@ -77,14 +77,21 @@ def test_build_reports_its_first_launch(lib):
     lib.fake_reset()
 
 
-def _patches(L, *fields):
-    nb, n = 3, len(fields)
+def _corr(L, nb, slop):
     o = [np.zeros(nb) for _ in range(8)]
     p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
     d, big = ctypes.c_double, sys.float_info.max
     c = ctypes.c_void_p()
-    assert L.tc_corr2_create(0, 0, 0, d(1.), d(10.), nb, d(np.log(10.) / nb), d(0.1), d(0.1), d(-big), d(big),
+    assert L.tc_corr2_create(0, 0, 0, d(1.), d(10.), nb, d(np.log(10.) / nb), d(slop), d(slop), d(-big), d(big),
                              d(0.), d(0.), d(0.), *map(p, o), ctypes.byref(c)) == 0
+    c.outputs = o
+    return c
+
+
+def _patches(L, *fields):
+    nb, n = 3, len(fields)
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    c = _corr(L, nb, 0.1)
     i, j, res, got = np.zeros(3, np.int32), np.zeros(3, np.int32), np.zeros((3, 8, nb)), ctypes.c_int(0)
     rc = L.tc_corr2_process_patches(c, (ctypes.c_void_p * n)(*fields), n, 1, 0, 3, p(i), p(j), p(res),
                                     ctypes.byref(got))
@@ -197,4 +204,18 @@ def test_assign_that_failed_leaves_the_callers_array(lib):
     assert rc != 0
     np.testing.assert_array_equal(out, np.arange(n) + 7)
     lib.fake_reset()
+    lib.tc_field_free(h)
+
+
+def test_shared_memory_is_only_raised(lib):
+    """The dynamic shared memory that a kernel may be launched with belongs to the kernel: a call with
+    fewer bins must not lower it under another thread's launch."""
+    lib.fake_reset()
+    h = _create(lib, 300)[1]
+    before = lib.fake_lowered()
+    for nb in (200, 20):
+        c = _corr(lib, nb, 0.)                       # the accurate mode
+        assert lib.tc_corr2_process_auto(c, h, 0, 0, 1) == 0, lib.tc_last_error()
+        lib.tc_corr2_free(c)
+    assert lib.fake_lowered() == before
     lib.tc_field_free(h)

@@ -117,6 +117,20 @@ void dev_free(void* p)
     if (p) cudaFreeAsync(p, g_stream.load(std::memory_order_acquire));
 }
 
+int allow_smem(const void* kernel, size_t bytes)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> allowed;     // per device and kernel
+    int dev = 0;
+    TC_CU(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& have = allowed[{dev, kernel}];
+    if (bytes <= have) return 0;
+    TC_CU(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    have = bytes;
+    return 0;
+}
+
 static const char* dev_err_msg(int code)
 {
     switch (code) {

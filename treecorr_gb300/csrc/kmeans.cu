@@ -1199,9 +1199,9 @@ int scratch_alloc(const KMField& F, int npatch, KMScratch& S, cudaStream_t st)
     if (nw < 1) { set_last_error("k-means: too many patches for the accumulators"); return TC_ERR_UNSUPPORTED; }
     S.acc_threads = 32 * nw;
     S.acc_smem = per_warp * nw;
-    TC_CU(cudaFuncSetAttribute(k_km_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KW_SMEM));
+    TC_TRY(allow_smem(k_km_walk, KW_SMEM));
     if (S.acc_smem > 48 * 1024)
-        TC_CU(cudaFuncSetAttribute(k_km_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.acc_smem));
+        TC_TRY(allow_smem(k_km_accum, S.acc_smem));
     return 0;
 }
 

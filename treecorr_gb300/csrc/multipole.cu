@@ -1608,7 +1608,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
     // (powers up to 32, or up to 64 in two rounds)
     auto* kfin = M + 1 <= 32 ? (P.three ? k_mp_finish<true, 1> : k_mp_finish<false, 1>)
                              : (P.three ? k_mp_finish<true, 2> : k_mp_finish<false, 2>);
-    TC_CU(cudaFuncSetAttribute(kfin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shbytes));
+    TC_TRY(allow_smem(kfin, shbytes));
     int per = 0;
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfin, MB, shbytes));
     if (per < 1) per = 1;
@@ -1620,7 +1620,7 @@ int run_multipole(MPParams& P, MPScratch& X, int ntop, cudaStream_t st, double* 
     const int chunk2 = (int)std::max<long long>(1, std::min<long long>(64, (48 * 1024) / (32LL * nb)));
     const size_t zsh2 = (size_t)chunk2 * nb * 32;
     // (with its static header array this can pass the 48 KB that needs no opt-in)
-    TC_CU(cudaFuncSetAttribute(k_mp_zscal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsh2));
+    TC_TRY(allow_smem(k_mp_zscal, zsh2));
     const int nsg = std::max(1, 2 * nsm / etiles);
     const long long recu = mp_rec_units(nb, M);
     const long long acc_cap = 4096;

@@ -38,6 +38,12 @@ void count_launch();
 int dev_alloc(void** p, size_t bytes);
 void dev_free(void* p);
 
+// The dynamic shared memory that a kernel may be launched with belongs to the kernel: several
+// threads launch it, with their own numbers of bins, so it is only ever raised.
+int allow_smem(const void* kernel, size_t bytes);
+template <class R, class... P>
+int allow_smem(R (*kernel)(P...), size_t bytes) { return allow_smem((const void*)kernel, bytes); }
+
 template <class T>
 int dalloc(T** p, size_t count)
 {

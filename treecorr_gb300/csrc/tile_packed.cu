@@ -848,7 +848,7 @@ int packed_grid(const TravParams& T, int* blocks, int* nwarps)
     TC_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const size_t sm = K.warp * PW;
     if (sm > 48 * 1024)
-        TC_CU(cudaFuncSetAttribute(K.run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TC_TRY(allow_smem(K.run, sm));
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, K.run, PB, sm));
     if (per < 1) per = 1;
     *blocks = nsm * per;

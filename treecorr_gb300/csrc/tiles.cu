@@ -710,7 +710,7 @@ int tiles_grid(const TravParams& T, int* blocks, int* nwarps)
     const size_t sm = edges_bytes(T.nbins) + warp_bytes(T.nqf, T.nbins) * TWPB;
     const TileKernel k = pick(T);
     if (sm > 48 * 1024)
-        TC_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TC_TRY(allow_smem(k, sm));
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, TPB, sm));
     if (per < 1) per = 1;
     *blocks = nsm * per;

@@ -999,7 +999,7 @@ int traverse_grid(int nq, int nb, int* blocks, int* nwarps)
     TC_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     size_t sm = traverse_smem_bytes(nq, nb);
     if (sm > 48 * 1024)
-        TC_CU(cudaFuncSetAttribute(k_traverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TC_TRY(allow_smem(k_traverse, sm));
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_traverse, TB, sm));
     if (per < 1) per = 1;
     *blocks = nsm * per;
@@ -1022,7 +1022,7 @@ template <int MODE, bool DET = false>
 static int set_expand_attr(size_t sm)
 {
     if (sm > 48 * 1024)
-        TC_CU(cudaFuncSetAttribute(k_expand<MODE, DET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TC_TRY(allow_smem(k_expand<MODE, DET>, sm));
     return 0;
 }
 

@@ -1306,8 +1306,7 @@ static int subtree_launch(int ntask, const BuildTask* tasks, Points P0, Points P
                           const BuildParams& BP, const Cells& C, int* tops, int* ntop,
                           WTask* wstack, int thread_t, int* err, cudaStream_t st)
 {
-    TC_CU(cudaFuncSetAttribute(k_subtree<FLATC, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SubShared)));
+    TC_TRY((allow_smem(k_subtree<FLATC, CPLX>, sizeof(SubShared))));
     count_launch();
     k_subtree<FLATC, CPLX><<<ntask, SB, sizeof(SubShared), st>>>(tasks, P0, P1, BP, C, tops, ntop,
                                                                  wstack, thread_t, err);

@@ -673,7 +673,7 @@ int walk_grid(const TravParams& T, int* blocks, int* nwarps)
     const size_t sm = walk_warp_bytes(walk_kind(T), T.nqf, T.nbins) * KW;
     const WalkKernel k = pick(T);
     if (sm > 48 * 1024)
-        TC_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        TC_TRY(allow_smem(k, sm));
     TC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, KB, sm));
     if (per < 1) per = 1;
     *blocks = nsm * per;

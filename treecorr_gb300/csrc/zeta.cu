@@ -272,7 +272,7 @@ int launch_zeta(const ZParams& Q, int nsm, cudaStream_t st)
 {
     const int chunk = std::min(64, std::max(1, ZIT * ZT / Q.nbins));
     const size_t sm = sizeof(float4) * 8 * (size_t)(chunk * Q.nbins + ZPAD);
-    TC_CU(cudaFuncSetAttribute(k_mp_zeta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    TC_TRY(allow_smem(k_mp_zeta, sm));
     TC_CU(cudaMemsetAsync(Q.count, 0, sizeof(int) * (size_t)Q.nbd * (Q.nbd + 1), st));
     const int blocks = (int)std::min<long long>(4LL * nsm, (Q.nrec + 255) / 256);
     count_launch();
