@@ -460,9 +460,11 @@ struct Events {
 };
 
 // field_build with its arrays there.
-int build_one(tc_field* f, const Events& ev, cudaStream_t st)
+int build_one(tc_field* f, cudaStream_t st)
 {
+    Events ev;
     TC_TRY(clear_cells(f->cells, 2 * f->n - 1, st));
+    TC_TRY(ev.make());
     TC_CU(cudaEventRecord(ev.a, st));
     const TreeBuild B = tree_of(f);
     BuildRun R;
@@ -487,11 +489,9 @@ int field_build(tc_field* f)
     cudaStream_t st;
     TC_TRY(stream_get(&st));
     if (f->n == 0) { f->built = true; return 0; }
-    Events ev;
-    TC_TRY(ev.make());
     int rc = build_arrays(f);
     if (rc) { drop_build_arrays(f); return rc; }    // (no kernel has run: it can be tried again)
-    rc = build_one(f, ev, st);
+    rc = build_one(f, st);
     if (rc) return build_broke(f, rc);
     set_built(f);
     return 0;
@@ -556,6 +556,8 @@ struct GroupBuild {
 int GroupBuild::run(cudaStream_t st)
 {
     TC_CU(cudaMemsetAsync(d_read, 0, sizeof(BuildRead) * f.size(), st));
+    TC_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    TC_TRY(time.make());
     TC_CU(cudaEventRecord(time.a, st));
     for (int k = 0; k < SIDES; ++k) TC_CU(cudaStreamWaitEvent(side[k], time.a, 0));
     for (size_t i = 0; i < f.size(); ++i) {
@@ -585,8 +587,6 @@ int build_group(const std::vector<tc_field*>& fields, size_t* taken)
     TC_TRY(stream_get(&st));
     GroupBuild G;
     TC_TRY(side_streams(G.side));
-    TC_CU(cudaEventCreateWithFlags(&G.ev, cudaEventDisableTiming));
-    TC_TRY(G.time.make());
     int64_t points = 0;
     for (tc_field* f : fields) {
         if (build_arrays(f)) { drop_build_arrays(f); break; }
