@@ -423,11 +423,12 @@ TreeBuild tree_of(tc_field* f)
     return B;
 }
 
-// The ordered tops onto the device, in place of the pairs they were made from (the host has
-// read those), and the check of the finished tree.
+// The ordered tops onto the device, and the check of the finished tree.
 int finish_tops(tc_field* f, cudaStream_t st)
 {
-    std::swap(f->d_tops, f->d_tops_raw);
+    // (Without memory, in place of the pairs they were made from, which the host has read: the
+    // build is too far to be tried again.)
+    if (dalloc(&f->d_tops, f->tops.size())) std::swap(f->d_tops, f->d_tops_raw);
     TC_CU(cudaMemcpyAsync(f->d_tops, f->tops.data(), f->tops.size() * sizeof(int),
                           cudaMemcpyHostToDevice, st));
     launch_validate_tree((int)(2 * f->n - 1), f->cells, f->d_tops, (int)f->tops.size(), f->d_err, st);
