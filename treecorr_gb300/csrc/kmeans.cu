@@ -117,16 +117,18 @@ __device__ __forceinline__ bool km_keep(double d, double s, double thresh, const
 constexpr int KM_SMALL = 16;
 
 __global__ void k_km_start(const int* tops, int ntop, int npatch, KMItem* items, int* pool,
-                           KMLevel* L, const KMCtl* ctl, const double* cen, float4* cen32)
+                           KMLevel* L, const KMCtl* ctl, const double* cen, const double* inertia,
+                           float4* cen32)
 {
     after_previous();
     if (ctl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < npatch) {                    // the centres as FP32 pairs
+    if (i < npatch) {                    // the centres as FP32 pairs, and their penalties
         const double x = cen[3 * i], y = cen[3 * i + 1], z = cen[3 * i + 2];
         const float hx = (float)x, hy = (float)y, hz = (float)z;
         cen32[2 * i] = make_float4(hx, hy, hz, fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))));
-        cen32[2 * i + 1] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.f);
+        cen32[2 * i + 1] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz),
+                                       inertia ? (float)inertia[i] : 0.f);
     }
     if (i < ntop) items[i] = KMItem{tops[i], npatch, 0};
     if (i < npatch) pool[i] = i;
@@ -166,33 +168,69 @@ __device__ __forceinline__ bool km_plain(float best, float thresh, float far)
 __device__ __forceinline__ bool km_close(float d, float best, float thresh)
 { return !(d > best * (1.f + 1e-5f) && fabsf(d - thresh) > 1e-5f * thresh); }
 
-// The closest candidate's place, and how many others can hold points of the cell, in FP32;
-// false: left to FP64.
+// The alternate form's rule in FP32, with the penalty I of a candidate at squared distance d from
+// a cell of size s (km_keep).  d is within 1e-6 and sqrt(d) within 6e-7 of itself, so that both
+// sides of the last comparison are within 1.5e-6 of thresh + d + I; penalties are not negative where
+// this is used.
+__device__ __forceinline__ float km_penalised(float d, float I, float s)
+{
+    const float dd = sqrtf(d);
+    return s > dd ? 0.f : (dd - s) * (dd - s) + I;
+}
+__device__ __forceinline__ bool km_alt_close(float d, float I, float s, float best, float thresh)
+{
+    const float dd = sqrtf(d);
+    const bool edge = fabsf(dd - s) > 1e-5f * dd;                 // on one side of s
+    const bool lim = s > dd || fabsf(km_penalised(d, I, s) - thresh) > 1e-5f * (thresh + d + I);
+    return !(d + I > best * (1.f + 1e-5f) && edge && lim);
+}
+
+// The closest candidate's place (by the distance with its penalty: ALT), and how many others can
+// hold points of the cell, in FP32; false: left to FP64.
+template <bool ALT>
 __device__ __forceinline__ bool km_item_warp32(const int* lst, int m, int lane, const KMPos& a, float s,
                                                const float4* cen32, int& bpos, int& nkeep, float& thresh)
 {
-    float best = 0.f, far = a.amax;
+    float best = 0.f, far = a.amax, dmin = 1e38f;
     bpos = INT_MAX;
+    bool sure = true;
     for (int j = lane; j < m; j += 32) {
-        const float d = km_dsq32(a, cen32, lst[j], far);
-        if (bpos == INT_MAX || d < best) { best = d; bpos = j; }
+        const int p = lst[j];
+        const float d = km_dsq32(a, cen32, p, far), I = ALT ? cen32[2 * p + 1].w : 0.f;
+        if (ALT) { dmin = fminf(dmin, d); sure = sure && I >= 0.f; }
+        if (bpos == INT_MAX || d + I < best) { best = d + I; bpos = j; }
     }
     unsigned key = bpos == INT_MAX ? 0xffffffffu : __float_as_uint(best);
     const unsigned mn = __reduce_min_sync(0xffffffffu, key);
     bpos = __reduce_min_sync(0xffffffffu, key == mn ? (unsigned)bpos : 0xffffffffu);
     best = __uint_as_float(mn);
     far = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(far)));
-    const float t = sqrtf(best) + 2.f * s;
-    thresh = t * t;
-    bool sure = km_plain(best, thresh, far);
+    if (ALT) {
+        if (!__all_sync(0xffffffffu, sure)) return false;         // (bpos may be none's)
+        const int cp = lst[bpos];
+        const float t = sqrtf(km_dsq32(a, cen32, cp, far)) + s;
+        thresh = t * t + cen32[2 * cp + 1].w;
+        sure = km_plain(dmin, thresh, far);
+    } else {
+        const float t = sqrtf(best) + 2.f * s;
+        thresh = t * t;
+        sure = km_plain(best, thresh, far);
+    }
     nkeep = 0;
     for (int j0 = 0; j0 < m; j0 += 32) {
         const int j = j0 + lane;
         bool keep = false;
         if (j < m && j != bpos) {
-            const float d = km_dsq32(a, cen32, lst[j], far);
-            sure = sure && !km_close(d, best, thresh);
-            keep = !(d > thresh);
+            const int p = lst[j];
+            const float d = km_dsq32(a, cen32, p, far);
+            if (ALT) {
+                const float I = cen32[2 * p + 1].w;
+                sure = sure && !km_alt_close(d, I, s, best, thresh);
+                keep = !(km_penalised(d, I, s) > thresh);
+            } else {
+                sure = sure && !km_close(d, best, thresh);
+                keep = !(d > thresh);
+            }
         }
         nkeep += __popc(__ballot_sync(0xffffffffu, keep));
     }
@@ -214,7 +252,8 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
     int bpos = INT_MAX, nkeep = 0;
     float thresh32 = 0.f, unused = 0.f;
     double thresh = 0.;
-    const bool sure = !inertia && km_item_warp32(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32);
+    const bool sure = inertia ? km_item_warp32<true>(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32)
+                              : km_item_warp32<false>(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32);
     if (!sure) {
         // The closest centre by the (penalised) distance: the first minimum in list order.
         double bmod = 0., bdsq = 0.;
@@ -277,9 +316,13 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
             int p = 0;
             if (j < m && j != bpos) {
                 p = lst[j];
-                keep = sure ? !(km_dsq32(pos, cen32, p, unused) > thresh32)
-                            : km_keep(dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]), s,
-                                      thresh, inertia, p);
+                if (sure) {
+                    const float d = km_dsq32(pos, cen32, p, unused);
+                    keep = !((inertia ? km_penalised(d, cen32[2 * p + 1].w, sf) : d) > thresh32);
+                } else {
+                    keep = km_keep(dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]), s, thresh,
+                                   inertia, p);
+                }
             }
             const unsigned bal = __ballot_sync(0xffffffffu, keep);
             if (keep) pool[off + base + __popc(bal & ((1u << lane) - 1u))] = p;
@@ -459,6 +502,7 @@ constexpr int KW_WARPS = KM_LTB / 32;
 constexpr int KW_BLOCKS = 3;        // per SM
 constexpr size_t KW_SMEM = sizeof(KMEntry) * KW_CAP * KW_WARPS;
 
+template <bool ALT>
 __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const double* cen, const float4* cen32, const double* inertia,
                                                     const KMItem* items, long long item_cap,
                                                     const int* pool, int* assign, int tag, KMLevel* L,
@@ -518,24 +562,32 @@ __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const do
                 left = C.left[c];
                 right = C.right[c];
                 int cp = 0;
-                bool sure = inertia == nullptr;
-                if (sure) {
+                bool sure = true;
+                {
                     const KMPos pos = km_pos(px, py, pz);
-                    float df[KM_SMALL], bd = 0.f, far = pos.amax;
+                    float df[KM_SMALL], best = 0.f, bd = 0.f, bI = 0.f, far = pos.amax, dmin = 1e38f;
 #pragma unroll
                     for (int j = 0; j < KM_SMALL; ++j) {
                         if (j < m) {
                             df[j] = km_dsq32(pos, cen32, cand[j], far);
-                            if (j == 0 || df[j] < bd) { bd = df[j]; bpos = j; cp = cand[j]; }
+                            const float I = ALT ? cen32[2 * cand[j] + 1].w : 0.f;
+                            if (ALT) { dmin = fminf(dmin, df[j]); sure = sure && I >= 0.f; }
+                            if (j == 0 || df[j] + I < best) { best = df[j] + I; bd = df[j]; bI = I; bpos = j; cp = cand[j]; }
                         }
                     }
-                    const float t = sqrtf(bd) + 2.f * sf, thresh = t * t;
-                    sure = km_plain(bd, thresh, far);
+                    const float t = sqrtf(bd) + (ALT ? 1.f : 2.f) * sf, thresh = ALT ? t * t + bI : t * t;
+                    sure = sure && km_plain(ALT ? dmin : bd, thresh, far);
 #pragma unroll
                     for (int j = 0; j < KM_SMALL; ++j) {
                         if (j < m && j != bpos) {
-                            sure = sure && !km_close(df[j], bd, thresh);
-                            if (!(df[j] > thresh)) kept |= 1u << j;
+                            if (ALT) {
+                                const float I = cen32[2 * cand[j] + 1].w;
+                                sure = sure && !km_alt_close(df[j], I, sf, best, thresh);
+                                if (!(km_penalised(df[j], I, sf) > thresh)) kept |= 1u << j;
+                            } else {
+                                sure = sure && !km_close(df[j], bd, thresh);
+                                if (!(df[j] > thresh)) kept |= 1u << j;
+                            }
                         }
                     }
                 }
@@ -1199,7 +1251,8 @@ int scratch_alloc(const KMField& F, int npatch, KMScratch& S, cudaStream_t st)
     if (nw < 1) { set_last_error("k-means: too many patches for the accumulators"); return TC_ERR_UNSUPPORTED; }
     S.acc_threads = 32 * nw;
     S.acc_smem = per_warp * nw;
-    TC_TRY(allow_smem(k_km_walk, KW_SMEM));
+    TC_TRY(allow_smem(k_km_walk<false>, KW_SMEM));
+    TC_TRY(allow_smem(k_km_walk<true>, KW_SMEM));
     if (S.acc_smem > 48 * 1024)
         TC_TRY(allow_smem(k_km_accum, S.acc_smem));
     return 0;
@@ -1245,13 +1298,18 @@ int enqueue_cells(const KMField& F, int npatch, const double* inertia, KMScratch
     TC_TRY(next_tag(F, S, st));
     const int nstart = std::max(F.ntop, npatch);
     TC_TRY(launch_chained(k_km_start, (nstart + 255) / 256, 256, 0, st, F.d_tops, F.ntop, npatch,
-                          S.items, S.pool, S.lvl, S.ctl, S.cen, S.cen32));
+                          S.items, S.pool, S.lvl, S.ctl, S.cen, inertia, S.cen32));
     for (int k = 0; k < S.pre; ++k) {
-        TC_TRY(launch_chained(k_km_level, nsm, KM_LTB, 0, st, F.cells, S.cen, S.cen32, inertia,
+        // A warp per item, of which a level holds twice as many as the one before at most.  A block
+        // per SM is enough for the first levels; with many patches some ten levels come before the
+        // walk (10^6 points in a box, 1000 patches, alternate: 116 ms at one block per SM throughout).
+        const long long items = (long long)F.ntop << std::min(k, 20);
+        const int blocks = (int)std::max<long long>(nsm, std::min<long long>(4LL * nsm, items / (KM_LTB / 32)));
+        TC_TRY(launch_chained(k_km_level, blocks, KM_LTB, 0, st, F.cells, S.cen, S.cen32, inertia,
                               S.items, S.item_cap, S.pool, S.pool_cap, S.assign, S.tag, S.lvl,
                               S.ctl));
     }
-    TC_TRY(launch_chained(k_km_walk, KW_BLOCKS * nsm, KM_LTB, KW_SMEM, st, F.cells, S.cen,
+    TC_TRY(launch_chained(inertia ? k_km_walk<true> : k_km_walk<false>, KW_BLOCKS * nsm, KM_LTB, KW_SMEM, st, F.cells, S.cen,
                           S.cen32, inertia, S.items, S.item_cap, S.pool, S.assign, S.tag, S.lvl,
                           S.ctl));
     TC_CU(cudaGetLastError());
@@ -1300,7 +1358,7 @@ int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S
         const int nstart = std::max(F.ntop, npatch);
         count_launch();
         k_km_start<<<(nstart + 255) / 256, 256, 0, st>>>(F.d_tops, F.ntop, npatch, S.items, S.pool, S.lvl, S.ctl,
-                                                     S.cen, S.cen32);
+                                                     S.cen, inertia, S.cen32);
         TC_CU(cudaGetLastError());
         KMLevel h{};
         bool done = false;
