@@ -198,7 +198,8 @@ __device__ __forceinline__ bool km_item_warp32(const int* lst, int m, int lane, 
         const int p = lst[j];
         const float d = km_dsq32(a, cen32, p, far), I = ALT ? cen32[2 * p + 1].w : 0.f;
         if (ALT) { dmin = fminf(dmin, d); sure = sure && I >= 0.f; }
-        if (bpos == INT_MAX || d + I < best) { best = d + I; bpos = j; }
+        const float mod = ALT ? d + I : d;
+        if (bpos == INT_MAX || mod < best) { best = mod; bpos = j; }
     }
     unsigned key = bpos == INT_MAX ? 0xffffffffu : __float_as_uint(best);
     const unsigned mn = __reduce_min_sync(0xffffffffu, key);
@@ -238,6 +239,7 @@ __device__ __forceinline__ bool km_item_warp32(const int* lst, int m, int lane, 
 }
 
 // The whole-warp form for one item with a long candidate list.
+template <bool ALT>
 __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* cen, const float4* cen32,
                              const double* inertia, KMItem* items, long long item_cap, int* pool,
                              long long pool_cap, int* assign, int tag, KMLevel* L)
@@ -252,8 +254,7 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
     int bpos = INT_MAX, nkeep = 0;
     float thresh32 = 0.f, unused = 0.f;
     double thresh = 0.;
-    const bool sure = inertia ? km_item_warp32<true>(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32)
-                              : km_item_warp32<false>(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32);
+    const bool sure = km_item_warp32<ALT>(lst, m, lane, pos, sf, cen32, bpos, nkeep, thresh32);
     if (!sure) {
         // The closest centre by the (penalised) distance: the first minimum in list order.
         double bmod = 0., bdsq = 0.;
@@ -318,7 +319,7 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
                 p = lst[j];
                 if (sure) {
                     const float d = km_dsq32(pos, cen32, p, unused);
-                    keep = !((inertia ? km_penalised(d, cen32[2 * p + 1].w, sf) : d) > thresh32);
+                    keep = !((ALT ? km_penalised(d, cen32[2 * p + 1].w, sf) : d) > thresh32);
                 } else {
                     keep = km_keep(dsq3(px, py, pz, cen[3 * p], cen[3 * p + 1], cen[3 * p + 2]), s, thresh,
                                    inertia, p);
@@ -344,6 +345,7 @@ __device__ void km_item_warp(const KMItem it, int lane, Cells C, const double* c
 // One level of FindCellsInPatches.  cen: npatch x 3 (z = 0 for Flat).  Items with short
 // lists are processed one per thread; their child items and new lists are reserved with one
 // atomic per warp.
+template <bool ALT>
 __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
                                                      const float4* cen32,
                                                      const double* inertia, KMItem* items,
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
         // A small level (the top of the tree, long lists): one item per warp.
         for (long long i = lo + (long long)blockIdx.x * (KM_LTB / 32) + (threadIdx.x >> 5); i < hi;
              i += nwarps)
-            km_item_warp(items[i], lane, C, cen, cen32, inertia, items, item_cap, pool, pool_cap, assign,
+            km_item_warp<ALT>(items[i], lane, C, cen, cen32, inertia, items, item_cap, pool, pool_cap, assign,
                          tag, L);
     } else
     for (long long base = lo + (long long)blockIdx.x * KM_LTB + (threadIdx.x & ~31); base < hi;
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(KM_LTB) k_km_level(Cells C, const double* cen,
             w.cell = __shfl_sync(0xffffffffu, it.cell, l);
             w.len = __shfl_sync(0xffffffffu, it.len, l);
             w.off = __shfl_sync(0xffffffffu, it.off, l);
-            km_item_warp(w, lane, C, cen, cen32, inertia, items, item_cap, pool, pool_cap, assign, tag, L);
+            km_item_warp<ALT>(w, lane, C, cen, cen32, inertia, items, item_cap, pool, pool_cap, assign, tag, L);
         }
     }
     // The last block to finish moves the level window to the appended items.
@@ -572,7 +574,8 @@ __global__ void __launch_bounds__(KM_LTB, KW_BLOCKS) k_km_walk(Cells C, const do
                             df[j] = km_dsq32(pos, cen32, cand[j], far);
                             const float I = ALT ? cen32[2 * cand[j] + 1].w : 0.f;
                             if (ALT) { dmin = fminf(dmin, df[j]); sure = sure && I >= 0.f; }
-                            if (j == 0 || df[j] + I < best) { best = df[j] + I; bd = df[j]; bI = I; bpos = j; cp = cand[j]; }
+                            const float mod = ALT ? df[j] + I : df[j];
+                            if (j == 0 || mod < best) { best = mod; bd = df[j]; bI = I; bpos = j; cp = cand[j]; }
                         }
                     }
                     const float t = sqrtf(bd) + (ALT ? 1.f : 2.f) * sf, thresh = ALT ? t * t + bI : t * t;
@@ -1305,7 +1308,7 @@ int enqueue_cells(const KMField& F, int npatch, const double* inertia, KMScratch
         // walk (10^6 points in a box, 1000 patches, alternate: 116 ms at one block per SM throughout).
         const long long items = (long long)F.ntop << std::min(k, 20);
         const int blocks = (int)std::max<long long>(nsm, std::min<long long>(4LL * nsm, items / (KM_LTB / 32)));
-        TC_TRY(launch_chained(k_km_level, blocks, KM_LTB, 0, st, F.cells, S.cen, S.cen32, inertia,
+        TC_TRY(launch_chained(inertia ? k_km_level<true> : k_km_level<false>, blocks, KM_LTB, 0, st, F.cells, S.cen, S.cen32, inertia,
                               S.items, S.item_cap, S.pool, S.pool_cap, S.assign, S.tag, S.lvl,
                               S.ctl));
     }
@@ -1353,6 +1356,7 @@ int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S
     }
     int nsm = 0;
     TC_TRY(sm_count(&nsm));
+    auto* level = inertia ? k_km_level<true> : k_km_level<false>;
     for (int attempt = 0; attempt < 6; ++attempt) {
         TC_TRY(next_tag(F, S, st));
         const int nstart = std::max(F.ntop, npatch);
@@ -1367,7 +1371,7 @@ int find_cells(const KMField& F, int npatch, const double* inertia, KMScratch& S
         for (int lev = 0; lev < F.ncap + 2 && !done; lev += batch, batch = KM_LEVELS_PER_CHECK) {
             for (int k = 0; k < batch; ++k) {
                 count_launch();
-                k_km_level<<<4 * nsm, KM_LTB, 0, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap,
+                level<<<4 * nsm, KM_LTB, 0, st>>>(F.cells, S.cen, S.cen32, inertia, S.items, S.item_cap,
                                                        S.pool, S.pool_cap, S.assign, S.tag, S.lvl, S.ctl);
             }
             TC_CU(cudaGetLastError());
